@@ -63,10 +63,12 @@ typedef struct sspp_params {
                                  reference); the pairs are the same in every mode   */
     int32_t model;            /* bit0 high-dimension guided clearing, bit1 collapse   */
     int32_t max_iteration;    /* candidates per simplex for guided clearing           */
-    int32_t ss_block_size;    /* initial spectral-sequence block size                 */
+    int32_t ss_block_size;    /* initial spectral-sequence block size (schedule 1 merges
+                                 blocks of fewer than 2^20 columns)                   */
     float growth;             /* block_size_growth_rate (>= 1)                        */
     int32_t queue_size;       /* concurrent column workers per launch                 */
-    int32_t level1_capacity;  /* per-worker on-chip column capacity (ints)            */
+    int32_t level1_capacity;  /* per-worker on-chip column capacity (ints; more than 64
+                                 counts as 64: longer columns go to the CTA tier)     */
     int32_t level2_capacity;  /* per-block on-chip column capacity (ints)             */
     int32_t autotune;         /* 0 off, 1 launch parameters, 2 also dualization     */
     int32_t heavy_threads;    /* threads per heavy-tier column: 128 or 256 (0 = 256)  */
@@ -106,8 +108,8 @@ typedef struct sspp_stats {
     int64_t heavy_additions;     /* additions done by the CTA tier                 */
     double build_ms;             /* last sspp_load_rips / sspp_load_lowerstar (host
                                     clock, input staging included), else 0          */
-    int64_t heavy_fast_inline;   /* CTA-tier additions of short apparent addends    */
-    int64_t heavy_fast_slot;     /* CTA-tier additions of short published addends   */
+    int64_t heavy_fast_inline;   /* CTA-tier additions of inline apparent columns in rounds */
+    int64_t heavy_fast_slot;     /* CTA-tier additions of published columns in rounds  */
 } sspp_stats;
 
 /* Replaces: the SpecSeqPlusPlus constructor's allocation (include/specseq.h:486-512). */

@@ -274,16 +274,30 @@ int64_t arena_need(const sspp_ctx* ctx) {
     return std::max(want, ctx->arena_request);
 }
 
+// Blocks of fewer columns are merged by the host loop of per-block launches.  A
+// block exists to bound the work in flight and to let a column wait for the
+// columns below its band; with rounds of additions a chain is no longer the
+// step's length, and a step costs its launches and its slowest column whatever
+// it holds.  64^3 (reference's blocks of 102400 growing by 1.05: 40 steps) 2.68 ms
+// of reduction in those blocks, 1.92 in 400 k, 1.74 in 1 M, 1.82 in one block per
+// dimension; 93^3 6.4 / 5.0 / 4.5 / 4.5 ms.  The pairs do not depend on it.
+constexpr int kMinBlock = 1 << 20;
+
 // SS schedule of one dimension, following include/specseq.h:603-697.
 struct Step {
     int32_t beg, end, minrow;
 };
 
-void ss_schedule(const sspp_params& P, int32_t ab, int32_t ae, int32_t minrow_dim, int32_t maxrow_dim,
+void ss_schedule(const sspp_params& P, int min_block, int32_t ab, int32_t ae, int32_t minrow_dim, int32_t maxrow_dim,
                  std::vector<Step>& out) {
     if (ae <= ab) return;
     const int kMaxSteps = 4096;
-    int64_t ss = std::max(1, P.ss_block_size);
+    int64_t ss = std::max(min_block, P.ss_block_size);
+    // one block that holds every column and every row is the completion sweep itself
+    if (ae - ab <= ss && int64_t(maxrow_dim) - minrow_dim <= ss) {
+        out.push_back({ab, ae, INT32_MIN});
+        return;
+    }
     int32_t b = ab;
     int32_t e = int32_t(std::min<int64_t>(int64_t(ab) + ss, ae));
     int64_t lo = int64_t(maxrow_dim) - ss, hi = lo + ss;
@@ -335,6 +349,12 @@ int level1_cap(const sspp_params& p) {
     c = std::min(c, 4096);
     return (c + 31) & ~31;
 }
+// The light tier's own bound on the level-1 capacity: a warp takes 32 rows a
+// round, a CTA 256, so longer columns finish sooner in the CTA tier, and small
+// buffers leave room for more warps.  Measured with 32 / 64 / 128 ints: 93^3 2.81 /
+// 3.14 / 3.73 ms of reduction, 64^3 1.19 / 1.22 / 1.20, the 1,200-point cloud 420 /
+// 360 / 353 us, 64 clouds in a batch 4.69 / 4.42 / 4.43 ms.
+constexpr int kLightCap = 64;
 int level2_cap(const sspp_params& p) {
     int c = std::max(level1_cap(p), p.level2_capacity);
     c = std::min(c, 18432);
@@ -634,21 +654,6 @@ int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2,
     const int light_max = std::max(1, ctx->num_sms * ctx->light_blocks_per_sm);
     const int heavy_grid = std::max(1, std::min(ctx->num_sms * ctx->heavy_blocks_per_sm, 2 * ctx->num_sms));
     const int q_blocks = std::max(1, (P.queue_size + 3) / 4);
-#ifndef SSPP_LIGHT_CHUNK
-#define SSPP_LIGHT_CHUNK 8
-#endif
-#ifndef SSPP_LIGHT_FILTER
-#define SSPP_LIGHT_FILTER 1
-#endif
-#ifndef SSPP_FILTER_CHUNK
-#define SSPP_FILTER_CHUNK 1
-#endif
-    // Each step first lists its runnable columns (k_light_filter, one thread
-    // per window entry), then warps take them SSPP_FILTER_CHUNK at a time;
-    // without the filter, warps walk the window SSPP_LIGHT_CHUNK entries at a
-    // time through one shared counter.
-    const bool filtered = SSPP_LIGHT_FILTER != 0;
-    const int chunk = filtered ? SSPP_FILTER_CHUNK : SSPP_LIGHT_CHUNK;
     // Heavy launches go to side streams (round robin) after their light step:
     // they overlap the following light steps and each other, so long chains of
     // different steps run concurrently.  Each dimension's completion sweep, and
@@ -667,8 +672,11 @@ int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2,
         CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         ctx->step_ev.push_back(ev);
     }
+    bool used[sspp_ctx::kSide] = {};  // side streams with launches since the last join
     auto join_sides = [&]() -> int {
         for (int q = 0; q < sspp_ctx::kSide; q++) {
+            if (!used[q]) continue;
+            used[q] = false;
             CK(cudaEventRecord(ctx->join_ev[q], ctx->side[q]));
             CK(cudaStreamWaitEvent(s, ctx->join_ev[q], 0));
         }
@@ -681,21 +689,15 @@ int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2,
             int rcj = join_sides();
             if (rcj) return rcj;
         }
-        int64_t chunks = (int64_t(st.end - st.beg) + chunk - 1) / chunk;
-        int grid = int(std::min<int64_t>(std::min<int64_t>((chunks + 3) / 4, light_max), q_blocks));
-        grid = std::max(grid, 1);
+        const int64_t window = int64_t(st.end) - st.beg;
+        const int grid = int(std::max<int64_t>(1, std::min<int64_t>({(window + 3) / 4, light_max, q_blocks})));
         int* ctr = D.step_ctr + kStepCtr * k;
         cudaEvent_t a = nullptr, b = nullptr;
         span_begin(ctx, a);
         int* ctr_next = k + 1 < steps.size() ? ctr + kStepCtr : nullptr;
-        if (filtered) {
-            const int fgrid = int(std::max<int64_t>(
-                1, std::min<int64_t>((int64_t(st.end - st.beg) + 255) / 256, int64_t(ctx->num_sms) * 8)));
-            reduce_light_filtered_launch(D, st.beg, st.end, st.minrow, cap1, chunk, ctr, ctr_next, fgrid, grid, s);
-            ctx->launches++;
-        } else {
-            reduce_light_launch(D, D.active, st.beg, st.end, st.minrow, cap1, chunk, ctr, ctr_next, grid, s);
-        }
+        const int fgrid = int(std::max<int64_t>(1, std::min<int64_t>((window + 255) / 256, int64_t(ctx->num_sms) * 8)));
+        reduce_light_launch(D, st.beg, st.end, st.minrow, cap1, ctr, ctr_next, fgrid, grid, s);
+        ctx->launches++;
         span_end(ctx, PH_LIGHT, a);
         if (overlap && (!last_of_dim || gate)) {
             // an idle side stream if there is one: a CTA-tier launch lasts as
@@ -712,6 +714,7 @@ int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2,
             }
 #endif
             cudaStream_t hs = ctx->side[q];
+            used[q] = true;
             CK(cudaEventRecord(ctx->step_ev[k], s));
             CK(cudaStreamWaitEvent(hs, ctx->step_ev[k], 0));
             span_begin(ctx, b, hs);
@@ -790,7 +793,7 @@ int run_queue(sspp_ctx* ctx, int dlo, int dhi, bool ascending, int cap1, int cap
             cap = std::max(cap, cnt);
             st.clear();
             const int32_t mr = mnr[int64_t(c) * kNumDims + d];
-            ss_schedule(P, ab, ae, mr == INT32_MAX ? 0 : mr, mxr[int64_t(c) * kNumDims + d], st);
+            ss_schedule(P, 1, ab, ae, mr == INT32_MAX ? 0 : mr, mxr[int64_t(c) * kNumDims + d], st);
             int32_t eprev = -1;
             const size_t d0 = items.size();
             for (const Step& x : st) {
@@ -913,7 +916,7 @@ int run_compute(sspp_ctx* ctx) {
         return SSPP_OK;
     }
     const sspp_params& P = ctx->params;
-    const int cap1 = level1_cap(P), cap2 = level2_cap(P);
+    const int cap1 = std::min(level1_cap(P), kLightCap), cap2 = level2_cap(P);
     const int ht = P.heavy_threads == 128 ? 128 : 256;
     if (cap1 != ctx->configured_cap1 || cap2 != ctx->configured_cap2 || ht != ctx->configured_ht) {
         CK(reduce_configure(cap1, cap2, ht, &ctx->light_blocks_per_sm, &ctx->heavy_blocks_per_sm));
@@ -932,7 +935,7 @@ int run_compute(sspp_ctx* ctx) {
         std::vector<Step> st;
         for (int k = 0; k <= dhi - dlo; k++) {
             const int d = ascending ? dlo + k : dhi - k;
-            ss_schedule(P, I.act_begin[d], I.act_end[d], I.min_row[d] == INT_MAX ? 0 : I.min_row[d], I.max_row[d], st);
+            ss_schedule(P, kMinBlock, I.act_begin[d], I.act_end[d], I.min_row[d] == INT_MAX ? 0 : I.min_row[d], I.max_row[d], st);
         }
         return st;
     };

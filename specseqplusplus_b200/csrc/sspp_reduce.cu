@@ -8,12 +8,13 @@
 //   CPU tail stage                     include/specseq.h:705-1046 (no counterpart here:
 //                                      every column is finished on the device)
 //
-// Two tiers, as in the reference's two phases.  Light tier: one warp reduces
-// one column whose entries fit in the warp's shared-memory buffers (level-1
-// capacity).  Heavy tier: a column that outgrows them is handed to a second
-// kernel in which a whole CTA reduces it with buffers of the level-2 capacity,
-// and beyond that in exact-size arena buffers.  Both tiers run the same
-// column routine, written once over a "group" (warp or CTA).
+// Two tiers, as in the reference's two phases.  Light tier: warps reduce the
+// columns whose entries fit in a warp's shared-memory buffers (level-1
+// capacity), four tiny ones at a time.  Heavy tier: a column that outgrows them
+// is handed to a second kernel in which a whole CTA reduces it with buffers of
+// the level-2 capacity, and beyond that in exact-size arena buffers.  Both tiers
+// add in rounds (below) and share the column routine, written once over a
+// "group" (warp or CTA).
 //
 // Pivot table.  pivot[row] holds the owning column and the arena slot of the
 // owner's version (pv_pack), so the owner's entries are one dependent load
@@ -29,13 +30,16 @@
 // those of any sequential one.  Claiming a row also clears the row's own
 // column (twist clearing).
 //
-// Addition.  The addend is staged into shared memory with 16-byte vector loads
-// (header and entries in one round when it fits).  The next lowest row is
-// known before the merge - it is the largest index at which the tops of the
-// two lists stop agreeing - so the pivot entry of that row is requested before
-// the merge starts and arrives while it runs.  The merge computes each
-// element's output slot from its rank in the other list minus twice the
-// cancelled pairs before it (one ballot/prefix per round for both lists): no
+// Additions.  A column in shared memory takes its additions in rounds: the
+// owners of all its top rows at once (round_adds).  What a round cannot take
+// (an addend of more than kRoundAddend entries, a sum that does not fit, a column
+// in the arena) goes one addition at a time: the addend is staged into shared
+// memory with 16-byte vector loads (header and entries in one pass when it fits);
+// the next lowest row is known before the merge - it is the largest index at
+// which the tops of the two lists stop agreeing - so the pivot entry of that row
+// is requested before the merge starts and arrives while it runs.  The merge
+// computes each element's output slot from its rank in the other list minus twice
+// the cancelled pairs before it (one ballot/prefix per round for both lists): no
 // atomics, no scratch in global memory.
 #include <climits>
 #include <mutex>
@@ -47,11 +51,9 @@ namespace sspp {
 
 struct ReduceArgs {
     int32_t ncols;
-    const int32_t* active;
-    int32_t beg, end;
+    const int32_t* active;  // light tier: the step's runnable columns
     int32_t minrow;
     int32_t cap;          // shared-memory capacity per buffer (ints), multiple of 32
-    int32_t chunk;        // light tier: window entries taken per fetch (1..32)
     int32_t* arena;
     int64_t arena_cap;
     unsigned long long* arena_top;
@@ -62,7 +64,7 @@ struct ReduceArgs {
     uint8_t* cleared;
     int* ctr;             // per step: [0] chunk counter, [1] [2] heavy pool range, [3] heavy pull counter,
                           // [4] warp-tier blocks finished, [5] runnable columns listed by k_light_filter
-    const int* count;     // when set, the work is active[beg, beg + *count) (a filtered list)
+    const int* count;     // light tier: how many columns `active` lists
     int* ctr_next;        // the next step's counters (its pool range starts where this step's ends), or null
     int32_t* heavy;       // heavy pool (columns handed to the CTA tier, appended in step order)
     int* pool_tail;
@@ -131,6 +133,7 @@ struct WarpG {
         tb = __popc(mb);
     }
     __device__ __forceinline__ int sum(int v) const { return warp_sum(v); }
+    __device__ __forceinline__ int min_all(int v) const { return __reduce_min_sync(kFull, v); }
     // exclusive prefix of v over lower ranks; tot = group total
     __device__ __forceinline__ int prefix_int(int v, int& tot) const {
         int inc = warp_inclusive_scan(v);
@@ -209,6 +212,16 @@ struct BlockG {
         __syncthreads();
         tot = b[kWarps];
         return b[wid] + inc - v;
+    }
+    __device__ __forceinline__ int min_all(int v) const {
+        int* b = scan_buf();
+        v = __reduce_min_sync(kFull, v);
+        if ((threadIdx.x & 31) == 0) b[threadIdx.x >> 5] = v;
+        __syncthreads();
+        int m = b[0];
+#pragma unroll
+        for (int k = 1; k < kWarps; k++) m = min(m, b[k]);
+        return m;
     }
     __device__ __forceinline__ int sum(int v) const {
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -539,656 +552,296 @@ enum Outcome { OUT_OWNER, OUT_ZERO, OUT_PARKED, OUT_DEFERRED, OUT_FAIL };
 // additions between two looks at a column's cleared flag
 constexpr int kClearCheck = 64;
 
-// Short addends in the CTA tier.  Along the long chains the CTA tier runs, the
-// working column holds hundreds to thousands of entries while the addends
-// (owners' versions) hold a handful, so rewriting the column for each addend
-// would cost O(column) per addition.  Warp 0 alone keeps the column as a
-// sorted bulk in shared memory plus a delta: up to 32 pending entries (sorted,
-// one per lane, in registers) whose xor with the bulk is the column.  The
-// lowest row only moves down, so it is always the larger of the two tops (equal
-// tops cancel); an addition removes that top and toggles the addend's other
-// entries in the delta (a ballot and a shuffle each).  The delta is folded
-// into the bulk when it fills and when the warp stops, by rewriting the bulk
-// from the lowest position a delta entry lands, one constant-shift segment per
-// delta entry, through the spare buffer.  The rest of the CTA waits at one
-// barrier.  The warp stops, leaving the step to the general path, when the row
-// must be claimed (no owner, or a larger one), the column is empty or below the
-// band, or the addend is longer than kShortAddend entries or would not fit.
-// Returns the additions done, or -1 after a failed self-check.
-constexpr int kShortAddend = 28;  // header + entries in one 32-lane load
+// Rounds of additions.  Every row of the working column that an earlier
+// column owns may take that owner's addition, not only the lowest one: an entry
+// above the final lowest row has to go anyway, and adding an earlier column is
+// a left-to-right operation whichever entry it cancels.  So one round takes the
+// column's top rows, one per thread (at most G::kSize of them), and adds the
+// owners of all rows that have one at once:
+//   - each thread reads its row's inline apparent column and pivot entry
+//     together, then a published owner's header and entries: one chain of
+//     dependent loads per round instead of one per addition;
+//   - the addends' other entries, and the rows that take no addition (no
+//     owner, a later one, or one longer than kRoundAddend entries), are
+//     gathered in shared memory and sorted (64 per warp in registers, then
+//     ranked across the warps' runs);
+//   - entries that occur an even number of times cancel, and the rest is merged
+//     into what is left of the column by ranks, as a symmetric difference.
+// A round ends the loop when the lowest row itself takes no addition (it must
+// be claimed, or its owner goes through the general path) or the column is
+// empty or below the band.
+// Bound: latency (about a dozen barriers and two or three dependent loads per
+// round); the point is the number of rounds.  On the 64^3 lower-star grid the
+// longest chain of 3,725 single additions takes 123 rounds of 32 rows with 3,807
+// additions, 40 rounds of 128 with 4,339.
+constexpr int kRoundAddend = 32;  // longest published addend taken in a round
 
-struct FastState {
-    unsigned long long e;
-    long long add_ints;
-    int len, L, adds, bad;
-};
-
-// a[0..nb) xor {dv on lanes 0..d-1, ascending} back into a; returns the new
-// length (the caller keeps it within the buffer) and pads with INT_MAX.  One
-// warp; tmp is a spare buffer of the same capacity.
-__device__ int fold_delta(int32_t* a, int nb, int dv, int d, int32_t* tmp, int* err) {
+// two values per lane, element 2 * lane + {0, 1} of 64: ascending bitonic sort
+__device__ __forceinline__ void warp_sort64(int& x0, int& x1) {
     const int lane = threadIdx.x & 31;
-    int pos = nb;
-    bool fnd = false;
-    if (lane < d) {
-        pos = lower_bound_t<false>(a, nb, dv);
-        fnd = pos < nb && lds(a + pos) == dv;
+#pragma unroll
+    for (int k = 2; k <= 64; k <<= 1) {
+        const bool up = ((2 * lane) & k) == 0;
+#pragma unroll
+        for (int j = k >> 1; j > 1; j >>= 1) {
+            const int y0 = __shfl_xor_sync(kFull, x0, j >> 1), y1 = __shfl_xor_sync(kFull, x1, j >> 1);
+            const bool keep_min = (((2 * lane) & j) == 0) == up;
+            x0 = keep_min ? min(x0, y0) : max(x0, y0);
+            x1 = keep_min ? min(x1, y1) : max(x1, y1);
+        }
+        const int lo = min(x0, x1), hi = max(x0, x1);
+        x0 = up ? lo : hi;
+        x1 = up ? hi : lo;
     }
-    const int pmin = warp_min(pos);
-    const unsigned fmask = __ballot_sync(kFull, lane < d && fnd);
-    const unsigned imask = __ballot_sync(kFull, lane < d && !fnd);
-    // segment j (j = -1 .. d-1) of the bulk suffix: from delta entry j's position
-    // (past the entry it cancels) to the next delta entry's; its entries move by
-    // the insertions minus the cancellations at or before it
-    for (int j = -1; j < d; j++) {
-        const int pj = j < 0 ? pmin : __shfl_sync(kFull, pos, j);
-        const bool fj = j >= 0 && ((fmask >> j) & 1);
-        const int lo = pj + (fj ? 1 : 0);
-        const int hi = j + 1 < d ? __shfl_sync(kFull, pos, j + 1) : nb;
-        const unsigned upto = j < 0 ? 0u : (j == 31 ? kFull : ((2u << j) - 1));
-        const int shift = __popc(imask & upto) - __popc(fmask & upto);
-        for (int i = lo + lane; i < hi; i += 32) {
-            const int t = i - pmin + shift;
-            tmp[t] = lds(a + i);
+}
+
+// one value per lane, ascending
+__device__ __forceinline__ void warp_sort32(int& x) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const int y = __shfl_xor_sync(kFull, x, j);
+            x = (((lane & j) == 0) == ((lane & k) == 0)) ? min(x, y) : max(x, y);
         }
     }
-    if (lane < d && !fnd) {  // inserted delta entries land before the bulk entry at their position
-        const unsigned lt = lanemask_lt();
-        const int t = pos - pmin + __popc(imask & lt) - __popc(fmask & lt);
-        tmp[t] = dv;
-    }
-    __syncwarp();
-    const int outl = nb - pmin + __popc(imask) - __popc(fmask);
-    for (int i = lane; i < outl; i += 32) a[pmin + i] = tmp[i];
-    const int nn = pmin + outl;
-    if (lane < int(pad4(nn) - nn)) a[nn + lane] = INT_MAX;
-    __syncwarp();
-    (void)err;
-    return nn;
 }
 
-// Runs of additions.  Lane j keeps the bulk entry a[cb-1-j] (cb: the bulk
-// length when the cache was filled) and that row's inline apparent column, all
-// loaded at once.  While the current low is the bulk top at cache lane h and
-// its owner is an inline apparent column, the additions of the bulk rows at
-// lanes h, h+1, ... follow one another without a look at the column: row
-// r_{i+1} is the next low after the additions of r_h..r_i exactly when every
-// entry those addends toggle, and the delta's top, lie below r_{i+1} (equal
-// would cancel it).  Such a run removes its rows from the bulk top at once and
-// toggles the addends' other entries into the delta; no dependent load waits
-// between its additions.
-constexpr int kCacheRefill = 16;  // cache lanes used before the cache is filled again
-#ifndef SSPP_FAST_PREFETCH
-#define SSPP_FAST_PREFETCH 1
-#endif
-#ifndef SSPP_FAST_TOGGLE3
-#define SSPP_FAST_TOGGLE3 0
-#endif
-#ifndef SSPP_FAST_PVPF
-#define SSPP_FAST_PVPF 0
-#endif
+// Shared memory of a group's rounds besides its column buffers: the sorted
+// entries and, per entry, the counts of kept and cancelled entries before it.
+template <class G>
+struct RoundMem {
+    static constexpr int kEntries = 2 * G::kSize;  // entries of one round
+    int32_t s[kEntries];
+    int32_t pre[kEntries + 1];  // kept before | cancelled before << 15 | cancels << 30
+};
 
-// Inline apparent columns of the delta's entries (SSPP_FAST_DAP): when an
-// entry enters the delta, its row's inline column is copied asynchronously
-// (cp.async) into a ring of shared-memory slots, and the entry's lane keeps
-// the insertion index with it as entries shift.  When the delta's top becomes
-// the lowest row, often many additions after it was inserted, its column is
-// already in shared memory: no dependent global load on the chain.  Copies are
-// committed once per addition (or run); a read waits only for the group its
-// entry was inserted in, and each commit first lets all but the last two
-// groups finish, so a slot is never reused while a copy to it is in flight
-// (two groups hold at most 2 x 96 insertions, the ring has 256 slots).
-#ifndef SSPP_FAST_DAP
-#define SSPP_FAST_DAP 1
-#endif
-#ifndef SSPP_FAST_TOGGLE_EAGER
-#define SSPP_FAST_TOGGLE_EAGER 1
-#endif
-constexpr int kDapSlots = 256;
-static_assert(!(SSPP_FAST_DAP && SSPP_FAST_TOGGLE3), "the three-entry toggle does not carry insertion indices");
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// largest entry of an inline apparent column below its top (-1 if none)
-__device__ __forceinline__ int app_max_below(int4 q) {
-    return q.x <= 0 ? -1 : (q.x == 1 ? q.y : (q.x == 2 ? q.z : q.w));
-}
-
-template <int T>
-__device__ int fast_adds(const BlockG<T>& g, const ReduceArgs& A, int32_t minrow, int col, Work& w, int& L,
-                         uint64_t& e, int32_t* tmp, int32_t* sb, long long& adds, long long& add_ints,
-                         int iters_left) {
-    __shared__ FastState fs;
-#if SSPP_FAST_DAP
-    __shared__ int4 s_dap[kDapSlots];
-#endif
-    (void)sb;
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        int32_t* a = w.buf;
-        int nb = w.len;         // bulk a[0..nb), ascending; its top is a[nb-1]
-        int d = 0;              // delta: dv on lanes 0..d-1, ascending, INT_MAX above
-        int dv = INT_MAX;
-        int Lc = L, done = 0, bad = 0;
-        bool top_in_bulk = true;  // Lc is a[nb-1] (else the delta's top)
-        uint64_t ec = e;
-        long long ai = 0;
-        int n_inline = 0;
-        // bulk cache: lane j holds cr = a[cb - 1 - j] and its inline apparent column ca
-        int cb = -1;
-        int cr = -1;
-        int4 ca = make_int4(-1, 0, 0, 0);
-        // inline apparent columns of the last addend's largest entries,
-        // loaded while that addition runs: one of them is usually the next low
-        int pf_row = -1;
-        int4 pf_ap = make_int4(-1, 0, 0, 0);
-        uint64_t pf_pv = kNoOwner;  // ... and their pivot entries (relaxed), for owners that are not inline
-        bool have_pf_pv = false;    // ec_pf below holds the current low's prefetched entry
-        uint64_t ec_pf = kNoOwner;
-        int next_clear = kClearCheck;  // additions before the next look at the cleared flag
-        bool have_e = true;  // ec is the pivot entry of Lc
-#if SSPP_FAST_DAP
-        int dslot = 0;  // insertion index of dv (lanes < d); its inline column is s_dap[dslot % kDapSlots]
-        int nslot = 0;  // insertions so far
-        int g_open = 0, g_last = 0, g_prev = 0;  // first insertion of the open, last and previous groups
-        auto dap_commit = [&]() {
-            cp_async_commit();
-            cp_async_wait<2>();  // every group before the last two has landed
-            g_prev = g_last;
-            g_last = g_open;
-            g_open = nslot;
-        };
-#endif
-        // toggles x in the delta (a fold into the bulk when the delta is full
-        // invalidates the bulk cache)
-        // (both outcomes' ballots and shuffles are issued together before the
-        // branch: they depend only on the delta, so their latencies overlap;
-        // SSPP_FAST_TOGGLE_EAGER 0 keeps them in dependent order.  Measured at
-        // 64^3: one block per dimension 5.38 -> 5.29 ms, the reference's block
-        // sizes 5.33 -> 5.30 ms.  The warp tier's register path keeps the
-        // dependent order: there the eager form spilled and measured slower)
-        auto toggle = [&](int x) {
-#if SSPP_FAST_TOGGLE_EAGER
-            const unsigned eq = __ballot_sync(kFull, lane < d && dv == x);
-            unsigned lt = __ballot_sync(kFull, lane < d && dv < x);
-            const int nx = __shfl_down_sync(kFull, dv, 1);
-            const int pv = __shfl_up_sync(kFull, dv, 1);
-#if SSPP_FAST_DAP
-            const int ns = __shfl_down_sync(kFull, dslot, 1);
-            const int ps = __shfl_up_sync(kFull, dslot, 1);
-#endif
-            if (eq) {
-                const int q = __ffs(eq) - 1;
-                if (lane >= q) {
-                    dv = lane + 1 < d ? nx : INT_MAX;
-#if SSPP_FAST_DAP
-                    dslot = ns;
-#endif
-                }
-                d--;
+// Returns the number of rounds done, or -1 after a failed self-check; *stop is
+// set when the column was cleared meanwhile.  The column moves between w.buf and
+// `other`; sp holds the gathered entries.
+template <class G>
+__device__ int round_adds(const G& g, const ReduceArgs& A, int32_t minrow, int col, Work& w, int32_t* other,
+                          int32_t* sp, RoundMem<G>& R, int& L, uint64_t& e, long long& adds, long long& add_ints,
+                          bool* cleared) {
+    constexpr int kS = G::kSize, kWarps = kS / 32, kM = RoundMem<G>::kEntries;
+    const int rank = g.rank(), lane = threadIdx.x & 31, wid = kWarps > 1 ? rank >> 5 : 0;
+    const int mlimit = min(kM, A.cap);
+    int32_t* a = w.buf;
+    int32_t* out = other;
+    int n = w.len, Lc = L, rounds = 0, n_inline = 0, n_slot = 0;
+    bool fail = false;
+    uint64_t ev = kNoOwner;
+    while (n > 0 && Lc >= minrow) {
+        // ---- the top rows and their owners
+        const int idx = n - 1 - rank;
+        const int r = idx >= 0 ? lds(a + idx) : -1;
+        const bool valid = r >= 0 && r >= minrow && r < A.ncols;
+        int4 q = make_int4(-1, 0, 0, 0);
+        ev = kNoOwner;
+        unsigned clr = 0;
+        if (valid) {
+            q = __ldg(A.app + r);
+            ev = ld_acquire_u64(A.pivot + r);
+        }
+        if (rank == 0) clr = ld_acquire_u8(A.cleared + col);
+        const bool inl = q.x >= 0;
+        bool own = inl;
+        int cnt = inl ? q.x : 0;
+        const int32_t* src = nullptr;
+        if (!inl && pv_col(ev) < col && pv_slot(ev) + 2 * kHdr <= uint64_t(A.arena_cap)) {
+            src = A.arena + pv_slot(ev);
+            const int4 h = __ldcg(reinterpret_cast<const int4*>(src));
+            q = __ldcg(reinterpret_cast<const int4*>(src) + 1);  // the first entries (a slot without any is not an owner's)
+            if (h.x >= 1 && h.x <= kRoundAddend && h.y == pv_col(ev) &&
+                int64_t(pv_slot(ev)) + slot_ints(h.x) <= A.arena_cap) {
+                own = true;
+                cnt = h.x - 1;
+            }
+        } else if (inl) {
+            q = make_int4(q.y, q.z, q.w, 0);
+        }
+        // ---- how many rows this round takes: what they leave must fit the buffers
+        const int c = idx >= 0 ? (own ? cnt : 1) : 0;
+        int tot;
+        const int pre = g.prefix_int(c, tot);
+        const bool ok = idx >= 0 && pre + c <= mlimit && idx + pre + c <= A.cap && (rank > 0 || own);
+        const int K = g.min_all(clr ? -1 : (ok ? kS : rank));
+        if (K <= 0) {
+            *cleared = K < 0;
+            break;
+        }
+        // ---- gather
+        if (rank < K) {
+            if (!own) {
+                sp[pre] = r;
             } else {
-                if (d == 32) {  // full: the bulk absorbs the delta, then x goes in first
-                    nb = fold_delta(a, nb, dv, d, tmp, A.err);
-                    d = 0;
-                    dv = INT_MAX;
-                    cb = -1;
-                    lt = 0;
+                if (cnt > 0) sp[pre] = q.x;
+                if (cnt > 1) sp[pre + 1] = q.y;
+                if (cnt > 2) sp[pre + 2] = q.z;
+                if (cnt > 3) {
+                    sp[pre + 3] = q.w;
+                    for (int k = 4; k < cnt; k++) sp[pre + k] = __ldcg(src + kHdr + k);
                 }
-                const int q = __popc(lt);
-                if (lane > q && lane <= d) {  // never after a fold (d == 0): pv is not stale there
-                    dv = pv;
-#if SSPP_FAST_DAP
-                    dslot = ps;
-#endif
-                }
-                if (lane == q) {
-                    dv = x;
-#if SSPP_FAST_DAP
-                    dslot = nslot;
-                    int4* dst = s_dap + (nslot & (kDapSlots - 1));
-                    if (x >= 0 && x < A.ncols) cp_async16(dst, A.app + x);
-                    else *dst = make_int4(-1, 0, 0, 0);
-#endif
-                }
-#if SSPP_FAST_DAP
-                nslot++;
-#endif
-                d++;
+                n_inline += inl;
+                n_slot += !inl;
             }
-#else
-            const unsigned eq = __ballot_sync(kFull, lane < d && dv == x);
-            if (eq) {
-                const int q = __ffs(eq) - 1;
-                const int nx = __shfl_down_sync(kFull, dv, 1);
-#if SSPP_FAST_DAP
-                const int ns = __shfl_down_sync(kFull, dslot, 1);
-                if (lane >= q) {
-                    dv = lane + 1 < d ? nx : INT_MAX;
-                    dslot = ns;
-                }
-#else
-                if (lane >= q) dv = lane + 1 < d ? nx : INT_MAX;
-#endif
-                d--;
-            } else {
-                if (d == 32) {  // full: the bulk absorbs the delta
-                    nb = fold_delta(a, nb, dv, d, tmp, A.err);
-                    d = 0;
-                    dv = INT_MAX;
-                    cb = -1;
-                }
-                const int q = __popc(__ballot_sync(kFull, lane < d && dv < x));
-                const int pv = __shfl_up_sync(kFull, dv, 1);
-#if SSPP_FAST_DAP
-                const int ps = __shfl_up_sync(kFull, dslot, 1);
-                if (lane > q && lane <= d) {
-                    dv = pv;
-                    dslot = ps;
-                }
-                if (lane == q) {
-                    dv = x;
-                    dslot = nslot;
-                    int4* dst = s_dap + (nslot & (kDapSlots - 1));
-                    if (x >= 0 && x < A.ncols) cp_async16(dst, A.app + x);
-                    else *dst = make_int4(-1, 0, 0, 0);
-                }
-                nslot++;
-#else
-                if (lane > q && lane <= d) dv = pv;
-                if (lane == q) dv = x;
-#endif
-                d++;
-            }
-#endif
-        };
-        // toggles up to three ascending entries x0 < x1 < x2 at once: entries
-        // found in the delta are removed, the others inserted; every output
-        // lane finds its source with bit counts and one shuffle gathers it
-        auto toggle3 = [&](int q, int x0, int x1, int x2) {
-            if (d + q > 32) {  // the bulk absorbs the delta first
-                nb = fold_delta(a, nb, dv, d, tmp, A.err);
-                d = 0;
-                dv = INT_MAX;
-                cb = -1;
-            }
-            const unsigned below_d = d >= 32 ? kFull : ((1u << d) - 1);
-            unsigned del = 0;
-            int e0 = 64, e1 = 64, e2 = 64;  // output slots of the inserted entries (64: not inserted)
-            int ninsb = 0;                  // entries inserted so far (all smaller than the next one)
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                if (j >= q) break;
-                const int x = j == 0 ? x0 : (j == 1 ? x1 : x2);
-                const unsigned eq = __ballot_sync(kFull, dv == x) & below_d;
-                if (eq) {
-                    del |= eq;
-                } else {
-                    const unsigned lt = __ballot_sync(kFull, dv < x) & below_d;
-                    const int e = __popc(lt) - __popc(del & lt) + ninsb;
-                    if (j == 0) e0 = e;
-                    else if (j == 1) e1 = e;
-                    else e2 = e;
-                    ninsb++;
-                }
-            }
-            // output lane t: an inserted entry, or the (t - inserted before t)-th kept entry
-            const int kt = (e0 < lane) + (e1 < lane) + (e2 < lane);
-            int src = lane - kt;
-            unsigned dm = del;
-            while (dm) {
-                const int pdel = __ffs(dm) - 1;
-                if (pdel > src) break;
-                src++;
-                dm &= dm - 1;
-            }
-            const int g = __shfl_sync(kFull, dv, src & 31);
-            const int nd = d - __popc(del) + ninsb;
-            int v = src < d ? g : INT_MAX;
-            if (lane == e0) v = x0;
-            else if (lane == e1) v = x1;
-            else if (lane == e2) v = x2;
-            dv = lane < nd ? v : INT_MAX;
-            d = nd;
-        };
-        while (done < iters_left && nb + d > 0 && Lc >= minrow) {
-            if (done >= next_clear) {  // cleared meanwhile: the general path stops the column
-                next_clear = done + kClearCheck;
-                unsigned c = 0;
-                if (lane == 0) c = ld_acquire_u8(A.cleared + col);
-                if (__shfl_sync(kFull, c, 0)) break;
-            }
-            // the inline apparent column of the current low: from the bulk
-            // cache when the low is the bulk top, else one load
-            have_pf_pv = false;  // set below only when the prefetch holds this low's entry
-            int4 ap;
-            int h = -1;
-            if (top_in_bulk) {
-                if (cb < 0 || cb - nb >= kCacheRefill) {
-                    cb = nb;
-                    const int idx = nb - 1 - lane;
-                    cr = idx >= 0 ? lds(a + idx) : -1;
-                    ca = (cr >= 0 && cr < A.ncols) ? __ldg(A.app + cr) : make_int4(-1, 0, 0, 0);
-                }
-                h = cb - nb;
-                ap.x = __shfl_sync(kFull, ca.x, h);
-                ap.y = __shfl_sync(kFull, ca.y, h);
-                ap.z = __shfl_sync(kFull, ca.z, h);
-                ap.w = __shfl_sync(kFull, ca.w, h);
-                if (__shfl_sync(kFull, cr, h) != Lc) {  // self-check: the cache lane holds the bulk top
-                    bad = 1;
-                    break;
-                }
-            } else {
-#if SSPP_FAST_DAP
-                // the low is the delta's top (lane d - 1): its column is in the ring
-                const int idx = __shfl_sync(kFull, dslot, d - 1);
-                if (idx >= g_last) cp_async_wait<0>();
-                else if (idx >= g_prev) cp_async_wait<1>();
-                __syncwarp();
-                ap = s_dap[idx & (kDapSlots - 1)];
-#else
-                const unsigned pm = __ballot_sync(kFull, pf_row == Lc);
-                const int src = pm ? __ffs(pm) - 1 : 31;
-                ap = pf_ap;
-                if (!pm) {
-                    ap = make_int4(-1, 0, 0, 0);
-                    if (lane == 31 && Lc >= 0 && Lc < A.ncols) ap = __ldg(A.app + Lc);
-                }
-                ap.x = __shfl_sync(kFull, ap.x, src);
-                ap.y = __shfl_sync(kFull, ap.y, src);
-                ap.z = __shfl_sync(kFull, ap.z, src);
-                ap.w = __shfl_sync(kFull, ap.w, src);
-                have_pf_pv = pm != 0 && ap.x < 0 && SSPP_FAST_PREFETCH && SSPP_FAST_PVPF;
-                if (have_pf_pv) ec_pf = __shfl_sync(kFull, (unsigned long long)pf_pv, src);
-#endif
-            }
-            if (top_in_bulk && ap.x >= 0) {
-                // a run from cache lane h: lane l (> h) joins while lanes h..l-1
-                // all joined, its row has an inline apparent column, and the
-                // delta top and every entry the run toggled so far lie below it
-                const int td = d > 0 ? __shfl_sync(kFull, dv, d - 1) : -1;
-                const bool mine = lane >= h && cr >= 0 && ca.x >= 0;
-                int mx = mine ? app_max_below(ca) : -1;
-                mx = mx > td ? mx : td;
-                int M = mx;  // inclusive prefix max over lanes h..lane
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(kFull, M, o);
-                    if (lane >= o && lane - o >= h) M = t > M ? t : M;
-                }
-                const int mprev = __shfl_up_sync(kFull, M, 1);   // prefix max up to lane - 1
-                const int mcnt = mine ? ca.x : 0;
-                // entries toggled by lanes h..lane (inclusive), for the capacity bound
-                int csum = mcnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(kFull, csum, o);
-                    if (lane >= o && lane - o >= h) csum += t;
-                }
-                const bool join = lane == h || (lane > h && mine && mprev < cr);
-                const bool fits = nb + d + csum <= A.cap && lane - h < iters_left - done;
-                const unsigned stop = __ballot_sync(kFull, lane >= h && !(join && fits));
-                // lanes h .. first stopping lane - 1 form the run; lane h always
-                // joins, so the run is empty only when lane h does not fit
-                const unsigned above = stop & (kFull << h);
-                const int end = above ? __ffs(above) - 1 : 32;
-                const int P = end - h;
-                if (P > 0) {
-                    const int rlast = __shfl_sync(kFull, cr, end - 1);
-                    nb -= P;
-                    for (int i = h; i < end; i++) {
-                        const int qx = __shfl_sync(kFull, ca.x, i);
-                        const int qy = __shfl_sync(kFull, ca.y, i);
-                        const int qz = __shfl_sync(kFull, ca.z, i);
-                        const int qw = __shfl_sync(kFull, ca.w, i);
-                        if (SSPP_FAST_TOGGLE3) {
-                            if (qx > 0) toggle3(qx, qy, qz, qw);
-                        } else {
-                            if (qx > 0) toggle(qy);
-                            if (qx > 1) toggle(qz);
-                            if (qx > 2) toggle(qw);
-                        }
-                        ai += 2 * (nb + d) + qx + 2;
-                    }
-                    done += P;
-                    n_inline += P;
-                    pf_row = -1;
-#if SSPP_FAST_DAP
-                    dap_commit();
-#endif
-                    // the next lowest row: the larger top; equal tops cancel
-                    int nl = -1;
-                    while (true) {
-                        const int tb = nb > 0 ? lds(a + nb - 1) : -1;
-                        const int tdd = d > 0 ? __shfl_sync(kFull, dv, d - 1) : -1;
-                        if (tb >= 0 && tb == tdd) {
-                            nb--;
-                            d--;
-                            if (lane == d) dv = INT_MAX;
-                            continue;
-                        }
-                        top_in_bulk = tb > tdd;
-                        nl = top_in_bulk ? tb : tdd;
-                        break;
-                    }
-                    if (nl >= rlast || nl >= A.ncols) {  // self-check: the lowest row only moves down
-                        bad = 1;
-                        break;
-                    }
-                    Lc = nl;
-                    have_e = false;
-                    ec = kNoOwner;  // unknown; the general path's claim retries with the real entry
-                    continue;
-                }
-            }
-            int plen, bj;
-            if (ap.x >= 0) {  // apparent owner: permanent, its entries are at hand
-                plen = ap.x + 1;
-                bj = lane == 0 ? ap.y : (lane == 1 ? ap.z : ap.w);
-            } else {
-                if (!have_e) {
-                    if (have_pf_pv) {
-                        // read early (relaxed): an older entry still names an earlier
-                        // column with this low, whose published versions never change;
-                        // the fence orders the slot reads after it
-                        ec = ec_pf;
-                        __threadfence();
-                    } else {
-                        uint64_t t = 0;
-                        if (lane == 0) t = ld_acquire_u64(A.pivot + Lc);
-                        ec = __shfl_sync(kFull, (unsigned long long)t, 0);
-                    }
-                    have_e = true;
-                }
-                if (pv_col(ec) >= col) break;                         // claim: the general path
-                if (pv_slot(ec) + kHdr > uint64_t(A.arena_cap)) break;  // the general path reports it
-                const int v = __ldcg(A.arena + pv_slot(ec) + lane);      // header and the first 28 entries
-                plen = __shfl_sync(kFull, v, 0);
-                const int hcol = __shfl_sync(kFull, v, 1);
-                if (plen < 1 || plen > kShortAddend || hcol != pv_col(ec)) break;
-                if (__shfl_sync(kFull, v, (kHdr + plen - 1) & 31) != Lc) break;  // the general path reports it
-                bj = __shfl_sync(kFull, v, (lane + kHdr) & 31);
-            }
-            const int m = plen - 1;  // addend entries below the common top
-            if (nb + d + m > A.cap) break;  // the folded column might not fit
-            // the addend's three largest other entries: their inline apparent
-            // columns load while this addition runs
-            pf_row = -1;
-            if (SSPP_FAST_PREFETCH && !SSPP_FAST_DAP && lane < m && lane >= m - 3 && bj >= 0 && bj < A.ncols) {
-                pf_row = bj;
-                pf_ap = __ldg(A.app + bj);
-                if (SSPP_FAST_PVPF) pf_pv = ld_relaxed_u64(A.pivot + bj);
-            }
-            if (top_in_bulk) {  // the tops cancel
-                nb--;
-            } else {
-                d--;
-                if (lane == d) dv = INT_MAX;
-            }
-            // toggle the addend's other entries in the delta
-            if (SSPP_FAST_TOGGLE3 && ap.x >= 0) {
-                if (m > 0) toggle3(m, ap.y, ap.z, ap.w);
-            } else {
-                for (int j = 0; j < m; j++) toggle(__shfl_sync(kFull, bj, j));
-            }
-#if SSPP_FAST_DAP
-            dap_commit();
-#endif
-            // the next lowest row: the larger top; equal tops cancel
-            int nl = -1;
-            while (true) {
-                const int tb = nb > 0 ? lds(a + nb - 1) : -1;
-                const int td = d > 0 ? __shfl_sync(kFull, dv, d - 1) : -1;
-                if (tb >= 0 && tb == td) {
-                    nb--;
-                    d--;
-                    if (lane == d) dv = INT_MAX;
-                    continue;
-                }
-                top_in_bulk = tb > td;
-                nl = top_in_bulk ? tb : td;
-                break;
-            }
-            ai += 2 * (nb + d) + plen + 1;
-            done++;
-            if (ap.x >= 0) n_inline++;
-            if (nl >= Lc || nl >= A.ncols) {  // self-check: the lowest row only moves down
-                bad = 1;
+            if (rank == K - 1) R.pre[kM] = pre + c;  // entries of the rows taken
+        }
+        g.sync();
+        const int m = lds(R.pre + kM);
+        const int nc = n - K;
+        if (kWarps == 1 && nc == 0 && m <= 32) {
+            // a warp's short column, all of it taken: one entry per lane, sorted and
+            // cancelled in registers
+            int x = lane < m ? lds(sp + lane) : INT_MAX;
+            warp_sort32(x);
+            const int up = __shfl_up_sync(kFull, x, 1);
+            const unsigned in = m == 32 ? kFull : (1u << m) - 1;
+            const unsigned head = __ballot_sync(kFull, lane < m && (lane == 0 || x != up));
+            // a run goes on to the next head (or the end); odd runs keep one entry
+            const unsigned later = lane == 31 ? 0u : head & (kFull << (lane + 1));
+            const int end = later ? __ffs(later) - 1 : __popc(in);
+            const unsigned keep = __ballot_sync(kFull, ((head >> lane) & 1) && ((end - lane) & 1));
+            const int nn = __popc(keep), at = __popc(keep & lanemask_lt());
+            if ((keep >> lane) & 1) out[at] = x;
+            if (lane < int(pad4(nn) - nn)) out[nn + lane] = INT_MAX;
+            const int nl = keep ? __shfl_sync(kFull, x, 31 - __clz(keep)) : -1;
+            __syncwarp();
+            add_ints += n + m + nn;
+            n = nn;
+            int32_t* t = a;
+            a = out;
+            out = t;
+            rounds++;
+            if (nl >= Lc) {
+                if (g.leader()) atomicOr(A.err, ERRB_CHECK);
+                fail = true;
                 break;
             }
             Lc = nl;
-            have_e = false;
-            ec = kNoOwner;  // unknown; the general path's claim retries with the real entry
+            continue;
         }
-        if (d > 0) nb = fold_delta(a, nb, dv, d, tmp, A.err);
-#if SSPP_FAST_DAP
-        cp_async_wait<0>();  // no copy may land in the ring after this call
-#endif
-        if (lane == 0) {
-            fs.len = nb;
-            fs.L = nb > 0 ? lds(a + nb - 1) : -1;
-            fs.e = ec;
-            fs.adds = done;
-            fs.add_ints = ai;
-            fs.bad = bad || (fs.L != (nb > 0 ? Lc : -1) && done > 0);
-            if (fs.bad) atomicOr(A.err, ERRB_CHECK);
-            if (done) {
-                cnt_add(&A.counters[CNT_FAST_INLINE], n_inline);
-                cnt_add(&A.counters[CNT_FAST_SLOT], done - n_inline);
+        // ---- sort
+        const int i0 = 2 * rank;
+        int x0 = INT_MAX, x1 = INT_MAX;
+        if (kWarps == 1 || 64 * wid < m) {
+            if (i0 < m) x0 = lds(sp + i0);
+            if (i0 + 1 < m) x1 = lds(sp + i0 + 1);
+            warp_sort64(x0, x1);
+            if (kWarps == 1) {
+                R.s[i0] = x0;
+                R.s[i0 + 1] = x1;
             }
         }
-    }
-    __syncthreads();
-    const int done = fs.adds;
-    if (fs.bad) return -1;
-    if (done > 0) {
-        w.len = fs.len;
-        w.dirty = true;
-        L = fs.L;
-        e = fs.e;
-        adds += done;
-        add_ints += fs.add_ints;
-    }
-    __syncthreads();  // fs is rewritten by the next call
-    return done;
-}
-
-// Warp tier, inline apparent addends.  A working column of at most 32 entries
-// is held in registers, one entry per lane, ascending; while the owner of its
-// lowest row is an inline apparent column (Device::app), an addition removes
-// the top and toggles the addend's other entries in place (a ballot and a
-// shuffle each), with no staging and no shared-memory merge, and the inline
-// columns of the addend's entries load during the addition (one of them is
-// usually the next low).  Stops at a row without such an owner, below the
-// band, or when the column would outgrow 32 entries or the buffer; the column
-// goes back to w.buf.  Returns the additions done, or -1 after a failed
-// self-check.
-#ifndef SSPP_WARP_REG
-#define SSPP_WARP_REG 1
-#endif
-__device__ int warp_adds(const ReduceArgs& A, int32_t minrow, Work& w, int& L, uint64_t& e, int4 ap, long long& adds,
-                         long long& add_ints, int iters_left) {
-    const int lane = threadIdx.x & 31;
-    int len = w.len;
-    int ev = lane < len ? lds(w.buf + lane) : INT_MAX;
-    int Lc = L, done = 0;
-    bool bad = false;
-    long long ai = 0;
-    int pf_row = -1;
-    int4 pf_ap = make_int4(-1, 0, 0, 0);
-    while (done < iters_left && ap.x >= 0) {
-        const int m = ap.x;
-        if (len - 1 + m > 32 || len - 1 + m > A.cap) break;
-        const int bj = lane == 0 ? ap.y : (lane == 1 ? ap.z : ap.w);
-        pf_row = -1;
-        if (lane < m && bj >= 0 && bj < A.ncols) {
-            pf_row = bj;
-            pf_ap = __ldg(A.app + bj);
-        }
-        len--;  // the tops cancel
-        if (lane == len) ev = INT_MAX;
-        for (int j = 0; j < m; j++) {
-            const int x = j == 0 ? ap.y : (j == 1 ? ap.z : ap.w);
-            const unsigned eq = __ballot_sync(kFull, lane < len && ev == x);
-            if (eq) {
-                const int q = __ffs(eq) - 1;
-                const int nx = __shfl_down_sync(kFull, ev, 1);
-                if (lane >= q) ev = lane + 1 < len ? nx : INT_MAX;
-                len--;
+        if constexpr (kWarps > 1) {
+            const int runs = (m + 63) >> 6;
+            if (runs == 1) {
+                if (wid == 0) {
+                    R.s[i0] = x0;
+                    R.s[i0 + 1] = x1;
+                }
             } else {
-                const int q = __popc(__ballot_sync(kFull, lane < len && ev < x));
-                const int pv = __shfl_up_sync(kFull, ev, 1);
-                if (lane > q && lane <= len) ev = pv;
-                if (lane == q) ev = x;
-                len++;
+                __syncthreads();  // every gathered entry is in registers
+                if (wid < runs) {
+                    if (i0 < mlimit) sp[i0] = x0;
+                    if (i0 + 1 < mlimit) sp[i0 + 1] = x1;
+                }
+                __syncthreads();
+                if (wid < runs) {
+                    // ranks over the other runs (equal entries of earlier runs come first); the last
+                    // run's padding stays behind every entry
+                    int p0 = 2 * lane, p1 = 2 * lane + 1;
+                    for (int k = 0; k < runs; k++) {
+                        if (k == wid) continue;
+                        const int len = min(64, m - 64 * k);
+                        const int bump = k < wid ? 1 : 0;
+                        if (x0 != INT_MAX) p0 += lower_bound_t<false>(sp + 64 * k, len, x0 + bump);
+                        if (x1 != INT_MAX) p1 += lower_bound_t<false>(sp + 64 * k, len, x1 + bump);
+                    }
+                    if (x0 != INT_MAX) R.s[p0] = x0;
+                    if (x1 != INT_MAX) R.s[p1] = x1;
+                }
             }
         }
-        ai += 2 * len + m + 2;
-        done++;
-        const int nl = len > 0 ? __shfl_sync(kFull, ev, (len - 1) & 31) : -1;
+        g.sync();
+        // ---- parity of each entry, and whether the rest of the column holds it
+        int kept0 = 0, canc0 = 0, kept1 = 0, canc1 = 0, rc0 = 0, rc1 = 0;
+        auto look = [&](int i, int& x, int& rc, int& kept, int& canc) {
+            if (i >= m) return;
+            x = lds(R.s + i);
+            if (i > 0 && lds(R.s + i - 1) == x) return;
+            int j = i + 1;
+            while (j < m && lds(R.s + j) == x) j++;
+            if (((j - i) & 1) == 0) return;
+            rc = lower_bound_t<false>(a, nc, x);
+            canc = rc < nc && lds(a + rc) == x;
+            kept = !canc;
+        };
+        look(i0, x0, rc0, kept0, canc0);
+        look(i0 + 1, x1, rc1, kept1, canc1);
+        int tp;
+        const int pp = g.prefix_int((kept0 + kept1) | ((canc0 + canc1) << 15), tp);
+        const int pp1 = pp + (kept0 | (canc0 << 15));
+        if (i0 < m) R.pre[i0] = pp | (canc0 << 30);
+        if (i0 + 1 < m) R.pre[i0 + 1] = pp1 | (canc1 << 30);
+        const int kept_all = tp & 0x7fff, canc_all = tp >> 15;
+        // self-check on every store: positions stay inside the buffer (sorted lists never leave it)
+        auto put = [&](int pos, int x) {
+            if (unsigned(pos) < unsigned(A.cap)) out[pos] = x;
+            else atomicOr(A.err, ERRB_CHECK);
+        };
+        if (kept0) put(rc0 - (pp >> 15) + (pp & 0x7fff), x0);
+        if (kept1) put(rc1 - (pp1 >> 15) + (pp1 & 0x7fff), x1);
+        g.sync();
+        // ---- the rest of the column, shifted by the entries kept and cancelled below each
+        const int s0 = m > 0 ? lds(R.s) : INT_MAX;
+        for (int j = rank; j < nc; j += kS) {
+            const int y = lds(a + j);
+            if (y < s0) {
+                out[j] = y;
+                continue;
+            }
+            const int p = lower_bound_t<false>(R.s, m, y);
+            if (p == m) {
+                put(j - canc_all + kept_all, y);
+            } else {
+                const int v = lds(R.pre + p);
+                if (!(v >> 30) || lds(R.s + p) != y) put(j - ((v >> 15) & 0x7fff) + (v & 0x7fff), y);
+            }
+        }
+        const int nn = nc - canc_all + kept_all;
+        if (rank < int(pad4(nn) - nn)) out[nn + rank] = INT_MAX;
+        g.sync();
+        add_ints += n + m + nn;
+        n = nn;
+        int32_t* t = a;
+        a = out;
+        out = t;
+        rounds++;
+        const int nl = n > 0 ? lds(a + n - 1) : -1;
         if (nl >= Lc) {  // self-check: the lowest row only moves down
-            bad = true;
+            if (g.leader()) atomicOr(A.err, ERRB_CHECK);
+            fail = true;
             break;
         }
         Lc = nl;
-        if (Lc < 0 || Lc < minrow) break;
-        const unsigned pm = __ballot_sync(kFull, pf_row == Lc);
-        const int src = pm ? __ffs(pm) - 1 : 31;
-        int4 q4 = pf_ap;
-        if (!pm) {
-            q4 = make_int4(-1, 0, 0, 0);
-            if (lane == 31 && Lc < A.ncols) q4 = __ldg(A.app + Lc);
-        }
-        ap.x = __shfl_sync(kFull, q4.x, src);
-        ap.y = __shfl_sync(kFull, q4.y, src);
-        ap.z = __shfl_sync(kFull, q4.z, src);
-        ap.w = __shfl_sync(kFull, q4.w, src);
     }
-    if (bad) {
-        if (lane == 0) atomicOr(A.err, ERRB_CHECK);
-        return -1;
-    }
-    if (done > 0) {
-        if (lane < pad4(len)) w.buf[lane] = lane < len ? ev : INT_MAX;
-        __syncwarp();
-        w.len = len;
+    if (fail) return -1;
+    e = g.bcast64(ev);  // the entry of the row the rounds stopped at
+    if (rounds > 0) {
+        w.buf = a;
+        w.len = n;
         w.dirty = true;
         L = Lc;
-        uint64_t t = kNoOwner;
-        if (lane == 0 && Lc >= 0 && Lc >= minrow) t = ld_acquire_u64(A.pivot + Lc);
-        e = __shfl_sync(kFull, (unsigned long long)t, 0);
-        adds += done;
-        add_ints += ai;
+        const int ni = g.sum(n_inline), ns = g.sum(n_slot);
+        adds += ni + ns;
+        if (g.leader() && kWarps > 1) {
+            cnt_add(&A.counters[CNT_FAST_INLINE], ni);
+            cnt_add(&A.counters[CNT_FAST_SLOT], ns);
+        }
     }
-    return done;
+    return rounds;
 }
 
 // Reduces column `col` until it owns its lowest row, becomes zero, or its
@@ -1199,7 +852,7 @@ __device__ int warp_adds(const ReduceArgs& A, int32_t minrow, Work& w, int& L, u
 // if none).  sp holds kHdr + cap ints (staged addend with its header).
 template <class G>
 __device__ Outcome reduce_column(const G& g, const ReduceArgs& A, const Band& band, int col, int32_t* sw0,
-                                 int32_t* sw1, int32_t* sp, bool defer, int* displaced) {
+                                 int32_t* sw1, int32_t* sp, RoundMem<G>& rm, bool defer, int* displaced) {
     const int32_t minrow = band.minrow;
     *displaced = -1;
     uint64_t d = 0;
@@ -1242,8 +895,7 @@ __device__ Outcome reduce_column(const G& g, const ReduceArgs& A, const Band& ba
     }
     // inline apparent column of row r (every thread loads it: one transaction per warp)
     auto app_of = [&](int r) { return (r >= 0 && r >= minrow) ? __ldg(A.app + r) : make_int4(-1, 0, 0, 0); };
-    int4 apc = app_of(L);
-    if (L >= minrow) {
+    if (w.global && L >= minrow) {
         if (g.leader()) e = ld_acquire_u64(A.pivot + L);
         e = g.bcast64(e);
     }
@@ -1251,22 +903,29 @@ __device__ Outcome reduce_column(const G& g, const ReduceArgs& A, const Band& ba
     const int first4 = min(G::kSize, (kHdr + A.cap) >> 2);
     int next_check = 0;
     for (int iter = 0;; iter++) {
-        if (iter >= next_check) {
-            // Cleared meanwhile: a column of the next higher dimension claimed this
-            // column's row, so the column is positive and zero once reduced (and a row
-            // never loses its owner, so it stays cleared).  It owns no row now (a claim
-            // ends the reduction), so it stops here as zero.
+        bool clr = false;
+        if (!w.global) {  // rounds of additions; they end with the entry of the row they stop at
+            const int done = round_adds(g, A, minrow, col, w, w.buf == sw0 ? sw1 : sw0, sp, rm, L, e, adds, add_ints,
+                                        &clr);
+            if (done < 0) break;
+            iter += done;
+        } else if (iter >= next_check) {
             next_check = iter + kClearCheck;
             int c = 0;
             if (g.leader()) c = int(ld_acquire_u8(A.cleared + col));
-            if (g.bcast(c)) {
-                if (g.leader()) {
-                    A.desc[col] = pack_desc(0, 0);
-                    A.low[col] = -1;
-                }
-                res = OUT_ZERO;
-                break;
+            clr = g.bcast(c) != 0;
+        }
+        // Cleared meanwhile: a column of the next higher dimension claimed this
+        // column's row, so the column is positive and zero once reduced (and a row
+        // never loses its owner, so it stays cleared).  It owns no row now (a claim
+        // ends the reduction), so it stops here as zero.
+        if (clr) {
+            if (g.leader()) {
+                A.desc[col] = pack_desc(0, 0);
+                A.low[col] = -1;
             }
+            res = OUT_ZERO;
+            break;
         }
         if (w.len == 0) {
             if (g.leader()) {
@@ -1314,14 +973,10 @@ __device__ Outcome reduce_column(const G& g, const ReduceArgs& A, const Band& ba
             e = old;  // someone else changed the owner; look again
             continue;
         }
-        // looked at on every pass once the chain is long enough: the register
-        // path adds many additions to iter at once, so iter seldom lands on a
-        // multiple of the limit (a test on multiples misses most long chains;
-        // measured at 64^3: 5.90 -> 5.38 ms per reduction with every pass)
+        // long chains of the warp tier: once the step's window is handed out they
+        // only hold up the step's tail, and the CTA tier continues them on a side
+        // stream while the next step runs (iter counts rounds here)
         if (defer && band.drain_ctr && A.light_chain > 0 && iter >= A.light_chain) {
-            // once the step's window is handed out, a long chain in the warp tier
-            // only holds up the step's tail: the CTA tier continues it on a side
-            // stream while the next step runs
             int drained = 0;
             if (g.leader()) drained = __ldcg(band.drain_ctr) >= band.drain_total;
             if (g.bcast(drained)) {
@@ -1330,38 +985,13 @@ __device__ Outcome reduce_column(const G& g, const ReduceArgs& A, const Band& ba
                 break;
             }
         }
-        if constexpr (G::kSize > 32) {  // CTA tier: short addends by one warp
-            if (!w.global) {
-                const int done = fast_adds(g, A, minrow, col, w, L, e, w.buf == sw0 ? sw1 : sw0, sp, adds, add_ints,
-                                           kMaxMergesPerColumn - iter);
-                if (done < 0) break;
-                if (done > 0) {
-                    iter += done;
-                    apc = app_of(L);
-                    continue;
-                }
-            }
-        } else if (SSPP_WARP_REG) {  // warp tier: the column in registers
-            if (!w.global && apc.x >= 0 && w.len <= 32) {
-#ifndef SSPP_WARP_RUN_CAP
-#define SSPP_WARP_RUN_CAP kClearCheck
-#endif
-                const int done = warp_adds(A, minrow, w, L, e, apc, adds, add_ints,
-                                           min(SSPP_WARP_RUN_CAP, kMaxMergesPerColumn - iter));
-                if (done < 0) break;
-                if (done > 0) {
-                    iter += done;
-                    apc = app_of(L);
-                    continue;
-                }
-            }
-        }
         // add the owner's version (p < col, same lowest row): stage header + entries
         if (pv_slot(e) + kHdr > uint64_t(A.arena_cap)) {  // self-check: entry inside the arena
             if (g.leader()) atomicOr(A.err, ERRB_CHECK);
             break;
         }
         const int32_t* src = A.arena + pv_slot(e);
+        const int4 apc = app_of(L);
         int plen;
         if (apc.x >= 0) {  // apparent owner: its entries are inline, no arena read
             plen = apc.x + 1;
@@ -1415,7 +1045,6 @@ __device__ Outcome reduce_column(const G& g, const ReduceArgs& A, const Band& ba
         // element, so its acquire load completes while the others merge
         uint64_t pref = kNoOwner;
         if (g.rank() == G::kSize - 1 && L2 >= minrow && L2 >= 0) pref = ld_acquire_u64(A.pivot + L2);
-        const int4 apn = app_of(L2);
         int out_len;
         const int bound = w.len + plen - 2;
         if (bound <= A.cap) {
@@ -1478,7 +1107,6 @@ __device__ Outcome reduce_column(const G& g, const ReduceArgs& A, const Band& ba
         w.dirty = true;
         L = L2;
         e = g.bcast64_last(pref);
-        apc = apn;
     }
     if (g.leader() && adds) {
         cnt_add(&A.counters[CNT_ADDITIONS], adds);
@@ -1567,54 +1195,328 @@ __device__ void light_block_done(const ReduceArgs& A) {
     }
 }
 
-// Light tier: warps take `chunk` window entries at a time and reduce the
-// runnable ones (active, not cleared, lowest row inside the band).
-// At least 9 blocks per SM: the compiler then keeps the kernel at 56 registers
-// with nothing spilled (left free, it spilled 16 bytes at the same count);
-// measured 64^3 5.79 -> 5.60 ms per reduction.
-#ifndef SSPP_LIGHT_MIN_BLOCKS
-#define SSPP_LIGHT_MIN_BLOCKS 9
-#endif
-__global__ void __launch_bounds__(128, SSPP_LIGHT_MIN_BLOCKS) k_reduce_light(ReduceArgs A) {
-    extern __shared__ __align__(16) int32_t smem[];
-    WarpG g;
-    const int lane = g.rank();
-    int32_t* sw0 = smem + size_t(threadIdx.x >> 5) * (3 * A.cap + kHdr);
-    int32_t* sw1 = sw0 + A.cap;
-    int32_t* sp = sw1 + A.cap;
-    const int count = A.count ? __ldcg(A.count) : A.end - A.beg;
-    const int end = A.beg + count;
-    const int chunk = A.chunk;
-    const Band band{A.minrow, A.ctr, count};
-    bool stop = false;  // warp-uniform: a failure ends this warp's work
-    while (!stop) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(A.ctr, chunk);
-        base = g.bcast(base);
-        if (base >= count) break;
-        const int idx = A.beg + base + lane;
-        int c = -1;
-        bool run = false;
-        if (lane < chunk && idx < end) {
-            c = A.active[idx];
-            run = ld_acquire_u8(A.state + c) == ST_ACTIVE && !ld_acquire_u8(A.cleared + c) &&
-                  __ldcg(A.low + c) >= A.minrow;
+// Light tier.  Most columns a step lists are tiny: at 64^3, 99% of them hold at
+// most 8 entries throughout and need one round of additions (two to four
+// addends) before they claim a row.  A warp therefore reduces four columns at a
+// time, eight lanes each with one entry per lane (largest first), in lockstep:
+// every pass of the loop refills idle groups, reads all groups' rows' inline
+// columns and pivot entries together, sorts what the addends leave (at most 16
+// entries a group) in registers, and publishes and claims for the groups that
+// reached a row to claim.  The dependent loads and the instructions of a pass
+// are shared by four columns.  A column that outgrows its group (more than 8
+// entries, more than 16 gathered, or a long addend) is published and finished
+// by the whole warp (reduce_column).
+constexpr int kGroup = 8;            // lanes and entries of a tiny column
+constexpr int kGroupGather = 16;     // entries a tiny column's round may gather
+
+// two values per lane over 8 lanes, element 2 * (lane & 7) + {0, 1}: descending bitonic sort of 16
+__device__ __forceinline__ void group_sort16(int& x0, int& x1) {
+    const int gl = threadIdx.x & (kGroup - 1);
+#pragma unroll
+    for (int k = 2; k <= 16; k <<= 1) {
+        const bool down = ((2 * gl) & k) == 0;
+#pragma unroll
+        for (int j = k >> 1; j > 1; j >>= 1) {
+            const int y0 = __shfl_xor_sync(kFull, x0, j >> 1), y1 = __shfl_xor_sync(kFull, x1, j >> 1);
+            const bool keep_max = (((2 * gl) & j) == 0) == down;
+            x0 = keep_max ? max(x0, y0) : min(x0, y0);
+            x1 = keep_max ? max(x1, y1) : min(x1, y1);
         }
-        unsigned m = __ballot_sync(kFull, run);
-        while (m && !stop) {
-            const int src = __ffs(m) - 1;
-            m &= m - 1;
-            int col = __shfl_sync(kFull, c, src);
-            while (col >= 0) {  // the column, then any owner it displaced
-                int next = -1;
-                Outcome o = reduce_column(g, A, band, col, sw0, sw1, sp, true, &next);
-                if (!settle(g, A, col, o)) {
+        const int lo = min(x0, x1), hi = max(x0, x1);
+        x0 = down ? hi : lo;
+        x1 = down ? lo : hi;
+    }
+}
+
+// bit i of an 8-bit mask to bit 2i
+__device__ __forceinline__ unsigned spread8(unsigned b) {
+    b = (b | (b << 4)) & 0x0f0fu;
+    b = (b | (b << 2)) & 0x3333u;
+    return (b | (b << 1)) & 0x5555u;
+}
+
+// At least 6 blocks per SM (80 registers, nothing spilled).  64^3, one block per
+// dimension: 8 / 7 / 6 / 5 blocks 1,228 / 1,192 / 1,223 / 1,250 us of reduction; small
+// inputs prefer few blocks (1,200-point cloud 396 / 375 / 360 / 356 us).
+constexpr int kLightMinBlocks = 6;
+__global__ void __launch_bounds__(128, kLightMinBlocks) k_reduce_light(ReduceArgs A) {
+    extern __shared__ __align__(16) int32_t smem[];
+    __shared__ RoundMem<WarpG> s_rm[4];
+    RoundMem<WarpG>& rm = s_rm[threadIdx.x >> 5];
+    WarpG g;
+    const int lane = g.rank(), gl = lane & (kGroup - 1), lead = lane & ~(kGroup - 1);
+    int32_t* sw0 = smem + size_t(threadIdx.x >> 5) * (3 * A.cap + kHdr);
+    int32_t* gbuf = rm.s + 2 * lead;  // 16 entries per group
+    const int count = __ldcg(A.count);
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    // list entries a warp takes at a time: enough to keep its groups busy, few enough to share a short list
+    const int chunk = max(4, min(32, count / (2 * warps)));
+    const Band band{A.minrow, A.ctr, count};
+    long long n_adds = 0, n_ints = 0, n_pub = 0;
+    int n_disp = 0;
+    // the chunk: lane i holds its i-th column and descriptor; avail marks the lanes not handed out yet
+    int ck_col = -1;
+    uint64_t ck_desc = 0;
+    unsigned avail = 0;
+    bool more = true, stop = false;
+    // the group's column: entries v (descending, -1 beyond n), the arena slot of its published version
+    int col = -1, n = 0, v = -1;
+    int64_t slot = 0;
+    bool dirty = false, displaced = false;
+    while (!stop) {
+        // ---- refill
+        unsigned idle = __ballot_sync(kFull, col < 0 && gl == 0);
+        if (idle && !avail && more) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(A.ctr, chunk);
+            base = __shfl_sync(kFull, base, 0);
+            more = base < count;
+            bool run = false;
+            if (lane < chunk && base + lane < count) {
+                ck_col = A.active[base + lane];
+                ck_desc = ld_cg_u64(A.desc + ck_col);
+                run = ld_acquire_u8(A.state + ck_col) == ST_ACTIVE && !ld_acquire_u8(A.cleared + ck_col) &&
+                      __ldcg(A.low + ck_col) >= A.minrow;
+            }
+            avail = __ballot_sync(kFull, run);
+            if (!avail && more) continue;
+        }
+        if (idle == 0x01010101u && !avail) break;
+        bool fresh = displaced;
+        int src = -1;
+#pragma unroll
+        for (int q = 0; q < 32; q += kGroup) {
+            if (((idle >> q) & 1) && avail) {
+                const int s = __ffs(avail) - 1;
+                avail &= avail - 1;
+                if (lead == q) src = s;
+            }
+        }
+        uint64_t d = __shfl_sync(kFull, (unsigned long long)ck_desc, src & 31);
+        const int c2 = __shfl_sync(kFull, ck_col, src & 31);
+        if (src >= 0) {
+            col = c2;
+            fresh = true;
+        } else if (displaced) {
+            d = ld_cg_u64(A.desc + col);
+        }
+        displaced = false;
+        bool bad = false, ovf = false;
+        if (fresh) {
+            n = int(desc_len(d));
+            slot = int64_t(desc_off(d));
+            dirty = false;
+            v = -1;
+            bad = slot + slot_ints(n) > A.arena_cap;  // self-check: descriptor inside the arena
+            ovf = n > kGroup;
+            if (!bad && !ovf && gl < n) v = __ldcg(A.arena + slot + kHdr + n - 1 - gl);
+        }
+        int L = __shfl_sync(kFull, v, lead);
+        bad = bad || L >= A.ncols;  // self-check: row index in range
+        if (__any_sync(kFull, bad)) {
+            if (bad && gl == 0) atomicOr(A.err, ERRB_CHECK);
+            stop = true;
+            break;
+        }
+        // ---- rows' owners
+        bool act = col >= 0 && !ovf && n > 0 && L >= A.minrow;
+        int4 q4 = make_int4(-1, 0, 0, 0);
+        uint64_t ev = kNoOwner;
+        unsigned clr = 0;
+        if (act && gl < n && v >= A.minrow) {
+            q4 = __ldg(A.app + v);
+            ev = ld_acquire_u64(A.pivot + v);
+            if (gl == 0) clr = ld_acquire_u8(A.cleared + col);
+        }
+        bool own = q4.x >= 0;
+        int cnt = own ? q4.x : 1;  // a row without an addend stays
+        const int32_t* as = nullptr;
+        if (!own && pv_col(ev) < col && pv_slot(ev) + 2 * kHdr <= uint64_t(A.arena_cap)) {
+            as = A.arena + pv_slot(ev);
+            const int4 h = __ldcg(reinterpret_cast<const int4*>(as));
+            q4 = __ldcg(reinterpret_cast<const int4*>(as) + 1);
+            if (h.x >= 1 && h.x <= kGroupGather && h.y == pv_col(ev) &&
+                int64_t(pv_slot(ev)) + slot_ints(h.x) <= A.arena_cap) {
+                own = true;
+                cnt = h.x - 1;
+            }
+        } else if (own) {
+            q4 = make_int4(q4.y, q4.z, q4.w, 0);
+        }
+        if (!act || gl >= n) cnt = 0;
+        int pre = cnt;
+#pragma unroll
+        for (int o = 1; o < kGroup; o <<= 1) {
+            const int t = __shfl_up_sync(kFull, pre, o, kGroup);
+            if (gl >= o) pre += t;
+        }
+        const int m = __shfl_sync(kFull, pre, lead + kGroup - 1);
+        pre -= cnt;
+        const bool low_own = __shfl_sync(kFull, own ? 1 : 0, lead) != 0;
+        const uint64_t e = __shfl_sync(kFull, (unsigned long long)ev, lead);
+        const bool cleared = __shfl_sync(kFull, clr, lead) != 0;
+        bool claim = act && !cleared && !low_own && pv_col(e) > col;
+        bool round = act && !cleared && low_own && m <= kGroupGather;
+        ovf = ovf || (act && !cleared && !claim && !round);
+        // ---- one round for the groups whose lowest row has an owner
+        if (__any_sync(kFull, round)) {
+            const unsigned owned = __ballot_sync(kFull, round && own && gl < n);
+            if (round && gl < n) {
+                if (!own) {
+                    gbuf[pre] = v;
+                } else {
+                    if (cnt > 0) gbuf[pre] = q4.x;
+                    if (cnt > 1) gbuf[pre + 1] = q4.y;
+                    if (cnt > 2) gbuf[pre + 2] = q4.z;
+                    if (cnt > 3) {
+                        gbuf[pre + 3] = q4.w;
+                        for (int k = 4; k < cnt; k++) gbuf[pre + k] = __ldcg(as + kHdr + k);
+                    }
+                }
+            }
+            __syncwarp();
+            int x0 = round && 2 * gl < m ? lds(gbuf + 2 * gl) : -1;
+            int x1 = round && 2 * gl + 1 < m ? lds(gbuf + 2 * gl + 1) : -1;
+            group_sort16(x0, x1);
+            // runs of equal entries: odd ones keep one entry
+            const int mr = round ? m : 0;
+            const int up = __shfl_up_sync(kFull, x1, 1);
+            const bool h0 = 2 * gl < mr && (gl == 0 || x0 != up), h1 = 2 * gl + 1 < mr && x1 != x0;
+            const unsigned heads = spread8((__ballot_sync(kFull, h0) >> lead) & 0xffu) |
+                                   (spread8((__ballot_sync(kFull, h1) >> lead) & 0xffu) << 1) | (1u << mr);
+            const bool k0 = h0 && (__ffs(heads >> (2 * gl + 1)) & 1), k1 = h1 && (__ffs(heads >> (2 * gl + 2)) & 1);
+            const unsigned b0 = (__ballot_sync(kFull, k0) >> lead) & 0xffu, b1 = (__ballot_sync(kFull, k1) >> lead) & 0xffu;
+            const int nn = __popc(b0) + __popc(b1);
+            const unsigned lt = (1u << gl) - 1;
+            const int p0 = __popc(b0 & lt) + __popc(b1 & lt), p1 = p0 + (k0 ? 1 : 0);
+            __syncwarp();  // every gathered entry has been read
+            if (round && nn <= kGroup) {
+                if (k0) gbuf[p0] = x0;
+                if (k1) gbuf[p1] = x1;
+            }
+            __syncwarp();
+            if (round) {
+                if (nn <= kGroup) {
+                    if (gl == 0) {
+                        n_adds += __popc((owned >> lead) & 0xffu);
+                        n_ints += n + m + nn;
+                    }
+                    n = nn;
+                    v = gl < nn ? lds(gbuf + gl) : -1;
+                    dirty = true;
+                } else {
+                    ovf = true;
+                }
+            }
+            const int nl = __shfl_sync(kFull, v, lead);
+            bad = round && !ovf && nl >= L;  // self-check: the lowest row only moves down
+            if (__any_sync(kFull, bad)) {
+                if (bad && gl == 0) atomicOr(A.err, ERRB_CHECK);
+                stop = true;
+                break;
+            }
+            L = nl;
+        }
+        // ---- what the group's column has come to
+        const bool zero = col >= 0 && !ovf && (n == 0 || cleared);
+        const bool park = col >= 0 && !ovf && !zero && L < A.minrow;
+        const bool pub = dirty && (claim || park || ovf);
+        if (__any_sync(kFull, pub)) {  // one allocation for all groups
+            const int want = pub && gl == 0 ? int(slot_ints(n)) : 0;
+            const int inc = warp_inclusive_scan(want);
+            const int tot = __shfl_sync(kFull, inc, 31);
+            unsigned long long off = 0;
+            if (lane == 0) {
+                off = atomicAdd(A.arena_top, (unsigned long long)tot);
+                if (int64_t(off) + tot > A.arena_cap) {
+                    atomicOr(A.err, ERRB_CAPACITY);
+                    off = ~0ull;
+                }
+                n_pub += tot;
+            }
+            off = __shfl_sync(kFull, off, 0);
+            if (off == ~0ull) {
+                stop = true;
+                break;
+            }
+            const int64_t so = int64_t(off) + __shfl_sync(kFull, inc - want, lead);
+            if (pub) {
+                slot = so;
+                dirty = false;
+                if (gl < n) A.arena[so + kHdr + n - 1 - gl] = v;
+                else if (gl < int(pad4(n))) A.arena[so + kHdr + gl] = INT_MAX;
+                if (gl == 0) {
+                    *reinterpret_cast<int4*>(A.arena + so) = make_int4(n, col, 0, 0);
+                    A.desc[col] = pack_desc(uint64_t(so), uint32_t(n));
+                }
+            }
+            __syncwarp();
+        }
+        int next = -1;  // leader: the owner the claim displaced; col when the claim failed
+        if (gl == 0 && (claim || park || zero)) {
+            if (claim) {
+                // the column's final state goes out before the claim: a group
+                // that later displaces it writes its own state after this one
+                A.low[col] = L;
+                A.state[col] = ST_OWNER;
+                __threadfence();
+                const uint64_t old = atomicCAS(reinterpret_cast<unsigned long long*>(A.pivot + L), (unsigned long long)e,
+                                               (unsigned long long)pv_pack(col, uint64_t(slot)));
+                if (old != e) {
+                    A.state[col] = ST_ACTIVE;
+                    next = col;  // someone else changed the owner; look again
+                } else if (e == kNoOwner) {
+                    A.cleared[L] = 1;  // twist clearing of the positive row column
+                } else {
+                    n_disp++;
+                    next = pv_col(e);
+                }
+            } else if (park) {
+                A.low[col] = L;
+                __threadfence();
+                st_release_u8(A.state + col, ST_ACTIVE);
+            } else {
+                A.desc[col] = pack_desc(0, 0);
+                A.low[col] = -1;
+                A.state[col] = ST_ZERO;
+            }
+        }
+        next = __shfl_sync(kFull, next, lead);
+        if (claim) {
+            if (next != col) {
+                col = next;  // idle, or the displaced owner
+                displaced = next >= 0;
+            }
+        } else if (park || zero) {
+            col = -1;
+        }
+        // ---- columns that outgrew their groups, one after another by the whole warp
+        unsigned big = __ballot_sync(kFull, ovf && gl == 0);
+        while (big && !stop) {
+            const int q = __ffs(big) - 1;
+            big &= big - 1;
+            int c = __shfl_sync(kFull, col, q);
+            while (c >= 0) {  // the column, then any owner it displaced
+                int nx = -1;
+                const Outcome o = reduce_column(g, A, band, c, sw0, sw0 + A.cap, sw0 + 2 * A.cap, rm, true, &nx);
+                if (!settle(g, A, c, o)) {
                     stop = true;
                     break;
                 }
-                col = next;
+                c = nx;
             }
+            if (lead == q) col = -1;
         }
+        if (ovf) n = 0;
+    }
+    n_adds = warp_sum(n_adds);
+    n_ints = warp_sum(n_ints);
+    n_disp = warp_sum(n_disp);
+    if (lane == 0) {
+        if (n_adds) cnt_add(&A.counters[CNT_ADDITIONS], n_adds);
+        if (n_ints) cnt_add(&A.counters[CNT_ADD_INTS], n_ints);
+        if (n_pub) cnt_add(&A.counters[CNT_PUBLISHED], n_pub);
+        if (n_disp) cnt_add(&A.counters[CNT_DISPLACED], (long long)n_disp);
     }
     light_block_done(A);
 }
@@ -1628,6 +1530,7 @@ __global__ void __launch_bounds__(T, 1) k_reduce_heavy(ReduceArgs A) {
     extern __shared__ __align__(16) int32_t smem[];
     __shared__ int gsm[2 * (T / 32 + 2)];
     __shared__ unsigned long long gsb[2];
+    __shared__ RoundMem<BlockG<T>> rm;
     BlockG<T> g;
     g.sm = gsm;
     g.sb = gsb;
@@ -1644,7 +1547,7 @@ __global__ void __launch_bounds__(T, 1) k_reduce_heavy(ReduceArgs A) {
         int col = __ldcg(A.heavy + k);
         while (col >= 0) {
             int next = -1;
-            Outcome o = reduce_column(g, A, band, col, sw0, sw1, sp, false, &next);
+            Outcome o = reduce_column(g, A, band, col, sw0, sw1, sp, rm, false, &next);
             if (!settle(g, A, col, o)) return;
             col = next;
         }
@@ -1755,7 +1658,7 @@ __device__ bool settle_q(const ReduceArgs& A, const QueueArgs& Q, int cc, int co
 }
 
 __device__ void queue_light(const ReduceArgs& A, const QueueArgs& Q, int32_t* sw0, int32_t* sw1, int32_t* sp,
-                            int warps_per_block) {
+                            RoundMem<WarpG>& rm, int warps_per_block) {
     WarpG g;
     const int lane = g.rank();
     const int wl = (blockIdx.x - Q.heavy_ctas) * warps_per_block + (threadIdx.x >> 5);
@@ -1856,7 +1759,7 @@ __device__ void queue_light(const ReduceArgs& A, const QueueArgs& Q, int32_t* sw
             int c2 = __shfl_sync(kFull, col, src);
             while (c2 >= 0) {  // the column, then any owner it displaced
                 int next = -1;
-                const Outcome o = reduce_column(g, A, band, c2, sw0, sw1, sp, true, &next);
+                const Outcome o = reduce_column(g, A, band, c2, sw0, sw1, sp, rm, true, &next);
                 if (!settle_q(A, Q, cc, c2, o, it, lout, lcap)) {
                     failed = true;
                     break;
@@ -1878,7 +1781,7 @@ __device__ void queue_light(const ReduceArgs& A, const QueueArgs& Q, int32_t* sw
 
 template <int T>
 __device__ void queue_heavy(const ReduceArgs& A, const QueueArgs& Q, const BlockG<T>& g, int32_t* sw0, int32_t* sw1,
-                            int32_t* sp) {
+                            int32_t* sp, RoundMem<BlockG<T>>& rm) {
     const Band band{INT32_MIN, nullptr, 0};
     long long idle = 0;
     while (true) {
@@ -1911,7 +1814,7 @@ __device__ void queue_heavy(const ReduceArgs& A, const QueueArgs& Q, const Block
         int col = int(uint32_t(pk));
         while (col >= 0) {
             int next = -1;
-            const Outcome o = reduce_column(g, A, band, col, sw0, sw1, sp, false, &next);
+            const Outcome o = reduce_column(g, A, band, col, sw0, sw1, sp, rm, false, &next);
             if (!settle(g, A, col, o)) {
                 if (g.leader()) queue_fail(A, Q, ERRB_CHECK);
                 return;
@@ -1931,14 +1834,18 @@ __global__ void __launch_bounds__(T, 1) k_reduce_queue(ReduceArgs Al, ReduceArgs
     extern __shared__ __align__(16) int32_t smem[];
     __shared__ int gsm[2 * (T / 32 + 2)];
     __shared__ unsigned long long gsb[2];
+    __shared__ union {
+        RoundMem<BlockG<T>> cta;
+        RoundMem<WarpG> warp[T / 32];
+    } rm;
     if (int(blockIdx.x) < Q.heavy_ctas) {
         BlockG<T> g;
         g.sm = gsm;
         g.sb = gsb;
-        queue_heavy<T>(Ah, Q, g, smem, smem + Ah.cap, smem + 2 * Ah.cap);
+        queue_heavy<T>(Ah, Q, g, smem, smem + Ah.cap, smem + 2 * Ah.cap, rm.cta);
     } else {
         int32_t* sw0 = smem + size_t(threadIdx.x >> 5) * (3 * Al.cap + kHdr);
-        queue_light(Al, Q, sw0, sw0 + Al.cap, sw0 + 2 * Al.cap, T / 32);
+        queue_light(Al, Q, sw0, sw0 + Al.cap, sw0 + 2 * Al.cap, rm.warp[threadIdx.x >> 5], T / 32);
     }
 }
 
@@ -1986,26 +1893,19 @@ int queue_complex_info(const Device& D, int32_t k, const int64_t* d_cstart, int3
 int light_smem_bytes(int cap) { return 4 * (3 * cap + kHdr) * 4; }
 int heavy_smem_bytes(int cap) { return (3 * cap + kHdr) * 4; }
 
-// Warp-tier additions per column after which, once its step's window is
-// fully handed out, the column moves to the CTA tier: a step's light launch
-// lasts as long as its longest chain, while CTA-tier launches overlap later
-// steps on side streams.  Handing chains over while the window still has work
-// would only move parallel work onto the (fewer) CTAs.
-#ifndef SSPP_LIGHT_CHAIN
-#define SSPP_LIGHT_CHAIN 8
-#endif
-constexpr int32_t kLightChain = SSPP_LIGHT_CHAIN;
+// Passes (rounds and single additions) of a warp-tier column after which, once
+// its step's window is fully handed out, it moves to the CTA tier: a step's light
+// launch lasts as long as its longest chain, while CTA-tier launches overlap
+// later steps on side streams.  Handing chains over while the window still has
+// work would only move parallel work onto the (fewer) CTAs.
+constexpr int32_t kLightChain = 8;
 
-static ReduceArgs make_args(const Device& D, const int32_t* active, int32_t beg, int32_t end, int32_t minrow, int cap,
-                            int chunk, int* ctr) {
+static ReduceArgs make_args(const Device& D, const int32_t* active, int32_t minrow, int cap, int* ctr) {
     ReduceArgs A;
     A.ncols = int32_t(D.n);
     A.active = active;
-    A.beg = beg;
-    A.end = end;
     A.minrow = minrow;
     A.cap = cap;
-    A.chunk = chunk;
     A.arena = D.arena;
     A.arena_cap = D.arena_cap;
     A.arena_top = D.arena_top;
@@ -2029,25 +1929,18 @@ static ReduceArgs make_args(const Device& D, const int32_t* active, int32_t beg,
     return A;
 }
 
-void reduce_light_launch(const Device& D, const int32_t* active, int32_t beg, int32_t end, int32_t minrow, int cap,
-                         int chunk, int* ctr, int* ctr_next, int grid, cudaStream_t s) {
-    ReduceArgs A = make_args(D, active, beg, end, minrow, cap, chunk, ctr);
-    A.ctr_next = ctr_next;
-    k_reduce_light<<<grid, 128, light_smem_bytes(cap), s>>>(A);
-}
-
-void reduce_light_filtered_launch(const Device& D, int32_t beg, int32_t end, int32_t minrow, int cap, int chunk,
-                                  int* ctr, int* ctr_next, int filter_grid, int grid, cudaStream_t s) {
+void reduce_light_launch(const Device& D, int32_t beg, int32_t end, int32_t minrow, int cap, int* ctr, int* ctr_next,
+                         int filter_grid, int grid, cudaStream_t s) {
     k_light_filter<<<filter_grid, kFilterThreads, 0, s>>>(D.active, beg, end, minrow, D.state, D.cleared, D.low,
                                                           D.runlist, ctr);
-    ReduceArgs A = make_args(D, D.runlist, 0, 0, minrow, cap, chunk, ctr);
+    ReduceArgs A = make_args(D, D.runlist, minrow, cap, ctr);
     A.ctr_next = ctr_next;
     A.count = ctr + 5;
     k_reduce_light<<<grid, 128, light_smem_bytes(cap), s>>>(A);
 }
 
 void reduce_heavy_launch(const Device& D, int cap, int threads, int* ctr, int grid, cudaStream_t s) {
-    ReduceArgs A = make_args(D, nullptr, 0, 0, INT32_MIN, cap, 1, ctr);
+    ReduceArgs A = make_args(D, nullptr, INT32_MIN, cap, ctr);
     if (threads == 256) k_reduce_heavy<256><<<grid, 256, heavy_smem_bytes(cap), s>>>(A);
     else k_reduce_heavy<128><<<grid, 128, heavy_smem_bytes(cap), s>>>(A);
 }
@@ -2092,8 +1985,8 @@ cudaError_t queue_configure(int cap1, int cap2, int threads, int* blocks_per_sm)
 
 cudaError_t reduce_queue_launch(const Device& D, int cap1, int cap2, int threads, const QueueArgs& Q, int grid,
                                 cudaStream_t s) {
-    ReduceArgs Al = make_args(D, D.active, 0, 0, INT32_MIN, cap1, 1, nullptr);
-    ReduceArgs Ah = make_args(D, nullptr, 0, 0, INT32_MIN, cap2, 1, nullptr);
+    ReduceArgs Al = make_args(D, D.active, INT32_MIN, cap1, nullptr);
+    ReduceArgs Ah = make_args(D, nullptr, INT32_MIN, cap2, nullptr);
     Al.gate_host = Ah.gate_host = nullptr;
     Al.heavy_done = Ah.heavy_done = nullptr;
     QueueArgs q = Q;
