@@ -67,11 +67,11 @@ void fill_i64(int64_t* p, int64_t v, int64_t n, cudaStream_t s) {
 }
 
 // Input validation before any index is used: dimensions in range and col_ptr
-// non-decreasing from 0 (device-resident inputs are only checked here).  Also
+// non-decreasing from 0 to nnz (device-resident inputs are only checked here).  Also
 // counts the columns of each dimension (dimtot, zeroed before), which give
 // the host the reordered dimension ranges with the same read as the error word.
-__global__ void __launch_bounds__(256) k_validate(const int32_t* dims, const int64_t* colptr, int64_t n, int* err,
-                                                  unsigned long long* dimtot) {
+__global__ void __launch_bounds__(256) k_validate(const int32_t* dims, const int64_t* colptr, int64_t n,
+                                                  int64_t nnz, int* err, unsigned long long* dimtot) {
     __shared__ unsigned s_cnt[kNumDims];
     if (threadIdx.x < kNumDims) s_cnt[threadIdx.x] = 0;
     __syncthreads();
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(256) k_validate(const int32_t* dims, const int
         if (j < n) {
             d = dims[j];
             const int64_t a = colptr[j], b = colptr[j + 1];
-            if (d < 0 || d > kMaxDim || b < a || b - a > kMaxColLen || (j == 0 && a != 0))
+            if (d < 0 || d > kMaxDim || b < a || b - a > kMaxColLen || (j == 0 && a != 0) || (j == n - 1 && b != nnz))
                 atomicOr(err, ERRB_BAD_INPUT);
         }
 #pragma unroll
@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(256) k_validate(const int32_t* dims, const int
 int validate(Device& D, cudaStream_t s) {
     if (D.n <= 0) return 0;
     cudaMemsetAsync(D.dimtot, 0, sizeof(unsigned long long) * kNumDims, s);
-    k_validate<<<grid_for(D.n, 256) > 4096 ? 4096 : grid_for(D.n, 256), 256, 0, s>>>(D.in_dims, D.in_colptr, D.n, D.err,
-                                                                                     D.dimtot);
+    k_validate<<<grid_for(D.n, 256) > 4096 ? 4096 : grid_for(D.n, 256), 256, 0, s>>>(D.in_dims, D.in_colptr, D.n, D.nnz,
+                                                                                     D.err, D.dimtot);
     return 1;
 }
 

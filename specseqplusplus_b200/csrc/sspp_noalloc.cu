@@ -33,16 +33,36 @@
 // dimensions must lie in 0..7, and each column's faces must be ascending, in
 // range and one dimension lower; anything else is SSPP_ERR_BAD_INPUT.
 //
-// The reduction is the standard twist (clearing) reduction, dimensions from
-// high to low, run by one thread block: columns one after another, each
-// addition a block-wide merge of two sorted index lists.  It is meant for
-// modest matrices; large ones belong on the context API.
+// Two ways.  While the engine's arrays (about 71 bytes per column and the padded
+// column arena) fit in the scratch array, its own passes run there on the
+// caller's stream (reduce_in_scratch): the same reorder, apparent pairs and
+// reduction kernels as the context API's, one block per dimension.  Otherwise,
+// and whenever that run does not end cleanly (malformed input, arena or fill-in
+// limit, or a matrix that is not a chain complex where the two could differ),
+// k_reduce_noalloc decides: the standard twist (clearing) reduction, dimensions
+// from high to low, run by one thread block: columns one after another, each
+// addition a block-wide merge of two sorted index lists.
+//
+// The pairs are the same for every well-formed matrix, chain complex or not: the
+// negative-row compression, the only pass that needs the boundary of a boundary
+// to be zero, is left out here, and a run in which a column is both a birth and a
+// death (possible only without that property, where the twist's clearing would
+// have come first) goes to k_reduce_noalloc.  The fill-in limit stays that of
+// k_reduce_noalloc: a run whose additions read and write more than the room it
+// would have goes there too, and gets its verdict.
+//
+// Measured (B200, device-resident input): 700 points (6,720 columns) 8.5 ms by one
+// block, 0.36 ms by the engine's passes.
+#include <algorithm>
 #include <climits>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
-#include "../../include/sspp.h"
+#include "sspp_kernels.cuh"
+#include "sspp_launch.h"
+#include "sspp_scan.cuh"
 
 namespace {
 
@@ -52,7 +72,6 @@ constexpr int64_t kFillReserve = int64_t(4) << 20;   // ints kept free for fill-
 constexpr int kCtl = 16;                            // control words at the start of the array
 constexpr int kMaxDevices = 64;
 constexpr int kThreads = 256;
-constexpr int kMaxDim = 7;                          // dimensions 0..7, as the context API
 
 // control words
 enum { C_ERR = 0, C_TOP_LO = 1, C_TOP_HI = 2, C_NPAIRS_LO = 3, C_NPAIRS_HI = 4, C_MAXDIM = 5 };
@@ -159,7 +178,7 @@ __global__ void __launch_bounds__(kThreads) k_reduce_noalloc(int32_t* S, int64_t
         const int d = dims[j];
         // every column's range must lie inside [0, nnz] before any entry is
         // read or copied (the copy runs in the same pass as the checks)
-        bool bad = b < 0 || e < b || e > nnz || d < 0 || d > kMaxDim;
+        bool bad = b < 0 || e < b || e > nnz || d < 0 || d > sspp::kMaxDim;
         for (int64_t k = b; k < e && !bad; k++) {
             const int32_t r = rows[k];
             if (r < 0 || r >= n || (k > b && r <= rows[k - 1]) || dims[r] != d - 1) bad = true;
@@ -233,6 +252,160 @@ __global__ void __launch_bounds__(kThreads) k_reduce_noalloc(int32_t* S, int64_t
     }
 }
 
+// ---------------------------------------------------------------------------
+// the engine's passes in the scratch array
+
+using namespace sspp;
+
+constexpr int kCap1 = 64;          // warp-tier column capacity (ints), as the context API's bound
+constexpr int kCap2 = 8192;        // CTA-tier column capacity
+constexpr int kStepInts = 8;       // counters per dimension's step (ReduceArgs::ctr)
+constexpr int64_t kGuard = 8192;   // ints after the arena: staging reads a first pass beyond a slot
+
+// what the host reads back, in one copy
+struct Status {
+    DimInfo info;
+    long long counters[CNT_NUM];
+    int err;
+    int pad[3];
+};
+
+// Engine arrays carved out of the scratch array; false when they leave too
+// little for the arena.  Buffers whose lifetimes do not meet share memory: the
+// pairs pass's death list lies in the inline columns, its essentials in the
+// column descriptors.
+bool carve(int32_t* scratch, int64_t n, int64_t nnz, Device& D, Status** status) {
+    char* p = reinterpret_cast<char*>(scratch);
+    char* const end = p + sizeof(int32_t) * kScratchInts;
+    auto take = [&](auto*& out, int64_t count) {
+        using T = std::remove_reference_t<decltype(*out)>;
+        out = reinterpret_cast<T*>(p);
+        p += (sizeof(T) * size_t(count) + 255) & ~size_t(255);
+    };
+    take(*status, 1);
+    take(D.dimtot, kNumDims);
+    take(D.arena_top, 1);
+    take(D.pool_tail, 1);
+    take(D.heavy_done, 1);
+    take(D.step_ctr, kStepInts * (kNumDims + 1));
+    take(D.dim, n);
+    take(D.perm, n);
+    take(D.newidx, n);
+    take(D.scratch64, n + 1);
+    take(D.desc, n + 1);
+    take(D.low, n);
+    take(D.pivot, n);
+    take(D.state, n);
+    take(D.cleared, n);
+    take(D.negative, n);
+    take(D.leftmost, n);
+    take(D.active, n);
+    take(D.runlist, n);
+    take(D.app, n);
+    take(D.blk, scan_blocks(n) + 2);
+    take(D.dimcnt, ((n + 255) / 256 + 1) * kNumDims);
+    D.pool_cap = n;
+    take(D.heavy, D.pool_cap);
+    D.arena = reinterpret_cast<int32_t*>(p);
+    D.arena_cap = p < end ? ((end - p) / int64_t(sizeof(int32_t)) - kGuard) & ~int64_t(3) : 0;
+    D.n = n;
+    D.nnz = nnz;
+    D.diminfo = &(*status)->info;
+    D.counters = (*status)->counters;
+    D.err = &(*status)->err;
+    D.death_of = reinterpret_cast<int64_t*>(D.app);
+    D.ess = reinterpret_cast<int64_t*>(D.desc);
+    // the input's slots, and as much again for the reduction's column versions
+    return D.arena_cap >= 2 * (nnz + (kHdr + 3) * n + 4);
+}
+
+// A column that owns a row and whose own row is owned (see the header).
+__global__ void k_check_complex(int64_t n, const uint64_t* pivot, const uint8_t* state, int* err) {
+    for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n; r += int64_t(gridDim.x) * blockDim.x)
+        if (pivot[r] != kNoOwner && state[r] == ST_OWNER) atomicOr(err, ERRB_CHECK);
+}
+
+// *npairs is written by a run that ends cleanly only.
+__global__ void k_store_npairs(const Status* st, int64_t room, int64_t* npairs) {
+    if (st->err == 0 && st->counters[CNT_ADD_INTS] <= room) *npairs = st->counters[CNT_NPAIRS];
+}
+
+// The device's multiprocessors and the reduction kernels' blocks per
+// multiprocessor, once per device.
+struct Launch {
+    int sms = 0, light = 0, heavy = 0;
+};
+
+cudaError_t launch_shape(int dev, Launch* out) {
+    static Launch known[kMaxDevices];
+    std::lock_guard<std::mutex> lock(g_setup_mu);
+    Launch& l = known[dev];
+    if (l.sms == 0) {
+        Launch f;
+        cudaError_t e = reduce_configure(kCap1, kCap2, 256, &f.light, &f.heavy);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&f.sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        if (f.light < 1 || f.heavy < 1) return cudaErrorInvalidConfiguration;
+        l = f;
+    }
+    *out = l;
+    return cudaSuccess;
+}
+
+// Runs the engine's passes in the scratch array.  *done: the pairs are in
+// place; otherwise the caller runs k_reduce_noalloc.
+cudaError_t reduce_in_scratch(int32_t* scratch, int dev, int64_t n, int64_t nnz, const int32_t* d_dims,
+                              const int64_t* d_col_ptr, const int32_t* d_rows, int64_t* d_pairs, int64_t* d_npairs,
+                              cudaStream_t s, bool* done) {
+    *done = false;
+    Device D;
+    Status* status = nullptr;
+    if (n < 1 || !carve(scratch, n, nnz, D, &status)) return cudaSuccess;
+    Launch shape;
+    cudaError_t e = launch_shape(dev, &shape);
+    if (e != cudaSuccess) return e;
+    D.in_dims = const_cast<int32_t*>(d_dims);
+    D.in_colptr = const_cast<int64_t*>(d_col_ptr);
+    D.in_rows = const_cast<int32_t*>(d_rows);
+    D.pairs = d_pairs;
+    Status h;
+    cudaMemsetAsync(status, 0, sizeof(Status), s);
+    validate(D, s);
+    cudaMemcpyAsync(&h.err, D.err, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+    if (h.err) return cudaSuccess;
+    reorder(D, true, s);
+    cudaMemcpyAsync(D.arena_top, D.blk + reorder_total_slot(D), sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s);
+    init_passes(D, true, s);
+    init_compress(D, nullptr, true, true, s);
+    active_list(D, true, s);
+    cudaMemsetAsync(D.step_ctr, 0, sizeof(int) * kStepInts * (kNumDims + 1), s);
+    cudaMemsetAsync(D.pool_tail, 0, sizeof(int), s);
+    cudaMemcpyAsync(&h, status, sizeof(Status), cudaMemcpyDeviceToHost, s);
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+    if (h.err) return cudaSuccess;
+    int* ctr = D.step_ctr;
+    for (int d = kMaxDim; d >= 1; d--) {
+        const int64_t b = h.info.act_begin[d], end = h.info.act_end[d], window = end - b;
+        if (window <= 0) continue;
+        const int grid = int(std::min<int64_t>((window + 3) / 4, int64_t(shape.sms) * shape.light));
+        const int fgrid = int(std::min<int64_t>((window + 255) / 256, int64_t(shape.sms) * 8));
+        reduce_light_launch(D, int32_t(b), int32_t(end), INT32_MIN, kCap1, ctr, ctr + kStepInts, fgrid, grid, s);
+        reduce_heavy_launch(D, kCap2, 256, ctr,
+                            int(std::min<int64_t>(int64_t(shape.sms) * std::min(shape.heavy, 2), window)), s);
+        ctr += kStepInts;
+    }
+    k_check_complex<<<unsigned(std::min<int64_t>((n + 255) / 256, 4096)), 256, 0, s>>>(n, D.pivot, D.state, D.err);
+    extract_pairs(D, 0, nullptr, s);
+    const int64_t room = kScratchInts - (kCtl + 3 * n) - nnz;  // k_reduce_noalloc's room for fill-in
+    k_store_npairs<<<1, 1, 0, s>>>(status, room, d_npairs);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    cudaMemcpyAsync(&h, status, sizeof(Status), cudaMemcpyDeviceToHost, s);
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+    *done = h.err == 0 && h.counters[CNT_ADD_INTS] <= room;
+    return cudaSuccess;
+}
+
 int32_t fail(char* msg, int32_t cap, int32_t code, const char* text) {
     if (msg && cap > 0) {
         std::strncpy(msg, text, size_t(cap) - 1);
@@ -270,9 +443,14 @@ extern "C" int32_t sspp_reduce_noalloc(int64_t ncols, int64_t nnz, const int32_t
         addr = g_scratch_addr[dev];
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    bool done = false;
+    cudaError_t e = reduce_in_scratch(static_cast<int32_t*>(addr), dev, ncols, nnz, d_dims, d_col_ptr, d_rows, d_pairs,
+                                      d_npairs, s, &done);
+    if (e != cudaSuccess) return fail(err_msg, err_cap, SSPP_ERR_CUDA, cudaGetErrorString(e));
+    if (done) return fail(err_msg, err_cap, SSPP_OK, "");
     k_reduce_noalloc<<<1, kThreads, 0, s>>>(static_cast<int32_t*>(addr), ncols, nnz, d_dims, d_col_ptr, d_rows,
                                             d_pairs, d_npairs);
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess) return fail(err_msg, err_cap, SSPP_ERR_CUDA, cudaGetErrorString(e));
     int32_t err = 0;
     e = cudaMemcpyAsync(&err, addr, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
