@@ -1032,32 +1032,59 @@ int ensure_own(sspp_ctx* ctx, int64_t n, int64_t nnz) {
     return SSPP_OK;
 }
 
-// A device pointer to `count` floats of the caller: the pointer itself when it
-// is device (or managed) memory of this context's device, else a copy in the
-// builder's input buffer.
-int stage_floats(sspp_ctx* ctx, const float* p, int64_t count, const float** out) {
+// Whether p is memory that kernels of this context's device read in place; an
+// error for another device's memory.
+int device_readable(sspp_ctx* ctx, const float* p, bool* yes) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         a.type = cudaMemoryTypeUnregistered;
     }
-    if (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged) {
-        if (a.type == cudaMemoryTypeDevice && a.device != ctx->cfg.device)
-            return set_err(ctx, SSPP_ERR_BAD_INPUT, "input is in another device's memory");
-        *out = p;
-        return SSPP_OK;
-    }
+    *yes = a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+    if (a.type == cudaMemoryTypeDevice && a.device != ctx->cfg.device)
+        return set_err(ctx, SSPP_ERR_BAD_INPUT, "input is in another device's memory");
+    return SSPP_OK;
+}
+
+// A device pointer to the floats of the caller's k arrays, one after another:
+// the pointer itself for one array that kernels can read in place, else a copy in
+// the builder's input buffer.
+struct Floats {
+    const float* p;
+    int64_t count;
+};
+int stage_floats(sspp_ctx* ctx, const Floats* in, int k, const float** out) {
+    *out = nullptr;
+    int64_t total = 0;
+    for (int i = 0; i < k; i++) total += in[i].count;
+    if (total == 0) return SSPP_OK;
     void* d = nullptr;
-    const size_t bytes = sizeof(float) * size_t(count);
-    CK(build_stage(ctx->bs, bytes, ctx->stream, &d));
-    CK(ctx->xfer.h2d({{p, d, bytes}}, ctx->stream));
+    std::vector<Piece> pcs;
+    int64_t at = 0;
+    for (int i = 0; i < k; i++) {
+        if (in[i].count == 0) continue;
+        bool resident = false;
+        int rc = device_readable(ctx, in[i].p, &resident);
+        if (rc) return rc;
+        if (resident && in[i].count == total) {
+            *out = in[i].p;
+            return SSPP_OK;
+        }
+        if (!d) CK(build_stage(ctx->bs, sizeof(float) * size_t(total), ctx->stream, &d));
+        float* dst = static_cast<float*>(d) + at;
+        const size_t bytes = sizeof(float) * size_t(in[i].count);
+        if (resident) CK(cudaMemcpyAsync(dst, in[i].p, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        else pcs.push_back({in[i].p, dst, bytes, 0});
+        at += in[i].count;
+    }
+    CK(ctx->xfer.h2d(pcs, ctx->stream));
     *out = static_cast<const float*>(d);
     return SSPP_OK;
 }
 
 int finish_build(sspp_ctx* ctx, int rc, const Built& b, const std::string& msg,
                  std::chrono::steady_clock::time_point t0) {
-    if (rc) return set_err(ctx, rc == -1 ? SSPP_ERR_BAD_INPUT : SSPP_ERR_CUDA, msg);
+    if (rc) return set_err(ctx, rc == BUILD_BAD_INPUT ? SSPP_ERR_BAD_INPUT : SSPP_ERR_CUDA, msg);
     rc = load_common(ctx, b.ncols, b.nnz);
     if (rc) return rc;
     ctx->D.in_dims = b.dims;
@@ -1278,13 +1305,13 @@ int32_t sspp_load_rips(sspp_ctx* ctx, int64_t npts, int32_t space_dim, const flo
     const auto t0 = std::chrono::steady_clock::now();
     ctx->loaded = false;  // the build reuses the buffers of an earlier build
     const float* dp = nullptr;
-    if (npts > 0) {
-        int rc = stage_floats(ctx, points, npts * space_dim, &dp);
-        if (rc) return rc;
-    }
+    const Floats in{points, npts * space_dim};
+    int rc0 = stage_floats(ctx, &in, 1, &dp);
+    if (rc0) return rc0;
     Built b;
     std::string msg;
-    const int rc = build_rips(ctx->bs, dp, npts, space_dim, radius, maxdim, ctx->stream, &b, &msg);
+    const Cloud c{npts, space_dim, maxdim, radius};
+    const int rc = build_clouds(ctx->bs, dp, &c, 1, ctx->stream, scratch_sink(ctx->bs, ctx->stream), nullptr, &b, &msg);
     return finish_build(ctx, rc, b, msg, t0);
 }
 
@@ -1298,11 +1325,12 @@ int32_t sspp_load_lowerstar(sspp_ctx* ctx, int64_t gx, int64_t gy, int64_t gz, c
     const auto t0 = std::chrono::steady_clock::now();
     ctx->loaded = false;
     const float* dv = nullptr;
-    int rc = stage_floats(ctx, values, gx * gy * gz, &dv);
+    const Floats in{values, gx * gy * gz};
+    int rc = stage_floats(ctx, &in, 1, &dv);
     if (rc) return rc;
     Built b;
     std::string msg;
-    rc = build_lowerstar(ctx->bs, dv, gx, gy, gz, maxdim, ctx->stream, &b, &msg);
+    rc = build_lowerstar(ctx->bs, dv, gx, gy, gz, maxdim, ctx->stream, scratch_sink(ctx->bs, ctx->stream), &b, &msg);
     return finish_build(ctx, rc, b, msg, t0);
 }
 
@@ -1355,53 +1383,75 @@ int32_t sspp_load_built_batch(sspp_ctx* ctx, int32_t k, const sspp_build_spec* s
     const auto t0 = std::chrono::steady_clock::now();
     ctx->loaded = false;
     cudaStream_t s = ctx->stream;
-    std::vector<int64_t> starts(size_t(2) * (size_t(k) + 1), 0);  // column starts, then entry starts
+    std::vector<int64_t> starts(size_t(k) + 1, 0);  // column starts
     int64_t* cst = starts.data();
-    int64_t* est = cst + k + 1;
-    // each complex is built in the builder's buffers, then appended to the
-    // context's input buffers (col_ptr entries and faces still local)
-    for (int32_t i = 0; i < k; i++) {
-        const sspp_build_spec& b = specs[i];
-        const int64_t nin = b.kind == SSPP_BUILD_RIPS ? b.size[0] * b.size[1] : b.size[0] * b.size[1] * b.size[2];
-        const float* din = nullptr;
-        if (nin > 0) {
-            int rc = stage_floats(ctx, b.data, nin, &din);
-            if (rc) return rc;
+    // complexes are written behind one another into the context's input buffers,
+    // indices already those of the block-diagonal matrix: consecutive point clouds
+    // as one build (fewer at a time when it asks for less), a field by itself
+    int64_t n = 0, nnz = 0;
+    bool too_many = false;
+    Sink sink;
+    sink.reserve = [&](int64_t nc, int64_t ne, Built* b) -> cudaError_t {
+        too_many = n + nc > INT32_MAX - 8;
+        if (too_many) return cudaErrorInvalidValue;
+        cudaError_t e = grow_own_cols(ctx, n + nc + 1, n, s);
+        if (e == cudaSuccess) e = grow_keep(ctx->own_rows, ctx->cap_own_nnz, std::max<int64_t>(nnz + ne, 1), nnz, s);
+        if (e == cudaSuccess) e = grow_keep(ctx->bvalues, ctx->cap_bvalues, std::max<int64_t>(n + nc, 1), n, s);
+        if (e != cudaSuccess) return e;
+        b->dims = ctx->own_dims + n;
+        b->col_ptr = ctx->own_colptr + n;
+        b->rows = ctx->own_rows + nnz;
+        b->values = ctx->bvalues + n;
+        return cudaSuccess;
+    };
+    std::vector<Floats> in;
+    std::vector<Cloud> clouds;
+    int32_t most = k;  // clouds per build
+    for (int32_t i = 0; i < k;) {
+        in.clear();
+        clouds.clear();
+        int32_t j = i;
+        if (specs[i].kind == SSPP_BUILD_RIPS) {
+            for (; j < k && j - i < most && specs[j].kind == SSPP_BUILD_RIPS; j++) {
+                const sspp_build_spec& b = specs[j];
+                in.push_back({b.data, b.size[0] * b.size[1]});
+                clouds.push_back({b.size[0], int32_t(b.size[1]), b.maxdim, b.radius});
+            }
+        } else {
+            in.push_back({specs[i].data, specs[i].size[0] * specs[i].size[1] * specs[i].size[2]});
+            j++;
         }
+        const float* din = nullptr;
+        int rc = stage_floats(ctx, in.data(), int(in.size()), &din);
+        if (rc) return rc;
+        sink.col0 = n;
+        sink.ent0 = nnz;
         Built out;
         std::string msg;
-        const int rc = b.kind == SSPP_BUILD_RIPS
-                           ? build_rips(ctx->bs, din, b.size[0], int(b.size[1]), b.radius, b.maxdim, s, &out, &msg)
-                           : build_lowerstar(ctx->bs, din, b.size[0], b.size[1], b.size[2], b.maxdim, s, &out, &msg);
-        if (rc) return set_err(ctx, rc == -1 ? SSPP_ERR_BAD_INPUT : SSPP_ERR_CUDA, msg);
-        const int64_t n0 = cst[i], e0 = est[i];
-        cst[i + 1] = n0 + out.ncols;
-        est[i + 1] = e0 + out.nnz;
-        if (cst[i + 1] > INT32_MAX - 8) return set_err(ctx, SSPP_ERR_CAPACITY, "more than 2^31 columns");
-        CK(grow_own_cols(ctx, cst[i + 1] + 1, n0, s));
-        CK(grow_keep(ctx->own_rows, ctx->cap_own_nnz, std::max<int64_t>(est[i + 1], 1), e0, s));
-        CK(grow_keep(ctx->bvalues, ctx->cap_bvalues, std::max<int64_t>(cst[i + 1], 1), n0, s));
-        if (out.ncols > 0) {
-            CK(cudaMemcpyAsync(ctx->own_dims + n0, out.dims, sizeof(int32_t) * size_t(out.ncols),
-                               cudaMemcpyDeviceToDevice, s));
-            CK(cudaMemcpyAsync(ctx->own_colptr + n0 + 1, out.col_ptr + 1, sizeof(int64_t) * size_t(out.ncols),
-                               cudaMemcpyDeviceToDevice, s));
-            CK(cudaMemcpyAsync(ctx->bvalues + n0, out.values, sizeof(float) * size_t(out.ncols),
-                               cudaMemcpyDeviceToDevice, s));
+        const sspp_build_spec& b0 = specs[i];
+        if (clouds.empty()) {
+            rc = build_lowerstar(ctx->bs, din, b0.size[0], b0.size[1], b0.size[2], b0.maxdim, s, sink, &out, &msg);
+            cst[j] = out.ncols;
+        } else {
+            rc = build_clouds(ctx->bs, din, clouds.data(), int(clouds.size()), s, sink, cst + i, &out, &msg);
         }
-        if (out.nnz > 0)
-            CK(cudaMemcpyAsync(ctx->own_rows + e0, out.rows, sizeof(int32_t) * size_t(out.nnz),
-                               cudaMemcpyDeviceToDevice, s));
+        if (rc == BUILD_SPLIT) {
+            most = std::max<int32_t>(1, (j - i) / 2);
+            continue;
+        }
+        if (too_many) return set_err(ctx, SSPP_ERR_CAPACITY, "more than 2^31 columns");
+        if (rc) return set_err(ctx, rc == BUILD_BAD_INPUT ? SSPP_ERR_BAD_INPUT : SSPP_ERR_CUDA, msg);
+        cst[i] = 0;
+        for (int32_t c = i; c <= j; c++) cst[c] += n;  // build_clouds and the field's count start at 0
+        n += out.ncols;
+        nnz += out.nnz;
+        i = j;
     }
-    const int64_t n = cst[k], nnz = est[k];
     CK(grow_own_cols(ctx, n + 1, n, s));
     if (!ctx->own_rows) CK(grow_keep(ctx->own_rows, ctx->cap_own_nnz, 1, 0, s));
     CK(cudaMemsetAsync(ctx->own_colptr, 0, sizeof(int64_t), s));
-    CK(grow(ctx->d_batch, ctx->cap_d_batch, 2 * int64_t(starts.size()) + 1, s));
+    CK(grow(ctx->d_batch, ctx->cap_d_batch, 4 * int64_t(starts.size()) + 1, s));
     CK(cudaMemcpyAsync(ctx->d_batch, starts.data(), sizeof(int64_t) * starts.size(), cudaMemcpyHostToDevice, s));
-    int* d_bad = reinterpret_cast<int*>(ctx->d_batch + starts.size());
-    CK(cudaMemsetAsync(d_bad, 0, sizeof(int), s));
-    batch_rebase(n, nnz, k, ctx->d_batch, ctx->d_batch + k + 1, ctx->own_colptr, ctx->own_rows, d_bad, s);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));
     int rc = load_common(ctx, n, nnz);

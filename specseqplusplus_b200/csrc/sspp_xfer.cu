@@ -9,6 +9,7 @@ namespace sspp {
 namespace {
 constexpr size_t kHalfBytes = size_t(32) << 20;    // each half of the pinned buffer
 constexpr size_t kDirectBytes = size_t(1) << 20;   // below this, plain copies
+constexpr size_t kDirectPieces = 8;                // more pieces than this are staged and move as one
 constexpr size_t kMinTaskBytes = size_t(1) << 20;  // smallest share of one host thread
 }  // namespace
 
@@ -161,7 +162,8 @@ cudaError_t Xfer::h2d(const std::vector<Piece>& pieces, cudaStream_t s) {
     for (const Piece& p : pieces) total += p.bytes;
     if (total == 0) return cudaSuccess;
     cudaError_t e;
-    if (total <= kDirectBytes || all_pinned(pieces, true)) {  // pinned sources: straight to the copy engine
+    // small: plain copies, unless many; pinned sources: straight to the copy engine
+    if ((total <= kDirectBytes && pieces.size() <= kDirectPieces) || all_pinned(pieces, true)) {
         for (const Piece& p : pieces)
             if (p.bytes && (e = cudaMemcpyAsync(p.dst, p.src, p.bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess)
                 return e;
