@@ -528,8 +528,6 @@ int run_init(sspp_ctx* ctx) {
     const bool guided = (ctx->params.model & 1) && ctx->params.max_iteration > 0;
     const bool early = guided && !(ctx->params.model & 2);
     ctx->launches += reorder(D, lows_in_reorder, s, early ? ctx->hc_fork : nullptr);
-    CK(cudaMemcpyAsync(D.arena_top, D.blk + reorder_total_slot(D), sizeof(unsigned long long),
-                       cudaMemcpyDeviceToDevice, s));
     if (ctx->user_params.autotune && !ctx->tune_locked) {
         int rc2 = autotune_choose(ctx);
         if (rc2) return rc2;
@@ -1825,8 +1823,6 @@ int32_t sspp_export_preprocessed(sspp_ctx* ctx, const sspp_params* p, const char
         CK(cudaStreamSynchronize(s));
         if (*ctx->h_err) return set_err(ctx, SSPP_ERR_BAD_INPUT, "dimension out of range 0..7 or malformed col_ptr");
         reorder(D, false, s);
-        CK(cudaMemcpyAsync(D.arena_top, D.blk + reorder_total_slot(D), sizeof(unsigned long long),
-                           cudaMemcpyDeviceToDevice, s));
         CK(cudaMemcpyAsync(ctx->h_err, D.err, sizeof(int), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         if (*ctx->h_err) return set_err(ctx, SSPP_ERR_BAD_INPUT, "malformed boundary matrix");

@@ -20,33 +20,6 @@
 
 namespace sspp {
 
-__global__ void __launch_bounds__(1024) k_scan_blocks(int64_t* blk, int64_t nb) {
-    __shared__ int64_t wt[32];
-    __shared__ int64_t carry;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (tid == 0) carry = 0;
-    __syncthreads();
-    for (int64_t base = 0; base < nb; base += 1024) {
-        int64_t i = base + tid;
-        int64_t v = i < nb ? blk[i] : 0;
-        int64_t inc = warp_inclusive_scan(v);
-        if (lane == 31) wt[wid] = inc;
-        __syncthreads();
-        if (wid == 0) {
-            int64_t t = wt[lane];
-            int64_t ti = warp_inclusive_scan(t);
-            wt[lane] = ti - t;
-        }
-        __syncthreads();
-        int64_t ex = carry + wt[wid] + inc - v;
-        if (i < nb) blk[i] = ex;
-        __syncthreads();
-        if (tid == 1023) carry = ex + v;
-        __syncthreads();
-    }
-    if (tid == 0) blk[nb] = carry;
-}
-
 template <typename T>
 __global__ void k_fill(T* p, T v, int64_t n) {
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) p[i] = v;
@@ -239,8 +212,14 @@ __global__ void __launch_bounds__(1024) k_dim_offsets(int32_t* dimcnt, int64_t n
     if (tid == 0) info->col_end[d] = int32_t(carry);
 }
 
-// per-dimension totals -> dimension ranges of the reordered columns
+// per-dimension totals -> dimension ranges of the reordered columns; also empties
+// the active segments and the row bounds that later passes fill
 __global__ void k_dim_starts(DimInfo* info) {
+    if (threadIdx.x < kNumDims) {
+        info->act_begin[threadIdx.x] = info->act_end[threadIdx.x] = 0;  // act_end counts first
+        info->min_row[threadIdx.x] = INT_MAX;
+        info->max_row[threadIdx.x] = -1;
+    }
     if (threadIdx.x == 0) {
         int32_t s = 0;
         for (int d = 0; d < kNumDims; d++) {
@@ -344,8 +323,6 @@ __global__ void k_scatter_cols(int64_t n, const int64_t* colptr, const int32_t* 
     }
 }
 
-int64_t reorder_total_slot(const Device& D) { return scan_blocks(D.n); }
-
 int reorder(Device& D, bool lows, cudaStream_t s, cudaEvent_t assigned) {
     const int64_t n = D.n;
     const int64_t nb = (n + kPartThreads - 1) / kPartThreads;
@@ -360,12 +337,14 @@ int reorder(Device& D, bool lows, cudaStream_t s, cudaEvent_t assigned) {
     if (assigned) cudaEventRecord(assigned, s);
     // padded column offsets in reordered order
     int64_t* off = D.scratch64;
+    unsigned long long* top = D.arena_top;
     scan([=] __device__(int64_t i) -> int64_t { return slot_ints(rlen[i]); },
-         [=] __device__(int64_t i, int64_t pre, int64_t) { off[i] = pre; }, n, D.blk, s);
+         [=] __device__(int64_t i, int64_t pre, int64_t) { off[i] = pre; }, n, D.blk, s,
+         [=] __device__(int64_t total) { *top = (unsigned long long)total; });
     k_scatter_cols<<<grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256), 256, 0, s>>>(
         n, D.in_colptr, D.in_rows, D.in_dims, D.newidx, off, D.diminfo, D.arena, D.desc, D.low, D.leftmost, lows,
         D.err);
-    return 8;
+    return 6;
 }
 
 // ------------------------------------------------------------- init passes
@@ -411,18 +390,19 @@ __global__ void k_init_apparent(int64_t n, const int32_t* arena, const uint64_t*
 // dimension row bounds of the schedule (min first row over non-empty columns,
 // max lowest row + 1 over active ones; ColumnShrink, include/specseq.h:374-398)
 // into info, whose bounds must start at INT_MAX / -1.
-__global__ void k_init_compress(int64_t cb, int64_t n, int32_t* arena, uint64_t* desc, int32_t* low, const uint64_t* pivot,
+__global__ void k_init_compress(int64_t n, int32_t* arena, uint64_t* desc, int32_t* low, const uint64_t* pivot,
                                 const uint8_t* cleared, const uint8_t* negative, uint8_t* state,
                                 const uint8_t* dropped, bool keep_rows, int4* app, const int32_t* rinfo,
                                 DimInfo* info, long long* counters, int* err) {
-    __shared__ int smin[kNumDims], smax[kNumDims];
+    __shared__ int smin[kNumDims], smax[kNumDims], sact[kNumDims];
     if (threadIdx.x < kNumDims) {
         smin[threadIdx.x] = INT_MAX;
         smax[threadIdx.x] = -1;
+        sact[threadIdx.x] = 0;
     }
     __syncthreads();
     long long ncl = 0, nact = 0;
-    for (int64_t i = cb + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
         if (app && pivot[i] == kNoOwner) app[i] = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
         uint64_t d = desc[i];
         int32_t* hdr = arena + desc_off(d);
@@ -463,7 +443,10 @@ __global__ void k_init_compress(int64_t cb, int64_t n, int32_t* arena, uint64_t*
         if (rinfo && m > 0) {
             const int dm = rinfo[i];
             atomicMin(&smin[dm], c[0]);
-            if (st == ST_ACTIVE) atomicMax(&smax[dm], l + 1);
+            if (st == ST_ACTIVE) {
+                atomicMax(&smax[dm], l + 1);
+                atomicAdd(&sact[dm], 1);
+            }
         }
         if (app && st == ST_OWNER) {
             int4 v = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
@@ -488,6 +471,7 @@ __global__ void k_init_compress(int64_t cb, int64_t n, int32_t* arena, uint64_t*
         if (threadIdx.x < kNumDims) {
             if (smin[threadIdx.x] != INT_MAX) atomicMin(&info->min_row[threadIdx.x], smin[threadIdx.x]);
             if (smax[threadIdx.x] >= 0) atomicMax(&info->max_row[threadIdx.x], smax[threadIdx.x]);
+            if (sact[threadIdx.x]) atomicAdd(&info->act_end[threadIdx.x], sact[threadIdx.x]);
         }
     }
 }
@@ -496,8 +480,8 @@ __global__ void k_init_compress(int64_t cb, int64_t n, int32_t* arena, uint64_t*
 // active columns (ColumnShrink, include/specseq.h:374-398)
 __global__ void k_dim_rows(int64_t n, const int32_t* rdim, const int32_t* arena, const uint64_t* desc,
                            const int32_t* low, const uint8_t* state, DimInfo* info) {
-    __shared__ int smin[kNumDims], smax[kNumDims];
-    if (threadIdx.x < kNumDims) { smin[threadIdx.x] = INT_MAX; smax[threadIdx.x] = -1; }
+    __shared__ int smin[kNumDims], smax[kNumDims], sact[kNumDims];
+    if (threadIdx.x < kNumDims) { smin[threadIdx.x] = INT_MAX; smax[threadIdx.x] = -1; sact[threadIdx.x] = 0; }
     __syncthreads();
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
         uint64_t d = desc[i];
@@ -505,18 +489,22 @@ __global__ void k_dim_rows(int64_t n, const int32_t* rdim, const int32_t* arena,
         if (!len) continue;
         int dm = rdim[i];
         atomicMin(&smin[dm], arena[desc_off(d) + kHdr]);
-        if (state[i] == ST_ACTIVE) atomicMax(&smax[dm], low[i] + 1);
+        if (state[i] == ST_ACTIVE) {
+            atomicMax(&smax[dm], low[i] + 1);
+            atomicAdd(&sact[dm], 1);
+        }
     }
     __syncthreads();
     if (threadIdx.x < kNumDims) {
         if (smin[threadIdx.x] != INT_MAX) atomicMin(&info->min_row[threadIdx.x], smin[threadIdx.x]);
         if (smax[threadIdx.x] >= 0) atomicMax(&info->max_row[threadIdx.x], smax[threadIdx.x]);
+        if (sact[threadIdx.x]) atomicAdd(&info->act_end[threadIdx.x], sact[threadIdx.x]);
     }
 }
 
 __global__ void k_diminfo_reset(DimInfo* info) {
     int d = threadIdx.x;
-    if (d < kNumDims) { info->min_row[d] = INT_MAX; info->max_row[d] = -1; }
+    if (d < kNumDims) { info->min_row[d] = INT_MAX; info->max_row[d] = -1; info->act_end[d] = 0; }
 }
 
 int init_passes(Device& D, bool lows_done, cudaStream_t s) {
@@ -528,17 +516,14 @@ int init_passes(Device& D, bool lows_done, cudaStream_t s) {
     return lows_done ? 1 : 2;
 }
 
-int init_compress(Device& D, const uint8_t* dropped, bool keep_rows, bool final, cudaStream_t s, int64_t cb,
-                  int64_t ce, bool reset) {
-    const int64_t n = ce < 0 ? D.n : ce;
-    if (n <= cb) return 0;
+int init_compress(Device& D, const uint8_t* dropped, bool keep_rows, bool final, cudaStream_t s) {
+    const int64_t n = D.n;
     // the row bounds go to the DimInfo through a few atomics per block: few blocks
-    const unsigned g = grid_for(n - cb, 256) > 4096 ? 4096 : grid_for(n - cb, 256);
-    if (final && reset) k_diminfo_reset<<<1, 32, 0, s>>>(D.diminfo);
-    k_init_compress<<<g, 256, 0, s>>>(cb, n, D.arena, D.desc, D.low, D.pivot, D.cleared, D.negative, D.state, dropped,
+    const unsigned g = grid_for(n, 256) > 4096 ? 4096 : grid_for(n, 256);
+    k_init_compress<<<g, 256, 0, s>>>(n, D.arena, D.desc, D.low, D.pivot, D.cleared, D.negative, D.state, dropped,
                                       keep_rows, final ? D.app : nullptr, final ? D.dim : nullptr, D.diminfo,
                                       D.counters, D.err);
-    return final && reset ? 2 : 1;
+    return 1;
 }
 
 // Inline copies of the short apparent columns, by row (see Device::app).
@@ -567,57 +552,92 @@ int build_apparent(Device& D, cudaStream_t s) {
     return 1;
 }
 
-// Active list in reordered order (dimension segments are contiguous) and the
-// per-dimension bounds.
-__global__ void k_act_segments(const int64_t* actpos, int64_t n, DimInfo* info) {
-    int d = threadIdx.x;
-    if (d < kNumDims) {
-        int32_t b = info->col_begin[d], e = info->col_end[d];
-        info->act_begin[d] = int32_t(b < n ? actpos[b] : actpos[n]);
-        info->act_end[d] = int32_t(e < n ? actpos[e] : actpos[n]);
-    }
-}
-
+// Active list in reordered order (dimension segments are contiguous).  act_end
+// holds each dimension's count of active columns, gathered with the row bounds;
+// the scan's end turns the counts into segments.
 int active_list(Device& D, bool rows_done, cudaStream_t s) {
     const int64_t n = D.n;
+    if (!rows_done) {
+        k_diminfo_reset<<<1, 32, 0, s>>>(D.diminfo);
+        const unsigned g = grid_for(n, 256) > 4096 ? 4096 : grid_for(n, 256);
+        k_dim_rows<<<g, 256, 0, s>>>(n, D.dim, D.arena, D.desc, D.low, D.state, D.diminfo);
+    }
     const uint8_t* state = D.state;
     int32_t* act = D.active;
-    int64_t* pos = D.scratch64;
-    scan([=] __device__(int64_t i) -> int64_t { return state[i] == ST_ACTIVE ? 1 : 0; },
-         [=] __device__(int64_t i, int64_t pre, int64_t v) {
-             pos[i] = pre;
-             if (v) act[pre] = int32_t(i);
+    DimInfo* info = D.diminfo;
+    scan([=] __device__(int64_t i) -> ScanClass { return {uint8_t(state[i] == ST_ACTIVE ? 1 : 0)}; },
+         [=] __device__(int64_t i, int64_t pre, ScanClass v) {
+             if (v.c) act[pre] = int32_t(i);
          },
-         n, D.blk, s);
-    // pos[n] = total
-    cudaMemcpyAsync(pos + n, D.blk + scan_blocks(n), sizeof(int64_t), cudaMemcpyDeviceToDevice, s);
-    k_act_segments<<<1, 32, 0, s>>>(pos, n, D.diminfo);
-    if (rows_done) return 4;
-    k_diminfo_reset<<<1, 32, 0, s>>>(D.diminfo);
-    const unsigned g = grid_for(n, 256) > 4096 ? 4096 : grid_for(n, 256);
-    k_dim_rows<<<g, 256, 0, s>>>(n, D.dim, D.arena, D.desc, D.low, D.state, D.diminfo);
-    return 6;
+         n, D.blk, s,
+         [=] __device__(int64_t) {
+             int32_t at = 0;
+             // reordered columns ascend with the dimension, or descend (dual)
+             const bool down = info->col_begin[0] > info->col_begin[kNumDims - 1];
+             for (int k = 0; k < kNumDims; k++) {
+                 const int d = down ? kNumDims - 1 - k : k;
+                 const int32_t c = info->act_end[d];
+                 info->act_begin[d] = at;
+                 info->act_end[d] = at += c;
+             }
+         });
+    return rows_done ? 1 : 3;
 }
 
 // ------------------------------------------------------------------- pairs
-// primal: row r (reordered) owned by column c -> (perm[r], perm[c]).
-// dual: the dual row r' owned by dual column c' maps back to the primal pair
-// (n-1-c', n-1-r') of the dualized matrix's own numbering; `dual_to_input`
-// then maps those primal reordered indices to input indices.
+// Primal: input simplex j (reordered i) is a birth when row i has an owner, whose
+// simplex is its death; it is a death when column i owns a row; neither, and not
+// dropped by an edge collapse: essential.  One scan in input order writes both
+// lists (births ascending, so the pairs come out sorted): it reads the maps and
+// the pivot table in two nearly sequential streams per dimension, and only the
+// deaths' input indices at random.  64^3: 92 us; a scatter by birth and two scans over
+// its marks took 250.
+struct PairsOut {
+    int64_t n;
+    const int32_t* newidx;
+    const int32_t* perm;
+    const uint64_t* pivot;
+    const uint8_t* state;
+    longlong2* pairs;
+    int64_t* ess;
+    long long* counters;
+};
+constexpr int64_t kBirths = (int64_t(1) << kScanClassShift) - 1;  // class 1: births, class 2: essentials
+
+struct PairsValue {
+    PairsOut o;
+    __device__ ScanClass operator()(int64_t j) const {
+        const int32_t i = o.newidx[j];
+        const uint64_t e = o.pivot[i];
+        const uint8_t st = o.state[i];
+        return {uint8_t(e != kNoOwner ? 1 : (st == ST_OWNER || st == ST_DROPPED ? 0 : 2))};
+    }
+};
+struct PairsSink {
+    PairsOut o;
+    __device__ void operator()(int64_t j, int64_t pre, ScanClass v) const {
+        if (v.c == 1) o.pairs[pre & kBirths] = make_longlong2(j, o.perm[pv_col(o.pivot[o.newidx[j]])]);
+        else if (v.c == 2) o.ess[pre >> kScanClassShift] = j;
+    }
+};
+struct PairsDone {
+    PairsOut o;
+    __device__ void operator()(int64_t total) const {
+        o.counters[CNT_NPAIRS] = total & kBirths;
+        o.counters[CNT_NESS] = total >> kScanClassShift;
+    }
+};
+
+// Dual: the dual row r' owned by dual column c' maps back to the primal pair
+// (n-1-c', n-1-r') of the dualized matrix's own numbering, and perm maps those
+// to input indices; scattered by birth first, since a column that owns a row from
+// the boundary matrix's pass (mode 2) is not marked as one.
 __global__ void k_pairs_scatter(int64_t n, const uint64_t* pivot, const int32_t* perm, int64_t* death_of,
-                                uint8_t* paired, int dual) {
+                                uint8_t* paired) {
     for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n; r += int64_t(gridDim.x) * blockDim.x) {
-        uint64_t e = pivot[r];
+        const uint64_t e = pivot[r];
         if (e == kNoOwner) continue;
-        int32_t c = pv_col(e);
-        int64_t birth, death;
-        if (!dual) {
-            birth = perm[r];
-            death = perm[c];
-        } else {
-            birth = perm[n - 1 - c];
-            death = perm[n - 1 - r];
-        }
+        const int64_t birth = perm[n - 1 - pv_col(e)], death = perm[n - 1 - r];
         death_of[birth] = death;
         paired[birth] = 1;
         paired[death] = 1;
@@ -631,31 +651,27 @@ __global__ void k_mark_dropped(int64_t n, const uint8_t* dropped, const int32_t*
 
 int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s) {
     const int64_t n = D.n;
+    longlong2* pairs = reinterpret_cast<longlong2*>(D.pairs);
+    const PairsOut o{n, D.newidx, D.perm, D.pivot, D.state, pairs, D.ess, D.counters};
+    if (!dual) {
+        scan(PairsValue{o}, PairsSink{o}, n, D.blk, s, PairsDone{o});
+        return 1;
+    }
     const unsigned g = grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256);
     fill_i64(D.death_of, -1, n, s);
     cudaMemsetAsync(D.negative, 0, n, s);  // reused as the "paired or dropped" mark
-    k_pairs_scatter<<<g, 256, 0, s>>>(n, D.pivot, D.perm, D.death_of, D.negative, dual);
+    k_pairs_scatter<<<g, 256, 0, s>>>(n, D.pivot, D.perm, D.death_of, D.negative);
     if (dropped) k_mark_dropped<<<g, 256, 0, s>>>(n, dropped, D.perm, D.negative);
     const int64_t* death_of = D.death_of;
-    int64_t* pairs = D.pairs;
-    scan([=] __device__(int64_t i) -> int64_t { return death_of[i] >= 0 ? 1 : 0; },
-         [=] __device__(int64_t i, int64_t pre, int64_t v) {
-             if (v) {
-                 pairs[2 * pre] = i;
-                 pairs[2 * pre + 1] = death_of[i];
-             }
-         },
-         n, D.blk, s);
-    cudaMemcpyAsync(&D.counters[CNT_NPAIRS], D.blk + scan_blocks(n), sizeof(int64_t), cudaMemcpyDeviceToDevice, s);
     const uint8_t* paired = D.negative;
     int64_t* ess = D.ess;
-    scan([=] __device__(int64_t i) -> int64_t { return paired[i] ? 0 : 1; },
-         [=] __device__(int64_t i, int64_t pre, int64_t v) {
-             if (v) ess[pre] = i;
+    scan([=] __device__(int64_t j) -> ScanClass { return {uint8_t(death_of[j] >= 0 ? 1 : (paired[j] ? 0 : 2))}; },
+         [=] __device__(int64_t j, int64_t pre, ScanClass v) {
+             if (v.c == 1) pairs[pre & kBirths] = make_longlong2(j, death_of[j]);
+             else if (v.c == 2) ess[pre >> kScanClassShift] = j;
          },
-         n, D.blk, s);
-    cudaMemcpyAsync(&D.counters[CNT_NESS], D.blk + scan_blocks(n), sizeof(int64_t), cudaMemcpyDeviceToDevice, s);
-    return 8 + (dropped ? 1 : 0);
+         n, D.blk, s, PairsDone{o});
+    return 3 + (dropped ? 1 : 0);
 }
 
 }  // namespace sspp

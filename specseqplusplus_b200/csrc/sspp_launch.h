@@ -23,7 +23,6 @@ int batch_rebase(int64_t n, int64_t nnz, int32_t k, const int64_t* d_cstart, con
 // assigned: recorded once perm / newidx / dim are written (before the columns
 // are scattered), or null
 int reorder(Device& D, bool lows, cudaStream_t s, cudaEvent_t assigned = nullptr);
-int64_t reorder_total_slot(const Device& D);  // index into D.blk of the arena total
 
 // per-complex slice starts (k+1 each) of the sorted pairs and essentials
 int batch_bounds(int32_t k, const int64_t* d_cstart, int64_t npairs, const int64_t* pairs, int64_t ness,
@@ -38,10 +37,7 @@ int init_passes(Device& D, bool lows_done, cudaStream_t s);
 // representative cycles); otherwise they are removed.
 // final (no dualization follows): also the inline apparent columns (as
 // build_apparent) and the per-dimension row bounds (as active_list)
-// columns [cb, ce) (ce < 0: to the end); reset: clear the row bounds first
-// (the first of the launches that together cover every column)
-int init_compress(Device& D, const uint8_t* dropped, bool keep_rows, bool final, cudaStream_t s, int64_t cb = 0,
-                  int64_t ce = -1, bool reset = true);
+int init_compress(Device& D, const uint8_t* dropped, bool keep_rows, bool final, cudaStream_t s);
 // rows_done: init_compress already gathered the row bounds
 int active_list(Device& D, bool rows_done, cudaStream_t s);
 // D.app from the pivot table as it stands (apparent pairs only)

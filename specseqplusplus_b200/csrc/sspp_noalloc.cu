@@ -375,7 +375,6 @@ cudaError_t reduce_in_scratch(int32_t* scratch, int dev, int64_t n, int64_t nnz,
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
     if (h.err) return cudaSuccess;
     reorder(D, true, s);
-    cudaMemcpyAsync(D.arena_top, D.blk + reorder_total_slot(D), sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s);
     init_passes(D, true, s);
     init_compress(D, nullptr, true, true, s);
     active_list(D, true, s);
