@@ -66,8 +66,9 @@ private:
     struct Seg {
         size_t piece, off, len, so;
     };
+    // `least`: smallest share of one host thread
     void parallel_copy(const std::vector<Piece>& pieces, const std::vector<Seg>& segs, size_t fill, uint8_t* stage,
-                       bool to_stage);
+                       bool to_stage, size_t least);
     uint8_t* stage_ = nullptr;  // pinned, two halves
     size_t half_ = 0;
     cudaEvent_t ev_[2] = {nullptr, nullptr};
