@@ -12,6 +12,7 @@
 #include <chrono>
 #include <climits>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -100,16 +101,14 @@ struct sspp_ctx {
     int64_t pool_request = 0;      // heavy pool entries requested (grows on CAPACITY)
     double init_ms = 0, compute_ms = 0;
     int64_t ss_steps = 0;
+    Ctl* h_ctl = nullptr;          // pinned mirror of Device::ctl
     int* h_err = nullptr;          // pinned
     int* h_gate = nullptr;         // mapped pinned: CTA-tier pool columns finished (mirror)
     int* d_gate = nullptr;         // its device address
     int* h_tail = nullptr;         // pinned: the pool tail after a dimension's sweep
     cudaEvent_t gate_ev = nullptr;
     cudaEvent_t hc_fork = nullptr, hc_join = nullptr;  // guided clearing beside the apparent-pair pass
-    long long* h_counters = nullptr;
-    unsigned long long* h_dimtot = nullptr;  // pinned: columns per dimension (validation pass)
-    DimInfo* h_info = nullptr;
-    unsigned long long* h_top = nullptr;
+    int64_t* h_top = nullptr;      // pinned: a device input's entry count
     uint8_t* dropped = nullptr;    // primal reordered numbering (model bit 2)
     int64_t cap_dropped = 0;
     // input buffers owned by the context (host loads); device loads are read in place
@@ -194,10 +193,9 @@ cudaError_t grow(T*& p, int64_t& cap, int64_t want, cudaStream_t s) {
 }
 
 void free_device(Device& D) {
-    void* ptrs[] = {D.dim, D.perm, D.newidx, D.scratch64, D.arena, D.arena_top,
-                    D.desc, D.low, D.pivot, D.state, D.cleared, D.negative, D.leftmost, D.active, D.blk, D.dimcnt,
-                    D.diminfo, D.err, D.counters, D.step_ctr, D.heavy, D.pool_tail, D.heavy_done, D.death_of, D.pairs,
-                    D.ess, D.misc, D.app, D.runlist, D.dimtot};
+    void* ptrs[] = {D.dim, D.perm, D.newidx, D.scratch64, D.arena,
+                    D.desc, D.low, D.pivot, D.state, D.cleared, D.negative, D.leftmost, D.active, D.ctl, D.dimcnt,
+                    D.step_ctr, D.heavy, D.death_of, D.pairs, D.ess, D.misc, D.app, D.runlist};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     D = Device();
@@ -233,21 +231,30 @@ int ensure_columns(sspp_ctx* ctx, int64_t n, int64_t nnz) {
         CK(g(D.ess, 1));
         CK(g(D.app, 1));
         D.cap_n = c;
-        int64_t nb = (c + 4095) / 4096 + 2;
-        CK(grow(D.blk, D.cap_blk, nb, ctx->stream));
-        int64_t nbp = (c + 255) / 256 + 1;
-        CK(grow(D.dimcnt, D.cap_dimcnt, nbp * kNumDims, ctx->stream));
+        // the control block and the scans' tile states (one per 4,096 columns, a total and room for one more)
+        D.blk_stride = (c + 4095) / 4096 + 2;
+        const int64_t ctl_words = int64_t((sizeof(Ctl) + 15) / 16) * 2;
+        int64_t* buf = reinterpret_cast<int64_t*>(D.ctl);
+        if (buf) CK(cudaFreeAsync(buf, ctx->stream));
+        buf = nullptr;
+        D.cap_blk = 0;
+        CK(grow(buf, D.cap_blk, ctl_words + 3 * D.blk_stride, ctx->stream));
+        D.ctl = reinterpret_cast<Ctl*>(buf);
+        D.blk = buf + ctl_words;
+        D.blk_zero = 0;
+        D.steps_zero = false;
+        D.diminfo = &D.ctl->info;
+        D.counters = D.ctl->counters;
+        D.arena_top = &D.ctl->arena_top;
+        D.err = &D.ctl->err;
+        D.pool_tail = &D.ctl->pool_tail;
+        D.heavy_done = &D.ctl->heavy_done;
+        D.cap_dimcnt = 0;
+        if (D.dimcnt) CK(cudaFreeAsync(D.dimcnt, ctx->stream));
+        D.dimcnt = nullptr;
+        CK(grow(D.dimcnt, D.cap_dimcnt, (part_tiles(c) + 1) * kNumDims, ctx->stream));
     }
-    if (!D.diminfo) {
-        CK(cudaMalloc(&D.diminfo, sizeof(DimInfo)));
-        CK(cudaMalloc(&D.err, sizeof(int)));
-        CK(cudaMalloc(&D.counters, sizeof(long long) * CNT_NUM));
-        CK(cudaMalloc(&D.arena_top, sizeof(unsigned long long)));
-        CK(cudaMalloc(&D.pool_tail, sizeof(int)));
-        CK(cudaMalloc(&D.heavy_done, sizeof(int)));
-        CK(cudaMalloc(&D.misc, sizeof(int64_t) * 8));
-        CK(cudaMalloc(&D.dimtot, sizeof(unsigned long long) * kNumDims));
-    }
+    if (!D.misc) CK(cudaMalloc(&D.misc, sizeof(int64_t) * 8));
     return SSPP_OK;
 }
 
@@ -282,6 +289,23 @@ int64_t arena_need(const sspp_ctx* ctx) {
 // of reduction in those blocks, 1.92 in 400 k, 1.74 in 1 M, 1.82 in one block per
 // dimension; 93^3 6.4 / 5.0 / 4.5 / 4.5 ms.  The pairs do not depend on it.
 constexpr int kMinBlock = 1 << 20;
+
+// Clears the control block and the scans' tile states.
+int clear_ctl(sspp_ctx* ctx) {
+    Device& D = ctx->D;
+    CK(cudaMemsetAsync(D.ctl, 0, size_t(reinterpret_cast<char*>(D.blk + 3 * D.blk_stride) - reinterpret_cast<char*>(D.ctl)),
+                       ctx->stream));
+    D.blk_zero = 7;
+    D.steps_zero = true;
+    return SSPP_OK;
+}
+
+// Reads the control block back (one copy, one synchronisation).
+int read_ctl(sspp_ctx* ctx) {
+    CK(cudaMemcpyAsync(ctx->h_ctl, ctx->D.ctl, offsetof(Ctl, step), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    return SSPP_OK;
+}
 
 // SS schedule of one dimension, following include/specseq.h:603-697.
 struct Step {
@@ -386,9 +410,9 @@ void span_collect(sspp_ctx* ctx) {
 // dropped[] of the edge collapse when it runs (model bit 2), else null
 const uint8_t* dropped_of(const sspp_ctx* ctx) { return (ctx->params.model & 2) ? ctx->dropped : nullptr; }
 
-// Edge collapse on the reordered matrix (needs host reads of the column
-// ranges, the edge count and the largest degree).
-int run_collapse(sspp_ctx* ctx) {
+// Edge collapse on the reordered matrix; info: its column ranges (it reads the
+// edge count and the largest degree back).
+int run_collapse(sspp_ctx* ctx, const DimInfo& info) {
     Device& D = ctx->D;
     cudaStream_t s = ctx->stream;
     if (D.n > ctx->cap_dropped) {
@@ -397,9 +421,6 @@ int run_collapse(sspp_ctx* ctx) {
         ctx->cap_dropped = 0;
         CK(grow(ctx->dropped, ctx->cap_dropped, D.n, s));
     }
-    CK(cudaMemcpyAsync(ctx->h_info, D.diminfo, sizeof(DimInfo), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    const DimInfo info = *ctx->h_info;
     const char* msg = nullptr;
     const int k = collapse(D, info, ctx->dropped, ctx->cs, s, &msg);
     if (k < 0) return set_err(ctx, SSPP_ERR_CUDA, msg ? msg : "edge collapse failed");
@@ -422,19 +443,9 @@ DimInfo ranges_of_counts(const unsigned long long* cnt) {
 }
 
 // Sizes the guided-clearing scratch from the per-dimension column ranges and
-// runs it on stream `s`.  `ranges` gives the ranges; without it they are read
-// back through the context's stream, whose work so far (the reorder) they
-// come from.
-int run_highclear(sspp_ctx* ctx, cudaStream_t s, const DimInfo* ranges = nullptr, bool from_input = false) {
+// runs it on stream `s`.
+int run_highclear(sspp_ctx* ctx, cudaStream_t s, const DimInfo& info, bool from_input) {
     Device& D = ctx->D;
-    DimInfo info;
-    if (ranges) {
-        info = *ranges;
-    } else {
-        CK(cudaMemcpyAsync(ctx->h_info, D.diminfo, sizeof(DimInfo), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        info = *ctx->h_info;
-    }
     HighclearScratch& S = ctx->hc;
     int top = -1;
     for (int d = kMaxDim; d >= 1; d--)
@@ -462,13 +473,10 @@ int run_highclear(sspp_ctx* ctx, cudaStream_t s, const DimInfo* ranges = nullptr
 }
 
 // Autotuned parameters for the loaded complex, chosen once its dimension
-// ranges are known (one host read): the shape key is the top dimension and
-// the quarter of the columns that lie in it.
-int autotune_choose(sspp_ctx* ctx) {
+// ranges are known: the shape key is the top dimension and the quarter of the
+// columns that lie in it.
+int autotune_choose(sspp_ctx* ctx, const DimInfo& I) {
     Device& D = ctx->D;
-    CK(cudaMemcpyAsync(ctx->h_info, D.diminfo, sizeof(DimInfo), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    const DimInfo& I = *ctx->h_info;
     int top = 0;
     for (int d = kMaxDim; d >= 0; d--)
         if (I.col_end[d] > I.col_begin[d]) { top = d; break; }
@@ -490,6 +498,8 @@ int autotune_choose(sspp_ctx* ctx) {
     return SSPP_OK;
 }
 
+const char* const kBadColumns = "dimension out of range 0..7 or malformed col_ptr";
+
 int run_init(sspp_ctx* ctx) {
     Device& D = ctx->D;
     cudaStream_t s = ctx->stream;
@@ -497,9 +507,9 @@ int run_init(sspp_ctx* ctx) {
     ctx->prof.reset();
     for (double& x : ctx->ph_ms) x = 0;
     ctx->launches = ctx->light_launches = ctx->heavy_launches = 0;
-    CK(cudaMemsetAsync(D.err, 0, sizeof(int), s));
-    CK(cudaMemsetAsync(D.counters, 0, sizeof(long long) * CNT_NUM, s));
-    int rc = ensure_arena(ctx, arena_need(ctx));
+    int rc = clear_ctl(ctx);
+    if (rc) return rc;
+    rc = ensure_arena(ctx, arena_need(ctx));
     if (rc) return rc;
     if (D.n == 0) {  // nothing to reduce
         std::memset(&ctx->hinfo, 0, sizeof(ctx->hinfo));
@@ -512,11 +522,17 @@ int run_init(sspp_ctx* ctx) {
     cudaEvent_t ev0 = nullptr;
     span_begin(ctx, ev0);
     ctx->launches += validate(D, s);
-    CK(cudaMemcpyAsync(ctx->h_err, D.err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(ctx->h_dimtot, D.dimtot, sizeof(unsigned long long) * kNumDims, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (*ctx->h_err) return set_err(ctx, SSPP_ERR_BAD_INPUT, "dimension out of range 0..7 or malformed col_ptr");
-    const DimInfo ranges = ranges_of_counts(ctx->h_dimtot);
+    // Guided clearing and the edge collapse need the dimension ranges on the host,
+    // the autotuner too, and the dualization reads what the passes leave whatever
+    // they find: these wait for the validation.  Every other run goes on, its passes
+    // look at the error word themselves, and the host reads it once, at the end.
+    const bool wait = ctx->params.model != 0 || ctx->user_params.autotune || ctx->params.dualize == 1;
+    DimInfo ranges{};
+    if (wait) {
+        if ((rc = read_ctl(ctx))) return rc;
+        if (ctx->h_ctl->err) return set_err(ctx, SSPP_ERR_BAD_INPUT, kBadColumns);
+        ranges = ranges_of_counts(ctx->h_ctl->dimtot);
+    }
     // the reorder also does the first init pass unless an edge collapse will
     // empty columns in between (the autotuner never changes the model)
     const bool lows_in_reorder = !(ctx->params.model & 2);
@@ -527,20 +543,21 @@ int run_init(sspp_ctx* ctx) {
     // has assigned the new indices (its tuples come from the input columns).
     const bool guided = (ctx->params.model & 1) && ctx->params.max_iteration > 0;
     const bool early = guided && !(ctx->params.model & 2);
-    ctx->launches += reorder(D, lows_in_reorder, s, early ? ctx->hc_fork : nullptr);
     if (ctx->user_params.autotune && !ctx->tune_locked) {
-        int rc2 = autotune_choose(ctx);
+        int rc2 = autotune_choose(ctx, ranges);
         if (rc2) return rc2;
     }
+    ctx->launches += reorder(D, lows_in_reorder, !lows_in_reorder || ctx->params.dualize == 1, s,
+                             early ? ctx->hc_fork : nullptr);
     if (ctx->params.model & 2) {  // collapse before everything else: dropped columns are emptied
-        int rc2 = run_collapse(ctx);
+        int rc2 = run_collapse(ctx, ranges);
         if (rc2) return rc2;
     }
     if (guided) {
         cudaStream_t hs = ctx->side[0];
         if (!early) CK(cudaEventRecord(ctx->hc_fork, s));  // after the collapse
         CK(cudaStreamWaitEvent(hs, ctx->hc_fork, 0));
-        int rc2 = run_highclear(ctx, hs, &ranges, early);
+        int rc2 = run_highclear(ctx, hs, ranges, early);
         CK(cudaEventRecord(ctx->hc_join, hs));
         if (rc2) {
             CK(cudaStreamWaitEvent(s, ctx->hc_join, 0));
@@ -557,20 +574,19 @@ int run_init(sspp_ctx* ctx) {
     ctx->launches += active_list(D, ctx->params.dualize != 1, s);
     span_end(ctx, PH_INIT, ev0);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(ctx->h_info, D.diminfo, sizeof(DimInfo), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(ctx->h_err, D.err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(ctx->h_counters, D.counters, sizeof(long long) * CNT_NUM, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    ctx->hinfo = *ctx->h_info;
-    std::memcpy(ctx->hcounters, ctx->h_counters, sizeof(ctx->hcounters));
+    if ((rc = read_ctl(ctx))) return rc;
+    const int err = ctx->h_ctl->err;
+    ctx->hinfo = ctx->h_ctl->info;
+    std::memcpy(ctx->hcounters, ctx->h_ctl->counters, sizeof(ctx->hcounters));
     ctx->init_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     span_collect(ctx);
-    if (*ctx->h_err & ERRB_BAD_INPUT)
+    if (err & ERRB_FACES)
         return set_err(ctx, SSPP_ERR_BAD_INPUT,
                        "malformed boundary matrix (a face index out of range, unsorted, duplicated, or of the "
                        "wrong dimension)");
-    if (*ctx->h_err & ERRB_CHECK) return set_err(ctx, SSPP_ERR_BAD_INPUT, "dualization self-check failed");
-    if (*ctx->h_err) return set_err(ctx, SSPP_ERR_CAPACITY, "init pass overflow");
+    if (err & ERRB_BAD_INPUT) return set_err(ctx, SSPP_ERR_BAD_INPUT, kBadColumns);
+    if (err & ERRB_CHECK) return set_err(ctx, SSPP_ERR_BAD_INPUT, "dualization self-check failed");
+    if (err) return set_err(ctx, SSPP_ERR_CAPACITY, "init pass overflow");
     ctx->inited = true;
     ctx->computed = false;
     return SSPP_OK;
@@ -626,19 +642,24 @@ int dimension_gate(sspp_ctx* ctx) {
     return SSPP_OK;
 }
 
-constexpr int kStepCtr = 8;  // counters per spectral-sequence step (see ReduceArgs::ctr)
-
 int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2, int ht) {
     Device& D = ctx->D;
     cudaStream_t s = ctx->stream;
     const sspp_params& P = ctx->params;
-    if (kStepCtr * int64_t(steps.size()) > D.cap_steps) {
-        if (D.step_ctr) cudaFreeAsync(D.step_ctr, s);
-        D.step_ctr = nullptr;
-        D.cap_steps = 0;
-        CK(grow(D.step_ctr, D.cap_steps, kStepCtr * int64_t(steps.size()) + 64, s));
+    // counters: the control block's while they are as the init passes cleared them
+    int* step_ctr = D.ctl->step;
+    if (!D.steps_zero || steps.size() > size_t(kCtlSteps)) {
+        if (kStepCtr * int64_t(steps.size()) > D.cap_steps) {
+            if (D.step_ctr) cudaFreeAsync(D.step_ctr, s);
+            D.step_ctr = nullptr;
+            D.cap_steps = 0;
+            CK(grow(D.step_ctr, D.cap_steps, kStepCtr * int64_t(steps.size()) + 64, s));
+        }
+        step_ctr = D.step_ctr;
+        if (!steps.empty()) CK(cudaMemsetAsync(step_ctr, 0, sizeof(int) * kStepCtr * steps.size(), s));
+        CK(cudaMemsetAsync(D.pool_tail, 0, 2 * sizeof(int), s));  // and heavy_done
     }
-    if (!steps.empty()) CK(cudaMemsetAsync(D.step_ctr, 0, sizeof(int) * kStepCtr * steps.size(), s));
+    D.steps_zero = false;
     // heavy pool: deferrals are rare (heavy columns and displaced owners); a
     // full pool sets the capacity bit and the run is repeated with a larger one
     const int64_t want_pool = std::max<int64_t>(ctx->pool_request, std::max<int64_t>(D.n / 4, 1 << 16));
@@ -648,7 +669,6 @@ int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2,
         D.pool_cap = 0;
         CK(grow(D.heavy, D.pool_cap, want_pool, s));
     }
-    CK(cudaMemsetAsync(D.pool_tail, 0, sizeof(int), s));
     const int light_max = std::max(1, ctx->num_sms * ctx->light_blocks_per_sm);
     const int heavy_grid = std::max(1, std::min(ctx->num_sms * ctx->heavy_blocks_per_sm, 2 * ctx->num_sms));
     const int q_blocks = std::max(1, (P.queue_size + 3) / 4);
@@ -663,7 +683,6 @@ int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2,
     D.gate_host = gate ? ctx->d_gate : nullptr;
     if (gate) {
         *reinterpret_cast<volatile int*>(ctx->h_gate) = 0;  // no CTA-tier launch of this context is running
-        CK(cudaMemsetAsync(D.heavy_done, 0, sizeof(int), s));
     }
     while (ctx->step_ev.size() < steps.size() + 1) {
         cudaEvent_t ev;
@@ -689,13 +708,12 @@ int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2,
         }
         const int64_t window = int64_t(st.end) - st.beg;
         const int grid = int(std::max<int64_t>(1, std::min<int64_t>({(window + 3) / 4, light_max, q_blocks})));
-        int* ctr = D.step_ctr + kStepCtr * k;
+        int* ctr = step_ctr + kStepCtr * k;
         cudaEvent_t a = nullptr, b = nullptr;
         span_begin(ctx, a);
         int* ctr_next = k + 1 < steps.size() ? ctr + kStepCtr : nullptr;
         const int fgrid = int(std::max<int64_t>(1, std::min<int64_t>((window + 255) / 256, int64_t(ctx->num_sms) * 8)));
-        reduce_light_launch(D, st.beg, st.end, st.minrow, cap1, ctr, ctr_next, fgrid, grid, s);
-        ctx->launches++;
+        ctx->launches += reduce_light_launch(D, st.beg, st.end, st.minrow, cap1, ctr, ctr_next, fgrid, grid, s);
         span_end(ctx, PH_LIGHT, a);
         if (overlap && (!last_of_dim || gate)) {
             // an idle side stream if there is one: a CTA-tier launch lasts as
@@ -725,7 +743,7 @@ int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2,
         }
         ctx->light_launches++;
         ctx->heavy_launches++;
-        ctx->launches += 2;
+        ctx->launches++;
         if (gate && last_of_dim && k + 1 < steps.size()) {
             int rcg = dimension_gate(ctx);
             if (rcg) return rcg;
@@ -955,9 +973,8 @@ int run_compute(sspp_ctx* ctx) {
         ctx->launches += dualize(D, 2, s);
         ctx->launches += build_apparent(D, s);
         ctx->launches += active_list(D, false, s);
-        CK(cudaMemcpyAsync(ctx->h_info, D.diminfo, sizeof(DimInfo), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        ctx->hinfo = *ctx->h_info;
+        if ((rc = read_ctl(ctx))) return rc;
+        ctx->hinfo = ctx->h_ctl->info;
         rc = phase(1, kMaxDim, true);
         if (rc) return rc;
         nsteps += ctx->ss_steps;
@@ -972,15 +989,12 @@ int run_compute(sspp_ctx* ctx) {
     ctx->launches += extract_pairs(D, P.dualize != 0, dropped_of(ctx), s);
     span_end(ctx, PH_PAIRS, ep);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(ctx->h_err, D.err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(ctx->h_counters, D.counters, sizeof(long long) * CNT_NUM, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(ctx->h_top, D.arena_top, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    std::memcpy(ctx->hcounters, ctx->h_counters, sizeof(ctx->hcounters));
-    ctx->arena_used = int64_t(*ctx->h_top);
+    if (int rc = read_ctl(ctx)) return rc;
+    std::memcpy(ctx->hcounters, ctx->h_ctl->counters, sizeof(ctx->hcounters));
+    ctx->arena_used = int64_t(ctx->h_ctl->arena_top);
     ctx->compute_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     span_collect(ctx);
-    const int e = *ctx->h_err;
+    const int e = ctx->h_ctl->err;
     if (e & ERRB_CAPACITY) return SSPP_ERR_CAPACITY;
     if (e & ERRB_LEN) return set_err(ctx, SSPP_ERR_CAPACITY, "a column exceeded 2^24 entries");
     if (e & ERRB_TIMEOUT) return set_err(ctx, SSPP_ERR_TIMEOUT, "per-column merge limit reached");
@@ -1185,10 +1199,8 @@ sspp_ctx* sspp_create(const sspp_config* cfg) {
         ctx->gate_ev = nullptr;
     }
     if (cudaMallocHost(&ctx->h_err, sizeof(int)) != cudaSuccess ||
-        cudaMallocHost(&ctx->h_counters, sizeof(long long) * CNT_NUM) != cudaSuccess ||
-        cudaMallocHost(&ctx->h_info, sizeof(DimInfo)) != cudaSuccess ||
-        cudaMallocHost(&ctx->h_dimtot, sizeof(unsigned long long) * kNumDims) != cudaSuccess ||
-        cudaMallocHost(&ctx->h_top, sizeof(unsigned long long)) != cudaSuccess) {
+        cudaMallocHost(&ctx->h_ctl, sizeof(Ctl)) != cudaSuccess ||
+        cudaMallocHost(&ctx->h_top, sizeof(int64_t)) != cudaSuccess) {
         delete ctx;
         return nullptr;
     }
@@ -1238,9 +1250,7 @@ void sspp_destroy(sspp_ctx* ctx) {
     if (ctx->gate_ev) cudaEventDestroy(ctx->gate_ev);
     if (ctx->hc_fork) cudaEventDestroy(ctx->hc_fork);
     if (ctx->hc_join) cudaEventDestroy(ctx->hc_join);
-    if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
-    if (ctx->h_info) cudaFreeHost(ctx->h_info);
-    if (ctx->h_dimtot) cudaFreeHost(ctx->h_dimtot);
+    if (ctx->h_ctl) cudaFreeHost(ctx->h_ctl);
     if (ctx->h_top) cudaFreeHost(ctx->h_top);
     delete ctx;
 }
@@ -1811,28 +1821,26 @@ int32_t sspp_export_preprocessed(sspp_ctx* ctx, const sspp_params* p, const char
         CK(cudaMemcpyAsync(cp.data(), D.in_colptr, 8 * (size_t(n) + 1), cudaMemcpyDeviceToHost, s));
     }
     if (nnz > 0) CK(cudaMemcpyAsync(rows.data(), D.in_rows, 4 * size_t(nnz), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemsetAsync(D.err, 0, sizeof(int), s));
-    CK(cudaMemsetAsync(D.counters, 0, sizeof(long long) * CNT_NUM, s));
+    if ((rc = clear_ctl(ctx))) return rc;
     CK(cudaStreamSynchronize(s));
     std::vector<uint8_t> drop(size_t(std::max<int64_t>(n, 1)), 0);
     if (n > 0 && (p->model & 3)) {
         rc = ensure_arena(ctx, arena_need(ctx));
         if (rc) return rc;
         validate(D, s);
-        CK(cudaMemcpyAsync(ctx->h_err, D.err, sizeof(int), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        if (*ctx->h_err) return set_err(ctx, SSPP_ERR_BAD_INPUT, "dimension out of range 0..7 or malformed col_ptr");
-        reorder(D, false, s);
-        CK(cudaMemcpyAsync(ctx->h_err, D.err, sizeof(int), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        if (*ctx->h_err) return set_err(ctx, SSPP_ERR_BAD_INPUT, "malformed boundary matrix");
+        if ((rc = read_ctl(ctx))) return rc;
+        if (ctx->h_ctl->err) return set_err(ctx, SSPP_ERR_BAD_INPUT, kBadColumns);
+        reorder(D, false, true, s);
+        if ((rc = read_ctl(ctx))) return rc;
+        if (ctx->h_ctl->err) return set_err(ctx, SSPP_ERR_BAD_INPUT, "malformed boundary matrix");
+        const DimInfo ranges = ctx->h_ctl->info;
         if (p->model & 2) {
-            rc = run_collapse(ctx);
+            rc = run_collapse(ctx, ranges);
             if (rc) return rc;
         }
         CK(cudaMemsetAsync(D.cleared, 0, size_t(n), s));
         if ((p->model & 1) && p->max_iteration > 0) {
-            rc = run_highclear(ctx, ctx->stream);
+            rc = run_highclear(ctx, ctx->stream, ranges, false);
             if (rc) return rc;
         }
         std::vector<int32_t> perm(static_cast<size_t>(n));
@@ -1840,10 +1848,9 @@ int32_t sspp_export_preprocessed(sspp_ctx* ctx, const sspp_params* p, const char
         CK(cudaMemcpyAsync(perm.data(), D.perm, 4 * size_t(n), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(cl.data(), D.cleared, size_t(n), cudaMemcpyDeviceToHost, s));
         if (p->model & 2) CK(cudaMemcpyAsync(dr.data(), ctx->dropped, size_t(n), cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(ctx->h_counters, D.counters, sizeof(long long) * CNT_NUM, cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
+        if ((rc = read_ctl(ctx))) return rc;
         CK(cudaGetLastError());
-        std::memcpy(ctx->hcounters, ctx->h_counters, sizeof(ctx->hcounters));
+        std::memcpy(ctx->hcounters, ctx->h_ctl->counters, sizeof(ctx->hcounters));
         for (int64_t i = 0; i < n; i++)
             if (cl[size_t(i)] || dr[size_t(i)]) drop[size_t(perm[size_t(i)])] = 1;
     }

@@ -40,40 +40,64 @@ void fill_i64(int64_t* p, int64_t v, int64_t n, cudaStream_t s) {
 }
 
 // Input validation before any index is used: dimensions in range and col_ptr
-// non-decreasing from 0 to nnz (device-resident inputs are only checked here).  Also
-// counts the columns of each dimension (dimtot, zeroed before), which give
-// the host the reordered dimension ranges with the same read as the error word.
-__global__ void __launch_bounds__(256) k_validate(const int32_t* dims, const int64_t* colptr, int64_t n,
-                                                  int64_t nnz, int* err, unsigned long long* dimtot) {
-    __shared__ unsigned s_cnt[kNumDims];
+// non-decreasing from 0 to nnz (device-resident inputs are only checked here).
+// The same pass counts the columns of each dimension, per tile for the reorder
+// (dimcnt) and in total for the host (dimtot, zeroed before), and finds the
+// longest column.  A warp takes 256 consecutive columns.
+constexpr int kPartThreads = 256;
+constexpr int kPartRounds = 8;
+constexpr int kPartTile = kPartThreads * kPartRounds;
+
+int64_t part_tiles(int64_t n) { return (n + kPartTile - 1) / kPartTile; }
+
+__global__ void __launch_bounds__(kPartThreads) k_validate(const int32_t* dims, const int64_t* colptr, int64_t n,
+                                                           int64_t nnz, int32_t* dimcnt, Ctl* ctl) {
+    __shared__ int s_cnt[kNumDims];
+    __shared__ int s_len, s_bad;
     if (threadIdx.x < kNumDims) s_cnt[threadIdx.x] = 0;
+    if (threadIdx.x == 0) s_len = s_bad = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    for (int64_t b0 = blockIdx.x * int64_t(blockDim.x); b0 < n; b0 += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t j = b0 + threadIdx.x;
+    const int64_t j0 = int64_t(blockIdx.x) * kPartTile + (threadIdx.x >> 5) * (32 * kPartRounds) + lane;
+    int mine = 0, longest = 0;
+    bool bad = false;
+#pragma unroll
+    for (int k = 0; k < kPartRounds; k++) {
+        const int64_t j = j0 + 32 * k;
         int d = -1;
         if (j < n) {
             d = dims[j];
-            const int64_t a = colptr[j], b = colptr[j + 1];
-            if (d < 0 || d > kMaxDim || b < a || b - a > kMaxColLen || (j == 0 && a != 0) || (j == n - 1 && b != nnz))
-                atomicOr(err, ERRB_BAD_INPUT);
+            const int64_t a = colptr[j], b = colptr[j + 1], len = b - a;
+            if (d < 0 || d > kMaxDim || len < 0 || len > kMaxColLen || (j == 0 && a != 0) || (j == n - 1 && b != nnz))
+                bad = true;
+            else
+                longest = max(longest, int(len));
         }
 #pragma unroll
         for (int q = 0; q < kNumDims; q++) {
             const unsigned m = __ballot_sync(kFull, d == q);
-            if (lane == 0 && m) atomicAdd(&s_cnt[q], unsigned(__popc(m)));
+            if (lane == q) mine += __popc(m);
         }
     }
+    if (lane < kNumDims && mine) atomicAdd(&s_cnt[lane], mine);
+    longest = __reduce_max_sync(kFull, longest);
+    if (lane == 0 && longest) atomicMax(&s_len, longest);
+    if (bad) s_bad = 1;
     __syncthreads();
-    if (threadIdx.x < kNumDims && s_cnt[threadIdx.x])
-        atomicAdd(dimtot + threadIdx.x, (unsigned long long)s_cnt[threadIdx.x]);
+    if (threadIdx.x < kNumDims) {
+        const int c = s_cnt[threadIdx.x];
+        dimcnt[int64_t(blockIdx.x) * kNumDims + threadIdx.x] = c;
+        if (c) atomicAdd(&ctl->dimtot[threadIdx.x], (unsigned long long)c);
+    }
+    if (threadIdx.x == 0) {
+        if (s_len > 0) atomicMax(&ctl->max_len, s_len);
+        if (s_bad) atomicOr(&ctl->err, ERRB_BAD_INPUT);
+    }
 }
 
 int validate(Device& D, cudaStream_t s) {
     if (D.n <= 0) return 0;
-    cudaMemsetAsync(D.dimtot, 0, sizeof(unsigned long long) * kNumDims, s);
-    k_validate<<<grid_for(D.n, 256) > 4096 ? 4096 : grid_for(D.n, 256), 256, 0, s>>>(D.in_dims, D.in_colptr, D.n, D.nnz,
-                                                                                     D.err, D.dimtot);
+    k_validate<<<unsigned(part_tiles(D.n)), kPartThreads, 0, s>>>(D.in_dims, D.in_colptr, D.n, D.nnz, D.dimcnt, D.ctl);
     return 1;
 }
 
@@ -166,103 +190,132 @@ int batch_localize(int64_t npairs, int64_t ness, int32_t k, const int64_t* d_cst
 }
 
 // ------------------------------------------------------------------ reorder
-constexpr int kPartThreads = 256;
+// The passes below run before the host has read the validation's verdict: each
+// leaves at once when the error word is set, so no unchecked index is used.
 
-// per-block count of columns of each dimension; flags dims out of range
-__global__ void __launch_bounds__(kPartThreads) k_dim_count(const int32_t* dims, int64_t n, int32_t* dimcnt, int* err) {
-    __shared__ int cnt[kNumDims];
-    if (threadIdx.x < kNumDims) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    int64_t j = int64_t(blockIdx.x) * kPartThreads + threadIdx.x;
-    if (j < n) {
-        int d = dims[j];
-        if (d < 0 || d > kMaxDim) atomicOr(err, ERRB_BAD_INPUT);
-        else atomicAdd(&cnt[d], 1);
+// Per-dimension totals -> dimension ranges of the reordered columns; also empties
+// the active segments (act_end counts first) and the row bounds that later passes
+// fill.
+__device__ void dim_ranges(const int64_t* total, DimInfo* info) {
+    int64_t at = 0;
+    for (int d = 0; d < kNumDims; d++) {
+        info->col_begin[d] = int32_t(at);
+        at += total[d];
+        info->col_end[d] = int32_t(at);
+        info->act_begin[d] = info->act_end[d] = 0;
+        info->min_row[d] = INT_MAX;
+        info->max_row[d] = -1;
     }
-    __syncthreads();
-    if (threadIdx.x < kNumDims) dimcnt[int64_t(blockIdx.x) * kNumDims + threadIdx.x] = cnt[threadIdx.x];
 }
 
-// one block per dimension: exclusive scan of that dimension's per-block
-// counts; the dimension's total goes to col_end[d] until k_dim_starts
-__global__ void __launch_bounds__(1024) k_dim_offsets(int32_t* dimcnt, int64_t nb, DimInfo* info) {
-    __shared__ int64_t wt[32];
-    __shared__ int64_t carry;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, d = blockIdx.x;
-    if (tid == 0) carry = 0;
+// First reordered index of each tile's columns of each dimension (dimcnt, in
+// place), and the ranges.  One block; thread (chunk, dimension) takes a chunk of
+// consecutive tiles.  Inputs of up to kInlineTiles tiles skip it: their tiles add
+// up the counts themselves.
+constexpr int kInlineTiles = 128;
+__global__ void __launch_bounds__(1024) k_dim_offsets(int32_t* dimcnt, int64_t nb, Ctl* ctl) {
+    if (ctl->err) return;
+    __shared__ int64_t s_sum[128][kNumDims];
+    __shared__ int64_t s_total[kNumDims];
+    const int d = threadIdx.x & 7, c = threadIdx.x >> 3;
+    const int64_t per = (nb + 127) / 128, b0 = c * per, b1 = b0 + per < nb ? b0 + per : nb;
+    int64_t sum = 0;
+    for (int64_t b = b0; b < b1; b++) sum += dimcnt[b * kNumDims + d];
+    s_sum[c][d] = sum;
     __syncthreads();
-    for (int64_t base = 0; base < nb; base += 1024) {
-        int64_t i = base + tid;
-        int64_t v = i < nb ? dimcnt[i * kNumDims + d] : 0;
-        int64_t inc = warp_inclusive_scan(v);
-        if (lane == 31) wt[wid] = inc;
-        __syncthreads();
-        if (wid == 0) {
-            int64_t t = wt[lane];
-            int64_t ti = warp_inclusive_scan(t);
-            wt[lane] = ti - t;
-        }
-        __syncthreads();
-        int64_t ex = carry + wt[wid] + inc - v;
-        if (i < nb) dimcnt[i * kNumDims + d] = int32_t(ex);
-        __syncthreads();
-        if (tid == 1023) carry = ex + v;
-        __syncthreads();
-    }
-    if (tid == 0) info->col_end[d] = int32_t(carry);
-}
-
-// per-dimension totals -> dimension ranges of the reordered columns; also empties
-// the active segments and the row bounds that later passes fill
-__global__ void k_dim_starts(DimInfo* info) {
     if (threadIdx.x < kNumDims) {
-        info->act_begin[threadIdx.x] = info->act_end[threadIdx.x] = 0;  // act_end counts first
-        info->min_row[threadIdx.x] = INT_MAX;
-        info->max_row[threadIdx.x] = -1;
-    }
-    if (threadIdx.x == 0) {
-        int32_t s = 0;
-        for (int d = 0; d < kNumDims; d++) {
-            const int32_t c = info->col_end[d];
-            info->col_begin[d] = s;
-            s += c;
-            info->col_end[d] = s;
+        int64_t run = 0;
+        for (int k = 0; k < 128; k++) {
+            const int64_t v = s_sum[k][threadIdx.x];
+            s_sum[k][threadIdx.x] = run;
+            run += v;
         }
+        s_total[threadIdx.x] = run;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) dim_ranges(s_total, &ctl->info);
+    int64_t run = s_sum[c][d];
+    for (int q = 0; q < d; q++) run += s_total[q];
+    for (int64_t b = b0; b < b1; b++) {
+        const int32_t v = dimcnt[b * kNumDims + d];
+        dimcnt[b * kNumDims + d] = int32_t(run);
+        run += v;
     }
 }
 
-// stable rank of each column inside its dimension -> reordered index
-// Also starts the init passes' per-column state of reordered column idx: no
-// leftmost column yet, no pivot owner, not cleared, not negative; and records
-// its length (rlen, read in this kernel's coalesced pass over col_ptr, so the
-// slot scan that follows reads it in reordered order without gathers).
+// Stable rank of each column inside its dimension -> reordered index.  Also
+// starts the init passes' per-column state of reordered column idx: no leftmost
+// column yet, no pivot owner, not cleared, not negative; and, unless every column
+// is short, records its length for the slot scan that follows.
 __global__ void __launch_bounds__(kPartThreads) k_dim_assign(const int32_t* dims, const int64_t* colptr, int64_t n,
-                                                             const int32_t* dimcnt, const DimInfo* info,
+                                                             int64_t nb, const int32_t* dimcnt, Ctl* ctl,
                                                              int32_t* newidx, int32_t* perm, int32_t* rdim,
                                                              int32_t* rlen, int32_t* leftmost, uint64_t* pivot,
                                                              uint8_t* cleared, uint8_t* negative) {
-    __shared__ int wcnt[kPartThreads / 32][kNumDims];
+    if (ctl->err) return;
+    constexpr int kWarps = kPartThreads / 32;
+    __shared__ int s_warp[kWarps][kNumDims];
+    __shared__ int64_t s_base[kNumDims], s_total[kNumDims];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int64_t j = int64_t(blockIdx.x) * kPartThreads + threadIdx.x;
-    int d = (j < n) ? dims[j] : -1;
-    if (d > kMaxDim) d = -1;
-    unsigned my_ballot = 0;
+    const int64_t tile = blockIdx.x;
+    const bool all_short = ctl->max_len <= kShortLen;
+    if (tile == 0 && threadIdx.x == 0 && all_short) ctl->arena_top = (unsigned long long)(kShortSlot * n);
+    const int64_t j0 = tile * kPartTile + wid * (32 * kPartRounds) + lane;
+    int d[kPartRounds], r[kPartRounds];
 #pragma unroll
-    for (int v = 0; v < kNumDims; v++) {
-        unsigned b = __ballot_sync(kFull, d == v);
-        if (d == v) my_ballot = b;
-        if (lane == 0) wcnt[wid][v] = __popc(b);
+    for (int k = 0; k < kPartRounds; k++) d[k] = j0 + 32 * k < n ? dims[j0 + 32 * k] : -1;
+    if (nb <= kInlineTiles) {  // warp q: dimension q
+        int64_t before = 0, total = 0;
+        for (int64_t b = lane; b < nb; b += 32) {
+            const int64_t v = dimcnt[b * kNumDims + wid];
+            total += v;
+            if (b < tile) before += v;
+        }
+        before = warp_sum(before);
+        total = warp_sum(total);
+        if (lane == 0) {
+            s_base[wid] = before;
+            s_total[wid] = total;
+        }
+    } else if (threadIdx.x < kNumDims) {
+        s_base[threadIdx.x] = dimcnt[tile * kNumDims + threadIdx.x];
     }
+    // rank within the warp's 256 columns, and the warp's counts
+    int run[kNumDims] = {};
+#pragma unroll
+    for (int k = 0; k < kPartRounds; k++) {
+        r[k] = 0;
+#pragma unroll
+        for (int q = 0; q < kNumDims; q++) {
+            const unsigned m = __ballot_sync(kFull, d[k] == q);
+            if (d[k] == q) r[k] = run[q] + __popc(m & lanemask_lt());
+            run[q] += __popc(m);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kNumDims; q++)
+        if (lane == q) s_warp[wid][q] = run[q];
     __syncthreads();
-    if (d >= 0) {
-        int r = __popc(my_ballot & lanemask_lt());
-        for (int w = 0; w < wid; w++) r += wcnt[w][d];
-        int32_t idx = info->col_begin[d] + dimcnt[int64_t(blockIdx.x) * kNumDims + d] + r;
+    if (nb <= kInlineTiles) {
+        if (tile == 0 && threadIdx.x == 0) dim_ranges(s_total, &ctl->info);
+        if (threadIdx.x < kNumDims) {
+            int64_t at = s_base[threadIdx.x];
+            for (int q = 0; q < threadIdx.x; q++) at += s_total[q];
+            s_base[threadIdx.x] = at;
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < kPartRounds; k++) {
+        if (d[k] < 0) continue;
+        const int64_t j = j0 + 32 * k;
+        int64_t at = s_base[d[k]] + r[k];
+        for (int w = 0; w < wid; w++) at += s_warp[w][d[k]];
+        const int32_t idx = int32_t(at);
         newidx[j] = idx;
         perm[idx] = int32_t(j);
-        rdim[idx] = d;
-        const int64_t len = colptr[j + 1] - colptr[j];  // validated: 0 <= len <= kMaxColLen
-        rlen[idx] = int32_t(len < 0 ? 0 : (len > kMaxColLen ? kMaxColLen : len));
+        rdim[idx] = d[k];
+        if (!all_short) rlen[idx] = int32_t(colptr[j + 1] - colptr[j]);
         leftmost[idx] = INT_MAX;
         pivot[idx] = kNoOwner;
         cleared[idx] = 0;
@@ -277,74 +330,108 @@ __global__ void __launch_bounds__(kPartThreads) k_dim_assign(const int32_t* dims
 // col_ptr and the faces are read in order and each slot is written whole.
 // With `lows` it also does the first init pass (include/kernel.h:444-457):
 // the column's lowest row, and each row's leftmost column by atomicMin (the
-// stable reorder keeps a column's rows ascending).
+// stable reorder keeps a column's rows ascending), read first: the columns of a
+// row come roughly in order, so most find an earlier one there.  Short columns
+// go through registers and are stored as two 16-byte halves of their slot; their
+// descriptors are left to the compression unless write_desc asks for them (they are
+// read before it, or also when it does not run).
 __global__ void k_scatter_cols(int64_t n, const int64_t* colptr, const int32_t* rows, const int32_t* dims,
-                               const int32_t* newidx, const int64_t* off, const DimInfo* info, int32_t* arena,
-                               uint64_t* desc, int32_t* low, int32_t* leftmost, bool lows, int* err) {
+                               const int32_t* newidx, const int64_t* off, Ctl* ctl, int32_t* arena,
+                               uint64_t* desc, int32_t* low, int32_t* leftmost, bool lows, bool write_desc) {
+    if (ctl->err & ~ERRB_FACES) return;
     __shared__ int32_t s_beg[kNumDims], s_end[kNumDims];
     if (threadIdx.x < kNumDims) {
-        s_beg[threadIdx.x] = info->col_begin[threadIdx.x];
-        s_end[threadIdx.x] = info->col_end[threadIdx.x];
+        s_beg[threadIdx.x] = ctl->info.col_begin[threadIdx.x];
+        s_end[threadIdx.x] = ctl->info.col_end[threadIdx.x];
     }
     __syncthreads();
+    const bool all_short = ctl->max_len <= kShortLen;
     for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < n; j += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t b = colptr[j], e = colptr[j + 1];
-        const int64_t len = e - b;
+        const int64_t b = colptr[j], len = colptr[j + 1] - b;
         const int32_t i = newidx[j];
-        const int64_t o = off[i];
+        const int64_t o = all_short ? int64_t(kShortSlot) * i : off[i];
         const int dj = dims[j];
         const int32_t fb = dj > 0 ? s_beg[dj - 1] : 0, fe = dj > 0 ? s_end[dj - 1] : 0;
-        bool bad = len < 0 || len > kMaxColLen;
-        int32_t prev = -1, last = -1;
-        int32_t* data = arena + o + kHdr;
-        for (int64_t k = 0; k < len && !bad; k++) {
-            const int32_t r = rows[b + k];
-            if (r < 0 || r >= n || r <= prev) { bad = true; break; }
-            const int32_t x = newidx[r];
-            if (x < fb || x >= fe) { bad = true; break; }
-            prev = r;
-            data[k] = x;
-            last = x;
-        }
-        if (bad) {
-            atomicOr(err, ERRB_BAD_INPUT);
-            desc[i] = pack_desc(uint64_t(o), 0);
-            *reinterpret_cast<int4*>(arena + o) = make_int4(0, int32_t(i), 0, 0);
-            if (lows) low[i] = -1;
-        } else {
-            for (int64_t k = len; k < pad4(len); k++) data[k] = INT_MAX;
-            desc[i] = pack_desc(uint64_t(o), uint32_t(len));
-            *reinterpret_cast<int4*>(arena + o) = make_int4(int32_t(len), int32_t(i), 0, 0);
-            if (lows) {
-                low[i] = len ? last : -1;
-                for (int64_t k = 0; k < len; k++) atomicMin(&leftmost[data[k]], int32_t(i));
+        bool bad = false;
+        int32_t last = -1;
+        if (all_short) {
+            int32_t r[kShortLen], x[kShortLen];
+#pragma unroll
+            for (int k = 0; k < kShortLen; k++) r[k] = k < len ? rows[b + k] : INT_MAX;
+#pragma unroll
+            for (int k = 0; k < kShortLen; k++) {
+                x[k] = INT_MAX;
+                if (k < len) {
+                    if (r[k] < 0 || r[k] >= n || (k > 0 && r[k] <= r[k - 1])) bad = true;
+                    else x[k] = newidx[r[k]];
+                }
             }
+#pragma unroll
+            for (int k = 0; k < kShortLen; k++)
+                if (k < len && !bad) {
+                    if (x[k] < fb || x[k] >= fe) bad = true;
+                    last = x[k];
+                }
+            const int32_t m = bad ? 0 : int32_t(len);
+            *reinterpret_cast<int4*>(arena + o) = make_int4(m, i, 0, 0);
+            *reinterpret_cast<int4*>(arena + o + kHdr) =
+                bad ? make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX) : make_int4(x[0], x[1], x[2], x[3]);
+            if (write_desc) desc[i] = pack_desc(uint64_t(o), uint32_t(m));
+            if (lows && !bad) {
+#pragma unroll
+                for (int k = 0; k < kShortLen; k++)
+                    if (k < len && __ldcg(leftmost + x[k]) > i) atomicMin(&leftmost[x[k]], i);
+            }
+        } else {
+            int32_t prev = -1;
+            int32_t* data = arena + o + kHdr;
+            for (int64_t k = 0; k < len && !bad; k++) {
+                const int32_t r = rows[b + k];
+                if (r < 0 || r >= n || r <= prev) { bad = true; break; }
+                const int32_t x = newidx[r];
+                if (x < fb || x >= fe) { bad = true; break; }
+                prev = r;
+                data[k] = x;
+                last = x;
+            }
+            const int64_t m = bad ? 0 : len;
+            for (int64_t k = m; k < pad4(m); k++) data[k] = INT_MAX;
+            *reinterpret_cast<int4*>(arena + o) = make_int4(int32_t(m), i, 0, 0);
+            desc[i] = pack_desc(uint64_t(o), uint32_t(m));
+            if (lows && !bad)
+                for (int64_t k = 0; k < len; k++)
+                    if (__ldcg(leftmost + data[k]) > i) atomicMin(&leftmost[data[k]], i);
         }
+        if (bad) atomicOr(&ctl->err, ERRB_FACES);
+        if (lows) low[i] = bad || len == 0 ? -1 : last;
     }
 }
 
-int reorder(Device& D, bool lows, cudaStream_t s, cudaEvent_t assigned) {
-    const int64_t n = D.n;
-    const int64_t nb = (n + kPartThreads - 1) / kPartThreads;
-    k_dim_count<<<unsigned(nb), kPartThreads, 0, s>>>(D.in_dims, n, D.dimcnt, D.err);
-    k_dim_offsets<<<kNumDims, 1024, 0, s>>>(D.dimcnt, nb, D.diminfo);
-    k_dim_starts<<<1, 32, 0, s>>>(D.diminfo);
+int reorder(Device& D, bool lows, bool write_desc, cudaStream_t s, cudaEvent_t assigned) {
+    const int64_t n = D.n, nb = part_tiles(n);
+    int launches = 3;
+    if (nb > kInlineTiles) {
+        k_dim_offsets<<<1, 1024, 0, s>>>(D.dimcnt, nb, D.ctl);
+        launches++;
+    }
     // the active list is built later: until then its buffer holds the reordered lengths
     int32_t* rlen = D.active;
-    k_dim_assign<<<unsigned(nb), kPartThreads, 0, s>>>(D.in_dims, D.in_colptr, n, D.dimcnt, D.diminfo, D.newidx,
-                                                       D.perm, D.dim, rlen, D.leftmost, D.pivot, D.cleared,
-                                                       D.negative);
+    k_dim_assign<<<unsigned(nb), kPartThreads, 0, s>>>(D.in_dims, D.in_colptr, n, nb, D.dimcnt, D.ctl, D.newidx, D.perm,
+                                                       D.dim, rlen, D.leftmost, D.pivot, D.cleared, D.negative);
     if (assigned) cudaEventRecord(assigned, s);
-    // padded column offsets in reordered order
+    // padded column offsets in reordered order, unless every column is short (or
+    // the input is refused: the limit then skips it too)
     int64_t* off = D.scratch64;
-    unsigned long long* top = D.arena_top;
-    scan([=] __device__(int64_t i) -> int64_t { return slot_ints(rlen[i]); },
-         [=] __device__(int64_t i, int64_t pre, int64_t) { off[i] = pre; }, n, D.blk, s,
-         [=] __device__(int64_t total) { *top = (unsigned long long)total; });
+    Ctl* ctl = D.ctl;
+    bool zeroed;
+    int64_t* blk = scan_region(D, 0, &zeroed);
+    scan([=] __device__(int64_t i) -> int64_t { return slot_ints(max(rlen[i], 0)); },
+         [=] __device__(int64_t i, int64_t pre, int64_t) { off[i] = pre; }, n, blk, s,
+         [=] __device__(int64_t total) { ctl->arena_top = (unsigned long long)total; }, zeroed, &ctl->max_len, kShortLen);
     k_scatter_cols<<<grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256), 256, 0, s>>>(
-        n, D.in_colptr, D.in_rows, D.in_dims, D.newidx, off, D.diminfo, D.arena, D.desc, D.low, D.leftmost, lows,
-        D.err);
-    return 6;
+        n, D.in_colptr, D.in_rows, D.in_dims, D.newidx, off, D.ctl, D.arena, D.desc, D.low, D.leftmost, lows,
+        write_desc);
+    return launches;
 }
 
 // ------------------------------------------------------------- init passes
@@ -360,26 +447,51 @@ __global__ void k_init_low(int64_t n, const int32_t* arena, const uint64_t* desc
     }
 }
 
+// A column's slot, length and entries (short columns: both halves of the slot in
+// two 16-byte loads, no descriptor).
+struct ColRef {
+    int64_t slot;
+    int len;
+    int4 q;  // the entries of a short column
+    __device__ __forceinline__ int32_t at(const int32_t* arena, int k, bool all_short) const {
+        return all_short ? (k == 0 ? q.x : k == 1 ? q.y : k == 2 ? q.z : q.w) : arena[slot + kHdr + k];
+    }
+};
+__device__ __forceinline__ ColRef col_ref(int64_t i, const int32_t* arena, const uint64_t* desc, bool all_short) {
+    ColRef c;
+    if (all_short) {
+        c.slot = int64_t(kShortSlot) * i;
+        c.len = arena[c.slot];
+        c.q = *reinterpret_cast<const int4*>(arena + c.slot + kHdr);
+    } else {
+        const uint64_t d = desc[i];
+        c.slot = int64_t(desc_off(d));
+        c.len = int(desc_len(d));
+        c.q = make_int4(0, 0, 0, 0);
+    }
+    return c;
+}
+
 __global__ void k_init_apparent(int64_t n, const int32_t* arena, const uint64_t* desc, const int32_t* low,
                                 const int32_t* leftmost, uint64_t* pivot, uint8_t* cleared, uint8_t* negative,
-                                long long* counters) {
+                                Ctl* ctl) {
+    if (ctl->err) return;
+    const bool all_short = ctl->max_len <= kShortLen;
     long long app = 0;
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        int32_t l = low[i];
+        const int32_t l = low[i];
         if (l < 0) continue;
         cleared[l] = 1;  // the youngest facet of any simplex is positive
-        uint64_t d = desc[i];
+        const ColRef c = col_ref(i, arena, desc, all_short);
         if (leftmost[l] == int32_t(i)) {
-            pivot[l] = pv_pack(int32_t(i), desc_off(d));  // no earlier column can ever reach row l
+            pivot[l] = pv_pack(int32_t(i), uint64_t(c.slot));  // no earlier column can ever reach row l
             app++;
         }
-        const int32_t* c = arena + desc_off(d) + kHdr;
-        uint32_t len = desc_len(d);
-        for (uint32_t k = 0; k < len; k++)
-            if (leftmost[c[k]] == int32_t(i)) { negative[i] = 1; break; }
+        for (int k = 0; k < c.len; k++)
+            if (leftmost[c.at(arena, k, all_short)] == int32_t(i)) { negative[i] = 1; break; }
     }
     app = warp_sum(app);
-    if ((threadIdx.x & 31) == 0 && app) cnt_add(&counters[CNT_APPARENT], app);
+    if ((threadIdx.x & 31) == 0 && app) cnt_add(&ctl->counters[CNT_APPARENT], app);
 }
 
 // Clears positive columns and removes negative rows in place.  With `app` it
@@ -392,8 +504,11 @@ __global__ void k_init_apparent(int64_t n, const int32_t* arena, const uint64_t*
 // into info, whose bounds must start at INT_MAX / -1.
 __global__ void k_init_compress(int64_t n, int32_t* arena, uint64_t* desc, int32_t* low, const uint64_t* pivot,
                                 const uint8_t* cleared, const uint8_t* negative, uint8_t* state,
-                                const uint8_t* dropped, bool keep_rows, int4* app, const int32_t* rinfo,
-                                DimInfo* info, long long* counters, int* err) {
+                                const uint8_t* dropped, bool keep_rows, int4* app, const int32_t* rinfo, Ctl* ctl) {
+    if (ctl->err) return;
+    DimInfo* info = &ctl->info;
+    long long* counters = ctl->counters;
+    const bool all_short = ctl->max_len <= kShortLen;
     __shared__ int smin[kNumDims], smax[kNumDims], sact[kNumDims];
     if (threadIdx.x < kNumDims) {
         smin[threadIdx.x] = INT_MAX;
@@ -404,60 +519,71 @@ __global__ void k_init_compress(int64_t n, int32_t* arena, uint64_t* desc, int32
     long long ncl = 0, nact = 0;
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
         if (app && pivot[i] == kNoOwner) app[i] = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
-        uint64_t d = desc[i];
-        int32_t* hdr = arena + desc_off(d);
-        int32_t* c = hdr + kHdr;
-        uint32_t len = desc_len(d);
-        if (dropped && dropped[i]) {
-            desc[i] = pack_desc(desc_off(d), 0);
-            hdr[0] = 0;
+        const bool drop = dropped && dropped[i];
+        if (drop || cleared[i]) {
+            const int64_t slot = all_short ? int64_t(kShortSlot) * i : int64_t(desc_off(desc[i]));
+            const int32_t l = low[i];
+            if (!drop && l >= 0 && pv_col(pivot[l]) == int32_t(i)) atomicOr(&ctl->err, ERRB_FACES);  // positive and negative
+            desc[i] = pack_desc(uint64_t(slot), 0);
+            arena[slot] = 0;
             low[i] = -1;
-            state[i] = ST_DROPPED;
+            state[i] = drop ? ST_DROPPED : ST_CLEARED;
+            ncl += !drop;
             continue;
         }
-        if (cleared[i]) {
-            if (len && pv_col(pivot[low[i]]) == int32_t(i)) atomicOr(err, ERRB_BAD_INPUT);  // positive and negative
-            desc[i] = pack_desc(desc_off(d), 0);
-            hdr[0] = 0;
-            low[i] = -1;
-            state[i] = ST_CLEARED;
-            ncl++;
-            continue;
-        }
-        uint32_t m = 0;
-        if (keep_rows) {
-            m = len;
+        ColRef c = col_ref(i, arena, desc, all_short);
+        int m = 0;
+        int32_t l = -1, first = INT_MAX;
+        int4 v = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);  // the inline column, should it own its row
+        if (all_short) {
+            int32_t y[kShortLen] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX};
+#pragma unroll
+            for (int k = 0; k < kShortLen; k++) {
+                const int32_t r = k == 0 ? c.q.x : k == 1 ? c.q.y : k == 2 ? c.q.z : c.q.w;
+                if (k < c.len && (keep_rows || !negative[r])) {
+                    if (m == 0) y[0] = r;
+                    else if (m == 1) y[1] = r;
+                    else if (m == 2) y[2] = r;
+                    else y[3] = r;
+                    m++;
+                    l = r;
+                }
+            }
+            first = y[0];
+            arena[c.slot] = m;
+            *reinterpret_cast<int4*>(arena + c.slot + kHdr) = make_int4(y[0], y[1], y[2], y[3]);
+            v = make_int4(m - 1, m > 1 ? y[0] : INT_MAX, m > 2 ? y[1] : INT_MAX, m > 3 ? y[2] : INT_MAX);
         } else {
-            for (uint32_t k = 0; k < len; k++) {
-                int32_t r = c[k];
-                if (!negative[r]) c[m++] = r;
+            int32_t* col = arena + c.slot + kHdr;
+            if (keep_rows) {
+                m = c.len;
+            } else {
+                for (int k = 0; k < c.len; k++) {
+                    const int32_t r = col[k];
+                    if (!negative[r]) col[m++] = r;
+                }
+            }
+            for (int k = m; k < c.len; k++) col[k] = INT_MAX;
+            arena[c.slot] = m;
+            if (m) {
+                l = col[m - 1];
+                first = col[0];
+                if (m <= 4) v = make_int4(m - 1, m > 1 ? col[0] : INT_MAX, m > 2 ? col[1] : INT_MAX, m > 3 ? col[2] : INT_MAX);
             }
         }
-        for (uint32_t k = m; k < len; k++) c[k] = INT_MAX;
-        desc[i] = pack_desc(desc_off(d), m);
-        hdr[0] = int32_t(m);
-        int32_t l = m ? c[m - 1] : -1;
+        desc[i] = pack_desc(uint64_t(c.slot), uint32_t(m));
         low[i] = l;
-        uint8_t st = (m == 0) ? ST_ZERO : (pv_col(pivot[l]) == int32_t(i) ? ST_OWNER : ST_ACTIVE);
+        const uint8_t st = (m == 0) ? ST_ZERO : (pv_col(pivot[l]) == int32_t(i) ? ST_OWNER : ST_ACTIVE);
         state[i] = st;
         if (rinfo && m > 0) {
             const int dm = rinfo[i];
-            atomicMin(&smin[dm], c[0]);
+            atomicMin(&smin[dm], first);
             if (st == ST_ACTIVE) {
                 atomicMax(&smax[dm], l + 1);
                 atomicAdd(&sact[dm], 1);
             }
         }
-        if (app && st == ST_OWNER) {
-            int4 v = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
-            if (m <= 4) {
-                v.x = int(m) - 1;
-                if (m > 1) v.y = c[0];
-                if (m > 2) v.z = c[1];
-                if (m > 3) v.w = c[2];
-            }
-            app[l] = v;
-        }
+        if (app && st == ST_OWNER) app[l] = v;
         nact += (st == ST_ACTIVE);
     }
     ncl = warp_sum(ncl);
@@ -511,8 +637,7 @@ int init_passes(Device& D, bool lows_done, cudaStream_t s) {
     const int64_t n = D.n;
     const unsigned g = grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256);
     if (!lows_done) k_init_low<<<g, 256, 0, s>>>(n, D.arena, D.desc, D.low, D.leftmost);
-    k_init_apparent<<<g, 256, 0, s>>>(n, D.arena, D.desc, D.low, D.leftmost, D.pivot, D.cleared, D.negative,
-                                      D.counters);
+    k_init_apparent<<<g, 256, 0, s>>>(n, D.arena, D.desc, D.low, D.leftmost, D.pivot, D.cleared, D.negative, D.ctl);
     return lows_done ? 1 : 2;
 }
 
@@ -521,8 +646,7 @@ int init_compress(Device& D, const uint8_t* dropped, bool keep_rows, bool final,
     // the row bounds go to the DimInfo through a few atomics per block: few blocks
     const unsigned g = grid_for(n, 256) > 4096 ? 4096 : grid_for(n, 256);
     k_init_compress<<<g, 256, 0, s>>>(n, D.arena, D.desc, D.low, D.pivot, D.cleared, D.negative, D.state, dropped,
-                                      keep_rows, final ? D.app : nullptr, final ? D.dim : nullptr, D.diminfo,
-                                      D.counters, D.err);
+                                      keep_rows, final ? D.app : nullptr, final ? D.dim : nullptr, D.ctl);
     return 1;
 }
 
@@ -565,11 +689,13 @@ int active_list(Device& D, bool rows_done, cudaStream_t s) {
     const uint8_t* state = D.state;
     int32_t* act = D.active;
     DimInfo* info = D.diminfo;
+    bool zeroed;
+    int64_t* blk = scan_region(D, 1, &zeroed);
     scan([=] __device__(int64_t i) -> ScanClass { return {uint8_t(state[i] == ST_ACTIVE ? 1 : 0)}; },
          [=] __device__(int64_t i, int64_t pre, ScanClass v) {
              if (v.c) act[pre] = int32_t(i);
          },
-         n, D.blk, s,
+         n, blk, s,
          [=] __device__(int64_t) {
              int32_t at = 0;
              // reordered columns ascend with the dimension, or descend (dual)
@@ -580,7 +706,8 @@ int active_list(Device& D, bool rows_done, cudaStream_t s) {
                  info->act_begin[d] = at;
                  info->act_end[d] = at += c;
              }
-         });
+         },
+         zeroed);
     return rows_done ? 1 : 3;
 }
 
@@ -653,8 +780,10 @@ int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s) {
     const int64_t n = D.n;
     longlong2* pairs = reinterpret_cast<longlong2*>(D.pairs);
     const PairsOut o{n, D.newidx, D.perm, D.pivot, D.state, pairs, D.ess, D.counters};
+    bool zeroed;
+    int64_t* blk = scan_region(D, 2, &zeroed);
     if (!dual) {
-        scan(PairsValue{o}, PairsSink{o}, n, D.blk, s, PairsDone{o});
+        scan(PairsValue{o}, PairsSink{o}, n, blk, s, PairsDone{o}, zeroed);
         return 1;
     }
     const unsigned g = grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256);
@@ -670,7 +799,7 @@ int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s) {
              if (v.c == 1) pairs[pre & kBirths] = make_longlong2(j, death_of[j]);
              else if (v.c == 2) ess[pre >> kScanClassShift] = j;
          },
-         n, D.blk, s, PairsDone{o});
+         n, blk, s, PairsDone{o}, zeroed);
     return 3 + (dropped ? 1 : 0);
 }
 

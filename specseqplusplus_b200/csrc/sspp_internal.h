@@ -55,6 +55,7 @@ enum : int {
     ERRB_TIMEOUT = 4,
     ERRB_LEN = 8,       // a column exceeded kMaxColLen
     ERRB_CHECK = 16,    // a self-check of the reduction failed (bad index skipped)
+    ERRB_FACES = 32,    // malformed input faces, found while the columns are copied
 };
 
 // Per-dimension summary after the init passes (in reordered numbering).
@@ -86,6 +87,28 @@ enum CounterIdx {
     CNT_NUM
 };
 
+// Small device state of a run, one block of memory: cleared at once before the
+// init passes and read back at once.
+constexpr int kCtlSteps = 16;  // spectral-sequence steps whose counters fit here
+constexpr int kStepCtr = 8;    // counters per step (see ReduceArgs::ctr)
+struct Ctl {
+    DimInfo info;
+    long long counters[CNT_NUM];
+    unsigned long long arena_top;
+    unsigned long long dimtot[kNumDims];  // input columns per dimension (validation pass)
+    int err;
+    int max_len;      // longest input column (validation pass)
+    int pool_tail;    // CTA-tier pool entries
+    int heavy_done;   // pool columns the CTA tier has finished
+    int step[kCtlSteps * kStepCtr];
+};
+
+// Columns of at most 4 entries (every simplicial complex up to dimension 3): when
+// no input column is longer, column i's slot is ints [8 i, 8 i + 8) of the arena,
+// and no offsets are computed or read.
+constexpr int kShortLen = 4;
+constexpr int kShortSlot = 8;
+
 struct Device {
     int64_t n = 0;        // columns
     int64_t nnz = 0;
@@ -114,15 +137,20 @@ struct Device {
     int32_t* active = nullptr;
     int32_t* runlist = nullptr;  // [n] a step's runnable columns (warp tier input)
     // block-scan scratch
-    int64_t* blk = nullptr;      // block sums
+    // one buffer: Ctl, then three regions of tile states (slot offsets and any
+    // other scan; active list; pair lists), cleared together before the init passes
+    Ctl* ctl = nullptr;
+    int64_t* blk = nullptr;      // region 0
+    int64_t blk_stride = 0;      // entries per region
+    unsigned blk_zero = 0;       // regions still as cleared (bits)
+    bool steps_zero = false;     // Ctl::pool_tail, heavy_done and step still as cleared
     int64_t cap_blk = 0;
     int32_t* dimcnt = nullptr;   // [nblocks * kNumDims]
     int64_t cap_dimcnt = 0;
     DimInfo* diminfo = nullptr;
-    unsigned long long* dimtot = nullptr;  // [kNumDims] input columns per dimension (validation pass)
     int* err = nullptr;
     long long* counters = nullptr;
-    int* step_ctr = nullptr;     // per-step work counters (8 ints per step)
+    int* step_ctr = nullptr;     // per-step work counters (kStepCtr ints per step) beyond Ctl's
     int32_t* heavy = nullptr;    // pool of columns handed to the CTA tier, appended step after step
     int64_t pool_cap = 0;
     int* pool_tail = nullptr;

@@ -10,10 +10,11 @@ void fill_i32(int32_t* p, int32_t v, int64_t n, cudaStream_t s);
 void fill_i64(int64_t* p, int64_t v, int64_t n, cudaStream_t s);
 
 // input (filtration order) -> dimension-sorted padded arena layout; writes
-// D.newidx, D.perm, D.dim, D.desc, D.diminfo->col_begin/col_end; D.blk[scan
-// total] holds the arena ints used.
+// D.newidx, D.perm, D.dim, D.desc, D.diminfo->col_begin/col_end and
+// D.arena_top (the arena ints used).
 // Each launcher returns the number of kernels it launched.
-int validate(Device& D, cudaStream_t s);  // sets ERRB_BAD_INPUT
+int64_t part_tiles(int64_t n);            // tiles of the validation and the reorder (D.dimcnt: kNumDims each)
+int validate(Device& D, cudaStream_t s);  // sets ERRB_BAD_INPUT; the passes after it leave when it is set
 // k complexes copied side by side (cstart/estart: k+1 column / entry starts on
 // the device): shifts each one's face indices and col_ptr entries; *d_bad = 1
 // when a face index lies outside its own complex
@@ -22,7 +23,9 @@ int batch_rebase(int64_t n, int64_t nnz, int32_t k, const int64_t* d_cstart, con
 // lows: also the lowest rows and leftmost columns (the first init pass);
 // assigned: recorded once perm / newidx / dim are written (before the columns
 // are scattered), or null
-int reorder(Device& D, bool lows, cudaStream_t s, cudaEvent_t assigned = nullptr);
+// write_desc: also the descriptors of short columns, which init_compress writes
+// otherwise (needed when anything reads them before it)
+int reorder(Device& D, bool lows, bool write_desc, cudaStream_t s, cudaEvent_t assigned = nullptr);
 
 // per-complex slice starts (k+1 each) of the sorted pairs and essentials
 int batch_bounds(int32_t k, const int64_t* d_cstart, int64_t npairs, const int64_t* pairs, int64_t ness,
@@ -104,12 +107,14 @@ cudaError_t reduce_queue_launch(const Device& D, int cap1, int cap2, int threads
 
 cudaError_t reduce_configure(int cap1, int cap2, int heavy_threads, int* light_blocks_per_sm,
                              int* heavy_blocks_per_sm);
-// One step's light tier in two launches: k_light_filter lists the window's
-// (active[beg, end)) runnable columns in D.runlist, then warps reduce them.
+// One step's light tier: k_light_filter lists the window's (active[beg, end))
+// runnable columns in D.runlist, then warps reduce them.
+// A step that takes the whole band (minrow INT32_MIN) takes the window as it is.
 // ctr: the step's 8 counters; the launch's last block also marks the step's
-// CTA-tier pool slice (ctr[2], and ctr_next[1] of the next step when given)
-void reduce_light_launch(const Device& D, int32_t beg, int32_t end, int32_t minrow, int cap, int* ctr, int* ctr_next,
-                         int filter_grid, int grid, cudaStream_t s);
+// CTA-tier pool slice (ctr[2], and ctr_next[1] of the next step when given).
+// Returns the kernels launched.
+int reduce_light_launch(const Device& D, int32_t beg, int32_t end, int32_t minrow, int cap, int* ctr, int* ctr_next,
+                        int filter_grid, int grid, cudaStream_t s);
 void reduce_heavy_launch(const Device& D, int cap, int threads, int* ctr, int grid, cudaStream_t s);
 
 }  // namespace sspp

@@ -55,6 +55,7 @@
 // block, 0.36 ms by the engine's passes.
 #include <algorithm>
 #include <climits>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -259,22 +260,13 @@ using namespace sspp;
 
 constexpr int kCap1 = 64;          // warp-tier column capacity (ints), as the context API's bound
 constexpr int kCap2 = 8192;        // CTA-tier column capacity
-constexpr int kStepInts = 8;       // counters per dimension's step (ReduceArgs::ctr)
 constexpr int64_t kGuard = 8192;   // ints after the arena: staging reads a first pass beyond a slot
-
-// what the host reads back, in one copy
-struct Status {
-    DimInfo info;
-    long long counters[CNT_NUM];
-    int err;
-    int pad[3];
-};
 
 // Engine arrays carved out of the scratch array; false when they leave too
 // little for the arena.  Buffers whose lifetimes do not meet share memory: the
 // pairs pass's death list lies in the inline columns, its essentials in the
 // column descriptors.
-bool carve(int32_t* scratch, int64_t n, int64_t nnz, Device& D, Status** status) {
+bool carve(int32_t* scratch, int64_t n, int64_t nnz, Device& D) {
     char* p = reinterpret_cast<char*>(scratch);
     char* const end = p + sizeof(int32_t) * kScratchInts;
     auto take = [&](auto*& out, int64_t count) {
@@ -282,12 +274,10 @@ bool carve(int32_t* scratch, int64_t n, int64_t nnz, Device& D, Status** status)
         out = reinterpret_cast<T*>(p);
         p += (sizeof(T) * size_t(count) + 255) & ~size_t(255);
     };
-    take(*status, 1);
-    take(D.dimtot, kNumDims);
-    take(D.arena_top, 1);
-    take(D.pool_tail, 1);
-    take(D.heavy_done, 1);
-    take(D.step_ctr, kStepInts * (kNumDims + 1));
+    // cleared together: the control block and the scans' tile states
+    take(D.ctl, 1);
+    D.blk_stride = scan_blocks(n) + 2;
+    take(D.blk, 3 * D.blk_stride);
     take(D.dim, n);
     take(D.perm, n);
     take(D.newidx, n);
@@ -302,17 +292,19 @@ bool carve(int32_t* scratch, int64_t n, int64_t nnz, Device& D, Status** status)
     take(D.active, n);
     take(D.runlist, n);
     take(D.app, n);
-    take(D.blk, scan_blocks(n) + 2);
-    take(D.dimcnt, ((n + 255) / 256 + 1) * kNumDims);
+    take(D.dimcnt, (part_tiles(n) + 1) * kNumDims);
     D.pool_cap = n;
     take(D.heavy, D.pool_cap);
     D.arena = reinterpret_cast<int32_t*>(p);
     D.arena_cap = p < end ? ((end - p) / int64_t(sizeof(int32_t)) - kGuard) & ~int64_t(3) : 0;
     D.n = n;
     D.nnz = nnz;
-    D.diminfo = &(*status)->info;
-    D.counters = (*status)->counters;
-    D.err = &(*status)->err;
+    D.diminfo = &D.ctl->info;
+    D.counters = D.ctl->counters;
+    D.arena_top = &D.ctl->arena_top;
+    D.err = &D.ctl->err;
+    D.pool_tail = &D.ctl->pool_tail;
+    D.heavy_done = &D.ctl->heavy_done;
     D.death_of = reinterpret_cast<int64_t*>(D.app);
     D.ess = reinterpret_cast<int64_t*>(D.desc);
     // the input's slots, and as much again for the reduction's column versions
@@ -326,7 +318,7 @@ __global__ void k_check_complex(int64_t n, const uint64_t* pivot, const uint8_t*
 }
 
 // *npairs is written by a run that ends cleanly only.
-__global__ void k_store_npairs(const Status* st, int64_t room, int64_t* npairs) {
+__global__ void k_store_npairs(const Ctl* st, int64_t room, int64_t* npairs) {
     if (st->err == 0 && st->counters[CNT_ADD_INTS] <= room) *npairs = st->counters[CNT_NPAIRS];
 }
 
@@ -359,8 +351,7 @@ cudaError_t reduce_in_scratch(int32_t* scratch, int dev, int64_t n, int64_t nnz,
                               cudaStream_t s, bool* done) {
     *done = false;
     Device D;
-    Status* status = nullptr;
-    if (n < 1 || !carve(scratch, n, nnz, D, &status)) return cudaSuccess;
+    if (n < 1 || !carve(scratch, n, nnz, D)) return cudaSuccess;
     Launch shape;
     cudaError_t e = launch_shape(dev, &shape);
     if (e != cudaSuccess) return e;
@@ -368,38 +359,34 @@ cudaError_t reduce_in_scratch(int32_t* scratch, int dev, int64_t n, int64_t nnz,
     D.in_colptr = const_cast<int64_t*>(d_col_ptr);
     D.in_rows = const_cast<int32_t*>(d_rows);
     D.pairs = d_pairs;
-    Status h;
-    cudaMemsetAsync(status, 0, sizeof(Status), s);
-    validate(D, s);
-    cudaMemcpyAsync(&h.err, D.err, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-    if (h.err) return cudaSuccess;
-    reorder(D, true, s);
+    Ctl h;
+    cudaMemsetAsync(D.ctl, 0, size_t(reinterpret_cast<char*>(D.blk + 3 * D.blk_stride) - reinterpret_cast<char*>(D.ctl)), s);
+    D.blk_zero = 7;
+    validate(D, s);  // the passes leave when it finds a fault
+    reorder(D, true, false, s);
     init_passes(D, true, s);
     init_compress(D, nullptr, true, true, s);
     active_list(D, true, s);
-    cudaMemsetAsync(D.step_ctr, 0, sizeof(int) * kStepInts * (kNumDims + 1), s);
-    cudaMemsetAsync(D.pool_tail, 0, sizeof(int), s);
-    cudaMemcpyAsync(&h, status, sizeof(Status), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(&h, D.ctl, offsetof(Ctl, step), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
     if (h.err) return cudaSuccess;
-    int* ctr = D.step_ctr;
+    int* ctr = D.ctl->step;  // cleared with the control block, one step per dimension
     for (int d = kMaxDim; d >= 1; d--) {
         const int64_t b = h.info.act_begin[d], end = h.info.act_end[d], window = end - b;
         if (window <= 0) continue;
         const int grid = int(std::min<int64_t>((window + 3) / 4, int64_t(shape.sms) * shape.light));
         const int fgrid = int(std::min<int64_t>((window + 255) / 256, int64_t(shape.sms) * 8));
-        reduce_light_launch(D, int32_t(b), int32_t(end), INT32_MIN, kCap1, ctr, ctr + kStepInts, fgrid, grid, s);
+        reduce_light_launch(D, int32_t(b), int32_t(end), INT32_MIN, kCap1, ctr, ctr + kStepCtr, fgrid, grid, s);
         reduce_heavy_launch(D, kCap2, 256, ctr,
                             int(std::min<int64_t>(int64_t(shape.sms) * std::min(shape.heavy, 2), window)), s);
-        ctr += kStepInts;
+        ctr += kStepCtr;
     }
     k_check_complex<<<unsigned(std::min<int64_t>((n + 255) / 256, 4096)), 256, 0, s>>>(n, D.pivot, D.state, D.err);
     extract_pairs(D, 0, nullptr, s);
     const int64_t room = kScratchInts - (kCtl + 3 * n) - nnz;  // k_reduce_noalloc's room for fill-in
-    k_store_npairs<<<1, 1, 0, s>>>(status, room, d_npairs);
+    k_store_npairs<<<1, 1, 0, s>>>(D.ctl, room, d_npairs);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    cudaMemcpyAsync(&h, status, sizeof(Status), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(&h, D.ctl, offsetof(Ctl, step), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
     *done = h.err == 0 && h.counters[CNT_ADD_INTS] <= room;
     return cudaSuccess;

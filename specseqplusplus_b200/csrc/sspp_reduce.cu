@@ -64,7 +64,8 @@ struct ReduceArgs {
     uint8_t* cleared;
     int* ctr;             // per step: [0] chunk counter, [1] [2] heavy pool range, [3] heavy pull counter,
                           // [4] warp-tier blocks finished, [5] runnable columns listed by k_light_filter
-    const int* count;     // light tier: how many columns `active` lists
+    const int* count;     // light tier: how many columns `active` lists (null: `listed`)
+    int32_t listed;
     int* ctr_next;        // the next step's counters (its pool range starts where this step's ends), or null
     int32_t* heavy;       // heavy pool (columns handed to the CTA tier, appended in step order)
     int* pool_tail;
@@ -1247,7 +1248,7 @@ __global__ void __launch_bounds__(128, kLightMinBlocks) k_reduce_light(ReduceArg
     const int lane = g.rank(), gl = lane & (kGroup - 1), lead = lane & ~(kGroup - 1);
     int32_t* sw0 = smem + size_t(threadIdx.x >> 5) * (3 * A.cap + kHdr);
     int32_t* gbuf = rm.s + 2 * lead;  // 16 entries per group
-    const int count = __ldcg(A.count);
+    const int count = A.count ? __ldcg(A.count) : A.listed;
     const int warps = gridDim.x * (blockDim.x >> 5);
     // list entries a warp takes at a time: enough to keep its groups busy, few enough to share a short list
     const int chunk = max(4, min(32, count / (2 * warps)));
@@ -1917,6 +1918,7 @@ static ReduceArgs make_args(const Device& D, const int32_t* active, int32_t minr
     A.ctr = ctr;
     A.ctr_next = nullptr;
     A.count = nullptr;
+    A.listed = 0;
     A.heavy = D.heavy;
     A.pool_tail = D.pool_tail;
     A.heavy_done = D.heavy_done;
@@ -1929,14 +1931,23 @@ static ReduceArgs make_args(const Device& D, const int32_t* active, int32_t minr
     return A;
 }
 
-void reduce_light_launch(const Device& D, int32_t beg, int32_t end, int32_t minrow, int cap, int* ctr, int* ctr_next,
-                         int filter_grid, int grid, cudaStream_t s) {
-    k_light_filter<<<filter_grid, kFilterThreads, 0, s>>>(D.active, beg, end, minrow, D.state, D.cleared, D.low,
-                                                          D.runlist, ctr);
+int reduce_light_launch(const Device& D, int32_t beg, int32_t end, int32_t minrow, int cap, int* ctr, int* ctr_next,
+                        int filter_grid, int grid, cudaStream_t s) {
     ReduceArgs A = make_args(D, D.runlist, minrow, cap, ctr);
     A.ctr_next = ctr_next;
-    A.count = ctr + 5;
+    if (minrow == INT32_MIN) {
+        // every column that is still active is runnable, and the warps look at the
+        // flags themselves: no list (it took 3-15 us and a launch)
+        A.active = D.active + beg;
+        A.count = nullptr;
+        A.listed = end - beg;
+    } else {
+        k_light_filter<<<filter_grid, kFilterThreads, 0, s>>>(D.active, beg, end, minrow, D.state, D.cleared, D.low,
+                                                              D.runlist, ctr);
+        A.count = ctr + 5;
+    }
     k_reduce_light<<<grid, 128, light_smem_bytes(cap), s>>>(A);
+    return A.count ? 2 : 1;
 }
 
 void reduce_heavy_launch(const Device& D, int cap, int threads, int* ctr, int grid, cudaStream_t s) {

@@ -102,7 +102,9 @@ struct ScanLane<ScanClass> {
 };
 
 template <class F, class G, class H>
-__global__ void __launch_bounds__(kScanThreads) k_scan(F value, G sink, H done, int64_t n, int64_t nb, int64_t* blk) {
+__global__ void __launch_bounds__(kScanThreads) k_scan(F value, G sink, H done, int64_t n, int64_t nb, int64_t* blk,
+                                                       const int* skip_upto, int skip_limit) {
+    if (skip_upto && *skip_upto <= skip_limit) return;
     using Lane = ScanLane<decltype(value(int64_t(0)))>;
     constexpr int kWarps = kScanThreads / 32;
     __shared__ int64_t s_warp[kWarps];
@@ -178,18 +180,28 @@ struct ScanNoop {
 };
 
 // Scratch (blk) must hold scan_blocks(n) + 1 entries; the total is left in
-// blk[scan_blocks(n)].
+// blk[scan_blocks(n)].  zeroed: the entries are zero already.  A launch whose
+// *skip_upto turns out to be at most skip_limit does nothing.
 inline int64_t scan_blocks(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
 
 template <class F, class G, class H = ScanNoop>
-void scan(F value, G sink, int64_t n, int64_t* blk, cudaStream_t s, H done = H()) {
+void scan(F value, G sink, int64_t n, int64_t* blk, cudaStream_t s, H done = H(), bool zeroed = false,
+          const int* skip_upto = nullptr, int skip_limit = 0) {
     const int64_t nb = scan_blocks(n);
     if (nb == 0) {
         cudaMemsetAsync(blk, 0, sizeof(int64_t), s);
         return;
     }
-    if (nb > 1) cudaMemsetAsync(blk, 0, sizeof(int64_t) * size_t(nb), s);
-    k_scan<<<unsigned(nb), kScanThreads, 0, s>>>(value, sink, done, n, nb, blk);
+    if (nb > 1 && !zeroed) cudaMemsetAsync(blk, 0, sizeof(int64_t) * size_t(nb), s);
+    k_scan<<<unsigned(nb), kScanThreads, 0, s>>>(value, sink, done, n, nb, blk, skip_upto, skip_limit);
+}
+
+// Tile states of one of a Device's regions, zero unless a scan used them since
+// the init passes' clearing (then *zeroed is false and the scan clears them).
+inline int64_t* scan_region(Device& D, int q, bool* zeroed) {
+    *zeroed = (D.blk_zero >> q) & 1;
+    D.blk_zero &= ~(1u << q);
+    return D.blk + q * D.blk_stride;
 }
 
 }  // namespace sspp
