@@ -74,14 +74,10 @@ struct sspp_ctx {
     std::string err;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
-#ifndef SSPP_SIDE_STREAMS
-#define SSPP_SIDE_STREAMS 64
-#endif
-    // CTA-tier launches in flight at once: each holds its stream until its
-    // longest chain ends, so a later launch needs a stream of its own
-    static constexpr int kSide = SSPP_SIDE_STREAMS;
-    cudaStream_t side[kSide] = {};     // heavy-tier launches overlap later light steps and each other
-    std::vector<cudaEvent_t> step_ev;  // light step k done
+    // a dimension's CTA-tier launch runs on its own stream beside the next dimensions
+    static constexpr int kSide = kNumDims;
+    cudaStream_t side[kSide] = {};
+    cudaEvent_t step_ev[kSide] = {};   // a dimension's light launch done
     cudaEvent_t join_ev[kSide] = {};   // side stream joins
     Device D;
     sspp_params params{};          // effective parameters (after autotuning)
@@ -195,7 +191,7 @@ cudaError_t grow(T*& p, int64_t& cap, int64_t want, cudaStream_t s) {
 void free_device(Device& D) {
     void* ptrs[] = {D.dim, D.perm, D.newidx, D.scratch64, D.arena,
                     D.desc, D.low, D.pivot, D.state, D.cleared, D.negative, D.leftmost, D.active, D.ctl, D.dimcnt,
-                    D.step_ctr, D.heavy, D.death_of, D.pairs, D.ess, D.misc, D.app, D.runlist};
+                    D.heavy, D.death_of, D.pairs, D.ess, D.misc, D.app};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     D = Device();
@@ -225,7 +221,6 @@ int ensure_columns(sspp_ctx* ctx, int64_t n, int64_t nnz) {
         CK(g(D.negative, 1));
         CK(g(D.leftmost, 1));
         CK(g(D.active, 1));
-        CK(g(D.runlist, 1));
         CK(g(D.death_of, 1));
         CK(g(D.pairs, 2));
         CK(g(D.ess, 1));
@@ -281,15 +276,6 @@ int64_t arena_need(const sspp_ctx* ctx) {
     return std::max(want, ctx->arena_request);
 }
 
-// Blocks of fewer columns are merged by the host loop of per-block launches.  A
-// block exists to bound the work in flight and to let a column wait for the
-// columns below its band; with rounds of additions a chain is no longer the
-// step's length, and a step costs its launches and its slowest column whatever
-// it holds.  64^3 (reference's blocks of 102400 growing by 1.05: 40 steps) 2.68 ms
-// of reduction in those blocks, 1.92 in 400 k, 1.74 in 1 M, 1.82 in one block per
-// dimension; 93^3 6.4 / 5.0 / 4.5 / 4.5 ms.  The pairs do not depend on it.
-constexpr int kMinBlock = 1 << 20;
-
 // Clears the control block and the scans' tile states.
 int clear_ctl(sspp_ctx* ctx) {
     Device& D = ctx->D;
@@ -312,11 +298,11 @@ struct Step {
     int32_t beg, end, minrow;
 };
 
-void ss_schedule(const sspp_params& P, int min_block, int32_t ab, int32_t ae, int32_t minrow_dim, int32_t maxrow_dim,
+void ss_schedule(const sspp_params& P, int32_t ab, int32_t ae, int32_t minrow_dim, int32_t maxrow_dim,
                  std::vector<Step>& out) {
     if (ae <= ab) return;
     const int kMaxSteps = 4096;
-    int64_t ss = std::max(min_block, P.ss_block_size);
+    int64_t ss = std::max(1, P.ss_block_size);
     // one block that holds every column and every row is the completion sweep itself
     if (ae - ab <= ss && int64_t(maxrow_dim) - minrow_dim <= ss) {
         out.push_back({ab, ae, INT32_MIN});
@@ -444,7 +430,7 @@ DimInfo ranges_of_counts(const unsigned long long* cnt) {
 
 // Sizes the guided-clearing scratch from the per-dimension column ranges and
 // runs it on stream `s`.
-int run_highclear(sspp_ctx* ctx, cudaStream_t s, const DimInfo& info, bool from_input) {
+int run_highclear(sspp_ctx* ctx, cudaStream_t s, const DimInfo& info) {
     Device& D = ctx->D;
     HighclearScratch& S = ctx->hc;
     int top = -1;
@@ -468,7 +454,7 @@ int run_highclear(sspp_ctx* ctx, cudaStream_t s, const DimInfo& info, bool from_
     while (slots < 2 * ntop) slots *= 2;
     CK(grow(S.table, S.cap_table, slots, s));
     S.mask = uint32_t(slots - 1);
-    ctx->launches += highclear(D, info, ctx->params.max_iteration, dropped_of(ctx), S, s, from_input);
+    ctx->launches += highclear(D, info, ctx->params.max_iteration, dropped_of(ctx), S, s);
     return SSPP_OK;
 }
 
@@ -536,28 +522,24 @@ int run_init(sspp_ctx* ctx) {
     // the reorder also does the first init pass unless an edge collapse will
     // empty columns in between (the autotuner never changes the model)
     const bool lows_in_reorder = !(ctx->params.model & 2);
-    // guided clearing reads only the matrix and marks top-dimension columns,
-    // the apparent-pair pass marks youngest facets (never of the top
+    // guided clearing reads only the reordered matrix and marks top-dimension
+    // columns, the apparent-pair pass marks youngest facets (never of the top
     // dimension): the two run side by side and the compression waits for both.
-    // Without an edge collapse guided clearing starts as soon as the reorder
-    // has assigned the new indices (its tuples come from the input columns).
     const bool guided = (ctx->params.model & 1) && ctx->params.max_iteration > 0;
-    const bool early = guided && !(ctx->params.model & 2);
     if (ctx->user_params.autotune && !ctx->tune_locked) {
         int rc2 = autotune_choose(ctx, ranges);
         if (rc2) return rc2;
     }
-    ctx->launches += reorder(D, lows_in_reorder, !lows_in_reorder || ctx->params.dualize == 1, s,
-                             early ? ctx->hc_fork : nullptr);
+    ctx->launches += reorder(D, lows_in_reorder, !lows_in_reorder || ctx->params.dualize == 1, s);
     if (ctx->params.model & 2) {  // collapse before everything else: dropped columns are emptied
         int rc2 = run_collapse(ctx, ranges);
         if (rc2) return rc2;
     }
     if (guided) {
         cudaStream_t hs = ctx->side[0];
-        if (!early) CK(cudaEventRecord(ctx->hc_fork, s));  // after the collapse
+        CK(cudaEventRecord(ctx->hc_fork, s));
         CK(cudaStreamWaitEvent(hs, ctx->hc_fork, 0));
-        int rc2 = run_highclear(ctx, hs, ranges, early);
+        int rc2 = run_highclear(ctx, hs, ranges);
         CK(cudaEventRecord(ctx->hc_join, hs));
         if (rc2) {
             CK(cudaStreamWaitEvent(s, ctx->hc_join, 0));
@@ -592,8 +574,6 @@ int run_init(sspp_ctx* ctx) {
     return SSPP_OK;
 }
 
-// Runs one spectral-sequence schedule: per step a light-tier launch on the
-// main stream and a heavy-tier launch for the columns it deferred.
 // Dimension gate.  The next dimension's columns are cleared by the claims of
 // this one, so it used to start only once every CTA-tier column of this
 // dimension was done; on large grids the last few of them are single long
@@ -615,7 +595,7 @@ constexpr double kGateMaxMs = 30000.0;
 constexpr double kGateSpinMs = 2.0;
 constexpr int kGateNapUs = 50;
 
-int dimension_gate(sspp_ctx* ctx) {
+int dimension_gate(sspp_ctx* ctx, int streams) {
     cudaStream_t s = ctx->stream;
     CK(cudaMemcpyAsync(ctx->h_tail, ctx->D.pool_tail, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaEventRecord(ctx->gate_ev, s));
@@ -627,7 +607,7 @@ int dimension_gate(sspp_ctx* ctx) {
         if (tail - done <= kGateLeft) break;
         if ((it & 63) == 0) {
             bool idle = true;
-            for (int q = 0; q < sspp_ctx::kSide && idle; q++) idle = cudaStreamQuery(ctx->side[q]) != cudaErrorNotReady;
+            for (int q = 0; q < streams && idle; q++) idle = cudaStreamQuery(ctx->side[q]) != cudaErrorNotReady;
             if (idle) break;
             const double waited =
                 std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -642,23 +622,27 @@ int dimension_gate(sspp_ctx* ctx) {
     return SSPP_OK;
 }
 
-int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2, int ht) {
+// Reduces dimensions [dlo, dhi] (ascending or descending): per dimension a
+// light-tier launch over its active columns and a CTA-tier launch for the columns
+// it deferred.  The whole dimension is one spectral-sequence block.  Smaller
+// blocks bound the work in flight and let a column wait for the columns below its
+// band; with rounds of additions a chain no longer is the step's length, and a
+// step costs its launches and its slowest column whatever it holds (the 40 blocks
+// of 102400 growing by 1.05 of 64^3 took 2.68 ms with rounds, blocks of 2^20 1.10, one
+// block per dimension 1.00; 93^3 6.4 / 3.0 / 2.3 ms).  The pairs do not depend on it.
+int run_dims(sspp_ctx* ctx, int dlo, int dhi, bool ascending, int cap1, int cap2, int ht) {
     Device& D = ctx->D;
     cudaStream_t s = ctx->stream;
     const sspp_params& P = ctx->params;
-    // counters: the control block's while they are as the init passes cleared them
-    int* step_ctr = D.ctl->step;
-    if (!D.steps_zero || steps.size() > size_t(kCtlSteps)) {
-        if (kStepCtr * int64_t(steps.size()) > D.cap_steps) {
-            if (D.step_ctr) cudaFreeAsync(D.step_ctr, s);
-            D.step_ctr = nullptr;
-            D.cap_steps = 0;
-            CK(grow(D.step_ctr, D.cap_steps, kStepCtr * int64_t(steps.size()) + 64, s));
-        }
-        step_ctr = D.step_ctr;
-        if (!steps.empty()) CK(cudaMemsetAsync(step_ctr, 0, sizeof(int) * kStepCtr * steps.size(), s));
-        CK(cudaMemsetAsync(D.pool_tail, 0, 2 * sizeof(int), s));  // and heavy_done
+    const DimInfo& I = ctx->hinfo;
+    int dims[kNumDims], nd = 0;
+    for (int k = 0; k <= dhi - dlo; k++) {
+        const int d = ascending ? dlo + k : dhi - k;
+        if (I.act_end[d] > I.act_begin[d]) dims[nd++] = d;
     }
+    // counters: the control block's, cleared again when an earlier pass used them
+    int* step_ctr = D.ctl->step;
+    if (!D.steps_zero) CK(cudaMemsetAsync(&D.ctl->pool_tail, 0, sizeof(Ctl) - offsetof(Ctl, pool_tail), s));
     D.steps_zero = false;
     // heavy pool: deferrals are rare (heavy columns and displaced owners); a
     // full pool sets the capacity bit and the run is repeated with a larger one
@@ -672,88 +656,44 @@ int run_steps(sspp_ctx* ctx, const std::vector<Step>& steps, int cap1, int cap2,
     const int light_max = std::max(1, ctx->num_sms * ctx->light_blocks_per_sm);
     const int heavy_grid = std::max(1, std::min(ctx->num_sms * ctx->heavy_blocks_per_sm, 2 * ctx->num_sms));
     const int q_blocks = std::max(1, (P.queue_size + 3) / 4);
-    // Heavy launches go to side streams (round robin) after their light step:
-    // they overlap the following light steps and each other, so long chains of
-    // different steps run concurrently.  Each dimension's completion sweep, and
-    // the next dimension, wait for all of them (twist clearing needs the
-    // finished dimension) -- on large inputs only until few of them are left
-    // (the dimension gate below).
-    const bool overlap = true;
+    // On large inputs a CTA-tier launch goes to a stream of its own and overlaps
+    // the next dimension, which starts once few of its columns are left (the
+    // dimension gate); on others the next dimension waits for it (twist clearing
+    // needs the finished dimension).
     const bool gate = D.n >= kGateMinCols && ctx->h_gate && ctx->d_gate && ctx->h_tail && ctx->gate_ev;
     D.gate_host = gate ? ctx->d_gate : nullptr;
-    if (gate) {
-        *reinterpret_cast<volatile int*>(ctx->h_gate) = 0;  // no CTA-tier launch of this context is running
-    }
-    while (ctx->step_ev.size() < steps.size() + 1) {
-        cudaEvent_t ev;
-        CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        ctx->step_ev.push_back(ev);
-    }
-    bool used[sspp_ctx::kSide] = {};  // side streams with launches since the last join
-    auto join_sides = [&]() -> int {
-        for (int q = 0; q < sspp_ctx::kSide; q++) {
-            if (!used[q]) continue;
-            used[q] = false;
-            CK(cudaEventRecord(ctx->join_ev[q], ctx->side[q]));
-            CK(cudaStreamWaitEvent(s, ctx->join_ev[q], 0));
-        }
-        return SSPP_OK;
-    };
-    for (size_t k = 0; k < steps.size(); k++) {
-        const Step& st = steps[k];
-        const bool last_of_dim = st.minrow == INT32_MIN;
-        if (overlap && last_of_dim && !gate) {  // join: everything heavy of this dimension is done
-            int rcj = join_sides();
-            if (rcj) return rcj;
-        }
-        const int64_t window = int64_t(st.end) - st.beg;
+    if (gate) *reinterpret_cast<volatile int*>(ctx->h_gate) = 0;  // no CTA-tier launch of this context is running
+    for (int k = 0; k < nd; k++) {
+        const int32_t b = I.act_begin[dims[k]], e = I.act_end[dims[k]];
+        const int64_t window = int64_t(e) - b;
         const int grid = int(std::max<int64_t>(1, std::min<int64_t>({(window + 3) / 4, light_max, q_blocks})));
         int* ctr = step_ctr + kStepCtr * k;
-        cudaEvent_t a = nullptr, b = nullptr;
-        span_begin(ctx, a);
-        int* ctr_next = k + 1 < steps.size() ? ctr + kStepCtr : nullptr;
-        const int fgrid = int(std::max<int64_t>(1, std::min<int64_t>((window + 255) / 256, int64_t(ctx->num_sms) * 8)));
-        ctx->launches += reduce_light_launch(D, st.beg, st.end, st.minrow, cap1, ctr, ctr_next, fgrid, grid, s);
-        span_end(ctx, PH_LIGHT, a);
-        if (overlap && (!last_of_dim || gate)) {
-            // an idle side stream if there is one: a CTA-tier launch lasts as
-            // long as its longest chain, and a launch queued behind it on the
-            // same stream would wait for that chain
-            int q = int(k % sspp_ctx::kSide);
-#ifndef SSPP_SIDE_RR
-            for (int t = 0; t < sspp_ctx::kSide; t++) {
-                const int c = int((k + t) % sspp_ctx::kSide);
-                if (cudaStreamQuery(ctx->side[c]) == cudaSuccess) {
-                    q = c;
-                    break;
-                }
-            }
-#endif
-            cudaStream_t hs = ctx->side[q];
-            used[q] = true;
+        cudaEvent_t ev = nullptr;
+        span_begin(ctx, ev);
+        reduce_light_launch(D, b, e, cap1, ctr, k + 1 < nd ? ctr + kStepCtr : nullptr, grid, s);
+        span_end(ctx, PH_LIGHT, ev);
+        cudaStream_t hs = s;
+        if (gate) {
+            hs = ctx->side[k];
             CK(cudaEventRecord(ctx->step_ev[k], s));
             CK(cudaStreamWaitEvent(hs, ctx->step_ev[k], 0));
-            span_begin(ctx, b, hs);
-            reduce_heavy_launch(D, cap2, ht, ctr, heavy_grid, hs);
-            span_end(ctx, PH_HEAVY, b, hs);
-        } else {
-            span_begin(ctx, b);
-            reduce_heavy_launch(D, cap2, ht, ctr, heavy_grid, s);
-            span_end(ctx, PH_HEAVY, b);
         }
+        span_begin(ctx, ev, hs);
+        reduce_heavy_launch(D, cap2, ht, ctr, heavy_grid, hs);
+        span_end(ctx, PH_HEAVY, ev, hs);
         ctx->light_launches++;
         ctx->heavy_launches++;
-        ctx->launches++;
-        if (gate && last_of_dim && k + 1 < steps.size()) {
-            int rcg = dimension_gate(ctx);
+        ctx->launches += 2;
+        if (gate && k + 1 < nd) {
+            int rcg = dimension_gate(ctx, k + 1);
             if (rcg) return rcg;
         }
     }
-    if (overlap) {  // nothing may still run on a side stream past this point
-        int rcj = join_sides();
-        if (rcj) return rcj;
+    for (int k = 0; gate && k < nd; k++) {  // nothing may still run on a side stream past this point
+        CK(cudaEventRecord(ctx->join_ev[k], ctx->side[k]));
+        CK(cudaStreamWaitEvent(s, ctx->join_ev[k], 0));
     }
-    ctx->ss_steps = int64_t(steps.size());
+    ctx->ss_steps = nd;
     return SSPP_OK;
 }
 
@@ -809,7 +749,7 @@ int run_queue(sspp_ctx* ctx, int dlo, int dhi, bool ascending, int cap1, int cap
             cap = std::max(cap, cnt);
             st.clear();
             const int32_t mr = mnr[int64_t(c) * kNumDims + d];
-            ss_schedule(P, 1, ab, ae, mr == INT32_MAX ? 0 : mr, mxr[int64_t(c) * kNumDims + d], st);
+            ss_schedule(P, ab, ae, mr == INT32_MAX ? 0 : mr, mxr[int64_t(c) * kNumDims + d], st);
             int32_t eprev = -1;
             const size_t d0 = items.size();
             for (const Step& x : st) {
@@ -942,20 +882,11 @@ int run_compute(sspp_ctx* ctx) {
         if (ctx->light_blocks_per_sm < 1 || ctx->heavy_blocks_per_sm < 1)
             return set_err(ctx, SSPP_ERR_CAPACITY, "level capacities too large for shared memory");
     }
-    // schedule: dimensions high to low, or low to high for the dual matrix
+    // dimensions high to low, or low to high for the dual matrix
     // (include/specseq.h:598-600).  dualize 2: the boundary matrix's edge
     // columns first (0-dimensional pairs), then the coboundary matrix from
     // dimension 1 up.
-    const DimInfo& I = ctx->hinfo;
-    auto schedule = [&](int dlo, int dhi, bool ascending) {
-        std::vector<Step> st;
-        for (int k = 0; k <= dhi - dlo; k++) {
-            const int d = ascending ? dlo + k : dhi - k;
-            ss_schedule(P, kMinBlock, I.act_begin[d], I.act_end[d], I.min_row[d] == INT_MAX ? 0 : I.min_row[d], I.max_row[d], st);
-        }
-        return st;
-    };
-    // schedule 1 (and 0): a host loop of per-block launches; 2: one persistent
+    // schedule 1 (and 0): launches per dimension; 2: one persistent
     // launch per phase draining the (complex, block) work queue.  The host loop
     // is the default: its warp-tier kernel keeps four times as many warps
     // resident as the persistent kernel, whose CTA-tier role sets the register
@@ -963,7 +894,7 @@ int run_compute(sspp_ctx* ctx) {
     const bool queue = P.schedule == 2;
     auto phase = [&](int dlo, int dhi, bool ascending) {
         return queue ? run_queue(ctx, dlo, dhi, ascending, cap1, cap2, ht)
-                     : run_steps(ctx, schedule(dlo, dhi, ascending), cap1, cap2, ht);
+                     : run_dims(ctx, dlo, dhi, ascending, cap1, cap2, ht);
     };
     int64_t nsteps = 0;
     if (P.dualize == 2) {
@@ -1167,6 +1098,7 @@ sspp_ctx* sspp_create(const sspp_config* cfg) {
     if (cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) != cudaSuccess) { delete ctx; return nullptr; }
     for (int q = 0; q < sspp_ctx::kSide; q++) {
         if (cudaStreamCreateWithFlags(&ctx->side[q], cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&ctx->step_ev[q], cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ctx->join_ev[q], cudaEventDisableTiming) != cudaSuccess) {
             delete ctx;
             return nullptr;
@@ -1238,8 +1170,8 @@ void sspp_destroy(sspp_ctx* ctx) {
     ctx->prof.release();
     for (int q = 0; q < sspp_ctx::kSide; q++)
         if (ctx->side[q]) cudaStreamSynchronize(ctx->side[q]);
-    for (auto ev : ctx->step_ev) cudaEventDestroy(ev);
     for (int q = 0; q < sspp_ctx::kSide; q++) {
+        if (ctx->step_ev[q]) cudaEventDestroy(ctx->step_ev[q]);
         if (ctx->join_ev[q]) cudaEventDestroy(ctx->join_ev[q]);
         if (ctx->side[q]) cudaStreamDestroy(ctx->side[q]);
     }
@@ -1840,7 +1772,7 @@ int32_t sspp_export_preprocessed(sspp_ctx* ctx, const sspp_params* p, const char
         }
         CK(cudaMemsetAsync(D.cleared, 0, size_t(n), s));
         if ((p->model & 1) && p->max_iteration > 0) {
-            rc = run_highclear(ctx, ctx->stream, ranges, false);
+            rc = run_highclear(ctx, ctx->stream, ranges);
             if (rc) return rc;
         }
         std::vector<int32_t> perm(static_cast<size_t>(n));

@@ -63,48 +63,24 @@ __device__ __forceinline__ void tuple_union(int d, int32_t c0, int32_t c1, int32
 
 // Vertex tuple of every column of dimension d >= 1 (sorted, d+1 vertices),
 // from the first two facets' tuples.  tup_d / tup_f point at the tuple arrays of
-// dims d and d-1 (dim-0 tuples are the vertex indices themselves).
+// dims d and d-1 (dim-0 tuples are the vertex indices themselves).  Columns come
+// from their slots, which lie in this kernel's order (short columns: without their
+// descriptors); read from the input columns through the index maps instead, so
+// that it could start before the slots were written, this took 182 us at 64^3 and
+// slowed the passes beside it.
 __global__ void k_tuples(int32_t cb, int32_t ce, int d, int32_t fb, const int32_t* arena, const uint64_t* desc,
-                         const int32_t* tup_f, int32_t* tup_d, int* err) {
+                         const Ctl* ctl, const int32_t* tup_f, int32_t* tup_d) {
+    const bool all_short = ctl->max_len <= kShortLen;
     for (int64_t i = cb + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < ce; i += int64_t(gridDim.x) * blockDim.x) {
-        uint64_t ds = desc[i];
-        const int32_t* c = arena + desc_off(ds) + kHdr;
+        const int32_t* slot = arena + (all_short ? int64_t(kShortSlot) * i : int64_t(desc_off(desc[i])));
+        const int len = all_short ? slot[0] : int(desc_len(desc[i]));
         int32_t* out = tup_d + (i - cb) * (d + 1);
-        if (desc_len(ds) < 2 || desc_len(ds) != uint32_t(d + 1)) {
+        if (len != d + 1) {
             // not a simplicial boundary (edge with < 2 vertices etc.): no tuple
             for (int k = 0; k <= d; k++) out[k] = -1;
             continue;
         }
-        tuple_union(d, c[0], c[1], fb, tup_f, out);
-    }
-}
-
-// The same tuples read from the input matrix through the reorder's index maps
-// (perm, newidx), so that they need only the dimension assignment, not the
-// reordered columns: a face index outside the input, or outside dimension
-// d-1, gives no tuple (the reorder reports such a matrix as malformed).
-__global__ void k_tuples_in(int32_t cb, int32_t ce, int d, int32_t fb, int32_t fe, const int32_t* perm,
-                            const int32_t* newidx, const int64_t* colptr, const int32_t* rows, int64_t n,
-                            const int32_t* tup_f, int32_t* tup_d) {
-    for (int64_t i = cb + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < ce; i += int64_t(gridDim.x) * blockDim.x) {
-        int32_t* out = tup_d + (i - cb) * (d + 1);
-        const int64_t j = perm[i], a = colptr[j];
-        bool ok = colptr[j + 1] - a == d + 1;
-        int32_t f0 = -1, f1 = -1;
-        if (ok) {
-            const int32_t r0 = rows[a], r1 = rows[a + 1];
-            ok = r0 >= 0 && r0 < n && r1 >= 0 && r1 < n;
-            if (ok) {
-                f0 = newidx[r0];
-                f1 = newidx[r1];
-                ok = f0 >= fb && f0 < fe && f1 >= fb && f1 < fe;
-            }
-        }
-        if (!ok) {
-            for (int k = 0; k <= d; k++) out[k] = -1;
-            continue;
-        }
-        tuple_union(d, f0, f1, fb, tup_f, out);
+        tuple_union(d, slot[kHdr], slot[kHdr + 1], fb, tup_f, out);
     }
 }
 
@@ -440,7 +416,7 @@ __global__ void __launch_bounds__(kHcThreads) k_highclear(int32_t cb, int32_t ce
 }
 
 int highclear(Device& D, const DimInfo& info, int max_iteration, const uint8_t* dropped, HighclearScratch& S,
-              cudaStream_t s, bool from_input) {
+              cudaStream_t s) {
     // top dimension with columns
     int top = -1;
     for (int d = kMaxDim; d >= 1; d--)
@@ -451,13 +427,8 @@ int highclear(Device& D, const DimInfo& info, int max_iteration, const uint8_t* 
     const int32_t* prev = nullptr;
     for (int d = 1; d <= top; d++) {
         int32_t cb = info.col_begin[d], ce = info.col_end[d];
-        if (from_input)
-            k_tuples_in<<<gridn(ce - cb, 256), 256, 0, s>>>(cb, ce, d, info.col_begin[d - 1], info.col_end[d - 1],
-                                                           D.perm, D.newidx, D.in_colptr, D.in_rows, D.n, prev,
-                                                           S.tup[d]);
-        else
-            k_tuples<<<gridn(ce - cb, 256), 256, 0, s>>>(cb, ce, d, info.col_begin[d - 1], D.arena, D.desc, prev,
-                                                        S.tup[d], D.err);
+        k_tuples<<<gridn(ce - cb, 256), 256, 0, s>>>(cb, ce, d, info.col_begin[d - 1], D.arena, D.desc, D.ctl, prev,
+                                                    S.tup[d]);
         launches++;
         prev = S.tup[d];
     }

@@ -43,15 +43,18 @@ void fill_i64(int64_t* p, int64_t v, int64_t n, cudaStream_t s) {
 // non-decreasing from 0 to nnz (device-resident inputs are only checked here).
 // The same pass counts the columns of each dimension, per tile for the reorder
 // (dimcnt) and in total for the host (dimtot, zeroed before), and finds the
-// longest column.  A warp takes 256 consecutive columns.
+// longest column.  It also starts the init passes' state of every column, in
+// order: no leftmost column yet, no pivot owner, not cleared, not negative.  A warp
+// takes 32 * kPartRounds consecutive columns.
 constexpr int kPartThreads = 256;
-constexpr int kPartRounds = 8;
+constexpr int kPartRounds = 4;  // 2, 4 and 8 measured alike on large inputs, 8 slower on small ones
 constexpr int kPartTile = kPartThreads * kPartRounds;
 
 int64_t part_tiles(int64_t n) { return (n + kPartTile - 1) / kPartTile; }
 
 __global__ void __launch_bounds__(kPartThreads) k_validate(const int32_t* dims, const int64_t* colptr, int64_t n,
-                                                           int64_t nnz, int32_t* dimcnt, Ctl* ctl) {
+                                                           int64_t nnz, int32_t* dimcnt, Ctl* ctl, int32_t* leftmost,
+                                                           uint64_t* pivot, uint8_t* cleared, uint8_t* negative) {
     __shared__ int s_cnt[kNumDims];
     __shared__ int s_len, s_bad;
     if (threadIdx.x < kNumDims) s_cnt[threadIdx.x] = 0;
@@ -72,6 +75,10 @@ __global__ void __launch_bounds__(kPartThreads) k_validate(const int32_t* dims, 
                 bad = true;
             else
                 longest = max(longest, int(len));
+            leftmost[j] = INT_MAX;
+            pivot[j] = kNoOwner;
+            cleared[j] = 0;
+            negative[j] = 0;
         }
 #pragma unroll
         for (int q = 0; q < kNumDims; q++) {
@@ -97,7 +104,8 @@ __global__ void __launch_bounds__(kPartThreads) k_validate(const int32_t* dims, 
 
 int validate(Device& D, cudaStream_t s) {
     if (D.n <= 0) return 0;
-    k_validate<<<unsigned(part_tiles(D.n)), kPartThreads, 0, s>>>(D.in_dims, D.in_colptr, D.n, D.nnz, D.dimcnt, D.ctl);
+    k_validate<<<unsigned(part_tiles(D.n)), kPartThreads, 0, s>>>(D.in_dims, D.in_colptr, D.n, D.nnz, D.dimcnt, D.ctl,
+                                                              D.leftmost, D.pivot, D.cleared, D.negative);
     return 1;
 }
 
@@ -212,7 +220,7 @@ __device__ void dim_ranges(const int64_t* total, DimInfo* info) {
 // place), and the ranges.  One block; thread (chunk, dimension) takes a chunk of
 // consecutive tiles.  Inputs of up to kInlineTiles tiles skip it: their tiles add
 // up the counts themselves.
-constexpr int kInlineTiles = 128;
+constexpr int kInlineTiles = 256;
 __global__ void __launch_bounds__(1024) k_dim_offsets(int32_t* dimcnt, int64_t nb, Ctl* ctl) {
     if (ctl->err) return;
     __shared__ int64_t s_sum[128][kNumDims];
@@ -243,15 +251,12 @@ __global__ void __launch_bounds__(1024) k_dim_offsets(int32_t* dimcnt, int64_t n
     }
 }
 
-// Stable rank of each column inside its dimension -> reordered index.  Also
-// starts the init passes' per-column state of reordered column idx: no leftmost
-// column yet, no pivot owner, not cleared, not negative; and, unless every column
-// is short, records its length for the slot scan that follows.
+// Stable rank of each column inside its dimension -> reordered index.  Unless
+// every column is short, also records its length for the slot scan that follows.
 __global__ void __launch_bounds__(kPartThreads) k_dim_assign(const int32_t* dims, const int64_t* colptr, int64_t n,
                                                              int64_t nb, const int32_t* dimcnt, Ctl* ctl,
                                                              int32_t* newidx, int32_t* perm, int32_t* rdim,
-                                                             int32_t* rlen, int32_t* leftmost, uint64_t* pivot,
-                                                             uint8_t* cleared, uint8_t* negative) {
+                                                             int32_t* rlen) {
     if (ctl->err) return;
     constexpr int kWarps = kPartThreads / 32;
     __shared__ int s_warp[kWarps][kNumDims];
@@ -316,10 +321,6 @@ __global__ void __launch_bounds__(kPartThreads) k_dim_assign(const int32_t* dims
         perm[idx] = int32_t(j);
         rdim[idx] = d[k];
         if (!all_short) rlen[idx] = int32_t(colptr[j + 1] - colptr[j]);
-        leftmost[idx] = INT_MAX;
-        pivot[idx] = kNoOwner;
-        cleared[idx] = 0;
-        negative[idx] = 0;
     }
 }
 
@@ -407,7 +408,7 @@ __global__ void k_scatter_cols(int64_t n, const int64_t* colptr, const int32_t* 
     }
 }
 
-int reorder(Device& D, bool lows, bool write_desc, cudaStream_t s, cudaEvent_t assigned) {
+int reorder(Device& D, bool lows, bool write_desc, cudaStream_t s) {
     const int64_t n = D.n, nb = part_tiles(n);
     int launches = 3;
     if (nb > kInlineTiles) {
@@ -417,8 +418,7 @@ int reorder(Device& D, bool lows, bool write_desc, cudaStream_t s, cudaEvent_t a
     // the active list is built later: until then its buffer holds the reordered lengths
     int32_t* rlen = D.active;
     k_dim_assign<<<unsigned(nb), kPartThreads, 0, s>>>(D.in_dims, D.in_colptr, n, nb, D.dimcnt, D.ctl, D.newidx, D.perm,
-                                                       D.dim, rlen, D.leftmost, D.pivot, D.cleared, D.negative);
-    if (assigned) cudaEventRecord(assigned, s);
+                                                       D.dim, rlen);
     // padded column offsets in reordered order, unless every column is short (or
     // the input is refused: the limit then skips it too)
     int64_t* off = D.scratch64;
@@ -482,13 +482,22 @@ __global__ void k_init_apparent(int64_t n, const int32_t* arena, const uint64_t*
         const int32_t l = low[i];
         if (l < 0) continue;
         cleared[l] = 1;  // the youngest facet of any simplex is positive
-        const ColRef c = col_ref(i, arena, desc, all_short);
-        if (leftmost[l] == int32_t(i)) {
-            pivot[l] = pv_pack(int32_t(i), uint64_t(c.slot));  // no earlier column can ever reach row l
+        if (leftmost[l] == int32_t(i)) {  // no earlier column can ever reach row l
+            pivot[l] = pv_pack(int32_t(i), all_short ? uint64_t(kShortSlot) * uint64_t(i) : desc_off(desc[i]));
+            negative[i] = 1;
             app++;
+            continue;  // its other entries need not be looked at
         }
-        for (int k = 0; k < c.len; k++)
-            if (leftmost[c.at(arena, k, all_short)] == int32_t(i)) { negative[i] = 1; break; }
+        const ColRef c = col_ref(i, arena, desc, all_short);
+        bool neg = false;
+        if (all_short) {  // the lowest entry's is known; the others' at once
+            const int32_t x = c.len > 1 ? leftmost[c.q.x] : -1, y = c.len > 2 ? leftmost[c.q.y] : -1,
+                          z = c.len > 3 ? leftmost[c.q.z] : -1;
+            neg = x == int32_t(i) || y == int32_t(i) || z == int32_t(i);
+        } else {
+            for (int k = 0; k < c.len && !neg; k++) neg = leftmost[c.at(arena, k, false)] == int32_t(i);
+        }
+        if (neg) negative[i] = 1;
     }
     app = warp_sum(app);
     if ((threadIdx.x & 31) == 0 && app) cnt_add(&ctl->counters[CNT_APPARENT], app);
@@ -524,8 +533,7 @@ __global__ void k_init_compress(int64_t n, int32_t* arena, uint64_t* desc, int32
             const int64_t slot = all_short ? int64_t(kShortSlot) * i : int64_t(desc_off(desc[i]));
             const int32_t l = low[i];
             if (!drop && l >= 0 && pv_col(pivot[l]) == int32_t(i)) atomicOr(&ctl->err, ERRB_FACES);  // positive and negative
-            desc[i] = pack_desc(uint64_t(slot), 0);
-            arena[slot] = 0;
+            desc[i] = pack_desc(uint64_t(slot), 0);  // its slot is not read any more
             low[i] = -1;
             state[i] = drop ? ST_DROPPED : ST_CLEARED;
             ncl += !drop;
@@ -550,8 +558,10 @@ __global__ void k_init_compress(int64_t n, int32_t* arena, uint64_t* desc, int32
                 }
             }
             first = y[0];
-            arena[c.slot] = m;
-            *reinterpret_cast<int4*>(arena + c.slot + kHdr) = make_int4(y[0], y[1], y[2], y[3]);
+            if (m != c.len) {
+                arena[c.slot] = m;
+                *reinterpret_cast<int4*>(arena + c.slot + kHdr) = make_int4(y[0], y[1], y[2], y[3]);
+            }
             v = make_int4(m - 1, m > 1 ? y[0] : INT_MAX, m > 2 ? y[1] : INT_MAX, m > 3 ? y[2] : INT_MAX);
         } else {
             int32_t* col = arena + c.slot + kHdr;
@@ -686,15 +696,11 @@ int active_list(Device& D, bool rows_done, cudaStream_t s) {
         const unsigned g = grid_for(n, 256) > 4096 ? 4096 : grid_for(n, 256);
         k_dim_rows<<<g, 256, 0, s>>>(n, D.dim, D.arena, D.desc, D.low, D.state, D.diminfo);
     }
-    const uint8_t* state = D.state;
     int32_t* act = D.active;
     DimInfo* info = D.diminfo;
     bool zeroed;
     int64_t* blk = scan_region(D, 1, &zeroed);
-    scan([=] __device__(int64_t i) -> ScanClass { return {uint8_t(state[i] == ST_ACTIVE ? 1 : 0)}; },
-         [=] __device__(int64_t i, int64_t pre, ScanClass v) {
-             if (v.c) act[pre] = int32_t(i);
-         },
+    scan(ScanBytes{D.state, ST_ACTIVE}, [=] __device__(int64_t i, int64_t pre) { act[pre] = int32_t(i); },
          n, blk, s,
          [=] __device__(int64_t) {
              int32_t at = 0;

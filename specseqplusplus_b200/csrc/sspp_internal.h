@@ -89,8 +89,7 @@ enum CounterIdx {
 
 // Small device state of a run, one block of memory: cleared at once before the
 // init passes and read back at once.
-constexpr int kCtlSteps = 16;  // spectral-sequence steps whose counters fit here
-constexpr int kStepCtr = 8;    // counters per step (see ReduceArgs::ctr)
+constexpr int kStepCtr = 8;  // counters per dimension's step (see ReduceArgs::ctr)
 struct Ctl {
     DimInfo info;
     long long counters[CNT_NUM];
@@ -100,7 +99,7 @@ struct Ctl {
     int max_len;      // longest input column (validation pass)
     int pool_tail;    // CTA-tier pool entries
     int heavy_done;   // pool columns the CTA tier has finished
-    int step[kCtlSteps * kStepCtr];
+    int step[kNumDims * kStepCtr];
 };
 
 // Columns of at most 4 entries (every simplicial complex up to dimension 3): when
@@ -135,7 +134,6 @@ struct Device {
     uint8_t* negative = nullptr;
     int32_t* leftmost = nullptr;
     int32_t* active = nullptr;
-    int32_t* runlist = nullptr;  // [n] a step's runnable columns (warp tier input)
     // block-scan scratch
     // one buffer: Ctl, then three regions of tile states (slot offsets and any
     // other scan; active list; pair lists), cleared together before the init passes
@@ -150,14 +148,12 @@ struct Device {
     DimInfo* diminfo = nullptr;
     int* err = nullptr;
     long long* counters = nullptr;
-    int* step_ctr = nullptr;     // per-step work counters (kStepCtr ints per step) beyond Ctl's
     int32_t* heavy = nullptr;    // pool of columns handed to the CTA tier, appended step after step
     int64_t pool_cap = 0;
     int* pool_tail = nullptr;
     int* heavy_done = nullptr;   // pool columns the CTA tier has finished (this run)
     int* gate_host = nullptr;    // device view of a mapped host word that mirrors heavy_done
                                  // (owned by the context; null: no mirror)
-    int64_t cap_steps = 0;
     // pairs output (input indices)
     int64_t* death_of = nullptr;   // [n]
     int64_t* pairs = nullptr;      // [2n]

@@ -20,12 +20,10 @@ int validate(Device& D, cudaStream_t s);  // sets ERRB_BAD_INPUT; the passes aft
 // when a face index lies outside its own complex
 int batch_rebase(int64_t n, int64_t nnz, int32_t k, const int64_t* d_cstart, const int64_t* d_estart,
                  int64_t* colptr, int32_t* rows, int* d_bad, cudaStream_t s);
-// lows: also the lowest rows and leftmost columns (the first init pass);
-// assigned: recorded once perm / newidx / dim are written (before the columns
-// are scattered), or null
+// lows: also the lowest rows and leftmost columns (the first init pass)
 // write_desc: also the descriptors of short columns, which init_compress writes
 // otherwise (needed when anything reads them before it)
-int reorder(Device& D, bool lows, bool write_desc, cudaStream_t s, cudaEvent_t assigned = nullptr);
+int reorder(Device& D, bool lows, bool write_desc, cudaStream_t s);
 
 // per-complex slice starts (k+1 each) of the sorted pairs and essentials
 int batch_bounds(int32_t k, const int64_t* d_cstart, int64_t npairs, const int64_t* pairs, int64_t ness,
@@ -107,14 +105,11 @@ cudaError_t reduce_queue_launch(const Device& D, int cap1, int cap2, int threads
 
 cudaError_t reduce_configure(int cap1, int cap2, int heavy_threads, int* light_blocks_per_sm,
                              int* heavy_blocks_per_sm);
-// One step's light tier: k_light_filter lists the window's (active[beg, end))
-// runnable columns in D.runlist, then warps reduce them.
-// A step that takes the whole band (minrow INT32_MIN) takes the window as it is.
-// ctr: the step's 8 counters; the launch's last block also marks the step's
-// CTA-tier pool slice (ctr[2], and ctr_next[1] of the next step when given).
-// Returns the kernels launched.
-int reduce_light_launch(const Device& D, int32_t beg, int32_t end, int32_t minrow, int cap, int* ctr, int* ctr_next,
-                        int filter_grid, int grid, cudaStream_t s);
+// One dimension's light tier: warps reduce the columns active[beg, end) that are
+// still active.  ctr: the step's counters; the launch's last block also marks the
+// step's CTA-tier pool slice (ctr[2], and ctr_next[1] of the next step when given).
+void reduce_light_launch(const Device& D, int32_t beg, int32_t end, int cap, int* ctr, int* ctr_next, int grid,
+                         cudaStream_t s);
 void reduce_heavy_launch(const Device& D, int cap, int threads, int* ctr, int grid, cudaStream_t s);
 
 }  // namespace sspp

@@ -33,7 +33,7 @@
 // dimensions must lie in 0..7, and each column's faces must be ascending, in
 // range and one dimension lower; anything else is SSPP_ERR_BAD_INPUT.
 //
-// Two ways.  While the engine's arrays (about 71 bytes per column and the padded
+// Two ways.  While the engine's arrays (about 67 bytes per column and the padded
 // column arena) fit in the scratch array, its own passes run there on the
 // caller's stream (reduce_in_scratch): the same reorder, apparent pairs and
 // reduction kernels as the context API's, one block per dimension.  Otherwise,
@@ -290,7 +290,6 @@ bool carve(int32_t* scratch, int64_t n, int64_t nnz, Device& D) {
     take(D.negative, n);
     take(D.leftmost, n);
     take(D.active, n);
-    take(D.runlist, n);
     take(D.app, n);
     take(D.dimcnt, (part_tiles(n) + 1) * kNumDims);
     D.pool_cap = n;
@@ -375,8 +374,7 @@ cudaError_t reduce_in_scratch(int32_t* scratch, int dev, int64_t n, int64_t nnz,
         const int64_t b = h.info.act_begin[d], end = h.info.act_end[d], window = end - b;
         if (window <= 0) continue;
         const int grid = int(std::min<int64_t>((window + 3) / 4, int64_t(shape.sms) * shape.light));
-        const int fgrid = int(std::min<int64_t>((window + 255) / 256, int64_t(shape.sms) * 8));
-        reduce_light_launch(D, int32_t(b), int32_t(end), INT32_MIN, kCap1, ctr, ctr + kStepCtr, fgrid, grid, s);
+        reduce_light_launch(D, int32_t(b), int32_t(end), kCap1, ctr, d > 1 ? ctr + kStepCtr : nullptr, grid, s);
         reduce_heavy_launch(D, kCap2, 256, ctr,
                             int(std::min<int64_t>(int64_t(shape.sms) * std::min(shape.heavy, 2), window)), s);
         ctr += kStepCtr;

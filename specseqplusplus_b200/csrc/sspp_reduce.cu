@@ -51,8 +51,7 @@ namespace sspp {
 
 struct ReduceArgs {
     int32_t ncols;
-    const int32_t* active;  // light tier: the step's runnable columns
-    int32_t minrow;
+    const int32_t* active;  // light tier: the step's columns
     int32_t cap;          // shared-memory capacity per buffer (ints), multiple of 32
     int32_t* arena;
     int64_t arena_cap;
@@ -63,9 +62,8 @@ struct ReduceArgs {
     uint8_t* state;
     uint8_t* cleared;
     int* ctr;             // per step: [0] chunk counter, [1] [2] heavy pool range, [3] heavy pull counter,
-                          // [4] warp-tier blocks finished, [5] runnable columns listed by k_light_filter
-    const int* count;     // light tier: how many columns `active` lists (null: `listed`)
-    int32_t listed;
+                          // [4] warp-tier blocks finished
+    int32_t listed;       // how many
     int* ctr_next;        // the next step's counters (its pool range starts where this step's ends), or null
     int32_t* heavy;       // heavy pool (columns handed to the CTA tier, appended in step order)
     int* pool_tail;
@@ -1138,48 +1136,6 @@ __device__ __forceinline__ bool settle(const G& g, const ReduceArgs& A, int col,
     return o != OUT_FAIL;
 }
 
-// The runnable columns of a step: window entries that are active, not cleared
-// and whose lowest row lies in the band (low >= minrow), listed in window
-// order within each block (one atomic per block pass) and counted in ctr[5].
-// One thread per entry reads the flags with independent loads, so the warp
-// tier then takes runnable columns one at a time instead of walking the whole
-// window with a shared counter.  A flag set concurrently (a cleared flag from
-// the previous dimension's CTA tier) is read again by the warp tier.
-constexpr int kFilterThreads = 256;
-
-__global__ void __launch_bounds__(kFilterThreads) k_light_filter(const int32_t* active, int32_t beg, int32_t end,
-                                                                 int32_t minrow, const uint8_t* state,
-                                                                 const uint8_t* cleared, const int32_t* low,
-                                                                 int32_t* out, int* ctr) {
-    __shared__ int s_warp[kFilterThreads / 32];
-    __shared__ int s_base;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int64_t b0 = beg + int64_t(blockIdx.x) * kFilterThreads; b0 < end; b0 += int64_t(gridDim.x) * kFilterThreads) {
-        const int64_t i = b0 + threadIdx.x;
-        int32_t c = -1;
-        bool r = false;
-        if (i < end) {
-            c = __ldcs(active + i);
-            r = __ldcg(state + c) == ST_ACTIVE && !__ldcg(cleared + c) && __ldcg(low + c) >= minrow;
-        }
-        const unsigned m = __ballot_sync(kFull, r);
-        if (lane == 0) s_warp[wid] = __popc(m);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int t = 0;
-            for (int w = 0; w < kFilterThreads / 32; w++) {
-                const int x = s_warp[w];
-                s_warp[w] = t;
-                t += x;
-            }
-            s_base = t ? atomicAdd(ctr + 5, t) : 0;
-        }
-        __syncthreads();
-        if (r) out[s_base + s_warp[wid] + __popc(m & ((1u << lane) - 1))] = c;
-        __syncthreads();  // s_warp and s_base are rewritten by the next pass
-    }
-}
-
 // The last warp-tier block of a step to finish marks the step's slice of the
 // CTA-tier pool: it ends at the pool tail, where the next step's slice starts
 // (every deferral of the step is appended before its block finishes).
@@ -1248,11 +1204,11 @@ __global__ void __launch_bounds__(128, kLightMinBlocks) k_reduce_light(ReduceArg
     const int lane = g.rank(), gl = lane & (kGroup - 1), lead = lane & ~(kGroup - 1);
     int32_t* sw0 = smem + size_t(threadIdx.x >> 5) * (3 * A.cap + kHdr);
     int32_t* gbuf = rm.s + 2 * lead;  // 16 entries per group
-    const int count = A.count ? __ldcg(A.count) : A.listed;
+    const int count = A.listed;
     const int warps = gridDim.x * (blockDim.x >> 5);
     // list entries a warp takes at a time: enough to keep its groups busy, few enough to share a short list
     const int chunk = max(4, min(32, count / (2 * warps)));
-    const Band band{A.minrow, A.ctr, count};
+    const Band band{INT32_MIN, A.ctr, count};  // the whole dimension is one block
     long long n_adds = 0, n_ints = 0, n_pub = 0;
     int n_disp = 0;
     // the chunk: lane i holds its i-th column and descriptor; avail marks the lanes not handed out yet
@@ -1276,8 +1232,7 @@ __global__ void __launch_bounds__(128, kLightMinBlocks) k_reduce_light(ReduceArg
             if (lane < chunk && base + lane < count) {
                 ck_col = A.active[base + lane];
                 ck_desc = ld_cg_u64(A.desc + ck_col);
-                run = ld_acquire_u8(A.state + ck_col) == ST_ACTIVE && !ld_acquire_u8(A.cleared + ck_col) &&
-                      __ldcg(A.low + ck_col) >= A.minrow;
+                run = ld_acquire_u8(A.state + ck_col) == ST_ACTIVE && !ld_acquire_u8(A.cleared + ck_col);
             }
             avail = __ballot_sync(kFull, run);
             if (!avail && more) continue;
@@ -1320,11 +1275,11 @@ __global__ void __launch_bounds__(128, kLightMinBlocks) k_reduce_light(ReduceArg
             break;
         }
         // ---- rows' owners
-        bool act = col >= 0 && !ovf && n > 0 && L >= A.minrow;
+        const bool act = col >= 0 && !ovf && n > 0;
         int4 q4 = make_int4(-1, 0, 0, 0);
         uint64_t ev = kNoOwner;
         unsigned clr = 0;
-        if (act && gl < n && v >= A.minrow) {
+        if (act && gl < n) {
             q4 = __ldg(A.app + v);
             ev = ld_acquire_u64(A.pivot + v);
             if (gl == 0) clr = ld_acquire_u8(A.cleared + col);
@@ -1356,8 +1311,8 @@ __global__ void __launch_bounds__(128, kLightMinBlocks) k_reduce_light(ReduceArg
         const bool low_own = __shfl_sync(kFull, own ? 1 : 0, lead) != 0;
         const uint64_t e = __shfl_sync(kFull, (unsigned long long)ev, lead);
         const bool cleared = __shfl_sync(kFull, clr, lead) != 0;
-        bool claim = act && !cleared && !low_own && pv_col(e) > col;
-        bool round = act && !cleared && low_own && m <= kGroupGather;
+        const bool claim = act && !cleared && !low_own && pv_col(e) > col;
+        const bool round = act && !cleared && low_own && m <= kGroupGather;
         ovf = ovf || (act && !cleared && !claim && !round);
         // ---- one round for the groups whose lowest row has an owner
         if (__any_sync(kFull, round)) {
@@ -1420,8 +1375,7 @@ __global__ void __launch_bounds__(128, kLightMinBlocks) k_reduce_light(ReduceArg
         }
         // ---- what the group's column has come to
         const bool zero = col >= 0 && !ovf && (n == 0 || cleared);
-        const bool park = col >= 0 && !ovf && !zero && L < A.minrow;
-        const bool pub = dirty && (claim || park || ovf);
+        const bool pub = dirty && (claim || ovf);
         if (__any_sync(kFull, pub)) {  // one allocation for all groups
             const int want = pub && gl == 0 ? int(slot_ints(n)) : 0;
             const int inc = warp_inclusive_scan(want);
@@ -1454,7 +1408,7 @@ __global__ void __launch_bounds__(128, kLightMinBlocks) k_reduce_light(ReduceArg
             __syncwarp();
         }
         int next = -1;  // leader: the owner the claim displaced; col when the claim failed
-        if (gl == 0 && (claim || park || zero)) {
+        if (gl == 0 && (claim || zero)) {
             if (claim) {
                 // the column's final state goes out before the claim: a group
                 // that later displaces it writes its own state after this one
@@ -1472,10 +1426,6 @@ __global__ void __launch_bounds__(128, kLightMinBlocks) k_reduce_light(ReduceArg
                     n_disp++;
                     next = pv_col(e);
                 }
-            } else if (park) {
-                A.low[col] = L;
-                __threadfence();
-                st_release_u8(A.state + col, ST_ACTIVE);
             } else {
                 A.desc[col] = pack_desc(0, 0);
                 A.low[col] = -1;
@@ -1488,7 +1438,7 @@ __global__ void __launch_bounds__(128, kLightMinBlocks) k_reduce_light(ReduceArg
                 col = next;  // idle, or the displaced owner
                 displaced = next >= 0;
             }
-        } else if (park || zero) {
+        } else if (zero) {
             col = -1;
         }
         // ---- columns that outgrew their groups, one after another by the whole warp
@@ -1901,11 +1851,10 @@ int heavy_smem_bytes(int cap) { return (3 * cap + kHdr) * 4; }
 // work would only move parallel work onto the (fewer) CTAs.
 constexpr int32_t kLightChain = 8;
 
-static ReduceArgs make_args(const Device& D, const int32_t* active, int32_t minrow, int cap, int* ctr) {
+static ReduceArgs make_args(const Device& D, const int32_t* active, int cap, int* ctr) {
     ReduceArgs A;
     A.ncols = int32_t(D.n);
     A.active = active;
-    A.minrow = minrow;
     A.cap = cap;
     A.arena = D.arena;
     A.arena_cap = D.arena_cap;
@@ -1917,7 +1866,6 @@ static ReduceArgs make_args(const Device& D, const int32_t* active, int32_t minr
     A.cleared = D.cleared;
     A.ctr = ctr;
     A.ctr_next = nullptr;
-    A.count = nullptr;
     A.listed = 0;
     A.heavy = D.heavy;
     A.pool_tail = D.pool_tail;
@@ -1931,27 +1879,16 @@ static ReduceArgs make_args(const Device& D, const int32_t* active, int32_t minr
     return A;
 }
 
-int reduce_light_launch(const Device& D, int32_t beg, int32_t end, int32_t minrow, int cap, int* ctr, int* ctr_next,
-                        int filter_grid, int grid, cudaStream_t s) {
-    ReduceArgs A = make_args(D, D.runlist, minrow, cap, ctr);
+void reduce_light_launch(const Device& D, int32_t beg, int32_t end, int cap, int* ctr, int* ctr_next, int grid,
+                         cudaStream_t s) {
+    ReduceArgs A = make_args(D, D.active + beg, cap, ctr);
+    A.listed = end - beg;
     A.ctr_next = ctr_next;
-    if (minrow == INT32_MIN) {
-        // every column that is still active is runnable, and the warps look at the
-        // flags themselves: no list (it took 3-15 us and a launch)
-        A.active = D.active + beg;
-        A.count = nullptr;
-        A.listed = end - beg;
-    } else {
-        k_light_filter<<<filter_grid, kFilterThreads, 0, s>>>(D.active, beg, end, minrow, D.state, D.cleared, D.low,
-                                                              D.runlist, ctr);
-        A.count = ctr + 5;
-    }
     k_reduce_light<<<grid, 128, light_smem_bytes(cap), s>>>(A);
-    return A.count ? 2 : 1;
 }
 
 void reduce_heavy_launch(const Device& D, int cap, int threads, int* ctr, int grid, cudaStream_t s) {
-    ReduceArgs A = make_args(D, nullptr, INT32_MIN, cap, ctr);
+    ReduceArgs A = make_args(D, nullptr, cap, ctr);
     if (threads == 256) k_reduce_heavy<256><<<grid, 256, heavy_smem_bytes(cap), s>>>(A);
     else k_reduce_heavy<128><<<grid, 128, heavy_smem_bytes(cap), s>>>(A);
 }
@@ -1996,8 +1933,8 @@ cudaError_t queue_configure(int cap1, int cap2, int threads, int* blocks_per_sm)
 
 cudaError_t reduce_queue_launch(const Device& D, int cap1, int cap2, int threads, const QueueArgs& Q, int grid,
                                 cudaStream_t s) {
-    ReduceArgs Al = make_args(D, D.active, INT32_MIN, cap1, nullptr);
-    ReduceArgs Ah = make_args(D, nullptr, INT32_MIN, cap2, nullptr);
+    ReduceArgs Al = make_args(D, D.active, cap1, nullptr);
+    ReduceArgs Ah = make_args(D, nullptr, cap2, nullptr);
     Al.gate_host = Ah.gate_host = nullptr;
     Al.heavy_done = Ah.heavy_done = nullptr;
     QueueArgs q = Q;

@@ -34,13 +34,14 @@ __device__ __forceinline__ void scan_store(unsigned long long* p, unsigned long 
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// The 16 values of a lane (items lane + 32 k of its warp's 512) and their
-// exclusive prefixes within the warp.
+// The 16 values of a lane (items lane + 32 k of its warp's 512, which start at
+// `begin`) and their exclusive prefixes within the warp.
 template <class T>
 struct ScanLane {  // numbers
     T v[kScanItems], ex[kScanItems];
     template <class F>
-    __device__ __forceinline__ int64_t load(const F& value, int64_t first, int64_t n) {
+    __device__ __forceinline__ int64_t load(const F& value, int64_t begin, int64_t n) {
+        const int64_t first = begin + (threadIdx.x & 31);
 #pragma unroll
         for (int k = 0; k < kScanItems; k++) v[k] = first + 32 * k < n ? value(first + 32 * k) : T(0);
         T run = 0;
@@ -53,12 +54,16 @@ struct ScanLane {  // numbers
         return int64_t(run);
     }
     template <class G>
-    __device__ __forceinline__ void store(const G& sink, int64_t first, int64_t n, int64_t base) const {
+    __device__ __forceinline__ void store(const G& sink, int64_t begin, int64_t n, int64_t base) const {
+        const int64_t first = begin + (threadIdx.x & 31);
 #pragma unroll
         for (int k = 0; k < kScanItems; k++)
             if (first + 32 * k < n) sink(first + 32 * k, base + int64_t(ex[k]), v[k]);
     }
-    static __device__ __forceinline__ int64_t number(T x) { return int64_t(x); }
+    template <class F>
+    static __device__ __forceinline__ int64_t number(const F& value, int64_t i, int64_t n) {
+        return int64_t(value(i));
+    }
 };
 
 // A selection: class 1 and class 2 of the items are counted side by side, in the
@@ -73,7 +78,8 @@ struct ScanLane<ScanClass> {
     unsigned one[kScanItems], two[kScanItems];
     static __device__ __forceinline__ int64_t pack(int a, int b) { return int64_t(a) | (int64_t(b) << kScanClassShift); }
     template <class F>
-    __device__ __forceinline__ int64_t load(const F& value, int64_t first, int64_t n) {
+    __device__ __forceinline__ int64_t load(const F& value, int64_t begin, int64_t n) {
+        const int64_t first = begin + (threadIdx.x & 31);
         uint8_t c[kScanItems];
 #pragma unroll
         for (int k = 0; k < kScanItems; k++) c[k] = first + 32 * k < n ? value(first + 32 * k).c : 0;
@@ -88,9 +94,10 @@ struct ScanLane<ScanClass> {
         return pack(a, b);
     }
     template <class G>
-    __device__ __forceinline__ void store(const G& sink, int64_t first, int64_t n, int64_t base) const {
+    __device__ __forceinline__ void store(const G& sink, int64_t begin, int64_t n, int64_t base) const {
         const unsigned lt = lanemask_lt();
         const int lane = threadIdx.x & 31;
+        const int64_t first = begin + lane;
 #pragma unroll
         for (int k = 0; k < kScanItems; k++) {
             const ScanClass v{uint8_t(((one[k] >> lane) & 1) | (((two[k] >> lane) & 1) << 1))};
@@ -98,7 +105,54 @@ struct ScanLane<ScanClass> {
             base += pack(__popc(one[k]), __popc(two[k]));
         }
     }
-    static __device__ __forceinline__ int64_t number(ScanClass x) { return pack(x.c == 1, x.c == 2); }
+    template <class F>
+    static __device__ __forceinline__ int64_t number(const F& value, int64_t i, int64_t n) {
+        const ScanClass x = value(i);
+        return pack(x.c == 1, x.c == 2);
+    }
+};
+
+// Selection by a byte array (16-byte aligned): items whose byte equals `want`.  A
+// lane takes 16 consecutive items with one load; the sink sees selected items only.
+struct ScanBytes {
+    const uint8_t* p;
+    uint8_t want;
+    __device__ __forceinline__ ScanBytes operator()(int64_t) const { return *this; }
+};
+template <>
+struct ScanLane<ScanBytes> {
+    unsigned sel;  // bit k: item 16 * lane + k
+    int pre;
+    template <class F>
+    __device__ __forceinline__ int64_t load(const F& value, int64_t begin, int64_t n) {
+        const int64_t first = begin + 16 * (threadIdx.x & 31);
+        sel = 0;
+        if (first + 16 <= n) {
+            const uint4 q = *reinterpret_cast<const uint4*>(value.p + first);
+            const unsigned w[4] = {q.x, q.y, q.z, q.w}, all = value.want * 0x01010101u;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const unsigned eq = __vcmpeq4(w[k], all) & 0x08040201u;  // one bit of each equal byte
+                sel |= ((eq | eq >> 8 | eq >> 16 | eq >> 24) & 15u) << (4 * k);
+            }
+        } else {
+            for (int k = 0; k < 16; k++)
+                if (first + k < n && value.p[first + k] == value.want) sel |= 1u << k;
+        }
+        const int cnt = __popc(sel), inc = warp_inclusive_scan(cnt);
+        pre = inc - cnt;
+        return __shfl_sync(kFull, inc, 31);
+    }
+    template <class G>
+    __device__ __forceinline__ void store(const G& sink, int64_t begin, int64_t, int64_t base) const {
+        const int64_t first = begin + 16 * (threadIdx.x & 31);
+        base += pre;
+        for (unsigned m = sel; m; m &= m - 1) sink(first + __ffs(m) - 1, base++);
+    }
+    template <class F>
+    static __device__ __forceinline__ int64_t number(const F& value, int64_t i, int64_t n) {
+        return value.p[i] == value.want;
+    }
 };
 
 template <class F, class G, class H>
@@ -113,9 +167,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(F value, G sink, H done, 
     unsigned long long* state = reinterpret_cast<unsigned long long*>(blk);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t tile = blockIdx.x;
-    const int64_t first = tile * kScanTile + int64_t(wid) * (32 * kScanItems) + lane;
+    const int64_t begin = tile * kScanTile + int64_t(wid) * (32 * kScanItems);
     Lane items;
-    const int64_t run = items.load(value, first, n);
+    const int64_t run = items.load(value, begin, n);
     if (lane == 0) s_warp[wid] = run;
     __syncthreads();
     int64_t mine = 0, sum = 0;  // sums of the warps before this one, and of the tile
@@ -151,7 +205,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(F value, G sink, H done, 
                 if (++polls < kScanPolls) continue;
                 // the predecessors do not answer: add their values up here
                 base = 0;
-                for (int64_t i = threadIdx.x; i < tile * kScanTile; i += kScanThreads) base += Lane::number(value(i));
+                for (int64_t i = threadIdx.x; i < tile * kScanTile; i += kScanThreads) base += Lane::number(value, i, n);
                 base = warp_sum(base);
                 __syncthreads();
                 if (lane == 0) s_look[wid] = base;
@@ -172,7 +226,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(F value, G sink, H done, 
             done(base + sum);
         }
     }
-    items.store(sink, first, n, base + mine);
+    items.store(sink, begin, n, base + mine);
 }
 
 struct ScanNoop {
