@@ -43,7 +43,7 @@ void fill_i64(int64_t* p, int64_t v, int64_t n, cudaStream_t s) {
 // non-decreasing from 0 to nnz (device-resident inputs are only checked here).
 // The same pass counts the columns of each dimension, per tile for the reorder
 // (dimcnt) and in total for the host (dimtot, zeroed before), and finds the
-// longest column.  It also starts the init passes' state of every column, in
+// longest column, and whether an edge has more than two faces.  It also starts the init passes' state of every column, in
 // order: no leftmost column yet, no pivot owner, not cleared, not negative.  A warp
 // takes 32 * kPartRounds consecutive columns.
 constexpr int kPartThreads = 256;
@@ -56,14 +56,14 @@ __global__ void __launch_bounds__(kPartThreads) k_validate(const int32_t* dims, 
                                                            int64_t nnz, int32_t* dimcnt, Ctl* ctl, int32_t* leftmost,
                                                            uint64_t* pivot, uint8_t* cleared, uint8_t* negative) {
     __shared__ int s_cnt[kNumDims];
-    __shared__ int s_len, s_bad;
+    __shared__ int s_len, s_bad, s_wide;
     if (threadIdx.x < kNumDims) s_cnt[threadIdx.x] = 0;
-    if (threadIdx.x == 0) s_len = s_bad = 0;
+    if (threadIdx.x == 0) s_len = s_bad = s_wide = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int64_t j0 = int64_t(blockIdx.x) * kPartTile + (threadIdx.x >> 5) * (32 * kPartRounds) + lane;
     int mine = 0, longest = 0;
-    bool bad = false;
+    bool bad = false, wide = false;
 #pragma unroll
     for (int k = 0; k < kPartRounds; k++) {
         const int64_t j = j0 + 32 * k;
@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(kPartThreads) k_validate(const int32_t* dims, 
                 bad = true;
             else
                 longest = max(longest, int(len));
+            wide = wide || (d == 1 && len > 2);
             leftmost[j] = INT_MAX;
             pivot[j] = kNoOwner;
             cleared[j] = 0;
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(kPartThreads) k_validate(const int32_t* dims, 
     longest = __reduce_max_sync(kFull, longest);
     if (lane == 0 && longest) atomicMax(&s_len, longest);
     if (bad) s_bad = 1;
+    if (wide) s_wide = 1;
     __syncthreads();
     if (threadIdx.x < kNumDims) {
         const int c = s_cnt[threadIdx.x];
@@ -99,6 +101,7 @@ __global__ void __launch_bounds__(kPartThreads) k_validate(const int32_t* dims, 
     if (threadIdx.x == 0) {
         if (s_len > 0) atomicMax(&ctl->max_len, s_len);
         if (s_bad) atomicOr(&ctl->err, ERRB_BAD_INPUT);
+        if (s_wide) ctl->wide_edges = 1;
     }
 }
 
@@ -734,6 +737,8 @@ struct PairsOut {
     longlong2* pairs;
     int64_t* ess;
     long long* counters;
+    int* err;
+    const DimInfo* edges;  // edges reduced beside the dimensions above them: the column ranges; otherwise null
 };
 constexpr int64_t kBirths = (int64_t(1) << kScanClassShift) - 1;  // class 1: births, class 2: essentials
 
@@ -743,6 +748,8 @@ struct PairsValue {
         const int32_t i = o.newidx[j];
         const uint64_t e = o.pivot[i];
         const uint8_t st = o.state[i];
+        if (o.edges && e != kNoOwner && st == ST_OWNER && i >= o.edges->col_begin[1] && i < o.edges->col_end[1])
+            atomicOr(o.err, ERRB_ORDER);
         return {uint8_t(e != kNoOwner ? 1 : (st == ST_OWNER || st == ST_DROPPED ? 0 : 2))};
     }
 };
@@ -785,7 +792,8 @@ __global__ void k_mark_dropped(int64_t n, const uint8_t* dropped, const int32_t*
 int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s) {
     const int64_t n = D.n;
     longlong2* pairs = reinterpret_cast<longlong2*>(D.pairs);
-    const PairsOut o{n, D.newidx, D.perm, D.pivot, D.state, pairs, D.ess, D.counters};
+    const PairsOut o{n, D.newidx, D.perm, D.pivot, D.state, pairs, D.ess, D.counters, D.err,
+                     D.edges_beside ? &D.ctl->info : nullptr};
     bool zeroed;
     int64_t* blk = scan_region(D, 2, &zeroed);
     if (!dual) {

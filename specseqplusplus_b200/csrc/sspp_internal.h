@@ -56,6 +56,7 @@ enum : int {
     ERRB_LEN = 8,       // a column exceeded kMaxColLen
     ERRB_CHECK = 16,    // a self-check of the reduction failed (bad index skipped)
     ERRB_FACES = 32,    // malformed input faces, found while the columns are copied
+    ERRB_ORDER = 64,    // an edge both owns a row and is one's (see sspp_edges.cu): run again in order
 };
 
 // Per-dimension summary after the init passes (in reordered numbering).
@@ -97,6 +98,7 @@ struct Ctl {
     unsigned long long dimtot[kNumDims];  // input columns per dimension (validation pass)
     int err;
     int max_len;      // longest input column (validation pass)
+    int wide_edges;   // a column of dimension 1 holds more than two entries (validation pass)
     int pool_tail;    // CTA-tier pool entries
     int heavy_done;   // pool columns the CTA tier has finished
     int step[kNumDims * kStepCtr];
@@ -141,6 +143,7 @@ struct Device {
     int64_t* blk = nullptr;      // region 0
     int64_t blk_stride = 0;      // entries per region
     unsigned blk_zero = 0;       // regions still as cleared (bits)
+    bool edges_beside = false;   // the edges were reduced beside the dimensions above them
     bool steps_zero = false;     // Ctl::pool_tail, heavy_done and step still as cleared
     int64_t cap_blk = 0;
     int32_t* dimcnt = nullptr;   // [nblocks * kNumDims]

@@ -48,6 +48,9 @@ int build_apparent(Device& D, cudaStream_t s);
 // mode 1: the whole matrix; mode 2: after the edge columns were reduced (the
 // 0-dimensional pairs are final, the vertices' dual columns are skipped)
 int dualize(Device& D, int mode, cudaStream_t s);
+// dimension 1 of the boundary matrix (active list entries [beg, end), no column of
+// more than two entries) over the vertices, the reordered rows [0, rows)
+int reduce_edges(Device& D, int32_t beg, int32_t end, int32_t rows, cudaStream_t s);
 int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s);
 
 // Device work queue of (complex, block) items (one persistent launch per
