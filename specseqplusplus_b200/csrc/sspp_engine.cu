@@ -69,6 +69,8 @@ struct Prof {
 };
 }  // namespace
 
+constexpr int64_t kPushCols = int64_t(1) << 16;  // up to here results go to pinned memory at once (1 MB of it)
+
 struct sspp_ctx {
     sspp_config cfg{};
     std::string err;
@@ -99,6 +101,11 @@ struct sspp_ctx {
     double init_ms = 0, compute_ms = 0;
     int64_t ss_steps = 0;
     Ctl* h_ctl = nullptr;          // pinned mirror of Device::ctl
+    int64_t* h_pairs = nullptr;    // pinned: the results of up to kPushCols columns (push_results)
+    int64_t* h_ess = nullptr;
+    bool pushed = false;           // they hold the last reduction's
+    cudaEvent_t load_ev = nullptr; // the last load on own_stream that was not waited for
+    bool loading = false;
     int* h_err = nullptr;          // pinned
     int* h_gate = nullptr;         // mapped pinned: CTA-tier pool columns finished (mirror)
     int* d_gate = nullptr;         // its device address
@@ -952,7 +959,14 @@ int run_compute(sspp_ctx* ctx) {
     ctx->launches += extract_pairs(D, P.dualize != 0, dropped_of(ctx), s);
     span_end(ctx, PH_PAIRS, ep);
     CK(cudaGetLastError());
-    if (int rc = read_ctl(ctx)) return rc;
+    ctx->pushed = D.n <= kPushCols;
+    if (ctx->pushed) {
+        ctx->launches += push_results(D, ctx->h_ctl, ctx->h_pairs, kPushCols / 2, ctx->h_ess, kPushCols, s);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(s));
+    } else if (int rc = read_ctl(ctx)) {
+        return rc;
+    }
     std::memcpy(ctx->hcounters, ctx->h_ctl->counters, sizeof(ctx->hcounters));
     ctx->arena_used = int64_t(ctx->h_ctl->arena_top);
     ctx->compute_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -1165,10 +1179,14 @@ sspp_ctx* sspp_create(const sspp_config* cfg) {
     }
     if (cudaMallocHost(&ctx->h_err, sizeof(int)) != cudaSuccess ||
         cudaMallocHost(&ctx->h_ctl, sizeof(Ctl)) != cudaSuccess ||
+        cudaMallocHost(&ctx->h_pairs, sizeof(int64_t) * 2 * kPushCols) != cudaSuccess ||
+        ctx->xfer.reserve_small() != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->load_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaMallocHost(&ctx->h_top, sizeof(int64_t)) != cudaSuccess) {
         delete ctx;
         return nullptr;
     }
+    ctx->h_ess = ctx->h_pairs + kPushCols;
     sspp_default_params(&ctx->params);
     return ctx;
 }
@@ -1216,6 +1234,8 @@ void sspp_destroy(sspp_ctx* ctx) {
     if (ctx->hc_fork) cudaEventDestroy(ctx->hc_fork);
     if (ctx->hc_join) cudaEventDestroy(ctx->hc_join);
     if (ctx->h_ctl) cudaFreeHost(ctx->h_ctl);
+    if (ctx->h_pairs) cudaFreeHost(ctx->h_pairs);
+    if (ctx->load_ev) cudaEventDestroy(ctx->load_ev);
     if (ctx->h_top) cudaFreeHost(ctx->h_top);
     delete ctx;
 }
@@ -1241,7 +1261,14 @@ int32_t sspp_load_csc(sspp_ctx* ctx, int64_t ncols, const int32_t* dims, const i
                                     {col_ptr, ctx->own_colptr, sizeof(int64_t) * size_t(ncols + 1)},
                                     {rows, ctx->own_rows, sizeof(int32_t) * size_t(nnz)}};
     CK(ctx->xfer.h2d(pcs, s));
-    CK(cudaStreamSynchronize(s));
+    // the caller's arrays have been read; what still runs is waited for by the stream
+    // that init is given (a caller's stream may be gone by then)
+    if (s == ctx->own_stream) {
+        CK(cudaEventRecord(ctx->load_ev, s));
+        ctx->loading = true;
+    } else {
+        CK(cudaStreamSynchronize(s));
+    }
     ctx->D.in_dims = ctx->own_dims;
     ctx->D.in_colptr = ctx->own_colptr;
     ctx->D.in_rows = ctx->own_rows;
@@ -1702,6 +1729,8 @@ int32_t sspp_init(sspp_ctx* ctx, const sspp_params* p, void* stream) {
     ctx->tune_locked = false;
     ctx->edges_last = false;
     ctx->stream = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
+    if (ctx->loading && ctx->stream != ctx->own_stream) CK(cudaStreamWaitEvent(ctx->stream, ctx->load_ev, 0));
+    ctx->loading = false;
     return run_init(ctx);
 }
 
@@ -1747,6 +1776,10 @@ int64_t sspp_pairs(sspp_ctx* ctx, int64_t* out, int64_t cap) {
     if (!ctx || !ctx->computed || cap < 0 || (!out && cap > 0)) return -1;
     cudaSetDevice(ctx->cfg.device);
     int64_t n = std::min<int64_t>(cap, ctx->hcounters[CNT_NPAIRS]);
+    if (n > 0 && ctx->pushed && host_memory(out)) {
+        std::memcpy(out, ctx->h_pairs, sizeof(int64_t) * 2 * size_t(n));
+        return n;
+    }
     if (n > 0 && ctx->xfer.d2h({{ctx->D.pairs, out, sizeof(int64_t) * 2 * size_t(n)}}, ctx->stream) != cudaSuccess) {
         set_err(ctx, SSPP_ERR_CUDA, "pairs copy failed");
         return -1;
@@ -1763,6 +1796,10 @@ int64_t sspp_essentials(sspp_ctx* ctx, int64_t* out, int64_t cap) {
     if (!ctx || !ctx->computed || cap < 0 || (!out && cap > 0)) return -1;
     cudaSetDevice(ctx->cfg.device);
     int64_t n = std::min<int64_t>(cap, ctx->hcounters[CNT_NESS]);
+    if (n > 0 && ctx->pushed && host_memory(out)) {
+        std::memcpy(out, ctx->h_ess, sizeof(int64_t) * size_t(n));
+        return n;
+    }
     if (n > 0 && cudaMemcpy(out, ctx->D.ess, sizeof(int64_t) * n, cudaMemcpyDeviceToHost) != cudaSuccess) {
         set_err(ctx, SSPP_ERR_CUDA, "essentials copy failed");
         return -1;

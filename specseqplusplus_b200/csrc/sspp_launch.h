@@ -48,6 +48,10 @@ int build_apparent(Device& D, cudaStream_t s);
 // mode 1: the whole matrix; mode 2: after the edge columns were reduced (the
 // 0-dimensional pairs are final, the vertices' dual columns are skipped)
 int dualize(Device& D, int mode, cudaStream_t s);
+// the control block up to its step counters and, as far as they fit, the pairs and
+// essentials into host memory that the device can write
+int push_results(const Device& D, Ctl* h_ctl, int64_t* h_pairs, int64_t max_pairs, int64_t* h_ess, int64_t max_ess,
+                 cudaStream_t s);
 // dimension 1 of the boundary matrix (active list entries [beg, end), no column of
 // more than two entries) over the vertices, the reordered rows [0, rows)
 int reduce_edges(Device& D, int32_t beg, int32_t end, int32_t rows, cudaStream_t s);

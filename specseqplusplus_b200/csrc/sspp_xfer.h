@@ -47,6 +47,9 @@ struct Piece {
     int group = -1;
 };
 
+// whether p is memory that the host itself reads and writes, pinned or not
+bool host_memory(const void* p);
+
 class Xfer {
 public:
     Xfer() = default;
@@ -58,6 +61,8 @@ public:
     cudaError_t h2d(const std::vector<Piece>& pieces, cudaStream_t s);
     // device -> host; returns when every byte has landed in host memory
     cudaError_t d2h(const std::vector<Piece>& pieces, cudaStream_t s);
+    // the pinned buffer of small copies; at creation, so that no request pays for it
+    cudaError_t reserve_small();
     HostPool& pool();
     void set_threads(int n) { threads_ = n; }  // before the first copy; 0 = all cores
 
@@ -69,6 +74,10 @@ private:
     // `least`: smallest share of one host thread
     void parallel_copy(const std::vector<Piece>& pieces, const std::vector<Seg>& segs, size_t fill, uint8_t* stage,
                        bool to_stage, size_t least);
+    cudaError_t fetch_small(const std::vector<Piece>& pieces, cudaStream_t s);
+    uint8_t* small_ = nullptr;  // pinned, for copies that one kernel fetches
+    cudaEvent_t small_ev_ = nullptr;
+    bool small_used_ = false;
     uint8_t* stage_ = nullptr;  // pinned, two halves
     size_t half_ = 0;
     cudaEvent_t ev_[2] = {nullptr, nullptr};
