@@ -558,10 +558,10 @@ int run_init(sspp_ctx* ctx) {
     if (guided) CK(cudaStreamWaitEvent(s, ctx->hc_join, 0));
     ctx->launches += init_compress(D, dropped_of(ctx), ctx->params.representatives != 0, ctx->params.dualize != 1, s);
     if (ctx->params.dualize == 1) {
-        ctx->launches += dualize(D, 1, s);
-        ctx->launches += build_apparent(D, s);
+        ctx->launches += dualize_begin(D, 1, s);
+        ctx->launches += dualize_end(D, 1, s);
     }
-    ctx->launches += active_list(D, ctx->params.dualize != 1, s);
+    ctx->launches += active_list(D, s);
     span_end(ctx, PH_INIT, ev0);
     CK(cudaGetLastError());
     if ((rc = read_ctl(ctx))) return rc;
@@ -937,12 +937,29 @@ int run_compute(sspp_ctx* ctx) {
     };
     int64_t nsteps = 0;
     if (P.dualize == 2) {
-        int rc = phase(1, 1, false);
-        if (rc) return rc;
+        // the edges' own reduction runs beside the dualization's first part
+        int rc = SSPP_OK;
+        const DimInfo& I = ctx->hinfo;
+        const bool beside = !queue && !ctx->h_ctl->wide_edges && I.act_end[1] > I.act_begin[1];
+        if (beside) {
+            cudaStream_t es = ctx->side[0];
+            CK(cudaEventRecord(ctx->step_ev[0], s));
+            CK(cudaStreamWaitEvent(es, ctx->step_ev[0], 0));
+            cudaEvent_t ev = nullptr;
+            span_begin(ctx, ev, es);
+            ctx->launches += reduce_edges(D, I.act_begin[1], I.act_end[1], I.col_end[0], es);
+            span_end(ctx, PH_LIGHT, ev, es);
+            CK(cudaEventRecord(ctx->join_ev[0], es));
+            ctx->light_launches++;
+            ctx->ss_steps = 1;
+        } else if ((rc = phase(1, 1, false))) {
+            return rc;
+        }
         nsteps += ctx->ss_steps;
-        ctx->launches += dualize(D, 2, s);
-        ctx->launches += build_apparent(D, s);
-        ctx->launches += active_list(D, false, s);
+        ctx->launches += dualize_begin(D, 2, s);
+        if (beside) CK(cudaStreamWaitEvent(s, ctx->join_ev[0], 0));
+        ctx->launches += dualize_end(D, 2, s);
+        ctx->launches += active_list(D, s);
         if ((rc = read_ctl(ctx))) return rc;
         ctx->hinfo = ctx->h_ctl->info;
         rc = phase(1, kMaxDim, true);

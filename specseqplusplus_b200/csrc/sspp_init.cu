@@ -615,37 +615,6 @@ __global__ void k_init_compress(int64_t n, int32_t* arena, uint64_t* desc, int32
     }
 }
 
-// per-dimension min first row over non-empty columns and max low + 1 over
-// active columns (ColumnShrink, include/specseq.h:374-398)
-__global__ void k_dim_rows(int64_t n, const int32_t* rdim, const int32_t* arena, const uint64_t* desc,
-                           const int32_t* low, const uint8_t* state, DimInfo* info) {
-    __shared__ int smin[kNumDims], smax[kNumDims], sact[kNumDims];
-    if (threadIdx.x < kNumDims) { smin[threadIdx.x] = INT_MAX; smax[threadIdx.x] = -1; sact[threadIdx.x] = 0; }
-    __syncthreads();
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        uint64_t d = desc[i];
-        uint32_t len = desc_len(d);
-        if (!len) continue;
-        int dm = rdim[i];
-        atomicMin(&smin[dm], arena[desc_off(d) + kHdr]);
-        if (state[i] == ST_ACTIVE) {
-            atomicMax(&smax[dm], low[i] + 1);
-            atomicAdd(&sact[dm], 1);
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < kNumDims) {
-        if (smin[threadIdx.x] != INT_MAX) atomicMin(&info->min_row[threadIdx.x], smin[threadIdx.x]);
-        if (smax[threadIdx.x] >= 0) atomicMax(&info->max_row[threadIdx.x], smax[threadIdx.x]);
-        if (sact[threadIdx.x]) atomicAdd(&info->act_end[threadIdx.x], sact[threadIdx.x]);
-    }
-}
-
-__global__ void k_diminfo_reset(DimInfo* info) {
-    int d = threadIdx.x;
-    if (d < kNumDims) { info->min_row[d] = INT_MAX; info->max_row[d] = -1; info->act_end[d] = 0; }
-}
-
 int init_passes(Device& D, bool lows_done, cudaStream_t s) {
     const int64_t n = D.n;
     const unsigned g = grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256);
@@ -663,42 +632,11 @@ int init_compress(Device& D, const uint8_t* dropped, bool keep_rows, bool final,
     return 1;
 }
 
-// Inline copies of the short apparent columns, by row (see Device::app).
-__global__ void k_build_apparent(int64_t n, const uint64_t* pivot, const int32_t* arena, int4* app) {
-    for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n; r += int64_t(gridDim.x) * blockDim.x) {
-        int4 v = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
-        const uint64_t e = pivot[r];
-        if (e != kNoOwner) {
-            const int32_t* h = arena + pv_slot(e);
-            const int len = h[0];
-            if (len >= 1 && len <= 4 && h[kHdr + len - 1] == int32_t(r)) {
-                v.x = len - 1;
-                if (len > 1) v.y = h[kHdr];
-                if (len > 2) v.z = h[kHdr + 1];
-                if (len > 3) v.w = h[kHdr + 2];
-            }
-        }
-        app[r] = v;
-    }
-}
-
-int build_apparent(Device& D, cudaStream_t s) {
-    const int64_t n = D.n;
-    if (n == 0) return 0;
-    k_build_apparent<<<grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256), 256, 0, s>>>(n, D.pivot, D.arena, D.app);
-    return 1;
-}
-
 // Active list in reordered order (dimension segments are contiguous).  act_end
 // holds each dimension's count of active columns, gathered with the row bounds;
 // the scan's end turns the counts into segments.
-int active_list(Device& D, bool rows_done, cudaStream_t s) {
+int active_list(Device& D, cudaStream_t s) {
     const int64_t n = D.n;
-    if (!rows_done) {
-        k_diminfo_reset<<<1, 32, 0, s>>>(D.diminfo);
-        const unsigned g = grid_for(n, 256) > 4096 ? 4096 : grid_for(n, 256);
-        k_dim_rows<<<g, 256, 0, s>>>(n, D.dim, D.arena, D.desc, D.low, D.state, D.diminfo);
-    }
     int32_t* act = D.active;
     DimInfo* info = D.diminfo;
     bool zeroed;
@@ -717,7 +655,7 @@ int active_list(Device& D, bool rows_done, cudaStream_t s) {
              }
          },
          zeroed);
-    return rows_done ? 1 : 3;
+    return 1;
 }
 
 // ------------------------------------------------------------------- pairs

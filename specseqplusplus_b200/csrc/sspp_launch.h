@@ -36,18 +36,19 @@ int batch_localize(int64_t npairs, int64_t ness, int32_t k, const int64_t* d_cst
 int init_passes(Device& D, bool lows_done, cudaStream_t s);
 // keep_rows: leave negative rows in the columns (whole reduced columns, for
 // representative cycles); otherwise they are removed.
-// final (no dualization follows): also the inline apparent columns (as
-// build_apparent) and the per-dimension row bounds (as active_list)
+// final (no dualization follows at once): also the inline apparent columns, the
+// per-dimension row bounds and the counts of active columns
 int init_compress(Device& D, const uint8_t* dropped, bool keep_rows, bool final, cudaStream_t s);
-// rows_done: init_compress already gathered the row bounds
-int active_list(Device& D, bool rows_done, cudaStream_t s);
-// D.app from the pivot table as it stands (apparent pairs only)
-int build_apparent(Device& D, cudaStream_t s);
+// (the row bounds and the counts of active columns were gathered with the states)
+int active_list(Device& D, cudaStream_t s);
 // anti-transpose of the compressed matrix behind the primal columns in the
-// arena; remaps pivots, states, dims and the per-dimension column ranges.
+// arena; remaps pivots, states, dims, inline columns, row bounds and the
+// per-dimension column ranges.
 // mode 1: the whole matrix; mode 2: after the edge columns were reduced (the
-// 0-dimensional pairs are final, the vertices' dual columns are skipped)
-int dualize(Device& D, int mode, cudaStream_t s);
+// 0-dimensional pairs are final, the vertices' dual columns are skipped).  The
+// first part reads no edge column in mode 2, so their reduction may still run.
+int dualize_begin(Device& D, int mode, cudaStream_t s);
+int dualize_end(Device& D, int mode, cudaStream_t s);
 // the control block up to its step counters and, as far as they fit, the pairs and
 // essentials into host memory that the device can write
 int push_results(const Device& D, Ctl* h_ctl, int64_t* h_pairs, int64_t max_pairs, int64_t* h_ess, int64_t max_ess,

@@ -365,7 +365,7 @@ cudaError_t reduce_in_scratch(int32_t* scratch, int dev, int64_t n, int64_t nnz,
     reorder(D, true, false, s);
     init_passes(D, true, s);
     init_compress(D, nullptr, true, true, s);
-    active_list(D, true, s);
+    active_list(D, s);
     cudaMemcpyAsync(&h, D.ctl, offsetof(Ctl, step), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
     if (h.err) return cudaSuccess;
