@@ -61,29 +61,6 @@ __device__ __forceinline__ void tuple_union(int d, int32_t c0, int32_t c1, int32
     }
 }
 
-// Vertex tuple of every column of dimension d >= 1 (sorted, d+1 vertices),
-// from the first two facets' tuples.  tup_d / tup_f point at the tuple arrays of
-// dims d and d-1 (dim-0 tuples are the vertex indices themselves).  Columns come
-// from their slots, which lie in this kernel's order (short columns: without their
-// descriptors); read from the input columns through the index maps instead, so
-// that it could start before the slots were written, this took 182 us at 64^3 and
-// slowed the passes beside it.
-__global__ void k_tuples(int32_t cb, int32_t ce, int d, int32_t fb, const int32_t* arena, const uint64_t* desc,
-                         const Ctl* ctl, const int32_t* tup_f, int32_t* tup_d) {
-    const bool all_short = ctl->max_len <= kShortLen;
-    for (int64_t i = cb + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < ce; i += int64_t(gridDim.x) * blockDim.x) {
-        const int32_t* slot = arena + (all_short ? int64_t(kShortSlot) * i : int64_t(desc_off(desc[i])));
-        const int len = all_short ? slot[0] : int(desc_len(desc[i]));
-        int32_t* out = tup_d + (i - cb) * (d + 1);
-        if (len != d + 1) {
-            // not a simplicial boundary (edge with < 2 vertices etc.): no tuple
-            for (int k = 0; k <= d; k++) out[k] = -1;
-            continue;
-        }
-        tuple_union(d, slot[kHdr], slot[kHdr + 1], fb, tup_f, out);
-    }
-}
-
 __device__ __forceinline__ uint32_t tuple_hash(const int32_t* t, int k) {
     uint64_t h = 0x9E3779B97F4A7C15ull;
     for (int i = 0; i < k; i++) {
@@ -94,16 +71,44 @@ __device__ __forceinline__ uint32_t tuple_hash(const int32_t* t, int k) {
     return uint32_t(h);
 }
 
-__global__ void k_hash_insert(int32_t cb, int32_t ce, int k, const int32_t* tup, const uint8_t* dropped, int32_t* table,
-                              uint32_t mask) {
+// Vertex tuple of every column of dimension d >= 1 (sorted, d+1 vertices),
+// from the first two facets' tuples.  tup_d / tup_f point at the tuple arrays of
+// dims d and d-1 (dim-0 tuples are the vertex indices themselves).  Columns come
+// from their slots, which lie in this kernel's order (short columns: without their
+// descriptors); read from the input columns through the index maps instead, so
+// that it could start before the slots were written, this took 182 us at 64^3 and
+// slowed the passes beside it.  The tuples of surviving edges are counted into their
+// vertices' degrees (deg), those of surviving top-dimension simplices entered into the
+// hash table (table), where they are at hand.
+__global__ void k_tuples(int32_t cb, int32_t ce, int d, int32_t fb, const int32_t* arena, const uint64_t* desc,
+                         const Ctl* ctl, const int32_t* tup_f, int32_t* tup_d, const uint8_t* dropped, int32_t* deg,
+                         int32_t* table, uint32_t mask) {
+    const bool all_short = ctl->max_len <= kShortLen;
     for (int64_t i = cb + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < ce; i += int64_t(gridDim.x) * blockDim.x) {
-        const int32_t* t = tup + (i - cb) * k;
+        const int32_t* slot = arena + (all_short ? int64_t(kShortSlot) * i : int64_t(desc_off(desc[i])));
+        const int len = all_short ? slot[0] : int(desc_len(desc[i]));
+        int32_t* out = tup_d + (i - cb) * (d + 1);
+        if (len != d + 1) {
+            // not a simplicial boundary (edge with < 2 vertices etc.): no tuple
+            for (int k = 0; k <= d; k++) out[k] = -1;
+            continue;
+        }
+        int32_t t[kMaxDim + 1];
+        tuple_union(d, slot[kHdr], slot[kHdr + 1], fb, tup_f, t);
+#pragma unroll
+        for (int k = 0; k <= kMaxDim; k++)
+            if (k <= d) out[k] = t[k];
         if (t[0] < 0 || (dropped && dropped[i])) continue;
-        uint32_t h = tuple_hash(t, k) & mask;
-        for (uint32_t probe = 0; probe <= mask; probe++) {
-            int32_t old = atomicCAS(table + h, -1, int32_t(i));
-            if (old == -1) break;
-            h = (h + 1) & mask;
+        if (deg) {
+            atomicAdd(deg + t[0], 1);
+            atomicAdd(deg + t[1], 1);
+        }
+        if (table) {
+            uint32_t h = tuple_hash(t, d + 1) & mask;
+            for (uint32_t probe = 0; probe <= mask; probe++) {
+                if (atomicCAS(table + h, -1, int32_t(i)) == -1) break;
+                h = (h + 1) & mask;
+            }
         }
     }
 }
@@ -126,15 +131,6 @@ __device__ int32_t hash_find(const int32_t* t, int k, const int32_t* table, uint
 
 // adjacency of the vertices (reordered vertex index = column index in [0, V))
 // (edges from their vertex tuples, tup1 = tuples of dimension 1)
-__global__ void k_degree(int32_t eb, int32_t ee, const int32_t* tup1, const uint8_t* dropped, int32_t* deg) {
-    for (int64_t i = eb + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < ee; i += int64_t(gridDim.x) * blockDim.x) {
-        const int2 c = reinterpret_cast<const int2*>(tup1)[i - eb];
-        if (c.x < 0 || (dropped && dropped[i])) continue;
-        atomicAdd(deg + c.x, 1);
-        atomicAdd(deg + c.y, 1);
-    }
-}
-
 __global__ void k_adj_fill(int32_t eb, int32_t ee, const int32_t* tup1, const uint8_t* dropped, const int64_t* adj_off,
                            int32_t* fill, int32_t* adj, int32_t* src) {
     for (int64_t i = eb + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < ee; i += int64_t(gridDim.x) * blockDim.x) {
@@ -416,27 +412,33 @@ __global__ void __launch_bounds__(kHcThreads) k_highclear(int32_t cb, int32_t ce
 }
 
 int highclear(Device& D, const DimInfo& info, int max_iteration, const uint8_t* dropped, HighclearScratch& S,
-              cudaStream_t s) {
+              cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEvent_t join) {
     // top dimension with columns
     int top = -1;
     for (int d = kMaxDim; d >= 1; d--)
         if (info.col_end[d] > info.col_begin[d]) { top = d; break; }
     if (top < 1 || max_iteration <= 0) return 0;
     int launches = 0;
-    // tuples of dims 1..top
-    const int32_t* prev = nullptr;
-    for (int d = 1; d <= top; d++) {
-        int32_t cb = info.col_begin[d], ce = info.col_end[d];
-        k_tuples<<<gridn(ce - cb, 256), 256, 0, s>>>(cb, ce, d, info.col_begin[d - 1], D.arena, D.desc, D.ctl, prev,
-                                                    S.tup[d]);
-        launches++;
-        prev = S.tup[d];
-    }
-    // adjacency
     const int64_t nv = info.col_end[0] - info.col_begin[0];
     cudaMemsetAsync(S.deg, 0, sizeof(int32_t) * (nv + 1), s);
-    k_degree<<<gridn(info.col_end[1] - info.col_begin[1], 256), 256, 0, s>>>(info.col_begin[1], info.col_end[1],
-                                                                            S.tup[1], dropped, S.deg);
+    cudaMemsetAsync(S.table, 0xff, sizeof(int32_t) * (size_t(S.mask) + 1), s);
+    // tuples of dims 1..top
+    auto tuples = [&](int d, cudaStream_t st) {
+        const int32_t cb = info.col_begin[d], ce = info.col_end[d];
+        k_tuples<<<gridn(ce - cb, 256), 256, 0, st>>>(cb, ce, d, info.col_begin[d - 1], D.arena, D.desc, D.ctl,
+                                                     d > 1 ? S.tup[d - 1] : nullptr, S.tup[d], dropped,
+                                                     d == 1 ? S.deg : nullptr, d == top ? S.table : nullptr, S.mask);
+        launches++;
+    };
+    tuples(1, s);
+    // The edges' adjacency and the higher tuples need nothing of one another: side by
+    // side (init of 64^3 1,056 us one after another, with the degrees and the hash table
+    // in passes of their own, 995 like this; 33^3 289 -> 245, 6^3 135 -> 114).
+    cudaEventRecord(fork, s);
+    cudaStreamWaitEvent(s2, fork, 0);
+    for (int d = 2; d <= top; d++) tuples(d, s2);
+    cudaEventRecord(join, s2);
+    // adjacency
     const int32_t* deg = S.deg;
     int64_t* adj_off = S.adj_off;
     scan([=] __device__(int64_t v) -> int64_t { return v < nv ? deg[v] : 0; },
@@ -446,20 +448,18 @@ int highclear(Device& D, const DimInfo& info, int max_iteration, const uint8_t* 
     k_adj_fill<<<gridn(info.col_end[1] - info.col_begin[1], 256), 256, 0, s>>>(
         info.col_begin[1], info.col_end[1], S.tup[1], dropped, S.adj_off, S.deg, S.adj, masks ? S.adj_src : nullptr);
     k_adj_sort<<<gridn(nv, 128), 128, 0, s>>>(nv, S.adj_off, S.adj);
-    launches += 6;
+    launches += 3;
     const int64_t ne2 = 2 * int64_t(info.col_end[1] - info.col_begin[1]);  // list entries, at most
     if (masks) {
         k_adj_masks<<<gridn(ne2, 256), 256, 0, s>>>(nv, S.adj_src, S.adj, S.adj_off, max_iteration, S.nmask);
         launches++;
     }
-    // hash of the top-dimension tuples
-    cudaMemsetAsync(S.table, 0xff, sizeof(int32_t) * (size_t(S.mask) + 1), s);
+    cudaStreamWaitEvent(s, join, 0);
     const int32_t cb = info.col_begin[top], ce = info.col_end[top];
-    k_hash_insert<<<gridn(ce - cb, 256), 256, 0, s>>>(cb, ce, top + 1, S.tup[top], dropped, S.table, S.mask);
     if (masks) {
         k_highclear_masks<<<gridn(ce - cb, 256), 256, 0, s>>>(cb, ce, top, S.tup[top], S.adj, S.adj_off, S.nmask,
                                                              S.table, S.mask, dropped, D.cleared, D.counters);
-        return launches + 2;
+        return launches + 1;
     }
     const int g = max_iteration <= 4 ? 4 : max_iteration <= 8 ? 8 : max_iteration <= 16 ? 16 : 32;
     const unsigned grid = gridn(int64_t(ce - cb) * g, kHcThreads, 148 * 64);
@@ -471,8 +471,7 @@ int highclear(Device& D, const DimInfo& info, int max_iteration, const uint8_t* 
     else if (g == 16) SSPP_HC(16);
     else SSPP_HC(32);
 #undef SSPP_HC
-    launches += 2;
-    return launches;
+    return launches + 1;
 }
 
 }  // namespace sspp

@@ -27,7 +27,8 @@ constexpr int kMaskCandidates = 64;
 
 // Sets cleared[] for the top-dimension columns the test proves positive;
 // returns the number of kernels launched.  Buffers must be sized by the caller.
+// s2: a second stream to work on, with two events to fork and join it.
 int highclear(Device& D, const DimInfo& info, int max_iteration, const uint8_t* dropped, HighclearScratch& S,
-              cudaStream_t s);
+              cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEvent_t join);
 
 }  // namespace sspp
