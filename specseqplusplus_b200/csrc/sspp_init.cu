@@ -339,7 +339,11 @@ __global__ void __launch_bounds__(kPartThreads) k_dim_assign(const int32_t* dims
 // go through registers and are stored as two 16-byte halves of their slot; their
 // descriptors are left to the compression unless write_desc asks for them (they are
 // read before it, or also when it does not run).
-__global__ void k_scatter_cols(int64_t n, const int64_t* colptr, const int32_t* rows, const int32_t* dims,
+// A column is a chain of four dependent trips to memory with little to do in between: at
+// 64^3 neither memory (29% of its bandwidth) nor L2 (43%) was busy.  The reads of a
+// trip go out together, of K columns on large inputs.
+template <int K>
+__global__ void __launch_bounds__(256) k_scatter_cols(int64_t n, const int64_t* colptr, const int32_t* rows, const int32_t* dims,
                                const int32_t* newidx, const int64_t* off, Ctl* ctl, int32_t* arena,
                                uint64_t* desc, int32_t* low, int32_t* leftmost, bool lows, bool write_desc) {
     if (ctl->err & ~ERRB_FACES) return;
@@ -350,44 +354,87 @@ __global__ void k_scatter_cols(int64_t n, const int64_t* colptr, const int32_t* 
     }
     __syncthreads();
     const bool all_short = ctl->max_len <= kShortLen;
-    for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < n; j += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t b = colptr[j], len = colptr[j + 1] - b;
-        const int32_t i = newidx[j];
-        const int64_t o = all_short ? int64_t(kShortSlot) * i : off[i];
-        const int dj = dims[j];
-        const int32_t fb = dj > 0 ? s_beg[dj - 1] : 0, fe = dj > 0 ? s_end[dj - 1] : 0;
-        bool bad = false;
-        int32_t last = -1;
+    for (int64_t j0 = blockIdx.x * int64_t(256 * K) + threadIdx.x; j0 < n; j0 += int64_t(gridDim.x) * (256 * K)) {
         if (all_short) {
-            int32_t r[kShortLen], x[kShortLen];
+            int len[K], i[K], dj[K];
+            int64_t b[K];
+            int32_t x[K][kShortLen];
+            unsigned bad = 0;
 #pragma unroll
-            for (int k = 0; k < kShortLen; k++) r[k] = k < len ? rows[b + k] : INT_MAX;
-#pragma unroll
-            for (int k = 0; k < kShortLen; k++) {
-                x[k] = INT_MAX;
-                if (k < len) {
-                    if (r[k] < 0 || r[k] >= n || (k > 0 && r[k] <= r[k - 1])) bad = true;
-                    else x[k] = newidx[r[k]];
+            for (int q = 0; q < K; q++) {
+                const int64_t j = j0 + 256 * q;
+                len[q] = 0;
+                i[q] = -1;
+                dj[q] = 0;
+                b[q] = 0;
+                if (j < n) {
+                    b[q] = colptr[j];
+                    len[q] = int(colptr[j + 1] - b[q]);
+                    i[q] = newidx[j];
+                    dj[q] = dims[j];
                 }
             }
 #pragma unroll
-            for (int k = 0; k < kShortLen; k++)
-                if (k < len && !bad) {
-                    if (x[k] < fb || x[k] >= fe) bad = true;
-                    last = x[k];
-                }
-            const int32_t m = bad ? 0 : int32_t(len);
-            *reinterpret_cast<int4*>(arena + o) = make_int4(m, i, 0, 0);
-            *reinterpret_cast<int4*>(arena + o + kHdr) =
-                bad ? make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX) : make_int4(x[0], x[1], x[2], x[3]);
-            if (write_desc) desc[i] = pack_desc(uint64_t(o), uint32_t(m));
-            if (lows && !bad) {
+            for (int q = 0; q < K; q++)
+#pragma unroll
+                for (int k = 0; k < kShortLen; k++) x[q][k] = k < len[q] ? rows[b[q] + k] : INT_MAX;
+#pragma unroll
+            for (int q = 0; q < K; q++)
 #pragma unroll
                 for (int k = 0; k < kShortLen; k++)
-                    if (k < len && __ldcg(leftmost + x[k]) > i) atomicMin(&leftmost[x[k]], i);
+                    if (k < len[q] && (x[q][k] < 0 || x[q][k] >= n || (k > 0 && x[q][k] <= x[q][k - 1]))) bad |= 1u << q;
+#pragma unroll
+            for (int q = 0; q < K; q++)
+#pragma unroll
+                for (int k = 0; k < kShortLen; k++)
+                    if (k < len[q] && !((bad >> q) & 1)) x[q][k] = newidx[x[q][k]];
+#pragma unroll
+            for (int q = 0; q < K; q++) {
+                if (i[q] < 0) continue;
+                const int32_t fb = dj[q] > 0 ? s_beg[dj[q] - 1] : 0, fe = dj[q] > 0 ? s_end[dj[q] - 1] : 0;
+                int32_t last = -1;
+#pragma unroll
+                for (int k = 0; k < kShortLen; k++)
+                    if (k < len[q]) {
+                        if (x[q][k] < fb || x[q][k] >= fe) bad |= 1u << q;
+                        last = x[q][k];
+                    }
+                const bool wrong = (bad >> q) & 1;
+                const int64_t o = int64_t(kShortSlot) * i[q];
+                const int32_t m = wrong ? 0 : len[q];
+                *reinterpret_cast<int4*>(arena + o) = make_int4(m, i[q], 0, 0);
+                *reinterpret_cast<int4*>(arena + o + kHdr) = wrong ? make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX)
+                                                                   : make_int4(x[q][0], x[q][1], x[q][2], x[q][3]);
+                if (write_desc) desc[i[q]] = pack_desc(uint64_t(o), uint32_t(m));
+                if (lows) low[i[q]] = m == 0 ? -1 : last;
+                len[q] = m;
             }
-        } else {
-            int32_t prev = -1;
+            if (bad) atomicOr(&ctl->err, ERRB_FACES);
+            if (lows) {
+                unsigned first = 0;  // rows whose leftmost column may be this one
+#pragma unroll
+                for (int q = 0; q < K; q++)
+#pragma unroll
+                    for (int k = 0; k < kShortLen; k++)
+                        if (k < len[q] && __ldcg(leftmost + x[q][k]) > i[q]) first |= 1u << (q * kShortLen + k);
+#pragma unroll
+                for (int q = 0; q < K; q++)
+#pragma unroll
+                    for (int k = 0; k < kShortLen; k++)
+                        if ((first >> (q * kShortLen + k)) & 1) atomicMin(&leftmost[x[q][k]], i[q]);
+            }
+            continue;
+        }
+        for (int q = 0; q < K; q++) {
+            const int64_t j = j0 + 256 * q;
+            if (j >= n) break;
+            const int64_t b = colptr[j], len = colptr[j + 1] - b;
+            const int32_t i = newidx[j];
+            const int64_t o = off[i];
+            const int dj = dims[j];
+            const int32_t fb = dj > 0 ? s_beg[dj - 1] : 0, fe = dj > 0 ? s_end[dj - 1] : 0;
+            bool bad = false;
+            int32_t last = -1, prev = -1;
             int32_t* data = arena + o + kHdr;
             for (int64_t k = 0; k < len && !bad; k++) {
                 const int32_t r = rows[b + k];
@@ -405,10 +452,22 @@ __global__ void k_scatter_cols(int64_t n, const int64_t* colptr, const int32_t* 
             if (lows && !bad)
                 for (int64_t k = 0; k < len; k++)
                     if (__ldcg(leftmost + data[k]) > i) atomicMin(&leftmost[data[k]], i);
+            if (bad) atomicOr(&ctl->err, ERRB_FACES);
+            if (lows) low[i] = bad || len == 0 ? -1 : last;
         }
-        if (bad) atomicOr(&ctl->err, ERRB_FACES);
-        if (lows) low[i] = bad || len == 0 ? -1 : last;
     }
+}
+
+// Columns per thread of two passes over all columns, from 2^17 columns up (below, one
+// each: apparent pairs of 55,000 columns 3.6 us with 1, 4.5 with 4; of 250,000 8.6 and
+// 4.9).  20.3 M columns (93^3):
+// apparent pairs 430 / 290 / 190 / 233 us with 1 / 2 / 4 / 8, the scatter 438 / 419 / 517
+// with 1 / 2 / 4 (530 when each read of a leftmost column was followed by its atomic);
+// 2.67 M (20,000 points) 70 / 46 / 36 / 41 and 73 / 73 / 85.
+constexpr int64_t kManyCols = int64_t(1) << 17;
+constexpr int kScatterCols = 2, kApparentCols = 4;
+unsigned cols_grid(int64_t n, int k, int64_t most) {
+    return unsigned(std::min<int64_t>((n + 256 * k - 1) / (256 * k), most));
 }
 
 int reorder(Device& D, bool lows, bool write_desc, cudaStream_t s) {
@@ -431,9 +490,9 @@ int reorder(Device& D, bool lows, bool write_desc, cudaStream_t s) {
     scan([=] __device__(int64_t i) -> int64_t { return slot_ints(max(rlen[i], 0)); },
          [=] __device__(int64_t i, int64_t pre, int64_t) { off[i] = pre; }, n, blk, s,
          [=] __device__(int64_t total) { ctl->arena_top = (unsigned long long)total; }, zeroed, &ctl->max_len, kShortLen);
-    k_scatter_cols<<<grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256), 256, 0, s>>>(
-        n, D.in_colptr, D.in_rows, D.in_dims, D.newidx, off, D.ctl, D.arena, D.desc, D.low, D.leftmost, lows,
-        write_desc);
+    const auto scatter = n < kManyCols ? k_scatter_cols<1> : k_scatter_cols<kScatterCols>;
+    scatter<<<cols_grid(n, n < kManyCols ? 1 : kScatterCols, 65536), 256, 0, s>>>(
+        n, D.in_colptr, D.in_rows, D.in_dims, D.newidx, off, D.ctl, D.arena, D.desc, D.low, D.leftmost, lows, write_desc);
     return launches;
 }
 
@@ -475,32 +534,58 @@ __device__ __forceinline__ ColRef col_ref(int64_t i, const int32_t* arena, const
     return c;
 }
 
-__global__ void k_init_apparent(int64_t n, const int32_t* arena, const uint64_t* desc, const int32_t* low,
-                                const int32_t* leftmost, uint64_t* pivot, uint8_t* cleared, uint8_t* negative,
-                                Ctl* ctl) {
+// Three dependent trips a column; bound by their latency (at 64^3 21% of the memory's
+// bandwidth, 14% of L2's), so a thread takes K columns at once on large inputs.
+template <int K>
+__global__ void __launch_bounds__(256) k_init_apparent(int64_t n, const int32_t* arena, const uint64_t* desc,
+                                                       const int32_t* low, const int32_t* leftmost, uint64_t* pivot,
+                                                       uint8_t* cleared, uint8_t* negative, Ctl* ctl) {
     if (ctl->err) return;
     const bool all_short = ctl->max_len <= kShortLen;
     long long app = 0;
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        const int32_t l = low[i];
-        if (l < 0) continue;
-        cleared[l] = 1;  // the youngest facet of any simplex is positive
-        if (leftmost[l] == int32_t(i)) {  // no earlier column can ever reach row l
-            pivot[l] = pv_pack(int32_t(i), all_short ? uint64_t(kShortSlot) * uint64_t(i) : desc_off(desc[i]));
-            negative[i] = 1;
-            app++;
-            continue;  // its other entries need not be looked at
+    for (int64_t i0 = blockIdx.x * int64_t(256 * K) + threadIdx.x; i0 < n; i0 += int64_t(gridDim.x) * (256 * K)) {
+        int32_t l[K], lm[K];
+        int4 e[K];
+        int len[K];
+#pragma unroll
+        for (int q = 0; q < K; q++) l[q] = i0 + 256 * q < n ? low[i0 + 256 * q] : -1;
+#pragma unroll
+        for (int q = 0; q < K; q++) lm[q] = l[q] >= 0 ? leftmost[l[q]] : -1;
+        // the entries of the columns that are not their lowest row's leftmost one
+#pragma unroll
+        for (int q = 0; q < K; q++) {
+            len[q] = 0;
+            e[q] = make_int4(0, 0, 0, 0);
+            if (all_short && l[q] >= 0 && lm[q] != int32_t(i0 + 256 * q)) {
+                const ColRef c = col_ref(i0 + 256 * q, arena, desc, true);
+                len[q] = c.len;
+                e[q] = c.q;
+            }
         }
-        const ColRef c = col_ref(i, arena, desc, all_short);
-        bool neg = false;
-        if (all_short) {  // the lowest entry's is known; the others' at once
-            const int32_t x = c.len > 1 ? leftmost[c.q.x] : -1, y = c.len > 2 ? leftmost[c.q.y] : -1,
-                          z = c.len > 3 ? leftmost[c.q.z] : -1;
-            neg = x == int32_t(i) || y == int32_t(i) || z == int32_t(i);
-        } else {
-            for (int k = 0; k < c.len && !neg; k++) neg = leftmost[c.at(arena, k, false)] == int32_t(i);
+        unsigned neg = 0;
+#pragma unroll
+        for (int q = 0; q < K; q++) {  // the lowest entry's is known; the others' at once
+            const int32_t i = int32_t(i0 + 256 * q);
+            const int32_t x = len[q] > 1 ? leftmost[e[q].x] : -1, y = len[q] > 2 ? leftmost[e[q].y] : -1,
+                          z = len[q] > 3 ? leftmost[e[q].z] : -1;
+            if (x == i || y == i || z == i) neg |= 1u << q;
         }
-        if (neg) negative[i] = 1;
+#pragma unroll
+        for (int q = 0; q < K; q++) {
+            const int64_t i = i0 + 256 * q;
+            if (l[q] < 0) continue;
+            cleared[l[q]] = 1;  // the youngest facet of any simplex is positive
+            bool is_neg = (neg >> q) & 1;
+            if (lm[q] == int32_t(i)) {  // no earlier column can ever reach row l
+                pivot[l[q]] = pv_pack(int32_t(i), all_short ? uint64_t(kShortSlot) * uint64_t(i) : desc_off(desc[i]));
+                is_neg = true;  // its other entries need not be looked at
+                app++;
+            } else if (!all_short) {
+                const ColRef c = col_ref(i, arena, desc, false);
+                for (int k = 0; k < c.len && !is_neg; k++) is_neg = leftmost[c.at(arena, k, false)] == int32_t(i);
+            }
+            if (is_neg) negative[i] = 1;
+        }
     }
     app = warp_sum(app);
     if ((threadIdx.x & 31) == 0 && app) cnt_add(&ctl->counters[CNT_APPARENT], app);
@@ -619,7 +704,8 @@ int init_passes(Device& D, bool lows_done, cudaStream_t s) {
     const int64_t n = D.n;
     const unsigned g = grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256);
     if (!lows_done) k_init_low<<<g, 256, 0, s>>>(n, D.arena, D.desc, D.low, D.leftmost);
-    k_init_apparent<<<g, 256, 0, s>>>(n, D.arena, D.desc, D.low, D.leftmost, D.pivot, D.cleared, D.negative, D.ctl);
+    const auto apparent = n < kManyCols ? k_init_apparent<1> : k_init_apparent<kApparentCols>;
+    apparent<<<cols_grid(n, n < kManyCols ? 1 : kApparentCols, 65536), 256, 0, s>>>(n, D.arena, D.desc, D.low, D.leftmost, D.pivot, D.cleared, D.negative, D.ctl);
     return lows_done ? 1 : 2;
 }
 
