@@ -171,22 +171,42 @@ __device__ __forceinline__ void read_mirror(const DualCols& D, int64_t j, Mirror
     m.state = D.state[j];
 }
 
+// Column c's slot and what its lane reads of it, all before either of the lane's columns
+// is worked on.
+struct Slot {
+    int64_t o, low_off;  // ints into the arena; the slot offset of the dual column that owns row c
+    int len;
+    int4 a, b;  // the first 8 entries of a column of at most 8
+};
+
+__device__ __forceinline__ void read_place(const DualCols& D, int64_t base, int64_t c, Slot& t) {
+    t.o = t.low_off = 0;
+    t.len = 0;
+    t.a = t.b = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
+    if (c < 0) return;
+    t.o = base + D.off[c];
+    t.len = D.cnt[c];
+}
+
+__device__ __forceinline__ void read_entries(const DualCols& D, const Mirror& m, Slot& t) {
+    if (t.len >= 1 && t.len <= 8) t.a = *reinterpret_cast<const int4*>(D.arena + t.o + kHdr);
+    if (t.len >= 5 && t.len <= 8) t.b = *reinterpret_cast<const int4*>(D.arena + t.o + kHdr + 4);
+    if (m.state == ST_OWNER) t.low_off = D.off[D.n - 1 - m.low];
+}
+
 // Dual column c of this lane (-1: none; the warp calls together): its entries sorted,
 // its header and padding, and everything else the reduction keeps of it.
-__device__ __forceinline__ void finish_columns(const DualCols& D, int64_t base, int64_t c, const Mirror& m, int32_t* s,
-                                               int* smin, int* smax, int* sact) {
+__device__ __forceinline__ void finish_columns(const DualCols& D, int64_t base, int64_t c, const Mirror& m,
+                                               const Slot& t, int32_t* s, int* smin, int* smax, int* sact) {
     const int lane = threadIdx.x & 31;
-    int len = 0;
-    int64_t o = 0;
+    const int len = t.len;
+    const int64_t o = t.o;
     int32_t first = INT_MAX, last = -1;
-    int4 a = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
+    int4 a = t.a;
     if (c >= 0) {
-        o = base + D.off[c];
-        len = D.cnt[c];
         *reinterpret_cast<int4*>(D.arena + o) = make_int4(len, int32_t(c), 0, 0);
         if (len >= 1 && len <= 8) {
             int4* d4 = reinterpret_cast<int4*>(D.arena + o + kHdr);
-            a = d4[0];
             if (len < 4) a.w = INT_MAX;
             if (len < 3) a.z = INT_MAX;
             if (len < 2) a.y = INT_MAX;
@@ -194,7 +214,7 @@ __device__ __forceinline__ void finish_columns(const DualCols& D, int64_t base, 
             if (len <= 4) {
                 last = len == 1 ? a.x : len == 2 ? a.y : len == 3 ? a.z : a.w;
             } else {
-                int4 b = d4[1];
+                int4 b = t.b;
                 if (len < 8) b.w = INT_MAX;
                 if (len < 7) b.z = INT_MAX;
                 if (len < 6) b.y = INT_MAX;
@@ -213,26 +233,46 @@ __device__ __forceinline__ void finish_columns(const DualCols& D, int64_t base, 
             first = a.x;
         }
     }
-    for (unsigned big = __ballot_sync(0xffffffffu, len > 8); big; big &= big - 1) {
+    // four columns of 9 to 32 entries at a time: their loads are under way together
+    for (unsigned mid = __ballot_sync(0xffffffffu, len > 8 && len <= 32); mid;) {
+        int q[4], ql[4];
+        int32_t *data[4], v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            q[u] = mid ? __ffs(mid) - 1 : -1;
+            mid &= mid - 1;
+            ql[u] = __shfl_sync(0xffffffffu, len, q[u] & 31);
+            data[u] = D.arena + __shfl_sync(0xffffffffu, o, q[u] & 31) + kHdr;
+            v[u] = q[u] >= 0 && lane < ql[u] ? data[u][lane] : INT_MAX;
+        }
+#pragma unroll
+        for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const bool keep_min = ((lane & j) == 0) == ((lane & k) == 0);
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int32_t x = __shfl_xor_sync(0xffffffffu, v[u], j);
+                    v[u] = keep_min ? min(v[u], x) : max(v[u], x);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int32_t bottom = __shfl_sync(0xffffffffu, v[u], 0), top = __shfl_sync(0xffffffffu, v[u], ql[u] - 1);
+            if (q[u] >= 0 && lane < int(pad4(ql[u]))) data[u][lane] = v[u];
+            if (lane == q[u]) {
+                first = bottom;
+                last = top;
+            }
+        }
+    }
+    for (unsigned big = __ballot_sync(0xffffffffu, len > 32); big; big &= big - 1) {
         const int q = __ffs(big) - 1;
         const int ql = __shfl_sync(0xffffffffu, len, q);
         int32_t* data = D.arena + __shfl_sync(0xffffffffu, o, q) + kHdr;
         int32_t bottom, top;
-        if (ql <= 32) {
-            int32_t v = lane < ql ? data[lane] : INT_MAX;
-#pragma unroll
-            for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    const int32_t x = __shfl_xor_sync(0xffffffffu, v, j);
-                    const bool keep_min = ((lane & j) == 0) == ((lane & k) == 0);
-                    v = keep_min ? min(v, x) : max(v, x);
-                }
-            }
-            if (lane < int(pad4(ql))) data[lane] = v;
-            bottom = __shfl_sync(0xffffffffu, v, 0);
-            top = __shfl_sync(0xffffffffu, v, ql - 1);
-        } else if (ql <= kWarpSortCap) {
+        if (ql <= kWarpSortCap) {
             const int p = next_pow2(ql);
             for (int i = lane; i < p; i += 32) s[i] = i < ql ? data[i] : INT_MAX;
             __syncwarp();
@@ -291,7 +331,7 @@ __device__ __forceinline__ void finish_columns(const DualCols& D, int64_t base, 
     uint64_t e = kNoOwner;
     if (negative) {
         const int64_t dc = D.n - 1 - m.low;
-        e = pv_pack(int32_t(dc), uint64_t(base + D.off[dc]));
+        e = pv_pack(int32_t(dc), uint64_t(base + t.low_off));
     } else {
         D.app[c] = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
     }
@@ -319,12 +359,13 @@ __device__ __forceinline__ void finish_columns(const DualCols& D, int64_t base, 
 // of vertices are never reduced.  Dual column c and dual row c come from primal row
 // and column n-1-c, so a lane takes a column and the mirrored one, reads what both
 // were and then writes both in place.  A warp takes 32 of each: columns of up to 8
-// entries (nearly all) are sorted by their own lanes in registers, the others one
-// after another by the whole warp (registers up to 32 entries, shared memory up to
-// kWarpSortCap; longer ones go to the long list, unsorted, but with their low known).
-// 20,000 points (2.67 M columns): 142 us, where sorting, remapping the pivots, inline
-// columns and row bounds in nine launches took 230; the whole dualization of a cloud
-// of 5,000 points 115 -> 61 us.
+// entries (nearly all) are sorted by their own lanes in registers, those of up to 32 by
+// the whole warp, four at a time, longer ones one after another in shared memory (up to
+// kWarpSortCap; the rest goes to the long list, unsorted, but with its low known).
+// Bound by the latency of its dependent reads (25% of the memory's bandwidth, 21% of
+// L2's): 20,000 points (2.67 M columns) 143 us with both columns' reads in turn and one
+// longer column at a time, 100 like this (and 230 where sorting, remapping the pivots,
+// inline columns and row bounds took nine launches); 64 requests 576 -> 446.
 __global__ void __launch_bounds__(kSortWarps * 32) k_dual_finish(const __grid_constant__ DualCols D) {
     __shared__ int32_t sm[kSortWarps][kWarpSortCap];
     __shared__ int smin[kNumDims], smax[kNumDims], sact[kNumDims];
@@ -345,8 +386,14 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_dual_finish(const __grid_co
         Mirror mc, mj;
         read_mirror(D, j, mc);
         read_mirror(D, c, mj);
-        finish_columns(D, base, c, mc, sm[w], smin, smax, sact);
-        finish_columns(D, base, j == c ? -1 : j, mj, sm[w], smin, smax, sact);
+        Slot tc, tj;
+        const int64_t j2 = j == c ? -1 : j;
+        read_place(D, base, c, tc);
+        read_place(D, base, j2, tj);
+        read_entries(D, mc, tc);
+        read_entries(D, mj, tj);
+        finish_columns(D, base, c, mc, tc, sm[w], smin, smax, sact);
+        finish_columns(D, base, j2, mj, tj, sm[w], smin, smax, sact);
     }
     __syncthreads();
     if (threadIdx.x < kNumDims) {
