@@ -686,7 +686,8 @@ int run_dims(sspp_ctx* ctx, int dlo, int dhi, bool ascending, int cap1, int cap2
         if (es != s) CK(cudaEventRecord(ctx->join_ev[kNumDims - 1], es));
         return int(SSPP_OK);
     };
-    D.edges_beside = es != s;
+    D.edge_begin = es != s ? I.col_begin[1] : 0;
+    D.edge_end = es != s ? I.col_end[1] : 0;
     // The edges depend on no other dimension: on a stream of their own, beside all of
     // them (launched after the first of them, which covers the launches), or, on large
     // inputs, where the passes fill the GPU and clear most of the edges, beside the last
@@ -931,7 +932,7 @@ int run_compute(sspp_ctx* ctx) {
     // resident as the persistent kernel, whose CTA-tier role sets the register
     // budget of every block
     const bool queue = P.schedule == 2;
-    D.edges_beside = false;
+    D.edge_begin = D.edge_end = 0;
     auto phase = [&](int dlo, int dhi, bool ascending) {
         return queue ? run_queue(ctx, dlo, dhi, ascending, cap1, cap2, ht)
                      : run_dims(ctx, dlo, dhi, ascending, cap1, cap2, ht);

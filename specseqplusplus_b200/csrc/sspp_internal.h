@@ -143,7 +143,7 @@ struct Device {
     int64_t* blk = nullptr;      // region 0
     int64_t blk_stride = 0;      // entries per region
     unsigned blk_zero = 0;       // regions still as cleared (bits)
-    bool edges_beside = false;   // the edges were reduced beside the dimensions above them
+    int32_t edge_begin = 0, edge_end = 0;  // the edges' columns, when reduced beside the dimensions above them
     bool steps_zero = false;     // Ctl::pool_tail, heavy_done and step still as cleared
     int64_t cap_blk = 0;
     int32_t* dimcnt = nullptr;   // [nblocks * kNumDims]
