@@ -755,7 +755,7 @@ int active_list(Device& D, cudaStream_t s) {
 // dropped by an edge collapse: essential.  One scan in input order writes both
 // lists (births ascending, so the pairs come out sorted): it reads the maps and
 // the pivot table in two nearly sequential streams per dimension, and only the
-// deaths' input indices at random.  64^3: 92 us; a scatter by birth and two scans over
+// deaths' input indices at random.  64^3: 81 us; a scatter by birth and two scans over
 // its marks took 250.
 struct PairsOut {
     int64_t n;
@@ -782,14 +782,27 @@ struct PairsValue {
 };
 struct PairsSink {
     PairsOut o;
-    __device__ void operator()(int64_t j, int64_t pre, ScanClass v) const {
-        if (v.c == 1) {
-            const int32_t c = pv_col(o.pivot[o.newidx[j]]);
-            o.pairs[pre & kBirths] = make_longlong2(j, o.perm[c]);
-            // an edge that owns a row may not be one itself (looked for here, at the vertices:
-            // in the value above it cost 30 us at 64^3)
-            if (c >= o.edge_begin && c < o.edge_end && o.pivot[c] != kNoOwner) atomicOr(o.err, ERRB_ORDER);
-        } else if (v.c == 2) o.ess[pre >> kScanClassShift] = j;
+    __device__ void operator()(int64_t j, const int64_t (&pre)[kScanBatch], const uint8_t (&cls)[kScanBatch]) const {
+        int32_t c[kScanBatch], death[kScanBatch];
+        bool twice = false;
+#pragma unroll
+        for (int u = 0; u < kScanBatch; u++) c[u] = cls[u] == 1 ? o.newidx[j + 32 * u] : -1;
+#pragma unroll
+        for (int u = 0; u < kScanBatch; u++)
+            if (c[u] >= 0) c[u] = pv_col(o.pivot[c[u]]);
+#pragma unroll
+        for (int u = 0; u < kScanBatch; u++) death[u] = c[u] >= 0 ? o.perm[c[u]] : -1;
+        // an edge that owns a row may not be one itself (looked for here, at the vertices: in
+        // the value above it cost 30 us at 64^3)
+#pragma unroll
+        for (int u = 0; u < kScanBatch; u++)
+            if (c[u] >= o.edge_begin && c[u] < o.edge_end) twice = twice || o.pivot[c[u]] != kNoOwner;
+#pragma unroll
+        for (int u = 0; u < kScanBatch; u++) {
+            if (cls[u] == 1) o.pairs[pre[u] & kBirths] = make_longlong2(j + 32 * u, death[u]);
+            else if (cls[u] == 2) o.ess[pre[u] >> kScanClassShift] = j + 32 * u;
+        }
+        if (twice) atomicOr(o.err, ERRB_ORDER);
     }
 };
 struct PairsDone {
@@ -867,9 +880,15 @@ int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s) {
     const uint8_t* paired = D.negative;
     int64_t* ess = D.ess;
     scan([=] __device__(int64_t j) -> ScanClass { return {uint8_t(death_of[j] >= 0 ? 1 : (paired[j] ? 0 : 2))}; },
-         [=] __device__(int64_t j, int64_t pre, ScanClass v) {
-             if (v.c == 1) pairs[pre & kBirths] = make_longlong2(j, death_of[j]);
-             else if (v.c == 2) ess[pre >> kScanClassShift] = j;
+         [=] __device__(int64_t j, const int64_t (&pre)[kScanBatch], const uint8_t (&cls)[kScanBatch]) {
+             int64_t death[kScanBatch];
+#pragma unroll
+             for (int u = 0; u < kScanBatch; u++) death[u] = cls[u] == 1 ? death_of[j + 32 * u] : -1;
+#pragma unroll
+             for (int u = 0; u < kScanBatch; u++) {
+                 if (cls[u] == 1) pairs[pre[u] & kBirths] = make_longlong2(j + 32 * u, death[u]);
+                 else if (cls[u] == 2) ess[pre[u] >> kScanClassShift] = j + 32 * u;
+             }
          },
          n, blk, s, PairsDone{o}, zeroed);
     return 3 + (dropped ? 1 : 0);

@@ -73,6 +73,11 @@ constexpr int kScanClassShift = 31;
 struct ScanClass {
     uint8_t c;
 };
+// Its sink takes kScanBatch items of a lane at a time (j, j + 32, ...: prefixes and
+// classes, 0 also beyond the end), so that what it reads for them is under way together
+// (pairs, a chain of three reads: 6,700 columns 12 us one item at a time, 8 by four, 8.5 by
+// eight; 6.57 M 97 / 81 / 102; 20.3 M 270 / 248 / 300, eight costing warps).
+constexpr int kScanBatch = 4;
 template <>
 struct ScanLane<ScanClass> {
     unsigned one[kScanItems], two[kScanItems];
@@ -99,10 +104,17 @@ struct ScanLane<ScanClass> {
         const int lane = threadIdx.x & 31;
         const int64_t first = begin + lane;
 #pragma unroll
-        for (int k = 0; k < kScanItems; k++) {
-            const ScanClass v{uint8_t(((one[k] >> lane) & 1) | (((two[k] >> lane) & 1) << 1))};
-            if (first + 32 * k < n) sink(first + 32 * k, base + pack(__popc(one[k] & lt), __popc(two[k] & lt)), v);
-            base += pack(__popc(one[k]), __popc(two[k]));
+        for (int k0 = 0; k0 < kScanItems; k0 += kScanBatch) {
+            int64_t pre[kScanBatch];
+            uint8_t c[kScanBatch];
+#pragma unroll
+            for (int u = 0; u < kScanBatch; u++) {
+                const unsigned a = one[k0 + u], b = two[k0 + u];
+                c[u] = uint8_t(((a >> lane) & 1) | (((b >> lane) & 1) << 1));
+                pre[u] = base + pack(__popc(a & lt), __popc(b & lt));
+                base += pack(__popc(a), __popc(b));
+            }
+            sink(first + 32 * k0, pre, c);
         }
     }
     template <class F>
