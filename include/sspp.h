@@ -63,8 +63,8 @@ typedef struct sspp_params {
                                  reference); the pairs are the same in every mode   */
     int32_t model;            /* bit0 high-dimension guided clearing, bit1 collapse   */
     int32_t max_iteration;    /* candidates per simplex for guided clearing           */
-    int32_t ss_block_size;    /* initial spectral-sequence block size (schedule 1 merges
-                                 blocks of fewer than 2^20 columns)                   */
+    int32_t ss_block_size;    /* initial spectral-sequence block size (schedule 2; schedules
+                                 0 and 1 take a dimension as one block)               */
     float growth;             /* block_size_growth_rate (>= 1)                        */
     int32_t queue_size;       /* concurrent column workers per launch                 */
     int32_t level1_capacity;  /* per-worker on-chip column capacity (ints; more than 64

@@ -32,10 +32,10 @@
 
 using namespace sspp;
 
-// CTA-tier launches of successive spectral-sequence steps run on separate side
-// streams.  The driver maps streams onto CUDA_DEVICE_MAX_CONNECTIONS hardware
-// work queues (8 by default), and launches on streams that share a queue wait
-// for each other: a short launch queued behind a long chain of another step.
+// A reduction's CTA-tier launches, its edges and the init passes' branches run on side
+// streams.  The driver maps streams onto CUDA_DEVICE_MAX_CONNECTIONS hardware work
+// queues (8 by default), and launches on streams that share a queue wait for each
+// other: a short launch queued behind a long chain of another dimension or context.
 // When the library is loaded, ask for the maximum (32) unless the variable is
 // set; it applies to a CUDA context created afterwards (for a program linked
 // against the library, every context).

@@ -30,6 +30,9 @@
 // those of any sequential one.  Claiming a row also clears the row's own
 // column (twist clearing).
 //
+// The boundary matrix's edges, columns of two entries at most, are reduced by a walk of
+// their own (sspp_edges.cu) when no longer column of dimension 1 is among them.
+//
 // Additions.  A column in shared memory takes its additions in rounds: the
 // owners of all its top rows at once (round_adds).  What a round cannot take
 // (an addend of more than kRoundAddend entries, a sum that does not fit, a column

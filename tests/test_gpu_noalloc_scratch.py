@@ -63,7 +63,7 @@ def test_columns_without_a_boundary(ncols):
 
 
 def test_larger_than_the_scratch_passes_take():
-    # 900,000 columns: 71 bytes each and their slots exceed the array, so the one-block kernel runs
+    # 900,000 columns: 67 bytes each and their slots exceed the array, so the one-block kernel runs
     torch = pytest.importorskip("torch")
     n = 450_000
     dims = np.concatenate([np.zeros(n, np.int32), np.ones(n, np.int32)])
