@@ -661,7 +661,7 @@ int scan_counts(BuildScratch& S, int64_t* a, int64_t n, cudaStream_t s, std::str
         return 0;
     }
     int64_t* blk;
-    BK(take(S, BuildScratch::BLK, scan_blocks(n) + 2, s, &blk));
+    BK(take(S, BuildScratch::BLK, scan_most_blocks(n) + 2, s, &blk));
     scan(ReadArr{a}, OffSink{a, n}, n, blk, s);
     BK(cudaGetLastError());
     return 0;
@@ -775,7 +775,7 @@ int build_flag(BuildScratch& S, int64_t nv, int64_t E, const float* vval, int ma
                                                          b.values, rank, &perm, err);
         if (rc) return rc;
         int64_t* blk;
-        BK(take(S, BuildScratch::BLK, scan_blocks(N) + 2, s, &blk));
+        BK(take(S, BuildScratch::BLK, scan_most_blocks(N) + 2, s, &blk));
         scan(ColLen{b.dims}, OffSink{b.col_ptr, N, sink.ent0}, N, blk, s);
         if (nnz > 0)
             k_rows<<<grid_for(N), kT, 0, s>>>(N, z, perm, rank, e_src, up_v, tri_f, tet_f, b.col_ptr, sink.ent0,
@@ -820,7 +820,7 @@ int build_lowerstar(BuildScratch& S, const float* d_values, int64_t gx, int64_t 
     k_canon<<<grid_for(nv), kT, 0, s>>>(d_values, vval, nv, flag);
     BK(take(S, BuildScratch::UP_OFF, nv + 1, s, &up_off));
     int64_t* blk;
-    BK(take(S, BuildScratch::BLK, scan_blocks(nv) + 2, s, &blk));
+    BK(take(S, BuildScratch::BLK, scan_most_blocks(nv) + 2, s, &blk));
     const Grid g{gx, gy, gz};
     scan(GridDegree{g}, OffSink{up_off, nv}, nv, blk, s);
     int64_t got[2];
@@ -891,7 +891,7 @@ int build_clouds(BuildScratch& S, const float* d_points, const Cloud* clouds, in
     if (n > 0) {
         k_cells<<<grid_for(n), kT, 0, s>>>(d_points, n, dc, k, count, pcell, pslot);
         int64_t* blk;
-        BK(take(S, BuildScratch::BLK, scan_blocks(std::max(cells, n)) + 2, s, &blk));
+        BK(take(S, BuildScratch::BLK, scan_most_blocks(std::max(cells, n)) + 2, s, &blk));
         scan(ReadI32{count}, OffSink{start, cells}, cells, blk, s);
         k_sort_points<<<grid_for(n), kT, 0, s>>>(d_points, n, dc, k, start, pcell, pslot, spt);
         k_nbrs<false><<<ng, kNbrWarps * 32, 0, s>>>(n, dc, k, start, spt, up_off, nullptr, nullptr, nullptr, false,

@@ -27,6 +27,7 @@
 #include "sspp_internal.h"
 #include "sspp_io.h"
 #include "sspp_launch.h"
+#include "sspp_scan.cuh"
 #include "sspp_tune.h"
 #include "sspp_xfer.h"
 
@@ -235,7 +236,7 @@ int ensure_columns(sspp_ctx* ctx, int64_t n, int64_t nnz) {
         CK(g(D.app, 1));
         D.cap_n = c;
         // the control block and the scans' tile states (one per 4,096 columns, a total and room for one more)
-        D.blk_stride = (c + 4095) / 4096 + 2;
+        D.blk_stride = scan_most_blocks(c) + 2;
         const int64_t ctl_words = int64_t((sizeof(Ctl) + 15) / 16) * 2;
         int64_t* buf = reinterpret_cast<int64_t*>(D.ctl);
         if (buf) CK(cudaFreeAsync(buf, ctx->stream));
@@ -450,7 +451,7 @@ int run_highclear(sspp_ctx* ctx, cudaStream_t s, const DimInfo& info) {
     const int64_t nv = info.col_end[0] - info.col_begin[0];
     const int64_t ne = info.col_end[1] - info.col_begin[1];
     CK(grow(S.deg, S.cap_deg, nv + 2, s));
-    CK(grow(S.blk, S.cap_blk, (nv + 1) / 4096 + 4, s));  // scan block sums (4,096 per block)
+    CK(grow(S.blk, S.cap_blk, scan_most_blocks(nv + 1) + 2, s));  // a scan's tile states
     CK(grow(S.adj_off, S.cap_adj_off, nv + 2, s));
     CK(grow(S.adj, S.cap_adj, 2 * ne + 1, s));
     if (ctx->params.max_iteration <= kMaskCandidates) {

@@ -276,7 +276,7 @@ bool carve(int32_t* scratch, int64_t n, int64_t nnz, Device& D) {
     };
     // cleared together: the control block and the scans' tile states
     take(D.ctl, 1);
-    D.blk_stride = scan_blocks(n) + 2;
+    D.blk_stride = scan_most_blocks(n) + 2;
     take(D.blk, 3 * D.blk_stride);
     take(D.dim, n);
     take(D.perm, n);

@@ -2,8 +2,8 @@
 // ScanClass for a selection), sink(i, exclusive prefix, value), and at the end
 // done(total).  Used for column offsets and stream compaction.
 //
-// Tiles of 4096 items per 256-thread block.  A warp takes 512 consecutive items,
-// 32 at a time, so that values are read and prefixes written coalesced.  Tiles
+// Tiles of 4096 items (1024 in mid-sized scans) per 256-thread block.  A warp takes 512
+// (128) consecutive items, 32 at a time, so that values are read and prefixes written coalesced.  Tiles
 // publish their sums and read their predecessors' (decoupled look-back, 256 tiles
 // at a time: with a warp's 32 the prefix needed 50 hops over 1,605 tiles, and the
 // pair lists took 217 us instead of 92), so every value is read once.  The three
@@ -12,13 +12,20 @@
 // three launches over a few thousand items, where this is one launch of 5 us (from
 // 4,097 items on with a clearing of the tile states before it).
 #pragma once
+#include <type_traits>
+
 #include "sspp_kernels.cuh"
 
 namespace sspp {
 
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 16;  // per lane
-constexpr int kScanTile = kScanThreads * kScanItems;
+// Items per lane.  A few items each put a scan of some ten thousand items on more SMs and
+// shorten each lane's chain; on large inputs they mean more tiles to look back over.
+// (Pairs of 6,700 columns 8 -> 4 us, of 55,000 9.5 -> 4.8, of 210,000 14 -> 11; whole
+// requests 2-6% below 2^18 columns.)
+constexpr int kScanItems = 16, kScanFewItems = 4;
+constexpr int64_t kScanOneTile = kScanThreads * kScanItems;  // a single tile needs no look-back
+constexpr int64_t kScanFewMax = int64_t(1) << 18;
 
 // A tile's published state: flag in the top two bits (0 nothing, 1 the tile's own
 // sum, 2 the sum up to and including it), the sum below.
@@ -34,19 +41,18 @@ __device__ __forceinline__ void scan_store(unsigned long long* p, unsigned long 
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// The 16 values of a lane (items lane + 32 k of its warp's 512, which start at
-// `begin`) and their exclusive prefixes within the warp.
-template <class T>
+// The values of a lane (items lane + 32 k of its warp's, which start at `begin`) and their exclusive prefixes within the warp.
+template <class T, int kItems>
 struct ScanLane {  // numbers
-    T v[kScanItems], ex[kScanItems];
+    T v[kItems], ex[kItems];
     template <class F>
     __device__ __forceinline__ int64_t load(const F& value, int64_t begin, int64_t n) {
         const int64_t first = begin + (threadIdx.x & 31);
 #pragma unroll
-        for (int k = 0; k < kScanItems; k++) v[k] = first + 32 * k < n ? value(first + 32 * k) : T(0);
+        for (int k = 0; k < kItems; k++) v[k] = first + 32 * k < n ? value(first + 32 * k) : T(0);
         T run = 0;
 #pragma unroll
-        for (int k = 0; k < kScanItems; k++) {
+        for (int k = 0; k < kItems; k++) {
             const T inc = warp_inclusive_scan(v[k]);
             ex[k] = run + inc - v[k];
             run += __shfl_sync(kFull, inc, 31);
@@ -57,7 +63,7 @@ struct ScanLane {  // numbers
     __device__ __forceinline__ void store(const G& sink, int64_t begin, int64_t n, int64_t base) const {
         const int64_t first = begin + (threadIdx.x & 31);
 #pragma unroll
-        for (int k = 0; k < kScanItems; k++)
+        for (int k = 0; k < kItems; k++)
             if (first + 32 * k < n) sink(first + 32 * k, base + int64_t(ex[k]), v[k]);
     }
     template <class F>
@@ -78,19 +84,19 @@ struct ScanClass {
 // (pairs, a chain of three reads: 6,700 columns 12 us one item at a time, 8 by four, 8.5 by
 // eight; 6.57 M 97 / 81 / 102; 20.3 M 270 / 248 / 300, eight costing warps).
 constexpr int kScanBatch = 4;
-template <>
-struct ScanLane<ScanClass> {
-    unsigned one[kScanItems], two[kScanItems];
+template <int kItems>
+struct ScanLane<ScanClass, kItems> {
+    unsigned one[kItems], two[kItems];
     static __device__ __forceinline__ int64_t pack(int a, int b) { return int64_t(a) | (int64_t(b) << kScanClassShift); }
     template <class F>
     __device__ __forceinline__ int64_t load(const F& value, int64_t begin, int64_t n) {
         const int64_t first = begin + (threadIdx.x & 31);
-        uint8_t c[kScanItems];
+        uint8_t c[kItems];
 #pragma unroll
-        for (int k = 0; k < kScanItems; k++) c[k] = first + 32 * k < n ? value(first + 32 * k).c : 0;
+        for (int k = 0; k < kItems; k++) c[k] = first + 32 * k < n ? value(first + 32 * k).c : 0;
         int a = 0, b = 0;
 #pragma unroll
-        for (int k = 0; k < kScanItems; k++) {
+        for (int k = 0; k < kItems; k++) {
             one[k] = __ballot_sync(kFull, c[k] == 1);
             two[k] = __ballot_sync(kFull, c[k] == 2);
             a += __popc(one[k]);
@@ -104,7 +110,7 @@ struct ScanLane<ScanClass> {
         const int lane = threadIdx.x & 31;
         const int64_t first = begin + lane;
 #pragma unroll
-        for (int k0 = 0; k0 < kScanItems; k0 += kScanBatch) {
+        for (int k0 = 0; k0 < kItems; k0 += kScanBatch) {
             int64_t pre[kScanBatch];
             uint8_t c[kScanBatch];
 #pragma unroll
@@ -131,8 +137,9 @@ struct ScanBytes {
     uint8_t want;
     __device__ __forceinline__ ScanBytes operator()(int64_t) const { return *this; }
 };
-template <>
-struct ScanLane<ScanBytes> {
+template <int kItems>
+struct ScanLane<ScanBytes, kItems> {
+    static_assert(kItems == 16, "one 16-byte load per lane");
     unsigned sel;  // bit k: item 16 * lane + k
     int pre;
     template <class F>
@@ -167,11 +174,12 @@ struct ScanLane<ScanBytes> {
     }
 };
 
-template <class F, class G, class H>
+template <int kItems, class F, class G, class H>
 __global__ void __launch_bounds__(kScanThreads) k_scan(F value, G sink, H done, int64_t n, int64_t nb, int64_t* blk,
                                                        const int* skip_upto, int skip_limit) {
     if (skip_upto && *skip_upto <= skip_limit) return;
-    using Lane = ScanLane<decltype(value(int64_t(0)))>;
+    using Lane = ScanLane<decltype(value(int64_t(0))), kItems>;
+    constexpr int kTile = kScanThreads * kItems;
     constexpr int kWarps = kScanThreads / 32;
     __shared__ int64_t s_warp[kWarps];
     __shared__ int64_t s_look[kWarps];
@@ -179,7 +187,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(F value, G sink, H done, 
     unsigned long long* state = reinterpret_cast<unsigned long long*>(blk);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t tile = blockIdx.x;
-    const int64_t begin = tile * kScanTile + int64_t(wid) * (32 * kScanItems);
+    const int64_t begin = tile * kTile + int64_t(wid) * (32 * kItems);
     Lane items;
     const int64_t run = items.load(value, begin, n);
     if (lane == 0) s_warp[wid] = run;
@@ -217,7 +225,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(F value, G sink, H done, 
                 if (++polls < kScanPolls) continue;
                 // the predecessors do not answer: add their values up here
                 base = 0;
-                for (int64_t i = threadIdx.x; i < tile * kScanTile; i += kScanThreads) base += Lane::number(value, i, n);
+                for (int64_t i = threadIdx.x; i < tile * kTile; i += kScanThreads) base += Lane::number(value, i, n);
                 base = warp_sum(base);
                 __syncthreads();
                 if (lane == 0) s_look[wid] = base;
@@ -245,21 +253,35 @@ struct ScanNoop {
     __device__ void operator()(int64_t) const {}
 };
 
-// Scratch (blk) must hold scan_blocks(n) + 1 entries; the total is left in
-// blk[scan_blocks(n)].  zeroed: the entries are zero already.  A launch whose
-// *skip_upto turns out to be at most skip_limit does nothing.
-inline int64_t scan_blocks(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
+// Tiles of a scan of numbers or classes over n items, and of any scan over up to n items
+// at most.
+inline bool scan_few(int64_t n) { return n > kScanOneTile && n <= kScanFewMax; }
+inline int64_t scan_blocks(int64_t n) {
+    const int64_t tile = kScanThreads * (scan_few(n) ? kScanFewItems : kScanItems);
+    return (n + tile - 1) / tile;
+}
+inline int64_t scan_most_blocks(int64_t n) {
+    return (n + kScanOneTile - 1) / kScanOneTile + kScanFewMax / (kScanThreads * kScanFewItems);
+}
 
+// Scratch (blk) must hold scan_blocks(n) + 1 entries (a selection by bytes: as many as
+// fewer); the total is left after the last tile's.  zeroed: the entries are zero already.
+// A launch whose *skip_upto turns out to be at most skip_limit does nothing.
 template <class F, class G, class H = ScanNoop>
 void scan(F value, G sink, int64_t n, int64_t* blk, cudaStream_t s, H done = H(), bool zeroed = false,
           const int* skip_upto = nullptr, int skip_limit = 0) {
-    const int64_t nb = scan_blocks(n);
+    constexpr bool bytes = std::is_same<F, ScanBytes>::value;
+    const int64_t nb = bytes ? (n + kScanOneTile - 1) / kScanOneTile : scan_blocks(n);
     if (nb == 0) {
         cudaMemsetAsync(blk, 0, sizeof(int64_t), s);
         return;
     }
     if (nb > 1 && !zeroed) cudaMemsetAsync(blk, 0, sizeof(int64_t) * size_t(nb), s);
-    k_scan<<<unsigned(nb), kScanThreads, 0, s>>>(value, sink, done, n, nb, blk, skip_upto, skip_limit);
+    if (!bytes && scan_few(n))
+        k_scan<bytes ? kScanItems : kScanFewItems>
+            <<<unsigned(nb), kScanThreads, 0, s>>>(value, sink, done, n, nb, blk, skip_upto, skip_limit);
+    else
+        k_scan<kScanItems><<<unsigned(nb), kScanThreads, 0, s>>>(value, sink, done, n, nb, blk, skip_upto, skip_limit);
 }
 
 // Tile states of one of a Device's regions, zero unless a scan used them since
