@@ -763,7 +763,7 @@ struct PairsOut {
     const int32_t* perm;
     const uint64_t* pivot;
     const uint8_t* state;
-    longlong2* pairs;
+    int64_t* pairs;
     int64_t* ess;
     long long* counters;
     int* err;
@@ -780,6 +780,9 @@ struct PairsValue {
         return {uint8_t(e != kNoOwner ? 1 : (st == ST_OWNER || st == ST_DROPPED ? 0 : 2))};
     }
 };
+// kWide: a pair is one 16-byte store (the context's buffer); otherwise two stores of 8
+// bytes, for a caller's buffer that only int64_t's alignment holds for.
+template <bool kWide>
 struct PairsSink {
     PairsOut o;
     __device__ void operator()(int64_t j, const int64_t (&pre)[kScanBatch], const uint8_t (&cls)[kScanBatch]) const {
@@ -799,8 +802,17 @@ struct PairsSink {
             if (c[u] >= o.edge_begin && c[u] < o.edge_end) twice = twice || o.pivot[c[u]] != kNoOwner;
 #pragma unroll
         for (int u = 0; u < kScanBatch; u++) {
-            if (cls[u] == 1) o.pairs[pre[u] & kBirths] = make_longlong2(j + 32 * u, death[u]);
-            else if (cls[u] == 2) o.ess[pre[u] >> kScanClassShift] = j + 32 * u;
+            if (cls[u] == 1) {
+                int64_t* p = o.pairs + 2 * (pre[u] & kBirths);
+                if constexpr (kWide) {
+                    *reinterpret_cast<longlong2*>(p) = make_longlong2(j + 32 * u, death[u]);
+                } else {
+                    p[0] = j + 32 * u;
+                    p[1] = death[u];
+                }
+            } else if (cls[u] == 2) {
+                o.ess[pre[u] >> kScanClassShift] = j + 32 * u;
+            }
         }
         if (twice) atomicOr(o.err, ERRB_ORDER);
     }
@@ -862,15 +874,19 @@ int push_results(const Device& D, Ctl* h_ctl, int64_t* h_pairs, int64_t max_pair
 
 int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s) {
     const int64_t n = D.n;
-    longlong2* pairs = reinterpret_cast<longlong2*>(D.pairs);
-    const PairsOut o{n, D.newidx, D.perm, D.pivot, D.state, pairs, D.ess, D.counters, D.err,
+    const PairsOut o{n, D.newidx, D.perm, D.pivot, D.state, D.pairs, D.ess, D.counters, D.err,
                      D.edge_begin, D.edge_end};
     bool zeroed;
     int64_t* blk = scan_region(D, 2, &zeroed);
     if (!dual) {
-        scan(PairsValue{o}, PairsSink{o}, n, blk, s, PairsDone{o}, zeroed);
+        if (reinterpret_cast<uintptr_t>(D.pairs) % sizeof(longlong2) == 0)
+            scan(PairsValue{o}, PairsSink<true>{o}, n, blk, s, PairsDone{o}, zeroed);
+        else
+            scan(PairsValue{o}, PairsSink<false>{o}, n, blk, s, PairsDone{o}, zeroed);
         return 1;
     }
+    // the dual's pairs are the context's own buffer
+    longlong2* pairs = reinterpret_cast<longlong2*>(D.pairs);
     const unsigned g = grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256);
     fill_i64(D.death_of, -1, n, s);
     cudaMemsetAsync(D.negative, 0, n, s);  // reused as the "paired or dropped" mark
