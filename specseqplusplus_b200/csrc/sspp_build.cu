@@ -267,7 +267,7 @@ __global__ void k_sort_points(const float* p, int64_t n, const CloudD* clouds, i
 // One warp per point, points in cell order (neighbouring warps read the same
 // cells).  The up to nine rows of three cells around a point are ranges of the
 // sorted points: lanes 0-8 read their bounds together, then all lanes test the
-// candidates.  FILL = false counts the point's upper neighbours into up_off[i]
+// candidates.  FILL = false counts the point's upper neighbours into count[i]
 // and the largest count into *most; FILL = true writes them from up_off[i]:
 // ascending (sorted by the warp, up to kNbrSort of them) or, with `raw`, as
 // found.  One thread per point, searching the sorted cells, took 111 us for the
@@ -277,8 +277,8 @@ constexpr int kNbrSort = 256;
 
 template <bool FILL>
 __global__ void __launch_bounds__(kNbrWarps * 32) k_nbrs(int64_t n, const CloudD* clouds, int k, const int64_t* start,
-                                                         const float4* spt, int64_t* up_off, int32_t* up_v, float* up_w,
-                                                         int32_t* e_src, bool raw, int* most) {
+                                                         const float4* spt, const int64_t* up_off, int32_t* count, int32_t* up_v,
+                                                         float* up_w, int32_t* e_src, bool raw, int* most) {
     __shared__ uint64_t s_buf[FILL ? kNbrWarps : 1][kNbrSort];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     uint64_t* buf = s_buf[FILL ? w : 0];
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kNbrWarps * 32) k_nbrs(int64_t n, const CloudD
             }
         }
         if (!FILL) {
-            if (lane == 0) up_off[i] = cnt;
+            if (lane == 0) count[i] = cnt;
             top = max(top, cnt);
             continue;
         }
@@ -408,12 +408,12 @@ struct DimLimit {
 // triangles (i, j, k), k > j, over edge e = (i, j)
 template <bool FILL>
 __global__ void k_tri(int64_t E, const int64_t* up_off, const int32_t* up_v, const float* up_w, const int32_t* e_src,
-                      DimLimit lim, int64_t* tri_off, int32_t* tri_k, int4* tri_f, float* tri_w) {
+                      DimLimit lim, const int64_t* tri_off, int32_t* count, int32_t* tri_k, int4* tri_f, float* tri_w) {
     GRID_STRIDE(e, E) {
         const int32_t i = e_src[e], j = up_v[e];
         int64_t a = e + 1, b = up_off[j];
         const int64_t ae = lim.below(i, 2) ? a : up_off[i + 1], be = up_off[j + 1];
-        int64_t cnt = 0;
+        int32_t cnt = 0;
         const int64_t base = FILL ? tri_off[e] : 0;
         const float we = FILL ? up_w[e] : 0.0f;
         while (a < ae && b < be) {
@@ -434,7 +434,7 @@ __global__ void k_tri(int64_t E, const int64_t* up_off, const int32_t* up_v, con
                 b++;
             }
         }
-        if (!FILL) tri_off[e] = cnt;
+        if (!FILL) count[e] = cnt;
     }
 }
 
@@ -453,13 +453,13 @@ __device__ __forceinline__ int32_t tri_of(const int64_t* tri_off, const int32_t*
 template <bool FILL>
 __global__ void k_tet(int64_t T, const int64_t* up_off, const int32_t* up_v, const float* up_w, const int64_t* tri_off,
                       const int32_t* tri_k, const int4* tri_f, const float* tri_w, const int32_t* e_src, DimLimit lim,
-                      int64_t* tet_off, int4* tet_f, float* tet_w) {
+                      const int64_t* tet_off, int32_t* count, int4* tet_f, float* tet_w) {
     GRID_STRIDE(t, T) {
         const int4 f = tri_f[t];
         const int32_t k = tri_k[t];
         int64_t a = t + 1, b = up_off[k];
         const int64_t ae = lim.clouds && lim.below(e_src[f.x], 3) ? a : tri_off[f.x + 1], be = up_off[k + 1];
-        int64_t cnt = 0;
+        int32_t cnt = 0;
         const int64_t base = FILL ? tet_off[t] : 0;
         const float wt = FILL ? tri_w[t] : 0.0f;
         while (a < ae && b < be) {
@@ -480,7 +480,7 @@ __global__ void k_tet(int64_t T, const int64_t* up_off, const int32_t* up_v, con
                 b++;
             }
         }
-        if (!FILL) tet_off[t] = cnt;
+        if (!FILL) count[t] = cnt;
     }
 }
 
@@ -582,11 +582,6 @@ struct ReadI32 {
     __device__ int64_t operator()(int64_t i) const { return a[i]; }
 };
 
-struct ReadArr {
-    const int64_t* a;
-    __device__ int64_t operator()(int64_t i) const { return a[i]; }
-};
-
 __global__ void k_rows(int64_t N, Sizes z, const int32_t* perm, const int32_t* rank, const int32_t* e_src,
                        const int32_t* up_v, const int4* tri_f, const int4* tet_f, const int64_t* col_ptr, int64_t ent0,
                        int32_t col0, int32_t* rows) {
@@ -654,15 +649,21 @@ int read_back(BuildScratch& S, std::initializer_list<const int64_t*> src, int64_
     return 0;
 }
 
-// Exclusive scan of a[0..n) in place, a[n] = total.
-int scan_counts(BuildScratch& S, int64_t* a, int64_t n, cudaStream_t s, std::string* err) {
+// Counts of n items, until scan_counts has read them (the ranks come later).
+int take_counts(BuildScratch& S, int64_t n, cudaStream_t s, int32_t** count, std::string* err) {
+    BK(take(S, BuildScratch::RANK, n, s, count));
+    return 0;
+}
+
+// off[0..n) = exclusive scan of count[0..n), off[n] = total.
+int scan_counts(BuildScratch& S, const int32_t* count, int64_t* off, int64_t n, cudaStream_t s, std::string* err) {
     if (n == 0) {
-        BK(cudaMemsetAsync(a, 0, sizeof(int64_t), s));
+        BK(cudaMemsetAsync(off, 0, sizeof(int64_t), s));
         return 0;
     }
     int64_t* blk;
     BK(take(S, BuildScratch::BLK, scan_most_blocks(n) + 2, s, &blk));
-    scan(ReadArr{a}, OffSink{a, n}, n, blk, s);
+    scan(ReadI32{count}, OffSink{off, n}, n, blk, s);
     BK(cudaGetLastError());
     return 0;
 }
@@ -726,27 +727,32 @@ int build_flag(BuildScratch& S, int64_t nv, int64_t E, const float* vval, int ma
     float* tri_w = nullptr;
     int4* tet_f = nullptr;
     float* tet_w = nullptr;
+    int32_t* count = nullptr;
     if (maxdim >= 2 && z.E > 0) {
         BK(take(S, BuildScratch::TRI_OFF, z.E + 1, s, &tri_off));
-        k_tri<false><<<grid_for(z.E), kT, 0, s>>>(z.E, up_off, up_v, up_w, e_src, lim, tri_off, nullptr, nullptr, nullptr);
-        if (scan_counts(S, tri_off, z.E, s, err)) return BUILD_CUDA;
+        if (take_counts(S, z.E, s, &count, err)) return BUILD_CUDA;
+        k_tri<false><<<grid_for(z.E), kT, 0, s>>>(z.E, up_off, up_v, up_w, e_src, lim, nullptr, count, nullptr, nullptr,
+                                                  nullptr);
+        if (scan_counts(S, count, tri_off, z.E, s, err)) return BUILD_CUDA;
         if (read_back(S, {tri_off + z.E}, &z.T, s, err)) return BUILD_CUDA;
         if (int rc = check_size(z.V + z.E + z.T)) return rc;
         BK(take(S, BuildScratch::TRI_K, z.T, s, &tri_k));
         BK(take(S, BuildScratch::TRI_F, z.T, s, &tri_f));
         BK(take(S, BuildScratch::TRI_W, z.T, s, &tri_w));
-        k_tri<true><<<grid_for(z.E), kT, 0, s>>>(z.E, up_off, up_v, up_w, e_src, lim, tri_off, tri_k, tri_f, tri_w);
+        k_tri<true><<<grid_for(z.E), kT, 0, s>>>(z.E, up_off, up_v, up_w, e_src, lim, tri_off, nullptr, tri_k, tri_f,
+                                                 tri_w);
         if (maxdim >= 3 && z.T > 0) {
             BK(take(S, BuildScratch::TET_OFF, z.T + 1, s, &tet_off));
+            if (take_counts(S, z.T, s, &count, err)) return BUILD_CUDA;
             k_tet<false><<<grid_for(z.T), kT, 0, s>>>(z.T, up_off, up_v, up_w, tri_off, tri_k, tri_f, tri_w, e_src, lim,
-                                                      tet_off, nullptr, nullptr);
-            if (scan_counts(S, tet_off, z.T, s, err)) return BUILD_CUDA;
+                                                      nullptr, count, nullptr, nullptr);
+            if (scan_counts(S, count, tet_off, z.T, s, err)) return BUILD_CUDA;
             if (read_back(S, {tet_off + z.T}, &z.Q, s, err)) return BUILD_CUDA;
             if (int rc = check_size(z.V + z.E + z.T + z.Q)) return rc;
             BK(take(S, BuildScratch::TET_F, z.Q, s, &tet_f));
             BK(take(S, BuildScratch::TET_W, z.Q, s, &tet_w));
             k_tet<true><<<grid_for(z.T), kT, 0, s>>>(z.T, up_off, up_v, up_w, tri_off, tri_k, tri_f, tri_w, e_src, lim,
-                                                     tet_off, tet_f, tet_w);
+                                                     tet_off, nullptr, tet_f, tet_w);
         }
     }
     const int64_t N = z.V + z.E + z.T + z.Q;
@@ -894,10 +900,11 @@ int build_clouds(BuildScratch& S, const float* d_points, const Cloud* clouds, in
         BK(take(S, BuildScratch::BLK, scan_most_blocks(std::max(cells, n)) + 2, s, &blk));
         scan(ReadI32{count}, OffSink{start, cells}, cells, blk, s);
         k_sort_points<<<grid_for(n), kT, 0, s>>>(d_points, n, dc, k, start, pcell, pslot, spt);
-        k_nbrs<false><<<ng, kNbrWarps * 32, 0, s>>>(n, dc, k, start, spt, up_off, nullptr, nullptr, nullptr, false,
-                                                    flag + 2);
+        // (there are at least four cells per point: the cells' counts have been scanned)
+        k_nbrs<false><<<ng, kNbrWarps * 32, 0, s>>>(n, dc, k, start, spt, nullptr, count, nullptr, nullptr, nullptr,
+                                                    false, flag + 2);
     }
-    if (scan_counts(S, up_off, n, s, err)) return BUILD_CUDA;
+    if (scan_counts(S, count, up_off, n, s, err)) return BUILD_CUDA;
     if (read_back(S, {up_off + n, reinterpret_cast<int64_t*>(flag), reinterpret_cast<int64_t*>(flag + 2)}, got, s, err))
         return BUILD_CUDA;
     if (got[1]) return fail(err, "non-finite point coordinate");
@@ -919,7 +926,8 @@ int build_clouds(BuildScratch& S, const float* d_points, const Cloud* clouds, in
             BK(take(S, BuildScratch::UP_V2, E, s, &v));
             BK(take(S, BuildScratch::UP_W2, E, s, &w));
         }
-        k_nbrs<true><<<ng, kNbrWarps * 32, 0, s>>>(n, dc, k, start, spt, up_off, v, w, e_src, raw, nullptr);
+        k_nbrs<true><<<ng, kNbrWarps * 32, 0, s>>>(n, dc, k, start, spt, up_off, nullptr, v, w, e_src, raw,
+                                                   nullptr);
         if (raw) {
             size_t sb = 0;
             BK(cub::DeviceSegmentedSort::StableSortPairs(nullptr, sb, v, up_v, w, up_w, int(E), int(n), up_off,

@@ -105,9 +105,9 @@ struct DualReserve {
     }
 };
 
-// scatter: cnt[] counts up again as the entries land (unsorted)
+// scatter: filled[] counts up as the entries land (unsorted)
 __global__ void k_dual_fill(int64_t n, const uint64_t* desc, int skip_edges, const DimInfo* info, const int64_t* off,
-                            const int64_t* misc, int32_t* cnt, int32_t* arena) {
+                            const int64_t* misc, int32_t* filled, int32_t* arena) {
     const int64_t base = misc[0];
     if (base < 0) return;
     for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < n; j += int64_t(gridDim.x) * blockDim.x) {
@@ -117,7 +117,7 @@ __global__ void k_dual_fill(int64_t n, const uint64_t* desc, int skip_edges, con
         const uint32_t len = desc_len(d);
         for (uint32_t k = 0; k < len; k++) {
             const int64_t c = n - 1 - col[k];
-            arena[base + off[c] + kHdr + atomicAdd(&cnt[c], 1)] = int32_t(n - 1 - j);
+            arena[base + off[c] + kHdr + atomicAdd(&filled[c], 1)] = int32_t(n - 1 - j);
         }
     }
 }
@@ -483,23 +483,25 @@ __global__ void __launch_bounds__(kLongThreads) k_dual_sort_long(const int64_t* 
     }
 }
 
+// [2 n], in the pairs' death list, which is free until they are extracted
+int32_t* dual_lengths(const Device& D) { return reinterpret_cast<int32_t*>(D.death_of); }
+
 }  // namespace
 
 int dualize_begin(Device& D, int mode, cudaStream_t s) {
     const int64_t n = D.n;
     const unsigned g = grid_of(n, 256, 65536);
-    int32_t* cnt = D.leftmost;  // free after the init passes
+    // the columns' lengths, and as many counters for the fill (the scan between the two
+    // reads the lengths, so they have to stay)
+    int32_t* cnt = dual_lengths(D);
+    int32_t* filled = cnt + n;
     int64_t* off = D.scratch64;
     const int skip = mode == 2;
-    cudaMemsetAsync(cnt, 0, sizeof(int32_t) * n, s);
+    cudaMemsetAsync(cnt, 0, 2 * sizeof(int32_t) * n, s);
     k_dual_count<<<g, 256, 0, s>>>(n, D.arena, D.desc, skip, D.diminfo, cnt);
     scan([=] __device__(int64_t c) -> int64_t { return slot_ints(cnt[c]); },
-         [=] __device__(int64_t c, int64_t pre, int64_t) {
-             off[c] = pre;
-             cnt[c] = 0;
-         },
-         n, D.blk, s, DualReserve{n, D.arena_top, D.arena_cap, D.misc, D.diminfo, D.err});
-    k_dual_fill<<<g, 256, 0, s>>>(n, D.desc, skip, D.diminfo, off, D.misc, cnt, D.arena);
+         [=] __device__(int64_t c, int64_t pre, int64_t) { off[c] = pre; }, n, D.blk, s, DualReserve{n, D.arena_top, D.arena_cap, D.misc, D.diminfo, D.err});
+    k_dual_fill<<<g, 256, 0, s>>>(n, D.desc, skip, D.diminfo, off, D.misc, filled, D.arena);
     return 3;
 }
 
@@ -507,7 +509,7 @@ int dualize_end(Device& D, int mode, cudaStream_t s) {
     const int64_t n = D.n;
     // the row bounds go to the DimInfo through a few atomics per block: few blocks
     k_dual_finish<<<grid_of((n + 1) / 2, kSortWarps * 32, 2048), kSortWarps * 32, 0, s>>>(
-        DualCols{n, D.scratch64, D.leftmost, D.misc, D.arena, D.active, D.desc, D.low, D.dim, D.pivot, D.state, D.cleared,
+        DualCols{n, D.scratch64, dual_lengths(D), D.misc, D.arena, D.active, D.desc, D.low, D.dim, D.pivot, D.state, D.cleared,
                  D.app, D.diminfo, D.err, mode == 2});
     // the pairs buffer (4n ints) is free until the pairs are extracted
     k_dual_sort_long<<<1, kLongThreads, 0, s>>>(D.scratch64, D.misc, D.arena, D.active,

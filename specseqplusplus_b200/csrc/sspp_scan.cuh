@@ -2,6 +2,10 @@
 // ScanClass for a selection), sink(i, exclusive prefix, value), and at the end
 // done(total).  Used for column offsets and stream compaction.
 //
+// value(i) must not read anything that a sink or done writes: a tile whose
+// predecessors do not answer (kScanPolls) takes their values itself, when other
+// tiles' sinks may have run already.
+//
 // Tiles of 4096 items (1024 in mid-sized scans) per 256-thread block.  A warp takes 512
 // (128) consecutive items, 32 at a time, so that values are read and prefixes written coalesced.  Tiles
 // publish their sums and read their predecessors' (decoupled look-back, 256 tiles
@@ -30,7 +34,10 @@ constexpr int64_t kScanFewMax = int64_t(1) << 18;
 // A tile's published state: flag in the top two bits (0 nothing, 1 the tile's own
 // sum, 2 the sum up to and including it), the sum below.
 constexpr unsigned long long kScanSum = 1ull << 62, kScanPrefix = 2ull << 62, kScanValue = kScanSum - 1;
-constexpr int kScanPolls = 1 << 22;
+#ifndef SSPP_SCAN_POLLS
+#define SSPP_SCAN_POLLS (1 << 22)
+#endif
+constexpr int kScanPolls = SSPP_SCAN_POLLS;
 
 __device__ __forceinline__ unsigned long long scan_load(const unsigned long long* p) {
     unsigned long long v;
