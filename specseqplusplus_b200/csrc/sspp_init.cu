@@ -607,17 +607,19 @@ __global__ void __launch_bounds__(256) k_init_apparent(int64_t n, const int32_t*
 __global__ void k_init_compress(int64_t n, int32_t* arena, uint64_t* desc, int32_t* low, const uint64_t* pivot,
                                 const uint8_t* cleared, const uint8_t* negative, uint8_t* state,
                                 const uint8_t* dropped, bool keep_rows, int4* app, const int32_t* rinfo, Ctl* ctl) {
-    if (ctl->err) return;
     DimInfo* info = &ctl->info;
     long long* counters = ctl->counters;
     const bool all_short = ctl->max_len <= kShortLen;
     __shared__ int smin[kNumDims], smax[kNumDims], sact[kNumDims];
+    __shared__ int s_err;  // one look per block: other blocks may set the error word meanwhile
+    if (threadIdx.x == 0) s_err = ctl->err;
     if (threadIdx.x < kNumDims) {
         smin[threadIdx.x] = INT_MAX;
         smax[threadIdx.x] = -1;
         sact[threadIdx.x] = 0;
     }
     __syncthreads();
+    if (s_err) return;
     long long ncl = 0, nact = 0;
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
         if (app && pivot[i] == kNoOwner) app[i] = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
