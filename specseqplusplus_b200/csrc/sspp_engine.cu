@@ -984,6 +984,8 @@ int run_compute(sspp_ctx* ctx) {
         ctx->launches += push_results(D, ctx->h_ctl, ctx->h_pairs, kPushCols / 2, ctx->h_ess, kPushCols, s);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(s));
+        // (in a matrix that is no chain complex a column may be in two pairs)
+        ctx->pushed = ctx->h_ctl->counters[CNT_NPAIRS] <= kPushCols / 2;
     } else if (int rc = read_ctl(ctx)) {
         return rc;
     }
