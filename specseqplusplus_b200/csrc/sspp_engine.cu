@@ -1713,11 +1713,16 @@ int32_t sspp_batch_copy(sspp_ctx* ctx, int64_t* const* pairs_out, int64_t* const
     const int64_t np = ctx->hcounters[CNT_NPAIRS], ne = ctx->hcounters[CNT_NESS];
     Device& D = ctx->D;
     cudaStream_t s = ctx->stream;
-    // local copies live in buffers the reduction no longer needs: 2 np <= n, ne <= n
+    // local copies live in buffers the reduction no longer needs: ne <= n, and 2 np <= n
+    // unless columns are in two pairs (a matrix that is no chain complex)
     int64_t* lp = D.death_of;
     int64_t* le = D.scratch64;
+    int64_t* more = nullptr;
+    if (2 * np > D.cap_n) {
+        CK(cudaMallocAsync(reinterpret_cast<void**>(&more), sizeof(int64_t) * 2 * size_t(np), s));
+        lp = more;
+    }
     batch_localize(np, ne, k, ctx->d_batch, D.pairs, D.ess, lp, le, s);
-    CK(cudaGetLastError());
     const int64_t* ps = ctx->batch_bounds.data();
     const int64_t* es = ps + k + 1;
     std::vector<Piece> pcs;
@@ -1731,7 +1736,10 @@ int32_t sspp_batch_copy(sspp_ctx* ctx, int64_t* const* pairs_out, int64_t* const
         const int64_t a = es[i], b = i + 1 < k ? es[i + 1] : ne;
         if (b > a && ess_out && ess_out[i]) pcs.push_back({le + a, ess_out[i], sizeof(int64_t) * size_t(b - a), -1});
     }
-    CK(ctx->xfer.d2h(pcs, s));
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = ctx->xfer.d2h(pcs, s);
+    if (more) cudaFreeAsync(more, s);
+    if (e != cudaSuccess) return set_err(ctx, SSPP_ERR_CUDA, std::string("batch results: ") + cudaGetErrorString(e));
     return SSPP_OK;
 }
 

@@ -38,3 +38,15 @@ def test_pairs_of_columns_that_are_in_two(k):
             assert e.num_pairs() == 3 * k
             assert np.array_equal(e.pairs(), want)
             assert np.array_equal(e.essentials(), ess)
+
+
+def test_batch_of_such_matrices():
+    sizes = [1, 2000, 70, 900, 5]
+    cases = [units(k) for k in sizes]
+    with Engine(0) as e:
+        for _ in range(2):
+            e.load_batch([m for m, _, _ in cases])
+            e.reduce(Params(representatives=1))
+            for (pairs, ess), (_, want, none) in zip(e.batch_results(), cases):
+                assert np.array_equal(pairs, want)
+                assert np.array_equal(ess, none)
