@@ -386,7 +386,8 @@ int32_t sspp_server_reset_stats(sspp_server* srv);
  * device pointers: d_pairs receives up to ncols (birth, death) int64 pairs
  * sorted by birth (room for 2 * ncols int64), *d_npairs their number.  Limits:
  * ncols <= 1048576 and 3 * ncols + nnz <= 12582896, else SSPP_ERR_BAD_INPUT;
- * fill-in beyond the array gives SSPP_ERR_CAPACITY; a col_ptr that does not
+ * fill-in beyond the array gives SSPP_ERR_CAPACITY, with nothing written to
+ * d_pairs and d_npairs; a col_ptr that does not
  * run from 0 to nnz without decreasing, a dimension outside 0..7, or faces that
  * are unsorted, out of range or not one dimension lower give
  * SSPP_ERR_BAD_INPUT.  The first call on a device looks up the array's address

@@ -874,7 +874,7 @@ int push_results(const Device& D, Ctl* h_ctl, int64_t* h_pairs, int64_t max_pair
     return 1;
 }
 
-int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s) {
+int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s, const int* unless) {
     const int64_t n = D.n;
     const PairsOut o{n, D.newidx, D.perm, D.pivot, D.state, D.pairs, D.ess, D.counters, D.err,
                      D.edge_begin, D.edge_end};
@@ -882,9 +882,9 @@ int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s) {
     int64_t* blk = scan_region(D, 2, &zeroed);
     if (!dual) {
         if (reinterpret_cast<uintptr_t>(D.pairs) % sizeof(longlong2) == 0)
-            scan(PairsValue{o}, PairsSink<true>{o}, n, blk, s, PairsDone{o}, zeroed);
+            scan(PairsValue{o}, PairsSink<true>{o}, n, blk, s, PairsDone{o}, zeroed, nullptr, 0, unless);
         else
-            scan(PairsValue{o}, PairsSink<false>{o}, n, blk, s, PairsDone{o}, zeroed);
+            scan(PairsValue{o}, PairsSink<false>{o}, n, blk, s, PairsDone{o}, zeroed, nullptr, 0, unless);
         return 1;
     }
     // the dual's pairs are the context's own buffer

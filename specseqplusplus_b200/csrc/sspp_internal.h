@@ -101,6 +101,8 @@ struct Ctl {
     int wide_edges;   // a column of dimension 1 holds more than two entries (validation pass)
     int pool_tail;    // CTA-tier pool entries
     int heavy_done;   // pool columns the CTA tier has finished
+    int fill_next;    // see FillArgs
+    unsigned long long fill;
     int step[kNumDims * kStepCtr];
 };
 

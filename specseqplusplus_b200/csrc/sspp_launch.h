@@ -56,7 +56,8 @@ int push_results(const Device& D, Ctl* h_ctl, int64_t* h_pairs, int64_t max_pair
 // dimension 1 of the boundary matrix (active list entries [beg, end), no column of
 // more than two entries) over the vertices, the reordered rows [0, rows)
 int reduce_edges(Device& D, int32_t beg, int32_t end, int32_t rows, cudaStream_t s);
-int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s);
+// unless (dual 0): a device word; when it is set, nothing is written
+int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s, const int* unless = nullptr);
 
 // Device work queue of (complex, block) items (one persistent launch per
 // schedule; see k_reduce_queue).  An item is one spectral-sequence block of
@@ -118,6 +119,10 @@ cudaError_t reduce_configure(int cap1, int cap2, int heavy_threads, int* light_b
 // step's CTA-tier pool slice (ctr[2], and ctr_next[1] of the next step when given).
 void reduce_light_launch(const Device& D, int32_t beg, int32_t end, int cap, int* ctr, int* ctr_next, int grid,
                          cudaStream_t s);
+// After a reduction with whole columns and no error: the ints that the additions of a
+// column-after-column reduction read, `listed` active columns, added up into ctl->fill;
+// sets ERRB_CAPACITY when they exceed `room`, or when it cannot tell.  ready: [n], zeroed.
+void fill_account_launch(const Device& D, int32_t listed, int64_t room, uint64_t* ready, int sms, cudaStream_t s);
 void reduce_heavy_launch(const Device& D, int cap, int threads, int* ctr, int grid, cudaStream_t s);
 
 }  // namespace sspp

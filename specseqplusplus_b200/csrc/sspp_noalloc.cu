@@ -14,8 +14,8 @@
 // output buffers, all in device memory; nothing else is allocated.  Limits:
 // at most kMaxCols columns, and 3 * ncols + nnz + fill-in must fit in the
 // array (the host rejects inputs that leave less than kFillReserve ints for
-// fill-in; a reduction whose fill-in still overflows returns
-// SSPP_ERR_CAPACITY).
+// fill-in; a reduction whose fill-in still overflows returns SSPP_ERR_CAPACITY and
+// writes neither pairs nor their number).
 //
 // The array's device address is looked up with cudaGetSymbolAddress the
 // first time the entry point runs on a device (with that device current) and
@@ -33,7 +33,7 @@
 // dimensions must lie in 0..7, and each column's faces must be ascending, in
 // range and one dimension lower; anything else is SSPP_ERR_BAD_INPUT.
 //
-// Two ways.  While the engine's arrays (about 67 bytes per column and the padded
+// Two ways.  While the engine's arrays (about 71 bytes per column and the padded
 // column arena) fit in the scratch array, its own passes run there on the
 // caller's stream (reduce_in_scratch): the same reorder, apparent pairs and
 // reduction kernels as the context API's, one block per dimension.  Otherwise,
@@ -47,12 +47,17 @@
 // negative-row compression, the only pass that needs the boundary of a boundary
 // to be zero, is left out here, and a run in which a column is both a birth and a
 // death (possible only without that property, where the twist's clearing would
-// have come first) goes to k_reduce_noalloc.  The fill-in limit stays that of
-// k_reduce_noalloc: a run whose additions read and write more than the room it
-// would have goes there too, and gets its verdict.
+// have come first) goes to k_reduce_noalloc.
 //
-// Measured (B200, device-resident input): 700 points (6,720 columns) 8.5 ms by one
-// block, 0.25 ms by the engine's passes.
+// The fill-in limit is that of k_reduce_noalloc, which takes new room for every single
+// addition.  The passes need far less (250 columns of 4,096 rows over rows owned by
+// short columns overflow it after four of them), and how much depends on the order in
+// which their blocks run, so their own additions say nothing about it: once the pairs
+// are known, k_fill_account adds up what k_reduce_noalloc's would take.  More than
+// its room is refused at once; where the account cannot tell, k_reduce_noalloc runs.
+//
+// Measured (B200, device-resident input): 700 points (7,678 columns) 9.5 ms by one
+// block, 0.29 ms by the engine's passes, of which the account is 0.04.
 #include <algorithm>
 #include <climits>
 #include <cstddef>
@@ -264,8 +269,7 @@ constexpr int64_t kGuard = 8192;   // ints after the arena: staging reads a firs
 
 // Engine arrays carved out of the scratch array; false when they leave too
 // little for the arena.  Buffers whose lifetimes do not meet share memory: the
-// pairs pass's death list lies in the inline columns, its essentials in the
-// column descriptors.
+// pairs pass's essentials lie in the column descriptors.
 bool carve(int32_t* scratch, int64_t n, int64_t nnz, Device& D) {
     char* p = reinterpret_cast<char*>(scratch);
     char* const end = p + sizeof(int32_t) * kScratchInts;
@@ -304,7 +308,6 @@ bool carve(int32_t* scratch, int64_t n, int64_t nnz, Device& D) {
     D.err = &D.ctl->err;
     D.pool_tail = &D.ctl->pool_tail;
     D.heavy_done = &D.ctl->heavy_done;
-    D.death_of = reinterpret_cast<int64_t*>(D.app);
     D.ess = reinterpret_cast<int64_t*>(D.desc);
     // the input's slots, and as much again for the reduction's column versions
     return D.arena_cap >= 2 * (nnz + (kHdr + 3) * n + 4);
@@ -317,8 +320,8 @@ __global__ void k_check_complex(int64_t n, const uint64_t* pivot, const uint8_t*
 }
 
 // *npairs is written by a run that ends cleanly only.
-__global__ void k_store_npairs(const Ctl* st, int64_t room, int64_t* npairs) {
-    if (st->err == 0 && st->counters[CNT_ADD_INTS] <= room) *npairs = st->counters[CNT_NPAIRS];
+__global__ void k_store_npairs(const Ctl* st, int64_t* npairs) {
+    if (st->err == 0) *npairs = st->counters[CNT_NPAIRS];
 }
 
 // The device's multiprocessors and the reduction kernels' blocks per
@@ -343,12 +346,15 @@ cudaError_t launch_shape(int dev, Launch* out) {
     return cudaSuccess;
 }
 
-// Runs the engine's passes in the scratch array.  *done: the pairs are in
-// place; otherwise the caller runs k_reduce_noalloc.
+// How a run of the engine's passes ended: the pairs are in place, or their fill-in is
+// refused, or k_reduce_noalloc has to run.
+enum class Ended { Done, Refused, Unknown };
+
+// Runs the engine's passes in the scratch array.
 cudaError_t reduce_in_scratch(int32_t* scratch, int dev, int64_t n, int64_t nnz, const int32_t* d_dims,
                               const int64_t* d_col_ptr, const int32_t* d_rows, int64_t* d_pairs, int64_t* d_npairs,
-                              cudaStream_t s, bool* done) {
-    *done = false;
+                              cudaStream_t s, Ended* ended) {
+    *ended = Ended::Unknown;
     Device D;
     if (n < 1 || !carve(scratch, n, nnz, D)) return cudaSuccess;
     Launch shape;
@@ -380,13 +386,18 @@ cudaError_t reduce_in_scratch(int32_t* scratch, int dev, int64_t n, int64_t nnz,
         ctr += kStepCtr;
     }
     k_check_complex<<<unsigned(std::min<int64_t>((n + 255) / 256, 4096)), 256, 0, s>>>(n, D.pivot, D.state, D.err);
-    extract_pairs(D, 0, nullptr, s);
+    // (the descriptors are not needed any more, and the essentials come later)
+    uint64_t* ready = D.desc;
+    cudaMemsetAsync(ready, 0, sizeof(uint64_t) * size_t(n), s);
     const int64_t room = kScratchInts - (kCtl + 3 * n) - nnz;  // k_reduce_noalloc's room for fill-in
-    k_store_npairs<<<1, 1, 0, s>>>(D.ctl, room, d_npairs);
+    fill_account_launch(D, h.info.act_end[kMaxDim], room, ready, shape.sms, s);
+    extract_pairs(D, 0, nullptr, s, D.err);  // nothing goes to the caller unless all is well
+    k_store_npairs<<<1, 1, 0, s>>>(D.ctl, d_npairs);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     cudaMemcpyAsync(&h, D.ctl, offsetof(Ctl, step), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-    *done = h.err == 0 && h.counters[CNT_ADD_INTS] <= room;
+    if (h.err == 0) *ended = Ended::Done;
+    else if (int64_t(h.fill) > room) *ended = Ended::Refused;
     return cudaSuccess;
 }
 
@@ -427,11 +438,13 @@ extern "C" int32_t sspp_reduce_noalloc(int64_t ncols, int64_t nnz, const int32_t
         addr = g_scratch_addr[dev];
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    bool done = false;
+    Ended ended;
     cudaError_t e = reduce_in_scratch(static_cast<int32_t*>(addr), dev, ncols, nnz, d_dims, d_col_ptr, d_rows, d_pairs,
-                                      d_npairs, s, &done);
+                                      d_npairs, s, &ended);
     if (e != cudaSuccess) return fail(err_msg, err_cap, SSPP_ERR_CUDA, cudaGetErrorString(e));
-    if (done) return fail(err_msg, err_cap, SSPP_OK, "");
+    const char* const kFillIn = "fill-in exceeded the 64 MiB allocation-free scratch array";
+    if (ended == Ended::Done) return fail(err_msg, err_cap, SSPP_OK, "");
+    if (ended == Ended::Refused) return fail(err_msg, err_cap, SSPP_ERR_CAPACITY, kFillIn);
     k_reduce_noalloc<<<1, kThreads, 0, s>>>(static_cast<int32_t*>(addr), ncols, nnz, d_dims, d_col_ptr, d_rows,
                                             d_pairs, d_npairs);
     e = cudaGetLastError();
@@ -444,6 +457,6 @@ extern "C" int32_t sspp_reduce_noalloc(int64_t ncols, int64_t nnz, const int32_t
         return fail(err_msg, err_cap, SSPP_ERR_BAD_INPUT,
                     "malformed boundary matrix (col_ptr, face order, range or dimension)");
     if (err & E_CAPACITY)
-        return fail(err_msg, err_cap, SSPP_ERR_CAPACITY, "fill-in exceeded the 64 MiB allocation-free scratch array");
+        return fail(err_msg, err_cap, SSPP_ERR_CAPACITY, kFillIn);
     return fail(err_msg, err_cap, SSPP_OK, "");
 }

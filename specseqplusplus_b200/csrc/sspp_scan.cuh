@@ -183,8 +183,9 @@ struct ScanLane<ScanBytes, kItems> {
 
 template <int kItems, class F, class G, class H>
 __global__ void __launch_bounds__(kScanThreads) k_scan(F value, G sink, H done, int64_t n, int64_t nb, int64_t* blk,
-                                                       const int* skip_upto, int skip_limit) {
+                                                       const int* skip_upto, int skip_limit, const int* unless) {
     if (skip_upto && *skip_upto <= skip_limit) return;
+    if (unless && *unless) return;
     using Lane = ScanLane<decltype(value(int64_t(0))), kItems>;
     constexpr int kTile = kScanThreads * kItems;
     constexpr int kWarps = kScanThreads / 32;
@@ -273,10 +274,11 @@ inline int64_t scan_most_blocks(int64_t n) {
 
 // Scratch (blk) must hold scan_blocks(n) + 1 entries (a selection by bytes: as many as
 // fewer); the total is left after the last tile's.  zeroed: the entries are zero already.
-// A launch whose *skip_upto turns out to be at most skip_limit does nothing.
+// A launch whose *skip_upto turns out to be at most skip_limit, or whose *unless is set,
+// does nothing (neither may change while it runs).
 template <class F, class G, class H = ScanNoop>
 void scan(F value, G sink, int64_t n, int64_t* blk, cudaStream_t s, H done = H(), bool zeroed = false,
-          const int* skip_upto = nullptr, int skip_limit = 0) {
+          const int* skip_upto = nullptr, int skip_limit = 0, const int* unless = nullptr) {
     constexpr bool bytes = std::is_same<F, ScanBytes>::value;
     const int64_t nb = bytes ? (n + kScanOneTile - 1) / kScanOneTile : scan_blocks(n);
     if (nb == 0) {
@@ -286,9 +288,10 @@ void scan(F value, G sink, int64_t n, int64_t* blk, cudaStream_t s, H done = H()
     if (nb > 1 && !zeroed) cudaMemsetAsync(blk, 0, sizeof(int64_t) * size_t(nb), s);
     if (!bytes && scan_few(n))
         k_scan<bytes ? kScanItems : kScanFewItems>
-            <<<unsigned(nb), kScanThreads, 0, s>>>(value, sink, done, n, nb, blk, skip_upto, skip_limit);
+            <<<unsigned(nb), kScanThreads, 0, s>>>(value, sink, done, n, nb, blk, skip_upto, skip_limit, unless);
     else
-        k_scan<kScanItems><<<unsigned(nb), kScanThreads, 0, s>>>(value, sink, done, n, nb, blk, skip_upto, skip_limit);
+        k_scan<kScanItems>
+            <<<unsigned(nb), kScanThreads, 0, s>>>(value, sink, done, n, nb, blk, skip_upto, skip_limit, unless);
 }
 
 // Tile states of one of a Device's regions, zero unless a scan used them since
