@@ -33,10 +33,11 @@
 // dimensions must lie in 0..7, and each column's faces must be ascending, in
 // range and one dimension lower; anything else is SSPP_ERR_BAD_INPUT.
 //
-// Two ways.  While the engine's arrays (about 71 bytes per column and the padded
-// column arena) fit in the scratch array, its own passes run there on the
-// caller's stream (reduce_in_scratch): the same reorder, apparent pairs and
-// reduction kernels as the context API's, one block per dimension.  Otherwise,
+// Two ways.  For more than kFewCols columns, and while the engine's arrays (about 71
+// bytes per column and the padded column arena) fit in the scratch array, its own
+// passes run there on the caller's stream (reduce_in_scratch): the same reorder,
+// apparent pairs and reduction kernels as the context API's, one block per dimension.
+// Otherwise,
 // and whenever that run does not end cleanly (malformed input, arena or fill-in
 // limit, or a matrix that is not a chain complex where the two could differ),
 // k_reduce_noalloc decides: the standard twist (clearing) reduction, dimensions
@@ -265,6 +266,10 @@ using namespace sspp;
 
 constexpr int kCap1 = 64;          // warp-tier column capacity (ints), as the context API's bound
 constexpr int kCap2 = 8192;        // CTA-tier column capacity
+// Up to here k_reduce_noalloc is done before the passes' launches and two waits are:
+// 51 / 92 / 134 / 201 columns 54 / 92 / 115 / 154 us against 90 / 145 / 155 / 173,
+// 226 / 293 / 410 columns 197 / 153 / 337 against 192 / 148 / 221.
+constexpr int64_t kFewCols = 224;
 constexpr int64_t kGuard = 8192;   // ints after the arena: staging reads a first pass beyond a slot
 
 // Engine arrays carved out of the scratch array; false when they leave too
@@ -356,7 +361,7 @@ cudaError_t reduce_in_scratch(int32_t* scratch, int dev, int64_t n, int64_t nnz,
                               cudaStream_t s, Ended* ended) {
     *ended = Ended::Unknown;
     Device D;
-    if (n < 1 || !carve(scratch, n, nnz, D)) return cudaSuccess;
+    if (n <= kFewCols || !carve(scratch, n, nnz, D)) return cudaSuccess;
     Launch shape;
     cudaError_t e = launch_shape(dev, &shape);
     if (e != cudaSuccess) return e;

@@ -10,6 +10,7 @@ import oracle
 from specseqplusplus_b200 import SsppError, gen
 from specseqplusplus_b200.engine import reduce_noalloc
 from specseqplusplus_b200.gen import BoundaryMatrix
+from test_gpu_noalloc_scratch import twist_pairs
 from test_zz_no_alloc import _noalloc_pairs
 
 pytestmark = pytest.mark.gpu
@@ -34,6 +35,32 @@ def test_pairs_on_any_eight_byte_boundary(npts, shift):
     # and nothing else of the pool
     rest = np.delete(got, np.r_[shift, 4 + shift:4 + shift + 2 * k])
     assert (rest == -7).all()
+
+
+@pytest.mark.parametrize("ncols", [1, 2, 51, 223, 224, 225, 226])  # up to 224: the one-block kernel alone
+def test_columns_around_the_smallest_of_the_passes(ncols):
+    torch = pytest.importorskip("torch")
+    m = gen.rips(64, 3, 5, 0.4, 3)
+    m = BoundaryMatrix(m.dims[:ncols], m.col_ptr[:ncols + 1], m.rows[:m.col_ptr[ncols]])  # a subcomplex
+    assert m.ncols == ncols
+    assert np.array_equal(_noalloc_pairs(m, torch), oracle.reduce(m).pairs)
+
+
+@pytest.mark.parametrize("seed", range(20))
+def test_larger_matrices_that_are_not_chain_complexes(seed):
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(seed)
+    layer = [int(rng.integers(120, 400)) for _ in range(int(rng.integers(2, 5)))]
+    dims, cols, begin = [], [], 0
+    for d, n in enumerate(layer):
+        for _ in range(n):
+            k = 0 if d == 0 else int(rng.integers(0, 7))
+            cols.append(begin + rng.choice(layer[d - 1], size=k, replace=False) if k else [])
+            dims.append(d)
+        if d:
+            begin += layer[d - 1]
+    m = BoundaryMatrix.from_columns(dims, cols)
+    assert m.ncols > 224 and np.array_equal(_noalloc_pairs(m, torch), twist_pairs(m))
 
 
 def _long_columns(k):
