@@ -161,8 +161,16 @@ struct CloudD {
     double lo[3];
     double side;
     int32_t n[3];
+    // while the bounding box is found (k_cloud_grid)
+    uint32_t key_lo[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, key_hi[3] = {0, 0, 0};
+    int32_t bad = 0, arrived = 0;
 };
 constexpr int kCellSlack = 64;
+constexpr int kBoxPoints = 2048, kBoxBlocks = 512;  // points a block at least, blocks a cloud at most
+__host__ __device__ inline int box_blocks(int64_t npts) {
+    const int64_t b = (npts + kBoxPoints - 1) / kBoxPoints;
+    return int(b < 1 ? 1 : b > kBoxBlocks ? kBoxBlocks : b);
+}
 
 __device__ __forceinline__ int32_t cell_coord(const CloudD& c, int d, float x) {
     const double t = floor((double(x) - c.lo[d]) / c.side);
@@ -170,13 +178,17 @@ __device__ __forceinline__ int32_t cell_coord(const CloudD& c, int d, float x) {
     return k < 0 ? 0 : (k >= c.n[d] ? c.n[d] - 1 : k);
 }
 
-// One block per cloud: the bounding box (also rejects non-finite coordinates)
-// and the cell grid.  Cells of side > radius: a margin of 2^-10 covers the rounding of
-// the float distance and of the cell coordinate; at most ~1000 per axis.
+// Cloud blockIdx.x's bounding box (also rejects non-finite coordinates), by box_blocks of
+// its size, and, by the last of them, its cell grid.  Cells of side > radius: a margin
+// of 2^-10 covers the rounding of the float distance and of the cell coordinate; at most
+// ~1000 per axis.  (One block whatever the size made loads of 300,000 and 1 M points
+// 1,146 and 4,307 us where they take 780 and 1,930 now.)
 __global__ void __launch_bounds__(kT) k_cloud_grid(const float* p, CloudD* clouds, int* flag) {
     __shared__ uint32_t s_lo[3], s_hi[3];
     __shared__ int s_bad;
     CloudD& c = clouds[blockIdx.x];
+    const int blocks = box_blocks(c.npts);
+    if (int(blockIdx.y) >= blocks) return;
     if (threadIdx.x < 3) {
         s_lo[threadIdx.x] = 0xFFFFFFFFu;
         s_hi[threadIdx.x] = 0;
@@ -186,7 +198,7 @@ __global__ void __launch_bounds__(kT) k_cloud_grid(const float* p, CloudD* cloud
     const int D = c.D;
     uint32_t lo[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, hi[3] = {0, 0, 0};
     bool bad = false;
-    for (int i = threadIdx.x; i < c.npts; i += kT) {
+    for (int i = blockIdx.y * kT + threadIdx.x; i < c.npts; i += blocks * kT) {
         for (int d = 0; d < D; d++) {
             const float x = p[c.f0 + int64_t(i) * D + d];
             if (!isfinite(x)) bad = true;
@@ -205,7 +217,24 @@ __global__ void __launch_bounds__(kT) k_cloud_grid(const float* p, CloudD* cloud
     }
     if (bad) s_bad = 1;
     __syncthreads();
+    if (threadIdx.x < 3 && blocks > 1) {
+        atomicMin(&c.key_lo[threadIdx.x], s_lo[threadIdx.x]);
+        atomicMax(&c.key_hi[threadIdx.x], s_hi[threadIdx.x]);
+        if (threadIdx.x == 0 && s_bad) atomicOr(&c.bad, 1);
+        __threadfence();
+    }
+    __syncthreads();
     if (threadIdx.x) return;
+    if (blocks > 1) {
+        __threadfence();
+        if (atomicAdd(&c.arrived, 1) != blocks - 1) return;
+        __threadfence();
+        for (int d = 0; d < 3; d++) {
+            s_lo[d] = __ldcg(&c.key_lo[d]);
+            s_hi[d] = __ldcg(&c.key_hi[d]);
+        }
+        s_bad = __ldcg(&c.bad);
+    }
     if (s_bad) atomicOr(flag, 1);
     double ext[3] = {0, 0, 0}, ext_max = 0.0;
     for (int d = 0; d < 3; d++) c.lo[d] = 0.0;
@@ -848,7 +877,7 @@ int build_clouds(BuildScratch& S, const float* d_points, const Cloud* clouds, in
                  int64_t* starts, Built* out, std::string* err) {
     std::vector<CloudD> h;
     h.reserve(size_t(k));
-    int64_t n = 0, f = 0;
+    int64_t n = 0, f = 0, most = 0;
     int maxdim = 0;
     bool mixed = false;
     for (int c = 0; c < k; c++) {
@@ -868,6 +897,7 @@ int build_clouds(BuildScratch& S, const float* d_points, const Cloud* clouds, in
         d.radius = q.radius;
         h.push_back(d);
         n += q.npts;
+        most = std::max(most, q.npts);
         f += q.npts * q.space_dim;
         mixed = mixed || (c > 0 && q.maxdim != clouds[0].maxdim);
         maxdim = std::max(maxdim, int(q.maxdim));
@@ -891,7 +921,7 @@ int build_clouds(BuildScratch& S, const float* d_points, const Cloud* clouds, in
     BK(cudaMemsetAsync(flag, 0, 4 * sizeof(int), s));
     BK(cudaMemcpyAsync(dc, h.data(), sizeof(CloudD) * h.size(), cudaMemcpyHostToDevice, s));
     BK(cudaMemsetAsync(count, 0, sizeof(int32_t) * size_t(cells), s));
-    k_cloud_grid<<<unsigned(k), kT, 0, s>>>(d_points, dc, flag);
+    k_cloud_grid<<<dim3(unsigned(k), unsigned(box_blocks(most))), kT, 0, s>>>(d_points, dc, flag);
     int64_t got[3] = {0, 0, 0};
     const unsigned ng = unsigned(std::max<int64_t>(1, std::min<int64_t>((n + kNbrWarps - 1) / kNbrWarps, 1 << 16)));
     if (n > 0) {
