@@ -189,6 +189,16 @@ __global__ void __launch_bounds__(kT) k_cloud_grid(const float* p, CloudD* cloud
     CloudD& c = clouds[blockIdx.x];
     const int blocks = box_blocks(c.npts);
     if (int(blockIdx.y) >= blocks) return;
+    if (c.maxdim == 0) {  // points alone: nobody is looked for, and any coordinate will do
+        if (blockIdx.y == 0 && threadIdx.x == 0) {
+            for (int d = 0; d < 3; d++) {
+                c.lo[d] = 0.0;
+                c.n[d] = 1;
+            }
+            c.side = 1.0;
+        }
+        return;
+    }
     if (threadIdx.x < 3) {
         s_lo[threadIdx.x] = 0xFFFFFFFFu;
         s_hi[threadIdx.x] = 0;
@@ -903,6 +913,13 @@ int build_clouds(BuildScratch& S, const float* d_points, const Cloud* clouds, in
         maxdim = std::max(maxdim, int(q.maxdim));
     }
     if (!S.h_misc) BK(cudaMallocHost(&S.h_misc, 8 * sizeof(int64_t)));
+    Clouds cl;
+    cl.k = k;
+    cl.mixed = mixed;
+    cl.starts = starts;
+    if (maxdim == 0 && k == 1) {  // points alone: no graph (and any coordinate will do)
+        return build_flag(S, n, 0, nullptr, 0, cl, s, sink, out, err);
+    }
     const int64_t cells = 4 * n + int64_t(kCellSlack) * k;
     int* flag;      // [0] non-finite coordinate, [2] largest upper degree
     CloudD* dc;
@@ -969,11 +986,7 @@ int build_clouds(BuildScratch& S, const float* d_points, const Cloud* clouds, in
         }
     }
     BK(cudaGetLastError());
-    Clouds cl;
     cl.d = dc;
-    cl.k = k;
-    cl.mixed = mixed;
-    cl.starts = starts;
     return build_flag(S, n, E, nullptr, maxdim, cl, s, sink, out, err);
 }
 

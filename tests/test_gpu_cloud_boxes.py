@@ -8,9 +8,29 @@ import numpy as np
 import pytest
 
 from specseqplusplus_b200 import Engine, SsppError, gen
-from test_gpu_build_joint import check, cloud
+from specseqplusplus_b200.gen import BoundaryMatrix
+import test_gpu_build_joint as joint
+from test_gpu_build_joint import cloud
 
 pytestmark = pytest.mark.gpu
+
+
+def check(requests, vertices=()):
+    """test_gpu_build_joint.check; the requests listed are vertices alone (the host builder wants finite points)"""
+    of = {id(requests[i]) for i in vertices}
+
+    def host(r):
+        n = len(r[1])
+        if id(r) in of:
+            return BoundaryMatrix(np.zeros(n, np.int32), np.zeros(n + 1, np.int64), np.zeros(0, np.int32),
+                                  np.zeros(n, np.float32))
+        return ordinary(r)
+
+    ordinary, joint.host = joint.host, host
+    try:
+        joint.check(requests)
+    finally:
+        joint.host = ordinary
 
 
 @pytest.mark.parametrize("n", [2047, 2048, 2049, 4096, 4097, 300_000])
@@ -44,3 +64,21 @@ def test_a_coordinate_that_is_not_finite(at, value):
             assert ei.value.code == 1 and "non-finite" in str(ei.value)
             e.load_rips(p, good, 2)
             assert e.input_matrix().ncols > 100_000
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf, 3e38])
+def test_points_alone_may_have_any_coordinate(value):
+    # without edges (maximal dimension 0) the coordinates are not looked at
+    rng = np.random.default_rng(11)
+    q = cloud(rng, 5000, 2)
+    q[[0, 2048, 4999], 1] = value
+    q[17, 0] = -value
+    check([("rips", cloud(rng, 60, 3), 0.4, 3), ("rips", q, 0.1, 0), ("rips", q[:0], 0.1, 0),
+           ("rips", cloud(rng, 3000, 2), 0.02, 2)], vertices=(1,))
+    check([("rips", q, 0.1, 0)] * 2, vertices=(0, 1))
+    with Engine(0) as e:
+        for _ in range(2):
+            e.load_rips(q, 0.1, 0)
+            m = e.input_matrix(values=True)
+            assert m.ncols == 5000 and m.nnz == 0
+            assert not m.dims.any() and not m.col_ptr.any() and not m.values.any()
