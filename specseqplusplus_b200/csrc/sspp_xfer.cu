@@ -243,6 +243,44 @@ cudaError_t Xfer::fetch_small(const std::vector<Piece>& pieces, cudaStream_t s) 
     return cudaSuccess;
 }
 
+// The staged segments from `stage` to their places: one DMA per run that is contiguous
+// on the device.
+cudaError_t Xfer::send(const std::vector<Piece>& pieces, const std::vector<Seg>& segs, const uint8_t* stage,
+                       cudaStream_t s) {
+    for (size_t k = 0; k < segs.size();) {
+        uint8_t* d0 = static_cast<uint8_t*>(pieces[segs[k].piece].dst) + segs[k].off;
+        size_t len = segs[k].len, k2 = k + 1;
+        const int grp = pieces[segs[k].piece].group;
+        while (k2 < segs.size() && grp >= 0 && pieces[segs[k2].piece].group == grp &&
+               static_cast<uint8_t*>(pieces[segs[k2].piece].dst) + segs[k2].off == d0 + len)
+            len += segs[k2++].len;
+        const cudaError_t e = cudaMemcpyAsync(d0, stage + segs[k].so, len, cudaMemcpyHostToDevice, s);
+        if (e != cudaSuccess) return e;
+        k = k2;
+    }
+    return cudaSuccess;
+}
+
+// Many small pieces (a batch of small matrices), through the buffer of small copies: the
+// large one, 64 MB of pinned memory, would cost a context's first batch 50 ms.
+cudaError_t Xfer::send_small(const std::vector<Piece>& pieces, cudaStream_t s) {
+    cudaError_t e;
+    if (small_used_ && (e = cudaEventSynchronize(small_ev_)) != cudaSuccess) return e;
+    std::vector<Seg> segs;
+    size_t at = 0;
+    for (size_t i = 0; i < pieces.size(); i++) {
+        const Piece& p = pieces[i];
+        if (!p.bytes) continue;
+        std::memcpy(small_ + at, p.src, p.bytes);
+        segs.push_back({i, 0, p.bytes, at});
+        at += p.bytes;
+    }
+    if ((e = send(pieces, segs, small_, s)) != cudaSuccess) return e;
+    if ((e = cudaEventRecord(small_ev_, s)) != cudaSuccess) return e;
+    small_used_ = true;
+    return cudaSuccess;
+}
+
 cudaError_t Xfer::h2d(const std::vector<Piece>& pieces, cudaStream_t s) {
     size_t total = 0;
     for (const Piece& p : pieces) total += p.bytes;
@@ -261,6 +299,7 @@ cudaError_t Xfer::h2d(const std::vector<Piece>& pieces, cudaStream_t s) {
                 return e;
         return cudaStreamSynchronize(s);  // pageable sources may be reused by the caller
     }
+    if (small_ && total <= kDirectBytes) return send_small(pieces, s);
     if ((e = ensure()) != cudaSuccess) return e;
     const bool small = total > kSmallChunk && total <= kManyChunks;
     const size_t chunk = small ? kSmallChunk : half_;
@@ -277,16 +316,7 @@ cudaError_t Xfer::h2d(const std::vector<Piece>& pieces, cudaStream_t s) {
         if (used_[h] && (e = cudaEventSynchronize(ev_[h])) != cudaSuccess) return e;
         uint8_t* st = stage_ + size_t(h) * half_;
         parallel_copy(pieces, segs, fill, st, true, small ? kMinTaskBytes / 4 : kMinTaskBytes);
-        for (size_t k = 0; k < segs.size();) {  // one DMA per run contiguous on the device
-            uint8_t* d0 = static_cast<uint8_t*>(pieces[segs[k].piece].dst) + segs[k].off;
-            size_t len = segs[k].len, k2 = k + 1;
-            const int grp = pieces[segs[k].piece].group;
-            while (k2 < segs.size() && grp >= 0 && pieces[segs[k2].piece].group == grp &&
-                   static_cast<uint8_t*>(pieces[segs[k2].piece].dst) + segs[k2].off == d0 + len)
-                len += segs[k2++].len;
-            if ((e = cudaMemcpyAsync(d0, st + segs[k].so, len, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
-            k = k2;
-        }
+        if ((e = send(pieces, segs, st, s)) != cudaSuccess) return e;
         if ((e = cudaEventRecord(ev_[h], s)) != cudaSuccess) return e;
         used_[h] = true;
         h ^= 1;

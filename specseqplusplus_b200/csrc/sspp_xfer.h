@@ -74,7 +74,9 @@ private:
     // `least`: smallest share of one host thread
     void parallel_copy(const std::vector<Piece>& pieces, const std::vector<Seg>& segs, size_t fill, uint8_t* stage,
                        bool to_stage, size_t least);
+    cudaError_t send(const std::vector<Piece>& pieces, const std::vector<Seg>& segs, const uint8_t* stage, cudaStream_t s);
     cudaError_t fetch_small(const std::vector<Piece>& pieces, cudaStream_t s);
+    cudaError_t send_small(const std::vector<Piece>& pieces, cudaStream_t s);
     uint8_t* small_ = nullptr;  // pinned, for copies that one kernel fetches
     cudaEvent_t small_ev_ = nullptr;
     bool small_used_ = false;
