@@ -12,22 +12,25 @@ namespace sspp {
 
 namespace {
 
-// Candidate launch settings, best first on the measured workloads (lower-
-// star grids and Rips complexes: one spectral-sequence block over the whole
-// dimension and 32-int warp columns were fastest or within a few percent).
+// Candidate launch settings.  What they differ in takes effect in every schedule: warp
+// columns of 32 or 64 ints, CTAs of 256 threads and 8,192 ints or 128 and 4,096 (block
+// size and growth, which schedules 0 and 1 do not look at, vary along with the last one
+// for schedule 2).  They lie within 15% of one another (reduction of 64^3 0.94 / 1.00 / 0.92 /
+// 0.99 ms, dualized 1.68 / 1.74 / 1.88 / 1.94; of a dualized 10,000-point Rips complex
+// 0.48 / 0.43 / 0.47 / 0.44).
 // queue_size only caps the light tier's grid, so it is set never to bind.
 const Knobs kCandidates[] = {
     {1 << 30, 1.0f, 1 << 20, 32, 8192, 256, 0},
-    {102400, 1.05f, 1 << 20, 32, 8192, 256, 0},
     {1 << 30, 1.0f, 1 << 20, 64, 8192, 256, 0},
     {1 << 30, 1.0f, 1 << 20, 32, 4096, 128, 0},
+    {102400, 1.05f, 1 << 20, 64, 4096, 128, 0},
 };
 constexpr int kNumBase = int(sizeof(kCandidates) / sizeof(kCandidates[0]));
 constexpr int kRetryEvery = 32;
 // Inputs this large explore only once their class has run kExploreMinRuns
 // times (a repeated workload, where what is learnt pays back): a poor
-// candidate on a one-off large input (a dual reduction of a large lower-star
-// grid takes four times as long) costs more than it could teach.  Until then
+// candidate on a one-off large input (a dual reduction of the 93^3 lower-star grid
+// takes 7.7 ms instead of 5.4) costs more than it could teach.  Until then
 // they take the lowest estimate: their own class's mean where measured, else
 // what similar smaller classes measured.
 constexpr int64_t kExploreMaxCols = int64_t(1) << 20;
