@@ -212,6 +212,7 @@ int ensure_columns(sspp_ctx* ctx, int64_t n, int64_t nnz) {
     if (n > INT32_MAX - 8) return set_err(ctx, SSPP_ERR_CAPACITY, "more than 2^31 columns");
     if (n > D.cap_n) {
         int64_t c = n;
+        D.cap_n = 0;  // until everything is there: a load after a failed one starts over
         auto g = [&](auto*& p, int64_t mult) {
             using T = std::remove_reference_t<decltype(*p)>;
             int64_t cap = 0;
@@ -234,13 +235,12 @@ int ensure_columns(sspp_ctx* ctx, int64_t n, int64_t nnz) {
         CK(g(D.pairs, 2));
         CK(g(D.ess, 1));
         CK(g(D.app, 1));
-        D.cap_n = c;
         // the control block and the scans' tile states (one per 4,096 columns, a total and room for one more)
         D.blk_stride = scan_most_blocks(c) + 2;
         const int64_t ctl_words = int64_t((sizeof(Ctl) + 15) / 16) * 2;
-        int64_t* buf = reinterpret_cast<int64_t*>(D.ctl);
-        if (buf) CK(cudaFreeAsync(buf, ctx->stream));
-        buf = nullptr;
+        if (D.ctl) CK(cudaFreeAsync(D.ctl, ctx->stream));
+        D.ctl = nullptr;
+        int64_t* buf = nullptr;
         D.cap_blk = 0;
         CK(grow(buf, D.cap_blk, ctl_words + 3 * D.blk_stride, ctx->stream));
         D.ctl = reinterpret_cast<Ctl*>(buf);
@@ -257,6 +257,7 @@ int ensure_columns(sspp_ctx* ctx, int64_t n, int64_t nnz) {
         if (D.dimcnt) CK(cudaFreeAsync(D.dimcnt, ctx->stream));
         D.dimcnt = nullptr;
         CK(grow(D.dimcnt, D.cap_dimcnt, (part_tiles(c) + 1) * kNumDims, ctx->stream));
+        D.cap_n = c;
     }
     if (!D.misc) CK(cudaMalloc(&D.misc, sizeof(int64_t) * 8));
     return SSPP_OK;
