@@ -711,7 +711,10 @@ constexpr int64_t kMaxCols = int64_t(1) << 31;
 
 // Several clouds are built as one up to this many columns (about 80 bytes of
 // scratch each); beyond it the caller takes fewer at a time.
-constexpr int64_t kMaxJointCols = int64_t(1) << 26;
+#ifndef SSPP_MAX_JOINT_COLS
+#define SSPP_MAX_JOINT_COLS (int64_t(1) << 26)
+#endif
+constexpr int64_t kMaxJointCols = SSPP_MAX_JOINT_COLS;
 
 // The clouds of a build (one, or a grid: k = 1 and no table).
 struct Clouds {

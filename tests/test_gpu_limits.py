@@ -1,8 +1,10 @@
-"""GPU parity when the scans' tiles do not wait for one another.
+"""GPU parity at limits that ordinary inputs do not reach.
 
 A tile of the one-pass scan that its predecessors do not answer in time takes
 their values itself.  That never happens by itself in a test, so the library is
 built here with a limit of one poll: every tile that is not answered at once does it.
+And point clouds are built together up to 2^26 columns; here up to 20,000, so that
+batches are built in several parts.
 """
 import os
 import subprocess
@@ -48,6 +50,32 @@ def check_reduced(e):
     assert np.array_equal(e.pairs(), want.pairs) and np.array_equal(e.essentials(), want.essential)
 
 
+def check_split(e):
+    import test_gpu_build_joint as joint
+
+    rng = np.random.default_rng(9)
+
+    def rips(n, d, degree, maxdim):
+        return ("rips", joint.cloud(rng, n, d), gen.rips_radius_for_degree(max(n, 2), d, degree), maxdim)
+
+    field = ("lowerstar", rng.normal(size=(5, 6, 7)).astype(np.float32), 3)
+    small = [rips(int(rng.integers(0, 400)), 2 + i % 2, 8.0, 2 + i % 2) for i in range(40)]
+    joint.check(small)
+    # one larger than the limit by itself, first, last and in the middle; parts that end at a field
+    large = rips(3000, 3, 14.0, 3)
+    joint.check([large] + small[:5] + [large, field] + small[5:9] + [rips(0, 2, 1.0, 2), large])
+    joint.check([large, large, large])
+    joint.check([rips(1500, 2, 9.0, i % 4) for i in range(9)])
+    # the batch's columns are those of its members, wherever the parts ended
+    requests = small[:20] + [field] + small[20:]
+    e.load_built_batch(requests)
+    e.reduce(Params())
+    for r, (pairs, ess) in zip(requests, e.batch_results(), strict=True):
+        m = joint.host(r)
+        want = oracle.reduce(m)
+        assert np.array_equal(pairs, want.pairs) and np.array_equal(ess, want.essential)
+
+
 def main(lib, check):
     from specseqplusplus_b200 import engine
 
@@ -58,21 +86,21 @@ def main(lib, check):
 
 
 @pytest.fixture(scope="module")
-def impatient(tmp_path_factory):
+def limited(tmp_path_factory):
     sys.path.insert(0, os.path.join(ROOT, "specseqplusplus_b200"))
     import build
 
-    d = tmp_path_factory.mktemp("impatient")
+    d = tmp_path_factory.mktemp("limited")
     lib = str(d / "libsspp.so")
-    build.build_engine(lib, str(d / "obj"), ["-DSSPP_SCAN_POLLS=1"])
+    build.build_engine(lib, str(d / "obj"), ["-DSSPP_SCAN_POLLS=1", "-DSSPP_MAX_JOINT_COLS=20000"])
     return lib
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("check", ["check_built", "check_reduced"])
-def test_tiles_that_take_the_earlier_values_themselves(impatient, check):
-    code = "import sys, test_gpu_scan_waits as t; t.main(sys.argv[1], sys.argv[2])"
+@pytest.mark.parametrize("check", ["check_built", "check_reduced", "check_split"])
+def test_with_small_limits(limited, check):
+    code = "import sys, test_gpu_limits as t; t.main(sys.argv[1], sys.argv[2])"
     path = os.pathsep.join([ROOT, os.path.join(ROOT, "oracle"), os.path.join(ROOT, "tests")])
-    r = subprocess.run([sys.executable, "-c", code, impatient, check], capture_output=True, text=True, timeout=300,
+    r = subprocess.run([sys.executable, "-c", code, limited, check], capture_output=True, text=True, timeout=300,
                        env=dict(os.environ, PYTHONPATH=path))
     assert r.returncode == 0, r.stdout + r.stderr
