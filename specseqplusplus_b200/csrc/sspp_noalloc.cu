@@ -73,9 +73,12 @@
 
 namespace {
 
-constexpr int64_t kScratchInts = int64_t(16) << 20;  // 64 MiB
+#ifndef SSPP_SCRATCH_INTS
+#define SSPP_SCRATCH_INTS (int64_t(16) << 20)
+#endif
+constexpr int64_t kScratchInts = SSPP_SCRATCH_INTS;  // 64 MiB
 constexpr int64_t kMaxCols = int64_t(1) << 20;
-constexpr int64_t kFillReserve = int64_t(4) << 20;   // ints kept free for fill-in
+constexpr int64_t kFillReserve = kScratchInts / 4;   // ints kept free for fill-in
 constexpr int kCtl = 16;                            // control words at the start of the array
 constexpr int kMaxDevices = 64;
 constexpr int kThreads = 256;

@@ -1887,8 +1887,9 @@ __global__ void __launch_bounds__(128) k_fill_account(const __grid_constant__ Fi
                 if (lane < pn) list[2][lane] = lane == q.x ? L : lane == 0 ? q.y : lane == 1 ? q.z : q.w;
                 __syncwarp();
             } else {
-                int64_t ps = slot_of(p);
-                if (lm != p) {  // listed: its reduced form, once it is there
+                // apparent: the leftmost column of its lowest row, never changed
+                pn = lm == p ? fetch(slot_of(p), list[2]) : 0;
+                if (pn == 0 || (pn > 0 && lds(list[2] + pn - 1) != L)) {  // listed: reduced, once it is there
                     unsigned long long r = 0;
                     if (lane == 0)
                         for (int polls = 0;
@@ -1897,11 +1898,11 @@ __global__ void __launch_bounds__(128) k_fill_account(const __grid_constant__ Fi
                     r = g.bcast64(r);
                     ok = r != 0;
                     if (!ok) break;
-                    ps = int64_t(r) - 1;
+                    __syncwarp();
+                    pn = fetch(int64_t(r) - 1, list[2]);
                 }
-                pn = fetch(ps, list[2]);
             }
-            ok = pn > 0 && n + pn - 2 <= kFillCap;
+            ok = pn > 0 && n + pn - 2 <= kFillCap && lds(list[2] + pn - 1) == L;
             if (!ok) break;
             cost += n + pn;
             n = merge(g, w, n, false, list[2], pn, false, o, kFillCap, err);
@@ -1909,6 +1910,7 @@ __global__ void __launch_bounds__(128) k_fill_account(const __grid_constant__ Fi
             w = o;
             o = x;
             added = true;
+            ok = n == 0 || lds(w + n - 1) < L;  // (the lowest row moves down with every addition)
         }
         if (ok && added && n > 0) {
             const int64_t ints = slot_ints(n);

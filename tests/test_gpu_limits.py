@@ -4,7 +4,9 @@ A tile of the one-pass scan that its predecessors do not answer in time takes
 their values itself.  That never happens by itself in a test, so the library is
 built here with a limit of one poll: every tile that is not answered at once does it.
 And point clouds are built together up to 2^26 columns; here up to 20,000, so that
-batches are built in several parts.
+batches are built in several parts.  The allocation-free call's array holds 2^20 ints
+instead of 2^24, so that matrices whose fill-in can be counted here end on either side
+of its room.
 """
 import os
 import subprocess
@@ -14,7 +16,7 @@ import numpy as np
 import pytest
 
 import oracle
-from specseqplusplus_b200 import Engine, Params, gen
+from specseqplusplus_b200 import Engine, Params, SsppError, gen
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -76,12 +78,38 @@ def check_split(e):
         assert np.array_equal(pairs, want.pairs) and np.array_equal(ess, want.essential)
 
 
+def check_fill(e):
+    import torch
+    from test_gpu_noalloc_buffers import fill_in
+    from test_zz_no_alloc import _noalloc_pairs
+
+    def left(m):  # room for fill-in that a column-after-column reduction leaves
+        took, room = fill_in(m)
+        return room - (16 << 20) + (1 << 20) - took
+
+    def first(m, n):
+        return gen.BoundaryMatrix(m.dims[:n], m.col_ptr[:n + 1], m.rows[:m.col_ptr[n]])
+
+    for npts, dim, degree in ((400, 2, 26.0), (150, 2, 40.0), (200, 2, 40.0)):
+        m = gen.rips(npts, dim, 3, gen.rips_radius_for_degree(npts, dim, degree), dim)
+        lo, hi = 1000, m.ncols  # the subcomplex of the first lo columns fits, that of the first hi does not
+        assert left(m) < 0 <= left(first(m, lo))
+        while hi - lo > 1:
+            n = (lo + hi) // 2
+            lo, hi = (n, hi) if left(first(m, n)) >= 0 else (lo, n)
+        for _ in range(2):
+            assert np.array_equal(_noalloc_pairs(first(m, lo), torch), oracle.reduce(first(m, lo)).pairs)
+            with pytest.raises(SsppError) as ei:
+                _noalloc_pairs(first(m, hi), torch)
+            assert ei.value.code == 2
+
+
 def main(lib, check):
     from specseqplusplus_b200 import engine
 
     engine.LIB_PATH = lib
     with Engine(0) as e:
-        for _ in range(3):
+        for _ in range(1 if check == "check_fill" else 3):
             globals()[check](e)
 
 
@@ -92,12 +120,13 @@ def limited(tmp_path_factory):
 
     d = tmp_path_factory.mktemp("limited")
     lib = str(d / "libsspp.so")
-    build.build_engine(lib, str(d / "obj"), ["-DSSPP_SCAN_POLLS=1", "-DSSPP_MAX_JOINT_COLS=20000"])
+    build.build_engine(lib, str(d / "obj"), ["-DSSPP_SCAN_POLLS=1", "-DSSPP_MAX_JOINT_COLS=20000",
+                                           "-DSSPP_SCRATCH_INTS=(1<<20)"])
     return lib
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("check", ["check_built", "check_reduced", "check_split"])
+@pytest.mark.parametrize("check", ["check_built", "check_reduced", "check_split", "check_fill"])
 def test_with_small_limits(limited, check):
     code = "import sys, test_gpu_limits as t; t.main(sys.argv[1], sys.argv[2])"
     path = os.pathsep.join([ROOT, os.path.join(ROOT, "oracle"), os.path.join(ROOT, "tests")])
