@@ -975,20 +975,27 @@ int run_compute(sspp_ctx* ctx) {
         nsteps += ctx->ss_steps;
     }
     ctx->ss_steps = nsteps;
-    cudaEvent_t ep = nullptr;
-    span_begin(ctx, ep);
-    ctx->launches += extract_pairs(D, P.dualize != 0, dropped_of(ctx), s);
-    span_end(ctx, PH_PAIRS, ep);
-    CK(cudaGetLastError());
-    ctx->pushed = D.n <= kPushCols;
-    if (ctx->pushed) {
-        ctx->launches += push_results(D, ctx->h_ctl, ctx->h_pairs, kPushCols / 2, ctx->h_ess, kPushCols, s);
+    for (bool marks : {false, true}) {
+        cudaEvent_t ep = nullptr;
+        span_begin(ctx, ep);
+        ctx->launches += extract_pairs(D, P.dualize != 0, dropped_of(ctx), s, marks);
+        span_end(ctx, PH_PAIRS, ep);
         CK(cudaGetLastError());
-        CK(cudaStreamSynchronize(s));
-        // (in a matrix that is no chain complex a column may be in two pairs)
-        ctx->pushed = ctx->h_ctl->counters[CNT_NPAIRS] <= kPushCols / 2;
-    } else if (int rc = read_ctl(ctx)) {
-        return rc;
+        ctx->pushed = D.n <= kPushCols;
+        if (ctx->pushed) {
+            ctx->launches += push_results(D, ctx->h_ctl, ctx->h_pairs, kPushCols / 2, ctx->h_ess, kPushCols, s);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(s));
+            // (in a matrix that is no chain complex a column may be in two pairs)
+            ctx->pushed = ctx->h_ctl->counters[CNT_NPAIRS] <= kPushCols / 2;
+        } else if (int rc = read_ctl(ctx)) {
+            return rc;
+        }
+        // every column a birth, a death, essential or dropped, unless the matrix is no chain
+        // complex: the pairs are then taken by marks
+        const long long* cnt = ctx->h_ctl->counters;
+        const int64_t dropped = dropped_of(ctx) ? cnt[CNT_DROPPED] : 0;
+        if (ctx->h_ctl->err || P.dualize || 2 * cnt[CNT_NPAIRS] + cnt[CNT_NESS] + dropped == D.n) break;
     }
     std::memcpy(ctx->hcounters, ctx->h_ctl->counters, sizeof(ctx->hcounters));
     ctx->arena_used = int64_t(ctx->h_ctl->arena_top);

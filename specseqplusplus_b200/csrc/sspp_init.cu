@@ -754,8 +754,11 @@ int active_list(Device& D, cudaStream_t s) {
 // ------------------------------------------------------------------- pairs
 // Primal: input simplex j (reordered i) is a birth when row i has an owner, whose
 // simplex is its death; it is a death when column i owns a row; neither, and not
-// dropped by an edge collapse: essential.  One scan in input order writes both
-// lists (births ascending, so the pairs come out sorted): it reads the maps and
+// dropped by an edge collapse: essential.  (A column that owns a row is marked as an
+// owner in every chain complex; in other matrices its marks may have gone with its lowest
+// row, when that row is negative.  The counts show it, every column being one of a
+// birth, a death, essential and dropped, and the pairs are then taken by the marks.)  One
+// scan in input order writes both lists (births ascending, so the pairs come out sorted): it reads the maps and
 // the pivot table in two nearly sequential streams per dimension, and only the
 // deaths' input indices at random.  64^3: 81 us; a scatter by birth and two scans over
 // its marks took 250.
@@ -827,16 +830,16 @@ struct PairsDone {
     }
 };
 
-// Dual: the dual row r' owned by dual column c' maps back to the primal pair
+// By marks.  Dual: the dual row r' owned by dual column c' maps back to the primal pair
 // (n-1-c', n-1-r') of the dualized matrix's own numbering, and perm maps those
 // to input indices; scattered by birth first, since a column that owns a row from
 // the boundary matrix's pass (mode 2) is not marked as one.
-__global__ void k_pairs_scatter(int64_t n, const uint64_t* pivot, const int32_t* perm, int64_t* death_of,
+__global__ void k_pairs_scatter(int64_t n, const uint64_t* pivot, const int32_t* perm, bool dual, int64_t* death_of,
                                 uint8_t* paired) {
     for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n; r += int64_t(gridDim.x) * blockDim.x) {
         const uint64_t e = pivot[r];
         if (e == kNoOwner) continue;
-        const int64_t birth = perm[n - 1 - pv_col(e)], death = perm[n - 1 - r];
+        const int64_t c = pv_col(e), birth = perm[dual ? n - 1 - c : r], death = perm[dual ? n - 1 - r : c];
         death_of[birth] = death;
         paired[birth] = 1;
         paired[death] = 1;
@@ -874,25 +877,25 @@ int push_results(const Device& D, Ctl* h_ctl, int64_t* h_pairs, int64_t max_pair
     return 1;
 }
 
-int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s, const int* unless) {
+int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s, bool marks, const int* unless) {
     const int64_t n = D.n;
     const PairsOut o{n, D.newidx, D.perm, D.pivot, D.state, D.pairs, D.ess, D.counters, D.err,
                      D.edge_begin, D.edge_end};
     bool zeroed;
     int64_t* blk = scan_region(D, 2, &zeroed);
-    if (!dual) {
+    if (!dual && !marks) {
         if (reinterpret_cast<uintptr_t>(D.pairs) % sizeof(longlong2) == 0)
             scan(PairsValue{o}, PairsSink<true>{o}, n, blk, s, PairsDone{o}, zeroed, nullptr, 0, unless);
         else
             scan(PairsValue{o}, PairsSink<false>{o}, n, blk, s, PairsDone{o}, zeroed, nullptr, 0, unless);
         return 1;
     }
-    // the dual's pairs are the context's own buffer
+    // (the context's own buffer)
     longlong2* pairs = reinterpret_cast<longlong2*>(D.pairs);
     const unsigned g = grid_for(n, 256) > 65536 ? 65536 : grid_for(n, 256);
     fill_i64(D.death_of, -1, n, s);
     cudaMemsetAsync(D.negative, 0, n, s);  // reused as the "paired or dropped" mark
-    k_pairs_scatter<<<g, 256, 0, s>>>(n, D.pivot, D.perm, D.death_of, D.negative);
+    k_pairs_scatter<<<g, 256, 0, s>>>(n, D.pivot, D.perm, dual != 0, D.death_of, D.negative);
     if (dropped) k_mark_dropped<<<g, 256, 0, s>>>(n, dropped, D.perm, D.negative);
     const int64_t* death_of = D.death_of;
     const uint8_t* paired = D.negative;

@@ -56,8 +56,11 @@ int push_results(const Device& D, Ctl* h_ctl, int64_t* h_pairs, int64_t max_pair
 // dimension 1 of the boundary matrix (active list entries [beg, end), no column of
 // more than two entries) over the vertices, the reordered rows [0, rows)
 int reduce_edges(Device& D, int32_t beg, int32_t end, int32_t rows, cudaStream_t s);
-// unless (dual 0): a device word; when it is set, nothing is written
-int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s, const int* unless = nullptr);
+// marks (always for a dual): by marking both columns of every pair, instead of by the
+// columns' states.  unless (neither dual nor marks): a device word; when it is set, nothing
+// is written
+int extract_pairs(Device& D, int dual, const uint8_t* dropped, cudaStream_t s, bool marks = false,
+                  const int* unless = nullptr);
 
 // Device work queue of (complex, block) items (one persistent launch per
 // schedule; see k_reduce_queue).  An item is one spectral-sequence block of

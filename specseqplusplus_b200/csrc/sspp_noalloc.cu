@@ -399,7 +399,7 @@ cudaError_t reduce_in_scratch(int32_t* scratch, int dev, int64_t n, int64_t nnz,
     cudaMemsetAsync(ready, 0, sizeof(uint64_t) * size_t(n), s);
     const int64_t room = kScratchInts - (kCtl + 3 * n) - nnz;  // k_reduce_noalloc's room for fill-in
     fill_account_launch(D, h.info.act_end[kMaxDim], room, ready, shape.sms, s);
-    extract_pairs(D, 0, nullptr, s, D.err);  // nothing goes to the caller unless all is well
+    extract_pairs(D, 0, nullptr, s, false, D.err);  // nothing goes to the caller unless all is well
     k_store_npairs<<<1, 1, 0, s>>>(D.ctl, d_npairs);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     cudaMemcpyAsync(&h, D.ctl, offsetof(Ctl, step), cudaMemcpyDeviceToHost, s);
