@@ -161,21 +161,33 @@ struct CloudD {
     double lo[3];
     double side;
     int32_t n[3];
+    // Radii below kTinyRadius: squares of such distances underflow, so points much further
+    // apart than the radius may have a distance that is not.  Edges are those between
+    // points of neighbouring cells of this grid, the host builder's.
+    double fine_side;
+    int32_t fine_n[3];
     // while the bounding box is found (k_cloud_grid)
     uint32_t key_lo[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, key_hi[3] = {0, 0, 0};
     int32_t bad = 0, arrived = 0;
 };
 constexpr int kCellSlack = 64;
+constexpr float kTinyRadius = 1e-19f;
 constexpr int kBoxPoints = 2048, kBoxBlocks = 512;  // points a block at least, blocks a cloud at most
 __host__ __device__ inline int box_blocks(int64_t npts) {
     const int64_t b = (npts + kBoxPoints - 1) / kBoxPoints;
     return int(b < 1 ? 1 : b > kBoxBlocks ? kBoxBlocks : b);
 }
 
-__device__ __forceinline__ int32_t cell_coord(const CloudD& c, int d, float x) {
-    const double t = floor((double(x) - c.lo[d]) / c.side);
+__device__ __forceinline__ int32_t cell_coord(double lo, double side, int32_t n, float x) {
+    const double t = floor((double(x) - lo) / side);
     const int32_t k = int32_t(t);
-    return k < 0 ? 0 : (k >= c.n[d] ? c.n[d] - 1 : k);
+    return k < 0 ? 0 : (k >= n ? n - 1 : k);
+}
+__device__ __forceinline__ int32_t cell_coord(const CloudD& c, int d, float x) {
+    return cell_coord(c.lo[d], c.side, c.n[d], x);
+}
+__device__ __forceinline__ bool fine_neighbours(const CloudD& c, int d, float x, float y) {
+    return abs(cell_coord(c.lo[d], c.fine_side, c.fine_n[d], x) - cell_coord(c.lo[d], c.fine_side, c.fine_n[d], y)) <= 1;
 }
 
 // Cloud blockIdx.x's bounding box (also rejects non-finite coordinates), by box_blocks of
@@ -256,6 +268,8 @@ __global__ void __launch_bounds__(kT) k_cloud_grid(const float* p, CloudD* cloud
         }
     }
     double side = fmax(fmax(double(c.radius) * (1.0 + 1.0 / 1024.0), ext_max / 1000.0), 1e-30);
+    c.fine_side = side;
+    for (int d = 0; d < 3; d++) c.fine_n[d] = d < D ? int32_t(fmin(1001.0, floor(ext[d] / side) + 1.0)) : 1;
     for (;; side *= 1.25) {
         int64_t total = 1;
         for (int d = 0; d < 3; d++) {
@@ -364,6 +378,9 @@ __global__ void __launch_bounds__(kNbrWarps * 32) k_nbrs(int64_t n, const CloudD
                         }
                         dist = __fsqrt_rn(s);
                         hit = dist <= radius;
+                        if (hit && radius < kTinyRadius)
+                            hit = fine_neighbours(c, 0, pi.x, pj.x) && (D < 2 || fine_neighbours(c, 1, pi.y, pj.y)) &&
+                                  (D < 3 || fine_neighbours(c, 2, pi.z, pj.z));
                     }
                 }
                 const unsigned hm = __ballot_sync(0xFFFFFFFFu, hit);

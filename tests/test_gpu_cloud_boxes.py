@@ -82,3 +82,13 @@ def test_points_alone_may_have_any_coordinate(value):
             m = e.input_matrix(values=True)
             assert m.ncols == 5000 and m.nnz == 0
             assert not m.dims.any() and not m.col_ptr.any() and not m.values.any()
+
+
+@pytest.mark.parametrize("d", [1, 2, 3])
+@pytest.mark.parametrize("scale", [1e-24, 1e-22, 1e-21, 3e-20, 1e-18, 1.0])
+@pytest.mark.parametrize("radius", [0.0, 1e-30, 2e-23, 4e-23, 3e-22, 9e-20, 1.1e-19])
+def test_distances_whose_squares_underflow(d, scale, radius):
+    rng = np.random.default_rng(d)
+    p = cloud(rng, 36, d, scale)
+    q = np.concatenate([cloud(rng, 40, d, scale), cloud(rng, 3, d)])  # and a few far away: larger cells
+    check([("rips", p, radius, 1), ("rips", q, radius, 1)])
