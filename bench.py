@@ -64,6 +64,7 @@ def workload_config(n, nnz):
                         f"ss_block_size {SS}, growth {GROWTH}",
             "ncols": n, "nnz": nnz, "grid": GRID, "sigma": SIGMA, "seed": SEED, "model": MODEL,
             "max_iteration": MAX_ITER, "ss_block_size": SS, "growth": GROWTH, "queue_size": QUEUE,
+            "blocks": "one per dimension (ss_block_size and growth take effect in schedule 2 only)",
             "level1_capacity": L1, "level2_capacity": L2, "dualize": 0, "index": "int32", "values": "float32",
             "l2": "flushed between steps (256 MiB write); inputs (149 MB) also exceed L2",
             "hw_queues": os.environ.get("CUDA_DEVICE_MAX_CONNECTIONS")}

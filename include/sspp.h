@@ -75,9 +75,10 @@ typedef struct sspp_params {
     int32_t representatives;  /* 1: keep whole reduced columns so that sspp_representative
                                  can return each pair's cycle (dualize 0 only; skips the
                                  negative-row compression, so the reduction does more work) */
-    int32_t schedule;         /* how the spectral-sequence blocks are driven: 1 a host
-                                 loop of per-block launches (as the reference's
-                                 GPU_Compute); 2 one persistent launch draining a device
+    int32_t schedule;         /* how the reduction is driven: 1 a host loop of launches
+                                 per dimension, each dimension one spectral-sequence
+                                 block (the reference's GPU_Compute loops over blocks);
+                                 2 one persistent launch draining a device
                                  queue of (complex, block) items, each complex with its
                                  own block order and dimension gate; 0 = 1.  The
                                  pairs are the same either way */

@@ -37,12 +37,12 @@ static void print_help() {
         "  3 - Enable both high-dimension guided clearing theorem and edge collapsing\n"
         "max_iteration[Only effective when model equals 1 or 3.]: candidates examined per top-dimension simplex "
         "by the high-dimension guided clearing\n"
-        "ss_block_size: Block size for ss (default 102400)\n"
-        "block_size_growth_rate: Block size growth rate (default 1.05)\n"
+        "ss_block_size: Block size for ss (default 102400); checked, but a dimension is reduced as one block\n"
+        "block_size_growth_rate: Block size growth rate (default 1.05); as ss_block_size\n"
         "queue_size: maximum number of concurrent column workers (default 65536)\n"
-        "level1_capacity: on-chip capacity (ints) of a column worker\n"
+        "level1_capacity: on-chip capacity (ints) of a column worker (more than 64 counts as 64)\n"
         "level2_capacity: on-chip capacity (ints) of a block worker\n"
-        "--auto: choose ss_block_size, growth, queue_size and capacities automatically\n"
+        "--auto: choose queue_size and capacities automatically\n"
         "--export-preprocessed: write the input with the model's clearing / collapse applied (cleared columns "
         "as dimension-only lines) to output_file instead of the pairs\n"
         "Example: ./specseq++ input.txt output.txt ascii ascii 0 1 10 1024000 1.05 65536 1000 2000\n");

@@ -930,9 +930,10 @@ int run_compute(sspp_ctx* ctx) {
     // dimension 1 up.
     // schedule 1 (and 0): launches per dimension; 2: one persistent
     // launch per phase draining the (complex, block) work queue.  The host loop
-    // is the default: its warp-tier kernel keeps four times as many warps
-    // resident as the persistent kernel, whose CTA-tier role sets the register
-    // budget of every block
+    // is the default: its warp tier takes four tiny columns a warp, 24 warps a
+    // multiprocessor, where the persistent kernel's warps take one each, and its
+    // CTA-tier role sets the register budget of every block (16 warps).  Reduction of
+    // 64^3 0.94 against 8.1 ms, of 512 Rips complexes 14 against 75
     const bool queue = P.schedule == 2;
     D.edge_begin = D.edge_end = 0;
     auto phase = [&](int dlo, int dhi, bool ascending) {

@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kPartThreads) k_dim_assign(const int32_t* dims
 // read before it, or also when it does not run).
 // A column is a chain of four dependent trips to memory with little to do in between: at
 // 64^3 neither memory (29% of its bandwidth) nor L2 (43%) was busy.  The reads of a
-// trip go out together, of K columns on large inputs.
+// trip go out together, of K columns on large inputs (K = 2: 32 registers, 4 bytes spilled).
 template <int K>
 __global__ void __launch_bounds__(256) k_scatter_cols(int64_t n, const int64_t* colptr, const int32_t* rows, const int32_t* dims,
                                const int32_t* newidx, const int64_t* off, Ctl* ctl, int32_t* arena,
@@ -486,8 +486,8 @@ int reorder(Device& D, bool lows, bool write_desc, cudaStream_t s) {
     int32_t* rlen = D.active;
     k_dim_assign<<<unsigned(nb), kPartThreads, 0, s>>>(D.in_dims, D.in_colptr, n, nb, D.dimcnt, D.ctl, D.newidx, D.perm,
                                                        D.dim, rlen);
-    // padded column offsets in reordered order, unless every column is short (or
-    // the input is refused: the limit then skips it too)
+    // padded column offsets in reordered order, unless every column is short (in a
+    // refused input they may be sums of old lengths; nobody reads them)
     int64_t* off = D.scratch64;
     Ctl* ctl = D.ctl;
     bool zeroed;

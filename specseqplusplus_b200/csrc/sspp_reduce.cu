@@ -1200,7 +1200,7 @@ __device__ __forceinline__ unsigned spread8(unsigned b) {
     return (b | (b << 1)) & 0x5555u;
 }
 
-// At least 6 blocks per SM (80 registers, nothing spilled).  64^3, one block per
+// At least 6 blocks per SM (80 registers, 20 bytes spilled).  64^3, one block per
 // dimension: 8 / 7 / 6 / 5 blocks 1,228 / 1,192 / 1,223 / 1,250 us of reduction; small
 // inputs prefer few blocks (1,200-point cloud 396 / 375 / 360 / 356 us).
 constexpr int kLightMinBlocks = 6;

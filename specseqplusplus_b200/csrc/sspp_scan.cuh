@@ -8,7 +8,8 @@
 //
 // Tiles of 4096 items (1024 in mid-sized scans) per 256-thread block.  A warp takes 512
 // (128) consecutive items, 32 at a time, so that values are read and prefixes written coalesced.  Tiles
-// publish their sums and read their predecessors' (decoupled look-back, 256 tiles
+// publish their sums and read their predecessors' (decoupled look-back: Merrill and
+// Garland, "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016; 256 tiles
 // at a time: with a warp's 32 the prefix needed 50 hops over 1,605 tiles, and the
 // pair lists took 217 us instead of 92), so every value is read once.  The three
 // passes it replaces (sums, sums of sums, prefixes with 16 consecutive items per

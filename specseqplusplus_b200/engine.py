@@ -77,15 +77,15 @@ class Params:
     dualize: int = 0
     model: int = 0
     max_iteration: int = 0
-    ss_block_size: int = 102400
-    growth: float = 1.05
+    ss_block_size: int = 102400  # schedule 2; the others take a dimension as one block
+    growth: float = 1.05  # as ss_block_size
     queue_size: int = 65536
-    level1_capacity: int = 1000
+    level1_capacity: int = 1000  # more than 64 counts as 64
     level2_capacity: int = 8000
     autotune: int = 0
     heavy_threads: int = 0
     representatives: int = 0
-    schedule: int = 0  # 1 (= 0) host loop of per-block launches, 2 one persistent device work-queue launch
+    schedule: int = 0  # 1 (= 0) host loop of launches per dimension, 2 one persistent device work-queue launch
 
     def _c(self) -> _Params:
         return _Params(*(getattr(self, f.name) for f in fields(self)))
